@@ -660,7 +660,10 @@ static int rhs_fff(ts_plan* p, const void* Uin, int mode, const StageArgs& a_in)
   a.eyf = p->eaxf[1];
   a.ezf = p->eaxf[2];
   const int rot = p->cfg.nlin_form == TS_NLIN_ROTATIONAL;
-  const int nin = rot ? 6 : 3, nout = rot ? 3 : 6;
+  // a conservative step takes the five products of form 7 (N up to a gradient, which the
+  // projection removes); the nonlinear term itself and the flux take the whole tensor
+  const int zform = rot ? 1 : (mode == MODE_STEP ? 7 : 0);
+  const int nin = rot ? 6 : 3, nout = z_nout(zform);
   // two-thirds dealiasing: after the x inverse only the columns with 3|ky| <= Ny and
   // 3 kz <= Nz can be nonzero, so the inverse x pass writes only those, the y
   // inverse transforms only kz <= Nz/3 and reads only the 3|ky| <= Ny rows, and the
@@ -677,10 +680,10 @@ static int rhs_fff(ts_plan* p, const void* Uin, int mode, const StageArgs& a_in)
   }
   {
     ProfScope ps(p, TS_KCLASS_Z, by(TS_KCLASS_Z));
-    CK(LAUNCH(p, z_fused, g, rot, p->P, p->twz, p->err_d, p->st, 1, 0, kept ? g.Nz / 3 : -1));
+    CK(LAUNCH(p, z_fused, g, zform, p->P, p->twz, p->err_d, p->st, 1, 0, kept ? g.Nz / 3 : -1));
   }
   { ProfScope ps(p, TS_KCLASS_Y_FWD, by(TS_KCLASS_Y_FWD)); CK(LAUNCH(p, strided, g, 1, -1, p->P, nout, p->twy, p->st)); }
-  { ProfScope ps(p, TS_KCLASS_FWD_X, by(TS_KCLASS_FWD_X)); CK(LAUNCH(p, fwd_x, g, rot, mode, p->P, a, p->twx, p->st)); }
+  { ProfScope ps(p, TS_KCLASS_FWD_X, by(TS_KCLASS_FWD_X)); CK(LAUNCH(p, fwd_x, g, zform, mode, p->P, a, p->twx, p->st)); }
   return TS_OK;
 }
 
@@ -769,20 +772,19 @@ static int adjoint_step_fff(ts_plan* p, const void* U0, const void* stages, void
     const void* cot = stage == 4 ? (const void*)lam : (const void*)p->Ucur;
     const double lsc = stage == 4 ? p->cfg.dt / 6.0 : 1.0;
     a.stage = stage;
+    {
+      ProfScope ps(p, TS_KCLASS_INV_X);
+      CK(LAUNCH(p, inv_x, g, 1, Uin, p->P, p->twx, nullptr, 0.0, p->st, kept));
+      CK(LAUNCH(p, inv_x, g, 4, Uin, p->P, p->twx, cot, lsc, p->st));
+    }
     if (kept) {
       // u, w (fields 0-5) on the kept columns only, as in rhs_fff; the cotangent fields 6-8 are full
-      {
-        ProfScope ps(p, TS_KCLASS_INV_X);
-        CK(LAUNCH(p, inv_x, g, 1, Uin, p->P, p->twx, nullptr, 0.0, p->st, 1));
-        CK(LAUNCH(p, inv_x, g, 4, Uin, p->P, p->twx, cot, lsc, p->st));
-      }
       {
         ProfScope ps(p, TS_KCLASS_Y_INV);
         CK(LAUNCH(p, strided, g, 1, +1, p->P, 6, p->twy, p->st, 0, 0, g.Nz / 3 + 1, 1));
         CK(LAUNCH(p, strided, g, 1, +1, (char*)p->P + 6 * g.S * (long long)p->cb, 3, p->twy, p->st));
       }
     } else {
-      { ProfScope ps(p, TS_KCLASS_INV_X); CK(LAUNCH(p, inv_x, g, 3, Uin, p->P, p->twx, cot, lsc, p->st)); }
       { ProfScope ps(p, TS_KCLASS_Y_INV); CK(LAUNCH(p, strided, g, 1, +1, p->P, 9, p->twy, p->st)); }
     }
     { ProfScope ps(p, TS_KCLASS_Z); CK(LAUNCH(p, z_fused, g, 3, p->P, p->twz, p->err_d, p->st, 1, 0, kept ? g.Nz / 3 : -1)); }
@@ -822,7 +824,7 @@ static int step_rbc(ts_plan* p, void* U0, void* T0) {
     { ProfScope ps(p, TS_KCLASS_INV_X); CK(LAUNCH(p, sff_inv_x, g, Uin, Tin, p->P, p->twq, p->st)); }
     { ProfScope ps(p, TS_KCLASS_Y_INV); CK(LAUNCH(p, strided, g, 1, +1, p->P, 4, p->twy, p->st)); }
     { ProfScope ps(p, TS_KCLASS_Z); CK(LAUNCH(p, z_fused, g, 2, p->P, p->twz, p->err_d, p->st)); }
-    { ProfScope ps(p, TS_KCLASS_Y_FWD); CK(LAUNCH(p, strided, g, 1, -1, p->P, 9, p->twy, p->st)); }
+    { ProfScope ps(p, TS_KCLASS_Y_FWD); CK(LAUNCH(p, strided, g, 1, -1, p->P, 8, p->twy, p->st)); }
     { ProfScope ps(p, TS_KCLASS_FWD_X); CK(LAUNCH(p, sff_fwd_x, g, p->P, a, p->twq, p->st)); }
   }
   if (p->cfg.reality_fix) {
@@ -884,10 +886,10 @@ static int step_scalar_fff(ts_plan* p, void* U0, void* T0) {
     }
     { ProfScope ps(p, TS_KCLASS_Y_INV); CK(LAUNCH(p, strided, g, 1, +1, p->P, 4, p->twy, p->st, 0, 0, kept ? g.Nz / 3 + 1 : 0, kept)); }
     { ProfScope ps(p, TS_KCLASS_Z); CK(LAUNCH(p, z_fused, g, 2, p->P, p->twz, p->err_d, p->st, 1, 0, kept ? g.Nz / 3 : -1)); }
-    { ProfScope ps(p, TS_KCLASS_Y_FWD); CK(LAUNCH(p, strided, g, 1, -1, p->P, 9, p->twy, p->st)); }
+    { ProfScope ps(p, TS_KCLASS_Y_FWD); CK(LAUNCH(p, strided, g, 1, -1, p->P, 8, p->twy, p->st)); }
     {
       ProfScope ps(p, TS_KCLASS_FWD_X);
-      CK(LAUNCH(p, strided, g, 0, -1, p->P, 9, p->twx, p->st));
+      CK(LAUNCH(p, strided, g, 0, -1, p->P, 8, p->twx, p->st));
       CK(LAUNCH(p, scalar_epi, g, p->P, a, p->st));
     }
   }
@@ -966,10 +968,10 @@ static int step_mhd_fff(ts_plan* p, void* U0, void* B0) {
     }
     { ProfScope ps(p, TS_KCLASS_Y_INV); CK(LAUNCH(p, strided, g, 1, +1, p->P, 6, p->twy, p->st, 0, 0, kept ? g.Nz / 3 + 1 : 0, kept)); }
     { ProfScope ps(p, TS_KCLASS_Z); CK(LAUNCH(p, z_fused, g, 5, p->P, p->twz, p->err_d, p->st, 1, 0, kept ? g.Nz / 3 : -1)); }
-    { ProfScope ps(p, TS_KCLASS_Y_FWD); CK(LAUNCH(p, strided, g, 1, -1, p->P, 9, p->twy, p->st)); }
+    { ProfScope ps(p, TS_KCLASS_Y_FWD); CK(LAUNCH(p, strided, g, 1, -1, p->P, 8, p->twy, p->st)); }
     {
       ProfScope ps(p, TS_KCLASS_FWD_X);
-      CK(LAUNCH(p, strided, g, 0, -1, p->P, 9, p->twx, p->st));
+      CK(LAUNCH(p, strided, g, 0, -1, p->P, 8, p->twx, p->st));
       CK(LAUNCH(p, mhd_epi, g, p->P, a, p->st));
     }
   }
@@ -1041,7 +1043,7 @@ static int step_ssf(ts_plan* p, void* U0, void* T0 = nullptr) {
   const Geo& g = p->g;
   const Geo gy = y_as_x(g);
   const long long cs = g.S * (long long)p->cb;  // bytes of one component
-  const int nf = T0 ? 4 : 3, np = T0 ? 9 : 6;
+  const int nf = T0 ? 4 : 3, np = T0 ? 8 : 5;
   char* P = (char*)p->P;
   StageArgs a;
   memset(&a, 0, sizeof(a));
@@ -1059,7 +1061,7 @@ static int step_ssf(ts_plan* p, void* U0, void* T0 = nullptr) {
   // products u1u1, u2u2, u3u3 (Vi2 = CCF), u1u2 (VxVy = SSF), u2u3 (VyVz = CSF),
   // u3u1 (VxVz = SCF), u1T (CCF), u2T (SSF), u3T (SCF)
   const int vx[4] = {1, 0, 0, 1}, vy[4] = {0, 1, 0, 0};
-  const int qx[9] = {0, 0, 0, 1, 0, 1, 0, 1, 1}, qy[9] = {0, 0, 0, 1, 1, 0, 0, 1, 0};
+  const int qx[8] = {0, 0, 1, 0, 1, 0, 1, 1}, qy[8] = {0, 0, 1, 1, 0, 0, 1, 0};
   const double sy = 1.0 / (2.0 * g.Ny), sx = 1.0 / (2.0 * g.Nx * (double)g.Nz);
   // the same letters as bit masks (bit c = field c), one batched launch per pass
   int mx_in = 0, my_in = 0, mx_out = 0, my_out = 0;
@@ -1073,13 +1075,16 @@ static int step_ssf(ts_plan* p, void* U0, void* T0 = nullptr) {
     b.Tin = Tin;
     {
       ProfScope ps(p, TS_KCLASS_INV_X);
-      if (T0 && stage > 1) {
-        CK(LAUNCH(p, dealias_copy, g, Uin, P, 4, p->st));  // U and T are adjacent in Ucur
-      } else {
-        CK(LAUNCH(p, dealias_copy, g, Uin, P, 3, p->st));
-        if (T0) CK(LAUNCH(p, dealias_copy, g, Tin, P + 3 * cs, 1, p->st));
-      }
-      CK(LAUNCH(p, sff_x, g, +1, P, 1, mx_in, 1.0, p->twq, p->st, nf, g.S));
+      // U and T dealiased as they are read
+      ScArgs x{};
+      x.s0 = Uin;
+      x.s3 = T0 ? Tin : nullptr;
+      x.d = P;
+      x.sF = x.dF = x.plane = g.S;
+      x.nplanes = 1;
+      x.smask = mx_in;
+      x.deal = 1;
+      CK(LAUNCH(p, sc_x, g, +1, x, p->twq, p->st, nf));
     }
     {
       ProfScope ps(p, TS_KCLASS_Y_INV);
@@ -1090,7 +1095,7 @@ static int step_ssf(ts_plan* p, void* U0, void* T0 = nullptr) {
       // or 2 in real space, forward; unnormalised) reads the nf spectra and writes the
       // np product spectra in place
       ProfScope ps(p, TS_KCLASS_Z);
-      CK(LAUNCH(p, z_fused, g, T0 ? 2 : 0, P, p->twz, p->err_d, p->st));
+      CK(LAUNCH(p, z_fused, g, T0 ? 2 : 7, P, p->twz, p->err_d, p->st));
     }
     {
       ProfScope ps(p, TS_KCLASS_Y_FWD);
@@ -1116,7 +1121,7 @@ static int step_sss(ts_plan* p, void* U0, void* T0 = nullptr) {
   const Geo& g = p->g;
   const Geo gy = y_as_x(g);
   const long long cs = g.S * (long long)p->cb;
-  const int nf = T0 ? 4 : 3, np = T0 ? 9 : 6;
+  const int nf = T0 ? 4 : 3, np = T0 ? 8 : 5;
   char* P = (char*)p->P;
   StageArgs a;
   memset(&a, 0, sizeof(a));
@@ -1133,8 +1138,8 @@ static int step_sss(ts_plan* p, void* U0, void* T0 = nullptr) {
   // sine (1) / cosine (0) letters: Vx = SCC, Vy = CSC, Vz = CCS, T = SCC; products u1u1,
   // u2u2, u3u3 (CCC), u1u2 (SSC), u2u3 (CSS), u3u1 (SCS), u1T (CCC), u2T (SSC), u3T (SCS)
   const int vx[4] = {1, 0, 0, 1}, vy[4] = {0, 1, 0, 0}, vz[4] = {0, 0, 1, 0};
-  const int qx[9] = {0, 0, 0, 1, 0, 1, 0, 1, 1}, qy[9] = {0, 0, 0, 1, 1, 0, 0, 1, 0};
-  const int qz[9] = {0, 0, 0, 0, 1, 1, 0, 0, 1};
+  const int qx[8] = {0, 0, 1, 0, 1, 0, 1, 1}, qy[8] = {0, 0, 1, 1, 0, 0, 1, 0};
+  const int qz[8] = {0, 0, 0, 1, 1, 0, 0, 1};
   // the same letters as bit masks (bit c = field c), one batched launch per pass
   int mx_in = 0, my_in = 0, mx_out = 0, my_out = 0;
   for (int c = 0; c < nf; ++c) mx_in |= vx[c] << c, my_in |= vy[c] << c;
@@ -1147,13 +1152,16 @@ static int step_sss(ts_plan* p, void* U0, void* T0 = nullptr) {
     b.Tin = Tin;
     {
       ProfScope ps(p, TS_KCLASS_INV_X);
-      if (T0 && stage > 1) {
-        CK(LAUNCH(p, sss_dealias_copy, g, Uin, P, 4, p->st));  // U and T are adjacent in Ucur
-      } else {
-        CK(LAUNCH(p, sss_dealias_copy, g, Uin, P, 3, p->st));
-        if (T0) CK(LAUNCH(p, sss_dealias_copy, g, Tin, P + 3 * cs, 1, p->st));
-      }
-      CK(LAUNCH(p, sff_x, g, +1, P, 1, mx_in, 1.0, p->twq, p->st, nf, g.S));
+      // U and T dealiased as they are read
+      ScArgs x{};
+      x.s0 = Uin;
+      x.s3 = T0 ? Tin : nullptr;
+      x.d = P;
+      x.sF = x.dF = x.plane = g.S;
+      x.nplanes = 1;
+      x.smask = mx_in;
+      x.deal = 1;
+      CK(LAUNCH(p, sc_x, g, +1, x, p->twq, p->st, nf));
     }
     {
       ProfScope ps(p, TS_KCLASS_Y_INV);
@@ -1165,7 +1173,7 @@ static int step_sss(ts_plan* p, void* U0, void* T0 = nullptr) {
       int zin = 0, zout = 0;
       for (int c = 0; c < nf; ++c) zin |= vz[c] << c;
       for (int f = 0; f < np; ++f) zout |= qz[f] << f;
-      CK(LAUNCH(p, sss_z_fused, g, T0 ? 2 : 0, P, p->twz, p->twqz, zin, zout, p->st));
+      CK(LAUNCH(p, sss_z_fused, g, T0 ? 2 : 7, P, p->twz, p->twqz, zin, zout, p->st));
     }
     {
       ProfScope ps(p, TS_KCLASS_Y_FWD);
@@ -1769,8 +1777,8 @@ int ts_fft_forward(ts_plan* p, const char* parity, const void* real_in, void* sp
   CK(LAUNCH(p, z_single, g, -1, real_in, spec_out, ncomp, p->twz, p->st));
   CK(LAUNCH(p, strided, g, 1, -1, spec_out, ncomp, p->twy, p->st));
   if (xp == 0) {
-    CK(LAUNCH(p, strided, g, 0, -1, spec_out, ncomp, p->twx, p->st));
-    CK(LAUNCH(p, scale, spec_out, ncomp * g.S, 1.0 / ((double)g.Nx * g.Ny * g.Nz), p->st));
+    CK(LAUNCH(p, strided, g, 0, -1, spec_out, ncomp, p->twx, p->st, 0, 0, 0, 0, nullptr,
+              1.0 / ((double)g.Nx * g.Ny * g.Nz)));
   } else {
     // sin/cos analysis / (2 Nx) along x (SFF_pencil_tr.cc:43-55), Fourier / (Ny Nz) along y, z
     CK(LAUNCH(p, sff_x, g, -1, spec_out, ncomp, xp == 1, 1.0 / (2.0 * g.Nx * (double)g.Ny * g.Nz), p->twq, p->st));
@@ -1789,12 +1797,12 @@ int ts_fft_inverse(ts_plan* p, const char* parity, const void* spec_in, void* re
   }
   if (!is_device_ptr(spec_in) || !is_device_ptr(real_out)) return TS_ERR_ARG;
   const Geo& g = p->g;
-  // the reference copies the input to X_transform first (FFF_pencil_tr.cc:59)
-  CK(cudaMemcpyAsync(p->P, spec_in, ncomp * g.S * p->cb, cudaMemcpyDeviceToDevice, p->st));
+  // the reference copies the input to X_transform first (FFF_pencil_tr.cc:59); here the x
+  // pass reads the input and writes the work fields
   if (zp) {
     const long long cs = g.S * (long long)p->cb, nl = (long long)ncomp * g.Nx * g.Ny;
     char* P = (char*)p->P;
-    CK(LAUNCH(p, sff_x, g, +1, P, ncomp, xp == 1, 1.0, p->twq, p->st));
+    CK(LAUNCH(p, sff_x, g, +1, P, ncomp, xp == 1, 1.0, p->twq, p->st, 1, 0, spec_in));
     CK(LAUNCH(p, sff_x, y_as_x(g), +1, P, ncomp * g.Nx, yp == 1, 1.0, p->twqy, p->st));
     CK(LAUNCH(p, sss_zpre_inv, P, P + 3 * cs, nl, g.Nz, zp == 1, p->twqz, p->st));
     CK(LAUNCH(p, z_single, g, +1, P + 3 * cs, P + 6 * cs, ncomp, p->twz, p->st));
@@ -1802,13 +1810,14 @@ int ts_fft_inverse(ts_plan* p, const char* parity, const void* spec_in, void* re
     return TS_OK;
   }
   if (yp) {
-    CK(LAUNCH(p, sff_x, g, +1, p->P, ncomp, xp == 1, 1.0, p->twq, p->st));
+    CK(LAUNCH(p, sff_x, g, +1, p->P, ncomp, xp == 1, 1.0, p->twq, p->st, 1, 0, spec_in));
     CK(LAUNCH(p, sff_x, y_as_x(g), +1, p->P, ncomp * g.Nx, yp == 1, 1.0, p->twqy, p->st));
     CK(LAUNCH(p, z_single, g, +1, p->P, real_out, ncomp, p->twz, p->st));
     return TS_OK;
   }
-  if (xp == 0) CK(LAUNCH(p, strided, g, 0, +1, p->P, ncomp, p->twx, p->st));
-  else CK(LAUNCH(p, sff_x, g, +1, p->P, ncomp, xp == 1, 1.0, p->twq, p->st));
+  if (xp == 0)
+    CK(LAUNCH(p, strided, g, 0, +1, const_cast<void*>(spec_in), ncomp, p->twx, p->st, 0, 0, 0, 0, p->P));
+  else CK(LAUNCH(p, sff_x, g, +1, p->P, ncomp, xp == 1, 1.0, p->twq, p->st, 1, 0, spec_in));
   CK(LAUNCH(p, strided, g, 1, +1, p->P, ncomp, p->twy, p->st));
   CK(LAUNCH(p, z_single, g, +1, p->P, real_out, ncomp, p->twz, p->st));
   return TS_OK;
@@ -1959,7 +1968,7 @@ static int step_rbc_group(ens_group& G) {
     CK(LAUNCH(p, sff_inv_x, g, Uin, Tin, G.P, p->twq, G.st, B, msUin, msTin, 9 * S));
     CK(LAUNCH(p, strided, g, 1, +1, G.P, 4 * B, p->twy, G.st, 4, 9 * S));
     CK(LAUNCH(p, z_fused, g, 2, G.P, p->twz, p->err_d, G.st, B, 9 * S));
-    CK(LAUNCH(p, strided, g, 1, -1, G.P, 9 * B, p->twy, G.st));
+    CK(LAUNCH(p, strided, g, 1, -1, G.P, 8 * B, p->twy, G.st, 8, 9 * S));
     CK(LAUNCH(p, sff_fwd_x, g, G.P, a, p->twq, G.st, B));
   }
   if (p->cfg.reality_fix) {

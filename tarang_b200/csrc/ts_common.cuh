@@ -52,6 +52,11 @@ template <> __device__ __forceinline__ float2 scale<float2, float>(float2 a, flo
 template <int SIGN, typename V> __device__ __forceinline__ V mul_i(V a) {
   return SIGN > 0 ? mk<V>(-a.y, a.x) : mk<V>(a.y, -a.x);
 }
+// a + i b (SIGN = +1) or a - i b (SIGN = -1): two plain adds, where mul_i and a packed
+// add would first have to swap and negate the halves of a register pair
+template <int SIGN, typename V> __device__ __forceinline__ V add_i(V a, V b) {
+  return SIGN > 0 ? mk<V>(a.x - b.y, a.y + b.x) : mk<V>(a.x + b.y, a.y - b.x);
+}
 // i * K * a for real K
 template <typename V, typename S> __device__ __forceinline__ V ik(S K, V a) { return mk<V>(-K * a.y, K * a.x); }
 
@@ -66,7 +71,14 @@ __device__ __forceinline__ double c32(int k) {
 }
 __device__ __forceinline__ double s32(int k) { return k <= 8 ? c32(8 - k) : c32(k - 8); }
 
-// In-register DFT of size R (2, 3, 4, 8, 16, 32), natural order in and out.
+// cos / sin of pi*k/6, k = 0..5
+__device__ __forceinline__ double c12(int k) {
+  const double t[6] = {1.0, 0.86602540378443864676, 0.5, 0.0, -0.5, -0.86602540378443864676};
+  return t[k];
+}
+__device__ __forceinline__ double s12(int k) { return k <= 3 ? c12(3 - k) : c12(k - 3); }
+
+// In-register DFT of size R (2, 3, 4, 6, 8, 12, 16, 32), natural order in and out.
 // DIR = -1: forward (e^{-2 pi i jk/R}), +1: inverse (unnormalised).
 template <int R, int DIR, typename V> struct DFT;
 template <int DIR, typename V> struct DFT<1, DIR, V> {
@@ -85,10 +97,10 @@ template <int DIR, typename V> struct DFT<3, DIR, V> {
     typedef decltype(V::x) S;
     const V a = v[0], s = add(v[1], v[2]), d = sub(v[1], v[2]);
     const V t = sub(a, scale(s, (S)0.5));
-    const V u = scale(mul_i<DIR>(d), (S)0.86602540378443864676);
+    const V u = scale(d, (S)0.86602540378443864676);
     v[0] = add(a, s);
-    v[1] = add(t, u);
-    v[2] = sub(t, u);
+    v[1] = add_i<DIR>(t, u);
+    v[2] = add_i<-DIR>(t, u);
   }
 };
 template <int R, int DIR, typename V> struct DFT {
@@ -103,11 +115,15 @@ template <int R, int DIR, typename V> struct DFT {
 #pragma unroll
     for (int k = 0; k < R / 2; ++k) {
       V t;
-      static_assert(R <= 32, "the twiddle table covers radices up to 32");
-      const int q = k * (32 / R);  // angle pi*q/16 = 2 pi k / R
+      static_assert(R % 3 == 0 ? R <= 12 : R <= 32, "the twiddle tables cover radices up to 32 (12 with a factor 3)");
+      const int q = R % 3 == 0 ? k * (12 / R) : k * (32 / R);  // angle pi*q/6 or pi*q/16 = 2 pi k / R
+      if (4 * k == R) {
+        v[k] = add_i<DIR>(e[k], o[k]);
+        v[k + R / 2] = add_i<-DIR>(e[k], o[k]);
+        continue;
+      }
       if (k == 0) t = o[k];
-      else if (4 * k == R) t = mul_i<DIR>(o[k]);
-      else t = mul(o[k], mk<V>((S)c32(q), (S)(DIR * s32(q))));
+      else t = mul(o[k], R % 3 == 0 ? mk<V>((S)c12(q), (S)(DIR * s12(q))) : mk<V>((S)c32(q), (S)(DIR * s32(q))));
       v[k] = add(e[k], t);
       v[k + R / 2] = sub(e[k], t);
     }
@@ -117,19 +133,25 @@ template <int R, int DIR, typename V> struct DFT {
 // ---------------------------------------------------------------------------
 // Stockham radix schedule for length L with at most E elements per thread.
 // ---------------------------------------------------------------------------
-// L = 2^a (or 3 * 2^a): the power-of-two part is split into passes of radix
-// min(lowbit(E), remaining); a factor 3 is one final radix-3 pass.  Every radix
+// L = 2^a: passes of radix min(lowbit(E), remaining).  L = 3 * 2^a: first one pass of
+// radix 3 * 2^b, b such that it divides E and is at most 12, then the rest as a power of
+// two (96 points with 24 elements per thread: 12, 8; 48 with 12: 12, 4).  Every radix
 // divides E, so a thread always owns whole butterflies.
 __host__ __device__ constexpr int lowbit(int x) { return x & (-x); }
 __host__ __device__ constexpr int rad2(int L2, int E2, int p) {
   return p == 0 ? (L2 < E2 ? L2 : E2) : rad2(L2 / (L2 < E2 ? L2 : E2), E2, p - 1);
 }
 __host__ __device__ constexpr int np2(int L2, int E2) { return L2 <= 1 ? 0 : 1 + np2(L2 / (L2 < E2 ? L2 : E2), E2); }
+// radix of the first pass of a length with a factor 3
+__host__ __device__ constexpr int rad3(int L, int E) {
+  const int b = lowbit(E) < lowbit(L) ? lowbit(E) : lowbit(L);
+  return 3 * (b < 4 ? b : 4);
+}
 __host__ __device__ constexpr int radix_at(int L, int E, int p) {
-  return p < np2(lowbit(L), lowbit(E)) ? rad2(lowbit(L), lowbit(E), p) : L / lowbit(L);
+  return L == lowbit(L) ? rad2(L, lowbit(E), p) : (p == 0 ? rad3(L, E) : rad2(L / rad3(L, E), lowbit(E), p - 1));
 }
 __host__ __device__ constexpr int npasses(int L, int E) {
-  return np2(lowbit(L), lowbit(E)) + (L != lowbit(L) ? 1 : 0);
+  return L == lowbit(L) ? np2(L, lowbit(E)) : 1 + np2(L / rad3(L, E), lowbit(E));
 }
 __host__ __device__ constexpr int ns_at(int L, int E, int p) {
   // product of the radices before pass p
@@ -280,43 +302,54 @@ __device__ __forceinline__ void fft_regs(V* v, int t, V* sm, int rs, int cs, con
   }
 }
 
-// ---------------------------------------------------------------------------
-// Shared-memory line FFTs with all threads of the block cooperating
-// (used by the contiguous-axis kernels, where lines are short and the real
-// transform pre/post-processing needs element pairs k, M-k).
-// Stockham ping-pong: reads src, writes dst, swaps; returns the buffer that
-// holds the result.  Lines are at src + l*ld.
-// ---------------------------------------------------------------------------
-template <int L, int E, int DIR, int P = 0, typename V>
-__device__ V* fft_smem_lines(V* src, V* dst, int nlines, int ld, const V* __restrict__ tw, int tws) {
-  typedef Pass<L, E, P> PP;
+// NB transforms of the same length at once: every pass's butterflies of all of them, then
+// one exchange (transform b through the slot sm + b * slot) between two barriers.  The
+// barriers and the twiddle loads are shared and NB times as many shared-memory accesses
+// are in flight between them.  WARP: the threads of a line sit in one warp, so a warp
+// barrier orders the exchange.
+template <bool WARP> __device__ __forceinline__ void fft_sync() {
+  if (WARP) __syncwarp();
+  else __syncthreads();
+}
+template <int L, int E, int P, int DIR, bool REV, int NB, typename V>
+__device__ __forceinline__ void pass_compute_b(V (&v)[NB][E], int t, const V* __restrict__ tw, int tws) {
+  typedef Pass<L, E, P, REV> PP;
   constexpr int R = PP::R, NS = PP::NS;
-  const int nb = nlines * (L / R);
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    const int line = b / (L / R);
-    const int j = b % (L / R);
-    const int k = j % NS;
-    V v[R];
-    const V* s = src + line * ld;
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = s[j + r * (L / R)];
+  for (int q = 0; q < PP::B; ++q) {
     if (NS > 1) {
+      const int j = t * PP::B + q;
+      const int k = j % NS;
 #pragma unroll
       for (int r = 1; r < R; ++r) {
         V w = tw[(r * k * (L / (NS * R))) * tws];
         if (DIR > 0) w.y = -w.y;
-        v[r] = mul(v[r], w);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) v[b][q * R + r] = mul(v[b][q * R + r], w);
       }
     }
-    DFT<R, DIR, V>::run(v);
-    V* d = dst + line * ld;
-    const int o = (j / NS) * NS * R + k;
 #pragma unroll
-    for (int r = 0; r < R; ++r) d[o + r * NS] = v[r];
+    for (int b = 0; b < NB; ++b) DFT<R, DIR, V>::run(v[b] + q * R);
   }
-  __syncthreads();
-  if constexpr (P + 1 < npasses(L, E)) return fft_smem_lines<L, E, DIR, P + 1>(dst, src, nlines, ld, tw, tws);
-  else return dst;
+}
+template <int L, int E, int DIR, int NB, bool WARP, int P = 0, bool PAD = false, bool REV = false, int SWK = 0,
+          typename V>
+__device__ __forceinline__ void fft_regs_b(V (&v)[NB][E], int t, V* sm, int slot, int rs, int cs,
+                                           const V* __restrict__ tw, int tws) {
+  pass_compute_b<L, E, P, DIR, REV, NB>(v, t, tw, tws);
+  if constexpr (P + 1 < npasses(L, E)) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int s = 0; s < E; ++s) sm[b * slot + xrow<PAD, SWK>(Pass<L, E, P, REV>::out_row(t, s)) * rs + cs] = v[b][s];
+    fft_sync<WARP>();
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int s = 0; s < E; ++s) v[b][s] = sm[b * slot + xrow<PAD, SWK>(Pass<L, E, P + 1, REV>::in_row(t, s)) * rs + cs];
+    fft_sync<WARP>();
+    fft_regs_b<L, E, DIR, NB, WARP, P + 1, PAD, REV, SWK>(v, t, sm, slot, rs, cs, tw, tws);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -327,6 +360,11 @@ template <typename V> __device__ __forceinline__ void cp_async(V* dst, const V* 
   const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
   if constexpr (sizeof(V) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(src) : "memory");
   else asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(src) : "memory");
+}
+// 16 bytes, both addresses 16-byte aligned
+template <typename V> __device__ __forceinline__ void cp_async16(V* dst, const V* src) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }

@@ -123,6 +123,45 @@ __global__ void __launch_bounds__(CW * (L / E), (CW * (L / E)) <= 256 ? 2 : 1)
 }
 
 // ---------------------------------------------------------------------------
+// strided-axis FFT, direct-load form: one tile of CW columns per block, every row of a
+// thread loaded straight into its registers (E loads in flight per thread, no staging
+// tile), one exchange tile of L x CW complex, so that two to four blocks share an SM and
+// overlap one another's loads, exchanges and stores.
+// The columns of all fields and outer planes are one run (column q = field, outer index,
+// column of the plane), so no tile is cut at a plane's end.  src == dst: in place (a
+// block's tile is wholly in registers before its first store).  Outputs are multiplied
+// by scl where SCALE.
+// ---------------------------------------------------------------------------
+template <typename T, int L, int E, int CW, int DIR, int MINB, bool SCALE>
+__global__ void __launch_bounds__(CW * (L / E), MINB)
+    k_strided_ld(const C<T>* src, C<T>* dst, unsigned ntot, unsigned nplane, unsigned inner, long long fstride,
+                 long long rstride, long long ostride, const C<T>* __restrict__ tw, unsigned per, long long mstride,
+                 int zero_hi, T scl) {
+  typedef C<T> V;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  V* xch = reinterpret_cast<V*>(smraw);
+  const int c = threadIdx.x % CW, t = threadIdx.x / CW;
+  const unsigned q = blockIdx.x * CW + c;
+  const bool ok = q < ntot;
+  const unsigned qq = ok ? q : 0;
+  const unsigned f = qq / nplane, r = qq - f * nplane, o = r / inner, col = r - o * inner;
+  const long long off = (long long)(f / per) * mstride + (long long)(f % per) * fstride + (long long)o * ostride + col;
+  const V* a = src + off;
+  V v[E];
+#pragma unroll
+  for (int s = 0; s < E; ++s) {
+    // zero_hi: rows with 3 |k| > L (two-thirds dealiased) are zero and were not written
+    const int row = load_row<L, E>(t, s);
+    v[s] = (ok && !(zero_hi && 3 * (row < L - row ? row : L - row) > L)) ? a[row * rstride] : mk<V>(0, 0);
+  }
+  fft_regs<L, E, DIR, 0, false, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
+  if (!ok) return;
+  V* d = dst + off;
+#pragma unroll
+  for (int s = 0; s < E; ++s) d[final_row<L, E>(t, s) * rstride] = SCALE ? scale(v[s], scl) : v[s];
+}
+
+// ---------------------------------------------------------------------------
 // inverse x pass: W_i = IFFT_x(D(U_i)); rotational form also W_{3+i} = IFFT_x(D(omega_i)),
 // omega = i K x D(U).  col = ly*Hz + lz; row = lx.
 // Persistent over column tiles.  Thread 0 streams the three components of a
@@ -346,6 +385,118 @@ __global__ void __launch_bounds__(CW * (L / E), (CW * (L / E)) <= 256 ? 2 : 1)
 
 
 // ---------------------------------------------------------------------------
+// inverse x pass, one output field per block: every row is loaded straight into registers
+// (as in k_strided_ld), a vorticity row is combined from the two components it needs, a
+// projected cotangent row from three.  The input components are read once per output field
+// that needs them; the blocks of a column tile's fields are neighbours (field fastest), so
+// all but the first read hit L2.  16 elements per thread and one field keep it at 64-80
+// registers and 24-32 warps per SM, where the form with all fields of a tile in one block
+// (k_inv_x_ld) holds U in registers, 8 elements per thread and 16 warps.
+// Fields and FORMs as k_inv_x_ld (FORM 0, 1, 4, 5).
+// ---------------------------------------------------------------------------
+// rows [lo, hi) of the column (ly, lz) are cleared by dealiasing (dealias_zero, basis 0)
+__device__ __forceinline__ void fff_zero_rows(int mode, int ly, int lz, int Nx, int Ny, int Nz, int& lo, int& hi) {
+  lo = hi = Nx;
+  if (mode == 1) {
+    if (ly >= Ny / 3 + 1 && ly <= 2 * Ny / 3 - 1 && lz >= Nz / 3 + 1) lo = Nx / 3 + 1, hi = 2 * Nx / 3;
+  } else if (mode == 2) {
+    const bool out = 3 * abs(kfft(ly, Ny)) > Ny || 3 * lz > Nz;
+    lo = out ? 0 : Nx / 3 + 1;
+    hi = out ? Nx : Nx - Nx / 3;
+  }
+}
+
+template <typename T, int L, int E, int CW, int FORM, int MINB>
+__global__ void __launch_bounds__(CW * (L / E), MINB)
+    k_inv_x_f(const C<T>* __restrict__ U, C<T>* __restrict__ W, Geo g, const C<T>* __restrict__ tw,
+              const C<T>* __restrict__ Lam, T lsc, int kept, double rad) {
+  typedef C<T> V;
+  static_assert(FORM == 0 || FORM == 1 || FORM == 4 || FORM == 5, "fluid forms, cotangent, flux giver");
+  constexpr unsigned NF = FORM == 1 || FORM == 5 ? 6 : 3;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  V* xch = reinterpret_cast<V*>(smraw);
+  const int c = threadIdx.x % CW, t = threadIdx.x / CW;
+  const unsigned inner = g.Ny * g.Hz;
+  const unsigned f = blockIdx.x % NF, q = (blockIdx.x / NF) * CW + c;
+  unsigned ly, lz;
+  bool ok;
+  if (kept) {
+    // two-thirds dealiasing: only the columns with 3|ky| <= Ny and 3 kz <= Nz can be
+    // nonzero; they are one run of columns here, the others are not written, and the y and
+    // z passes treat them as zero without reading them
+    const unsigned qy = g.Ny / 3, nzk = g.Nz / 3 + 1, iy = q / nzk;
+    lz = q - iy * nzk;
+    ok = iy <= 2 * qy;
+    ly = iy <= qy ? iy : iy + g.Ny - (2 * qy + 1);
+  } else {
+    ok = q < inner;
+    ly = q / g.Hz;
+    lz = q - ly * g.Hz;
+  }
+  if (!ok) ly = lz = 0;
+  const long long col = (long long)ly * g.Hz + lz, rstride = inner;
+  const T Ky = (T)(kfft(ly, g.Ny) * g.kf[1]), Kz = (T)(lz * g.kf[2]);
+  V v[E];
+  if constexpr (FORM == 4) {
+    // (P Lam)_i = Lam_i - K_i (K . Lam) / K^2, identity at K = 0
+    const T lw = (lz > 0 && 2 * (int)lz < g.Nz) ? lsc * (T)0.5 : lsc;
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int lx = load_row<L, E>(t, s);
+      const long long off = lx * rstride + col;
+      const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]);
+      v[s] = mk<V>(0, 0);
+      if (ok) {
+        const V l0 = Lam[off], l1 = Lam[g.S + off], l2 = Lam[2 * g.S + off];
+        const T K2 = (Kx * Kx + Ky * Ky) + Kz * Kz;
+        const V d = add(add(scale(l0, Kx), scale(l1, Ky)), scale(l2, Kz));
+        const V p = K2 > (T)0 ? mk<V>(d.x / K2, d.y / K2) : mk<V>(0, 0);
+        v[s] = scale(f == 0 ? sub(l0, scale(p, Kx)) : f == 1 ? sub(l1, scale(p, Ky)) : sub(l2, scale(p, Kz)), lw);
+      }
+    }
+  } else {
+    int zlo, zhi;
+    fff_zero_rows(g.dealias, ly, lz, g.Nx, g.Ny, g.Nz, zlo, zhi);
+    if (!ok) zlo = 0, zhi = L;
+    if (FORM == 0 || f < 3 || FORM == 5) {
+      const V* src = U + (f < 3 ? f : f - 3) * g.S + col;
+#pragma unroll
+      for (int s = 0; s < E; ++s) {
+        const int lx = load_row<L, E>(t, s);
+        v[s] = (lx >= zlo && lx < zhi) ? mk<V>(0, 0) : src[lx * rstride];
+      }
+      if (FORM == 5 && f >= 3) {
+        // inside |K| <= rad with |K| = sqrt((Kx^2 + Ky^2) + Kz^2) in FP64 (Kmagnitude)
+        const double Kyd = kfft(ly, g.Ny) * g.kf[1], Kzd = lz * g.kf[2];
+#pragma unroll
+        for (int s = 0; s < E; ++s) {
+          const double Kxd = kfft(load_row<L, E>(t, s), g.Nx) * g.kf[0];
+          if (!(sqrt((Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd) <= rad)) v[s] = mk<V>(0, 0);
+        }
+      }
+    } else {
+      // omega_i = i (K_{i+1} U_{i+2} - K_{i+2} U_{i+1})  (indices mod 3)
+      const int i = (int)f - 3, i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
+      const V *sa = U + i1 * g.S + col, *sb = U + i2 * g.S + col;
+#pragma unroll
+      for (int s = 0; s < E; ++s) {
+        const int lx = load_row<L, E>(t, s);
+        const bool z = lx >= zlo && lx < zhi;
+        const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]);
+        const T Ka = i1 == 0 ? Kx : (i1 == 1 ? Ky : Kz), Kb = i2 == 0 ? Kx : (i2 == 1 ? Ky : Kz);
+        const V ua = z ? mk<V>(0, 0) : sa[lx * rstride], ub = z ? mk<V>(0, 0) : sb[lx * rstride];
+        v[s] = mul_i<1>(sub(scale(ub, Ka), scale(ua, Kb)));
+      }
+    }
+  }
+  fft_regs<L, E, 1, 0, false, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
+  if (!ok) return;
+  V* d = W + (f + (FORM == 4 ? 6 : 0)) * g.S + col;
+#pragma unroll
+  for (int s = 0; s < E; ++s) d[final_row<L, E>(t, s) * rstride] = v[s];
+}
+
+// ---------------------------------------------------------------------------
 // inverse x pass with the tile's U staged in shared memory (two-thirds dealiasing,
 // FORM 0 / 1): one column tile per block (the kept-column mapping of k_inv_x_ld); every
 // thread stages the kept rows (3 |kx| <= Nx) of the three components that it will read
@@ -355,8 +506,8 @@ __global__ void __launch_bounds__(CW * (L / E), (CW * (L / E)) <= 256 ? 2 : 1)
 // Shared memory: 3 x LK x CW staged complex (LK = 2 (L/3) + 1 kept rows) + L x CW exchange.
 // ---------------------------------------------------------------------------
 template <int L> __host__ __device__ constexpr int ix_kept_rows() { return 2 * (L / 3) + 1; }
-template <typename T, int L, int E, int CW, int FORM>
-__global__ void __launch_bounds__(CW * (L / E), 1)
+template <typename T, int L, int E, int CW, int FORM, int MINB = 1>
+__global__ void __launch_bounds__(CW * (L / E), MINB)
     k_inv_x_st(const C<T>* __restrict__ U, C<T>* __restrict__ W, Geo g, const C<T>* __restrict__ tw) {
   typedef C<T> V;
   static_assert(FORM == 0 || FORM == 1, "the fluid forms");
@@ -367,12 +518,12 @@ __global__ void __launch_bounds__(CW * (L / E), 1)
   const int c = threadIdx.x % CW, t = threadIdx.x / CW;
   const int inner = g.Ny * g.Hz;
   const long long rstride = inner;
-  const int qy = g.Ny / 3, nzk = g.Nz / 3 + 1, ntz = (nzk + CW - 1) / CW;
-  const int iy = blockIdx.x / ntz, lzc = (blockIdx.x % ntz) * CW + c;
-  const int ky = iy <= qy ? iy : iy - (2 * qy + 1);
-  const bool ok = lzc < nzk;
-  const int col = ((ky + g.Ny) % g.Ny) * g.Hz + (ok ? lzc : 0);
-  const int lz = ok ? lzc : 0;
+  // the kept columns as one run, so no tile is cut at the end of a kept row
+  const unsigned qy = g.Ny / 3, nzk = g.Nz / 3 + 1, q0 = blockIdx.x * CW + c, iy0 = q0 / nzk;
+  const bool ok = iy0 <= 2 * qy;
+  const int iy = ok ? iy0 : 0, lz = ok ? q0 - iy0 * nzk : 0;
+  const int ky = iy <= (int)qy ? iy : iy - (int)(2 * qy + 1);
+  const int col = (ky < 0 ? ky + g.Ny : ky) * g.Hz + lz;
   const T Ky = (T)(ky * g.kf[1]), Kz = (T)(lz * g.kf[2]);
   // staged row of x row lx (kept rows only: lx <= Q or lx >= L - Q)
   auto krow = [](int lx) { return lx <= Q ? lx : lx - (L - 2 * Q - 1); };
@@ -536,20 +687,25 @@ __global__ void __launch_bounds__(CW * (L / E), 1)
 template <int M> __host__ __device__ constexpr int zslot() { return M + M / 16 + 1; }
 
 // Real-space product forms of the z pass.
-// FORM 0 (conservative):  in u1,u2,u3       -> u1u1,u2u2,u3u3,u1u2,u2u3,u3u1
+// FORM 0 (conservative, whole tensor): in u1,u2,u3 -> u1u1,u2u2,u3u3,u1u2,u2u3,u3u1
+// FORM 7 (conservative step): in u1,u2,u3 -> d1,d2,u1u2,u2u3,u3u1 with d1 = u1u1 - u3u3,
+//         d2 = u2u2 - u3u3: taking u3u3 off the diagonal changes N by the gradient of u3u3,
+//         which the projection removes, so a step needs one transform less
 // FORM 1 (rotational):    in u1..3,w1..3    -> u x w
-// FORM 2 (Boussinesq):    in u1,u2,u3,T     -> the six u_i u_j, then u1T,u2T,u3T
+// FORM 2 (scalar, Boussinesq): in u1,u2,u3,T -> the five of FORM 7, then u1T,u2T,u3T
 //                         (compute_diag_offdiag.cc:47-136)
 // FORM 3 (adjoint of the rotational form): in u, w, mu -> mu x u, then w x mu
-// FORM 5 (MHD):           in u1..3, b1..3      -> Zp_i Zm_j (f = 3 i + j), Zp = u + b, Zm = u - b
-//                         (compute_nlin_VF_MHD.cc:40-95, MHD.cc:75-84)
-// FORM 6 (flux giver):    in u1..3, g1..3      -> u_i g_j (f = 3 i + j), for the giver nonlinear
+// FORM 5 (MHD):           in u1..3, b1..3 -> the symmetric part S_ij = u_i u_j - b_i b_j of
+//         Zp_i Zm_j, Zp = u + b, Zm = u - b, as S11 - S33, S22 - S33, S12, S23, S31, and the
+//         antisymmetric part A_ij = b_i u_j - u_i b_j as A12, A23, A31: U.nlin is the
+//         divergence of S and B.nlin that of A (compute_nlin_VF_MHD.cc:40-95, MHD.cc:75-84,150-161)
+// FORM 6 (flux giver):    in u1..3, g1..3   -> u_i g_j (f = 3 i + j), for the giver nonlinear
 //                         term N_i = sum_j D_j F[u_j g_i] (compute_nlin_ET_VF.cc:71-87)
 __host__ __device__ constexpr int z_nin(int form) {
-  return form == 0 ? 3 : (form == 1 ? 6 : (form == 2 ? 4 : ((form == 5 || form == 6) ? 6 : 9)));
+  return (form == 0 || form == 7) ? 3 : (form == 2 ? 4 : (form == 3 ? 9 : 6));
 }
 __host__ __device__ constexpr int z_nout(int form) {
-  return form == 0 ? 6 : (form == 1 ? 3 : (form == 2 ? 9 : ((form == 5 || form == 6) ? 9 : 6)));
+  return form == 0 ? 6 : (form == 7 ? 5 : (form == 1 ? 3 : (form == 6 ? 9 : (form == 3 ? 6 : 8))));
 }
 
 // component f of a x b for real points packed two per complex (re, im independent)
@@ -557,23 +713,26 @@ template <typename V> __device__ __forceinline__ V cross_pk(int f, const V* a, c
   const int i = f == 2 ? 0 : f + 1, j = f == 0 ? 2 : f - 1;
   return mk<V>(a[i].x * b[j].x - a[j].x * b[i].x, a[i].y * b[j].y - a[j].y * b[i].y);
 }
-// factor indices (a, b) of product output f for FORM 0 / 2
-__host__ __device__ constexpr int z_pa(int f, int form = 0) {
-  return (form == 5 || form == 6) ? f / 3 : (f < 3 ? f : (f < 6 ? f - 3 : f - 6));
+template <typename V> __device__ __forceinline__ V prod_pk(V a, V b) { return mk<V>(a.x * b.x, a.y * b.y); }
+// a c - b d
+template <typename V> __device__ __forceinline__ V diff_pk(V a, V c, V b, V d) {
+  return mk<V>(a.x * c.x - b.x * d.x, a.y * c.y - b.y * d.y);
 }
-__host__ __device__ constexpr int z_pb(int f, int form = 0) {
-  return (form == 5 || form == 6) ? 3 + f % 3 : (f < 3 ? f : (f < 6 ? (f == 5 ? 0 : f - 2) : 3));
-}
-// FORM 5: the real lines of u and b (packed two points per complex) become the
-// Elsasser lines Zp = u + b, Zm = u - b in place
-template <int FORM, typename V> __device__ __forceinline__ void z_elsasser(V* in) {
-  if constexpr (FORM == 5) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const V u = in[c], b = in[c + 3];
-      in[c] = add(u, b);
-      in[c + 3] = sub(u, b);
-    }
+// product f of a form from its inputs at a point (f known at compile time; not FORM 3)
+template <int FORM, typename V> __device__ __forceinline__ V z_product(int f, const V* in) {
+  if constexpr (FORM == 1) {
+    return cross_pk(f, in, in + 3);
+  } else if constexpr (FORM == 0) {
+    return f < 3 ? prod_pk(in[f], in[f]) : prod_pk(in[f - 3], in[f == 5 ? 0 : f - 2]);
+  } else if constexpr (FORM == 6) {
+    return prod_pk(in[f / 3], in[3 + f % 3]);
+  } else if constexpr (FORM == 5) {
+    if (f < 2) return sub(diff_pk(in[f], in[f], in[3 + f], in[3 + f]), diff_pk(in[2], in[2], in[5], in[5]));
+    const int i = (f - 2) % 3, j = (i + 1) % 3;
+    return f < 5 ? diff_pk(in[i], in[j], in[3 + i], in[3 + j]) : diff_pk(in[3 + i], in[j], in[i], in[3 + j]);
+  } else {
+    if (f < 2) return diff_pk(in[f], in[f], in[2], in[2]);
+    return f < 5 ? prod_pk(in[f - 2], in[(f - 1) % 3]) : prod_pk(in[f - 5], in[3]);
   }
 }
 
@@ -622,21 +781,15 @@ __global__ void __launch_bounds__(256) k_z_fused(C<T>* __restrict__ P, Geo g, co
     V in[NIN];
 #pragma unroll
     for (int c = 0; c < NIN; ++c) in[c] = slot(c, ll)[m];
-    z_elsasser<FORM>(in);
     if constexpr (FORM == 3) {
 #pragma unroll
       for (int f = 0; f < 3; ++f) {
         slot(f, ll)[m] = cross_pk(f, in + 6, in);
         slot(3 + f, ll)[m] = cross_pk(f, in + 3, in + 6);
       }
-    } else if (FORM != 1) {
-#pragma unroll
-      for (int f = 0; f < NOUT; ++f)
-        slot(f, ll)[m] = mk<V>(in[z_pa(f, FORM)].x * in[z_pb(f, FORM)].x, in[z_pa(f, FORM)].y * in[z_pb(f, FORM)].y);
     } else {
-      slot(0, ll)[m] = mk<V>(in[1].x * in[5].x - in[2].x * in[4].x, in[1].y * in[5].y - in[2].y * in[4].y);
-      slot(1, ll)[m] = mk<V>(in[2].x * in[3].x - in[0].x * in[5].x, in[2].y * in[3].y - in[0].y * in[5].y);
-      slot(2, ll)[m] = mk<V>(in[0].x * in[4].x - in[1].x * in[3].x, in[0].y * in[4].y - in[1].y * in[3].y);
+#pragma unroll
+      for (int f = 0; f < NOUT; ++f) slot(f, ll)[m] = z_product<FORM>(f, in);
     }
   }
   __syncthreads();
@@ -661,114 +814,6 @@ __global__ void __launch_bounds__(256) k_z_fused(C<T>* __restrict__ P, Geo g, co
       const V s = scale(add(Z, Zp), (T)0.5);
       const V d = mul_i<-1>(mul(tw[k], scale(sub(Z, Zp), (T)0.5)));
       dst[e] = add(s, d);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// SSS z pass, fused: per z line of real coefficients (N + 2 reals, the padded real
-// layout), the sin/cos inverse of the NIN inputs, the real products of FORM 0 / 2,
-// and the sin/cos forward of the NOUT products, in place.  The sin/cos transforms are
-// the x / y passes' algorithm along z: a quarter-step twiddle (tq = e^{-i pi m / 2N})
-// on the half spectrum of the reordered line v (v_k = u_2k, v_{N-1-k} = +-u_{2k+1},
-// minus for a sine series) and one real FFT of length N, the same real FFT and slot
-// layout as k_z_fused.  The lines are never put back in natural order: the product of
-// two reordered lines is the reordered product with the product's own sign pattern
-// (sine x sine = cosine, sine x cosine = sine, and the sign flips multiply), so the
-// forward transform takes it as it is.  zin / zout: bit c set = input / output c is a
-// sine series along z; scl = 1 / (2N).
-//   inverse: V_m = conj(w_m) (c_m - i c_{N-m}) (cosine, V_0 = c_0),
-//            conj(w_m) (s_{N-m} - i s_m) (sine, V_0 = 0); real inverse FFT of V
-//   forward: Z = real FFT of v; c_m = 2 scl Re(w_m Z_m) (cosine), -2 scl Im(w_m Z_m)
-//            (sine), Z_m = conj(Z_{N-m}) above N/2; the two padding reals written 0
-// ---------------------------------------------------------------------------
-template <typename T, int NZ, int E, int FORM>
-__global__ void __launch_bounds__(256) k_sss_z_fused(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw,
-                                                     const C<T>* __restrict__ tq, int nl, int zin, int zout,
-                                                     T scl) {
-  typedef C<T> V;
-  constexpr int N = NZ, M = NZ / 2, H = M + 1, TPL = M / E, LDS = zslot<M>();
-  constexpr int NIN = z_nin(FORM), NOUT = z_nout(FORM);
-  static_assert(FORM == 0 || FORM == 2 || FORM == 6,
-                "SSS z pass: conservative products, with or without T, or the flux giver's products");
-  extern __shared__ __align__(16) unsigned char smraw[];
-  V* sm = reinterpret_cast<V*>(smraw);
-  const long long nlines = (long long)g.Nx * g.Ny;
-  const long long line0 = (long long)blockIdx.x * nl;
-  const int nh = (int)((nlines - line0) < nl ? (nlines - line0) : nl);
-  const int l = threadIdx.x / TPL, t = threadIdx.x % TPL;
-  const bool live = l < nh;
-  const long long lbase = (line0 + (live ? l : 0)) * H;
-  auto slot = [&](int c, int ll) { return sm + (c * nl + ll) * LDS; };
-
-  // A. inverse of each input line into its slot (real points packed two per complex)
-  for (int c = 0; c < NIN; ++c) {
-    const T* cl = reinterpret_cast<const T*>(P + c * g.S + lbase);  // reals 0 .. N-1 of the line
-    const bool sine = (zin >> c) & 1;
-    auto half = [&](int m) -> V {  // V_m, 0 <= m <= M
-      if (m == 0) return mk<V>(sine ? (T)0 : cl[0], (T)0);
-      const T a = sine ? cl[N - m] : cl[m], b = sine ? cl[m] : cl[N - m];
-      return mul(conjg(tq[m]), mk<V>(a, -b));
-    };
-    V v[E];
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-      const int k = load_row<M, E>(t, s);
-      V a = mk<V>(0, 0), b = mk<V>(0, 0);
-      if (live) {
-        a = half(k);
-        b = conjg(half(M - k));
-      }
-      if (k == 0) { a.y = 0; b.y = 0; }
-      v[s] = add(add(a, b), mul_i<1>(mul(conjg(tw[k]), sub(a, b))));
-    }
-    V* sl = slot(c, l < nl ? l : 0);
-    fft_regs<M, E, 1, 0, true>(v, t, sl, 1, 0, tw, 2);
-#pragma unroll
-    for (int s = 0; s < E; ++s) sl[prow<true>(final_row<M, E>(t, s))] = v[s];
-  }
-  __syncthreads();
-  // B + C. per product: the product of two input lines formed as the forward FFT loads
-  // it (the input slots stay intact), the FFT in the line's work slot, then the real
-  // sin/cos coefficients.  NIN + 1 slots per line instead of max(NIN, NOUT) keep more
-  // lines, and so more warps, per SM.
-  const int lw = l < nl ? l : 0;
-  for (int c = 0; c < NOUT; ++c) {
-    V* sl = slot(NIN, lw);
-    const V* sa = slot(z_pa(c, FORM), lw);
-    const V* sb = slot(z_pb(c, FORM), lw);
-    V v[E];
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-      const int r = prow<true>(load_row<M, E>(t, s));
-      v[s] = mk<V>(sa[r].x * sb[r].x, sa[r].y * sb[r].y);
-    }
-    __syncthreads();  // the previous product's coefficients have been read from the work slot
-    fft_regs<M, E, -1, 0, true>(v, t, sl, 1, 0, tw, 2);
-#pragma unroll
-    for (int s = 0; s < E; ++s) sl[prow<true>(final_row<M, E>(t, s))] = v[s];
-    __syncthreads();
-    const bool sine = (zout >> c) & 1;
-    V* dst = P + c * g.S + line0 * H;  // complex slot j holds reals 2j, 2j + 1
-    for (int e = threadIdx.x; e < nh * H; e += blockDim.x) {
-      const int ll = e / H, j = e % H;
-      const V* z = slot(NIN, ll);
-      T o[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int m = 2 * j + h;
-        o[h] = (T)0;
-        if (m < N) {
-          const int k = m <= M ? m : N - m;
-          const V Z = z[prow<true>(k == M ? 0 : k)];
-          const V Zp = conjg(z[prow<true>(k == 0 ? 0 : M - k)]);
-          V X = add(scale(add(Z, Zp), (T)0.5), mul_i<-1>(mul(tw[k], scale(sub(Z, Zp), (T)0.5))));
-          if (m > M) X = conjg(X);
-          const V w = mul(tq[m], X);
-          o[h] = sine ? (T)-2 * scl * w.y : (T)2 * scl * w.x;
-        }
-      }
-      dst[e] = mk<V>(o[0], o[1]);
     }
   }
 }
@@ -947,227 +992,400 @@ __global__ void __launch_bounds__(zreg_threads<FORM>(), zreg_min_blocks<NZ, EZ, 
     }
   }
   // real-space products; each complex register holds two real points
-  if constexpr (FORM == 5) {
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-      V col[6];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) col[c] = in[c][s];
-      z_elsasser<FORM>(col);
-#pragma unroll
-      for (int c = 0; c < 6; ++c) in[c][s] = col[c];
-    }
-  }
-  if (FORM == 1) {
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-      const V u1 = in[0][s], u2 = in[1][s], u3 = in[2][s], w1 = in[3][s], w2 = in[4][s], w3 = in[5][s];
-      in[0][s] = mk<V>(u2.x * w3.x - u3.x * w2.x, u2.y * w3.y - u3.y * w2.y);
-      in[1][s] = mk<V>(u3.x * w1.x - u1.x * w3.x, u3.y * w1.y - u1.y * w3.y);
-      in[2][s] = mk<V>(u1.x * w2.x - u2.x * w1.x, u1.y * w2.y - u2.y * w1.y);
-    }
-  }
 #pragma unroll
   for (int f = 0; f < NOUT; ++f) {
     V p[E];
 #pragma unroll
     for (int s = 0; s < E; ++s) {
-      if (FORM == 1) {
-        p[s] = in[f][s];
-      } else {
-        const int a = z_pa(f, FORM), b = z_pb(f, FORM);
-        p[s] = mk<V>(in[a][s].x * in[b][s].x, in[a][s].y * in[b][s].y);
-      }
+      V q[NIN];
+#pragma unroll
+      for (int c = 0; c < NIN; ++c) q[c] = in[c][s];
+      p[s] = z_product<FORM>(f, q);
     }
     zreg_forward_store<T, M, E, TPL>(p, P + f * g.S + (live ? line : 0) * H, live, t, partner, tw, xch);
   }
 }
 
 // ---------------------------------------------------------------------------
-// z pass of the adjoint right-hand side, register-resident (FP32 M <= 512, FP64 M <= 128).
-// Inputs per line: u (components 0-2), w (3-5), mu (6-8); outputs mu x u into
-// components 0-2 and w x mu into 3-5.  Staged so that at most six components
-// are live: mu and u are inverted, mu x u is transformed and stored over u,
-// then w is inverted into u's registers and w x mu is stored over w.
+// z pass, line-pair form: two neighbouring real lines a, b of a component ride in one
+// complex transform of the full length N = Nz (z_n = a_n + i b_n), so the real-transform
+// pre- and post-processing is additions only:
+//   inverse: Z_k = A_k + i B_k, Z_{N-k} = conj(A_k) + i conj(B_k)  (0 < k < M = N/2),
+//            Z_0 = Re A_0 + i Re B_0, Z_M = Re A_M + i Re B_M;
+//   forward: A_k = (Z_k + conj Z_{N-k}) / 2, B_k = -i (Z_k - conj Z_{N-k}) / 2.
+// A pair is held by TPL = N / E lanes, E elements each; the inverse (forward radix
+// schedule) leaves the points of every component in the order in which the forward
+// transform with the reversed schedule takes them, so the products (re and im: the points
+// of the two lines) are formed in registers.  All input components go through each
+// exchange together, the products in groups of NB.  A pair within a warp (TPL <= 32)
+// needs warp barriers only, and the mirrored rows N - k come from the partner lane by
+// shuffles (SH); otherwise they are read again (L1) and, on the way out, taken from the
+// exchange line.
 // ---------------------------------------------------------------------------
-template <typename T, int NZ>
-__global__ void __launch_bounds__(zreg_threads<3>(), sizeof(T) == 8 ? 3 : 6)
-    k_z_reg_adj(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw, int zkeep) {
+template <typename T, int NZ, int E> __host__ __device__ constexpr bool zpair_shfl() {
+  return radix_at(NZ, E, 0) == E && NZ / E <= 32 && E >= 2;
+}
+template <typename T> __host__ __device__ constexpr int zpair_slot(int NZ) { return NZ + NZ / 16 + 1; }
+
+// lines of exchange space per pair: the inputs go through it together, the products NB at a time
+__host__ __device__ constexpr int zpair_lines(int nin, int nb) { return nin > nb ? nin : nb; }
+
+// the two lines X, X + H of NC components (stride cs) as Z rows in registers, rows above zkeep
+// zero and not read; every load is issued before any of them is used
+template <typename T, int NZ, int E, int NC>
+__device__ __forceinline__ void zpair_load(const C<T>* X, long long cs, bool live0, bool live1, int t, int partner,
+                                           int zkeep, C<T> (&in)[NC][E]) {
   typedef C<T> V;
-  // 8 elements per thread in FP32, 4 in FP64 (six components live at once)
-  constexpr int M = NZ / 2, H = M + 1, E = sizeof(T) == 8 ? 4 : 8, TPL = M / E, LDX = zslot<M>();
-  static_assert(TPL >= 1 && TPL <= 64, "a line spans at most two warps");
-  constexpr int LPB = zreg_threads<3>() / TPL;
-  __shared__ __align__(16) V xch_all[LPB * LDX];
+  constexpr int M = NZ / 2, H = M + 1, TPL = NZ / E;
+  if constexpr (zpair_shfl<T, NZ, E>()) {
+    // slots s < E/2 hold rows t + s TPL < M, slot E/2 of lane 0 row M
+    V a[NC][E / 2], b[NC][E / 2], aM[NC], bM[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const V* x = X + c * cs;
+#pragma unroll
+      for (int s = 0; s < E / 2; ++s) {
+        const int k = t + s * TPL;
+        a[c][s] = (live0 && k <= zkeep) ? x[k] : mk<V>(0, 0);
+        b[c][s] = (live1 && k <= zkeep) ? x[H + k] : mk<V>(0, 0);
+      }
+      aM[c] = (live0 && t == 0 && M <= zkeep) ? x[M] : mk<V>(0, 0);
+      bM[c] = (live1 && t == 0 && M <= zkeep) ? x[H + M] : mk<V>(0, 0);
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      if (t == 0) a[c][0].y = b[c][0].y = 0;
+      V w[E / 2];
+#pragma unroll
+      for (int s = 0; s < E / 2; ++s) {
+        in[c][s] = mk<V>(a[c][s].x - b[c][s].y, a[c][s].y + b[c][s].x);
+        w[s] = mk<V>(a[c][s].x + b[c][s].y, b[c][s].x - a[c][s].y);  // conj(A) + i conj(B): row N - k
+      }
+      // slot s >= E/2 of lane t > 0 holds row N - (TPL - t) - (E-1-s) TPL; lane 0 holds row N - (E-s) TPL
+#pragma unroll
+      for (int s = E / 2; s < E; ++s) {
+        V z;
+        z.x = __shfl_sync(0xffffffffu, w[E - 1 - s].x, partner);
+        z.y = __shfl_sync(0xffffffffu, w[E - 1 - s].y, partner);
+        if (t == 0) z = s == E / 2 ? mk<V>(aM[c].x, bM[c].x) : w[(E - s) % (E / 2)];
+        in[c][s] = z;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const V* x = X + c * cs;
+#pragma unroll
+      for (int s = 0; s < E; ++s) {
+        const int r = load_row<NZ, E>(t, s), k = r <= M ? r : NZ - r;
+        V a = (live0 && k <= zkeep) ? x[k] : mk<V>(0, 0);
+        V b = (live1 && k <= zkeep) ? x[H + k] : mk<V>(0, 0);
+        if (k == 0 || k == M) a.y = b.y = 0;
+        if (r > M) a.y = -a.y, b.y = -b.y;
+        in[c][s] = mk<V>(a.x - b.y, a.y + b.x);
+      }
+    }
+  }
+}
+
+// forward transform of NB packed line pairs and the store of their rows 0 .. M
+template <typename T, int NZ, int E, int NB>
+__device__ __forceinline__ void zpair_forward_store(C<T> (&p)[NB][E], C<T>* X, long long cs, bool live0, bool live1,
+                                                    int t, int partner, const C<T>* __restrict__ tw, C<T>* xch) {
+  typedef C<T> V;
+  constexpr int M = NZ / 2, H = M + 1, TPL = NZ / E, LDX = zpair_slot<T>(NZ);
+  constexpr bool WARP = TPL <= 32;
+  fft_regs_b<NZ, E, -1, NB, WARP, 0, true, true>(p, t, xch, LDX, 1, 0, tw, 1);
+  if constexpr (zpair_shfl<T, NZ, E>()) {
+#pragma unroll
+    for (int f = 0; f < NB; ++f) {
+      V* Xo = X + f * cs;
+#pragma unroll
+      for (int s = 0; s < E / 2; ++s) {
+        V zp;
+        zp.x = __shfl_sync(0xffffffffu, p[f][E - 1 - s].x, partner);
+        zp.y = __shfl_sync(0xffffffffu, p[f][E - 1 - s].y, partner);
+        if (t == 0) zp = p[f][(E - s) % E];
+        const V z = p[f][s];
+        const int k = t + s * TPL;
+        if (live0) Xo[k] = mk<V>((T)0.5 * (z.x + zp.x), (T)0.5 * (z.y - zp.y));
+        if (live1) Xo[H + k] = mk<V>((T)0.5 * (z.y + zp.y), (T)0.5 * (zp.x - z.x));
+      }
+      if (t == 0) {
+        if (live0) Xo[M] = mk<V>(p[f][E / 2].x, (T)0);
+        if (live1) Xo[H + M] = mk<V>(p[f][E / 2].y, (T)0);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int f = 0; f < NB; ++f)
+#pragma unroll
+      for (int s = 0; s < E; ++s) xch[f * LDX + prow<true>(final_row<NZ, E, true>(t, s))] = p[f][s];
+    fft_sync<WARP>();
+#pragma unroll
+    for (int f = 0; f < NB; ++f) {
+      V* Xo = X + f * cs;
+      const V* zl = xch + f * LDX;
+      for (int k = t; k <= M; k += TPL) {
+        const V z = zl[prow<true>(k)], zp = zl[prow<true>((NZ - k) % NZ)];
+        if (live0) Xo[k] = mk<V>((T)0.5 * (z.x + zp.x), (T)0.5 * (z.y - zp.y));
+        if (live1) Xo[H + k] = mk<V>((T)0.5 * (z.y + zp.y), (T)0.5 * (zp.x - z.x));
+      }
+    }
+    fft_sync<WARP>();  // the exchange lines are used again by the next group
+  }
+}
+
+template <typename T, int NZ, int E, int FORM, int NTHR, int MINB, int NB>
+__global__ void __launch_bounds__(NTHR, MINB)
+    k_z_pair(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw, long long msP, int zkeep) {
+  typedef C<T> V;
+  constexpr int H = NZ / 2 + 1, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ);
+  constexpr int NIN = z_nin(FORM), NOUT = z_nout(FORM);
+  constexpr bool WARP = TPL <= 32;
+  static_assert(NOUT % NB == 0 && NTHR % TPL == 0 && (!WARP || 32 % TPL == 0), "whole pairs per warp or block");
+  extern __shared__ __align__(16) unsigned char smraw[];
+  P += blockIdx.y * msP;  // member blockIdx.y
+  const int l = threadIdx.x / TPL, t = threadIdx.x % TPL;
+  const int lane = threadIdx.x & 31;
+  const int partner = (lane - t) + (TPL - t) % TPL;  // lane holding the rows N - k
+  const long long nlines = (long long)g.Nx * g.Ny;
+  const long long line = 2 * ((long long)blockIdx.x * PPB + l);
+  const bool live0 = line < nlines, live1 = line + 1 < nlines;
+  V* xch = reinterpret_cast<V*>(smraw) + l * (zpair_lines(NIN, NB) * LDX);
+  V* Pl = P + (live0 ? line : 0) * H;
+
+  V in[NIN][E];
+  zpair_load<T, NZ, E, NIN>(Pl, g.S, live0, live1, t, partner, zkeep, in);
+  fft_regs_b<NZ, E, 1, NIN, WARP, 0, true, false>(in, t, xch, LDX, 1, 0, tw, 1);
+#pragma unroll
+  for (int f0 = 0; f0 < NOUT; f0 += NB) {
+    V p[NB][E];
+#pragma unroll
+    for (int s = 0; s < E; ++s)
+#pragma unroll
+      for (int f = 0; f < NB; ++f) {
+        V q[NIN];
+#pragma unroll
+        for (int c = 0; c < NIN; ++c) q[c] = in[c][s];
+        p[f][s] = z_product<FORM>(f0 + f, q);
+      }
+    zpair_forward_store<T, NZ, E, NB>(p, Pl + f0 * g.S, g.S, live0, live1, t, partner, tw, xch);
+  }
+}
+
+// line pairs, the points of the components in shared memory: component c is transformed
+// while the rows of component c + 1 are on their way, its points wait in slots that only
+// their own thread reads, and each product is formed from them as it is transformed.  One
+// component and one product are in registers at a time, so twice the warps of k_z_pair fit.
+template <typename T, int NZ, int E, int FORM, int NTHR, int MINB>
+__global__ void __launch_bounds__(NTHR, MINB)
+    k_z_pair_s(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw, long long msP, int zkeep) {
+  typedef C<T> V;
+  constexpr int H = NZ / 2 + 1, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ);
+  constexpr int NIN = z_nin(FORM), NOUT = z_nout(FORM);
+  constexpr bool WARP = TPL <= 32;
+  static_assert(NTHR % TPL == 0 && (!WARP || 32 % TPL == 0), "whole pairs per warp or block");
+  extern __shared__ __align__(16) unsigned char smraw[];
+  P += blockIdx.y * msP;  // member blockIdx.y
+  const int l = threadIdx.x / TPL, t = threadIdx.x % TPL;
+  const int lane = threadIdx.x & 31;
+  const int partner = (lane - t) + (TPL - t) % TPL;  // lane holding the rows N - k
+  const long long nlines = (long long)g.Nx * g.Ny;
+  const long long line = 2 * ((long long)blockIdx.x * PPB + l);
+  const bool live0 = line < nlines, live1 = line + 1 < nlines;
+  V* xch = reinterpret_cast<V*>(smraw) + l * LDX;
+  V* pts = reinterpret_cast<V*>(smraw) + PPB * LDX + threadIdx.x;  // point s of component c at (c E + s) NTHR
+  V* Pl = P + (live0 ? line : 0) * H;
+  V in[1][E], nx[1][E];
+  zpair_load<T, NZ, E, 1>(Pl, g.S, live0, live1, t, partner, zkeep, in);
+#pragma unroll
+  for (int c = 0; c < NIN; ++c) {
+    if (c + 1 < NIN) zpair_load<T, NZ, E, 1>(Pl + (c + 1) * g.S, g.S, live0, live1, t, partner, zkeep, nx);
+    fft_regs_b<NZ, E, 1, 1, WARP, 0, true, false>(in, t, xch, LDX, 1, 0, tw, 1);
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      pts[(c * E + s) * NTHR] = in[0][s];
+      in[0][s] = nx[0][s];
+    }
+  }
+  if constexpr (!WARP) __syncthreads();  // outputs overwrite rows that other threads of the pair have read
+#pragma unroll
+  for (int f = 0; f < NOUT; ++f) {
+    V p[1][E];
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      V q[NIN];
+#pragma unroll
+      for (int c = 0; c < NIN; ++c) q[c] = pts[(c * E + s) * NTHR];
+      p[0][s] = z_product<FORM>(f, q);
+    }
+    zpair_forward_store<T, NZ, E, 1>(p, Pl + f * g.S, g.S, live0, live1, t, partner, tw, xch);
+  }
+}
+
+// z pass of the adjoint right-hand side on line pairs: inputs u (components 0-2), w (3-5),
+// mu (6-8); mu x u into components 0-2 and w x mu into 3-5.  The points of mu wait in shared
+// memory (each thread reads back only its own), so one vector and one product are in
+// registers at a time.
+template <typename T, int NZ, int E, int NTHR, int MINB>
+__global__ void __launch_bounds__(NTHR, MINB)
+    k_z_pair_adj(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw, int zkeep) {
+  typedef C<T> V;
+  constexpr int M = NZ / 2, H = M + 1, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ);
+  constexpr bool WARP = TPL <= 32;
+  extern __shared__ __align__(16) unsigned char smraw[];
   const int l = threadIdx.x / TPL, t = threadIdx.x % TPL;
   const int lane = threadIdx.x & 31;
   const int partner = (lane - t) + (TPL - t) % TPL;
   const long long nlines = (long long)g.Nx * g.Ny;
-  const long long line = (long long)blockIdx.x * LPB + l;
-  const bool live = line < nlines;
-  const long long lo = (live ? line : 0) * H;
-  V* xch = xch_all + l * LDX;
-
-  V mu[3][E], w[3][E];
+  const long long line = 2 * ((long long)blockIdx.x * PPB + l);
+  const bool live0 = line < nlines, live1 = line + 1 < nlines;
+  V* xch = reinterpret_cast<V*>(smraw) + l * (3 * LDX);
+  V* mus = reinterpret_cast<V*>(smraw) + PPB * (3 * LDX) + threadIdx.x;  // slot (f, s) at (f E + s) NTHR
+  V* Pl = P + (live0 ? line : 0) * H;
+  V in[3][E];
+  zpair_load<T, NZ, E, 3>(Pl + 6 * g.S, g.S, live0, live1, t, partner, M, in);
+  fft_regs_b<NZ, E, 1, 3, WARP, 0, true, false>(in, t, xch, LDX, 1, 0, tw, 1);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) zreg_inverse<T, M, E, TPL>(P + (6 + c) * g.S + lo, live, t, partner, tw, xch, mu[c]);
+  for (int f = 0; f < 3; ++f)
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    V XM;
-    zreg_load<T, M, E, TPL>(P + c * g.S + lo, live, t, w[c], XM, zkeep);
-    zreg_inverse_loaded<T, M, E, TPL>(P + c * g.S + lo, live, t, partner, tw, xch, w[c], XM, zkeep);
-  }
+    for (int s = 0; s < E; ++s) mus[(f * E + s) * NTHR] = in[f][s];
 #pragma unroll
-  for (int f = 0; f < 3; ++f) {
-    V p[E];
+  for (int h = 0; h < 2; ++h) {
+    zpair_load<T, NZ, E, 3>(Pl + 3 * h * g.S, g.S, live0, live1, t, partner, zkeep, in);
+    fft_regs_b<NZ, E, 1, 3, WARP, 0, true, false>(in, t, xch, LDX, 1, 0, tw, 1);
 #pragma unroll
-    for (int s = 0; s < E; ++s) {
-      const V a[3] = {mu[0][s], mu[1][s], mu[2][s]}, b[3] = {w[0][s], w[1][s], w[2][s]};
-      p[s] = cross_pk(f, a, b);
+    for (int f = 0; f < 3; ++f) {
+      V p[1][E];
+#pragma unroll
+      for (int s = 0; s < E; ++s) {
+        const int i = f == 2 ? 0 : f + 1, j = f == 0 ? 2 : f - 1;
+        const V a = h == 0 ? mus[(i * E + s) * NTHR] : in[i][s], b = h == 0 ? in[j][s] : mus[(j * E + s) * NTHR];
+        const V c = h == 0 ? mus[(j * E + s) * NTHR] : in[j][s], d = h == 0 ? in[i][s] : mus[(i * E + s) * NTHR];
+        p[0][s] = mk<V>(a.x * b.x - c.x * d.x, a.y * b.y - c.y * d.y);
+      }
+      zpair_forward_store<T, NZ, E, 1>(p, Pl + (3 * h + f) * g.S, g.S, live0, live1, t, partner, tw, xch);
     }
-    zreg_forward_store<T, M, E, TPL>(p, P + f * g.S + lo, live, t, partner, tw, xch);
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    V XM;
-    zreg_load<T, M, E, TPL>(P + (3 + c) * g.S + lo, live, t, w[c], XM, zkeep);
-    zreg_inverse_loaded<T, M, E, TPL>(P + (3 + c) * g.S + lo, live, t, partner, tw, xch, w[c], XM, zkeep);
-  }
-#pragma unroll
-  for (int f = 0; f < 3; ++f) {
-    V p[E];
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-      const V a[3] = {w[0][s], w[1][s], w[2][s]}, b[3] = {mu[0][s], mu[1][s], mu[2][s]};
-      p[s] = cross_pk(f, a, b);
-    }
-    zreg_forward_store<T, M, E, TPL>(p, P + (3 + f) * g.S + lo, live, t, partner, tw, xch);
   }
 }
 
 // ---------------------------------------------------------------------------
-// z pass, bulk-copy variant: persistent over groups of LPB consecutive (x,y)
-// lines.  A group's input lines are contiguous per component (LPB*H complex,
-// 16-byte aligned), so thread 0 fetches each component with one 1-D
-// cp.async.bulk into shared memory, double buffered across groups.  Each line
-// is transformed by TPL = M/E lanes in registers (pair terms X[M-k] read from
-// shared memory on the way in, exchanged by warp shuffles on the way out); the
-// products are formed in registers and fed to the forward FFTs with the
-// reversed radix schedule.  Shared memory: 2 x NIN x LPB x H input + LPB
-// exchange lines.
+// SSS z pass, line-pair form: two neighbouring real lines a, b of a component as one
+// complex line p = a + i b.  The sin/cos transform of complex data is the algorithm of the
+// x / y passes (one complex FFT of the full length N with the quarter-step twiddles
+// w_m = e^{-i pi m / 2N}):
+//   inverse: V_m = conj(w_m) (p_m - i p_{N-m}) (cosine, V_0 = p_0), conj(w_m) (p_{N-m} - i p_m)
+//            (sine, V_0 = 0); inverse FFT, points left in the reordered order v;
+//   forward: Z = FFT(v); p_m = scl (w_m Z_m + conj(w_m) Z_{N-m}) (cosine),
+//            i scl (w_m Z_m - conj(w_m) Z_{N-m}) (sine).
+// Lines, registers, exchanges, mirrored rows and products as in k_z_pair; the product of two
+// reordered lines is the reordered product with the product's own sign pattern (sine x sine =
+// cosine, sine x cosine = sine, and the sign flips multiply), so the forward transform takes
+// it as it is.  zin / zout: bit c set = input / output c is a sine series along z;
+// scl = 1 / (2N).
 // ---------------------------------------------------------------------------
-template <typename T> __host__ __device__ constexpr int ztma_e() { return sizeof(T) == 4 ? 8 : 4; }
-template <typename T, int NZ> __host__ __device__ constexpr int ztma_lpb() { return 256 / ((NZ / 2) / ztma_e<T>()); }
-
-template <typename T, int NZ, int FORM>
-__global__ void __launch_bounds__(256, 1) k_z_tma(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw,
-                                                  int* err, long long msP, int zkeep) {
+template <typename T, int NZ, int E, int FORM, int NTHR, int MINB, int NB>
+__global__ void __launch_bounds__(NTHR, MINB)
+    k_sss_z_pair(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw, const C<T>* __restrict__ tq, int zin,
+                 int zout, T scl) {
   typedef C<T> V;
-  constexpr int M = NZ / 2, H = M + 1, E = ztma_e<T>(), TPL = M / E, LDX = zslot<M>();
-  constexpr int LPB = ztma_lpb<T, NZ>();
-  static_assert(TPL >= 1 && TPL <= 32, "line group must fit in a warp");
+  constexpr int H = NZ / 2 + 1, LD = NZ + 2, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ);
   constexpr int NIN = z_nin(FORM), NOUT = z_nout(FORM);
-  constexpr int GRP = LPB * H;  // complex per component per group
-  extern __shared__ __align__(128) unsigned char smraw_[];
-  unsigned char* smraw = smraw_ + ((128 - (smem_u32(smraw_) & 127)) & 127);
-  V* inb = reinterpret_cast<V*>(smraw);  // [2][NIN][GRP]
-  V* xch_all = inb + 2 * NIN * GRP;      // [LPB][LDX]
-  __shared__ __align__(8) uint64_t bar[2];
+  constexpr bool WARP = TPL <= 32, SH = zpair_shfl<T, NZ, E>();
+  static_assert(FORM == 7 || FORM == 2 || FORM == 6, "conservative products, with or without T, or the flux giver's");
+  static_assert(NOUT % NB == 0 && NTHR % TPL == 0, "whole pairs per block");
+  extern __shared__ __align__(16) unsigned char smraw[];
   const int l = threadIdx.x / TPL, t = threadIdx.x % TPL;
   const int lane = threadIdx.x & 31;
-  const int partner = (lane - t) + (TPL - t) % TPL;  // lane holding row M - k
-  const long long ngroups = (long long)g.Nx * g.Ny / LPB;
-  V* xch = xch_all + l * LDX;
-  P += blockIdx.y * msP;  // member blockIdx.y
-  if (threadIdx.x == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    fence_mbar_init();
+  const int partner = (lane - t) + (TPL - t) % TPL;  // lane holding the rows N - m (SH)
+  const long long nlines = (long long)g.Nx * g.Ny;
+  const long long line = 2 * ((long long)blockIdx.x * PPB + l);
+  const bool live0 = line < nlines, live1 = line + 1 < nlines;
+  V* xch = reinterpret_cast<V*>(smraw) + l * (zpair_lines(NIN, NB) * LDX);
+  T* Pl = reinterpret_cast<T*>(P + (live0 ? line : 0) * H);  // line a; line b follows at Pl + LD
+
+  V in[NIN][E];
+#pragma unroll
+  for (int c = 0; c < NIN; ++c) {
+    const T* X = Pl + 2 * c * g.S;
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int m = load_row<NZ, E>(t, s);
+      in[c][s] = mk<V>(live0 ? X[m] : (T)0, live1 ? X[LD + m] : (T)0);
+    }
   }
-  __syncthreads();
-  auto issue = [&](long long grp, int slot) {
-    if (grp >= ngroups) return;
-    mbar_expect_tx(&bar[slot], (unsigned)(NIN * GRP * sizeof(V)));
-    for (int c = 0; c < NIN; ++c)
-      bulk_load(inb + (slot * NIN + c) * GRP, P + c * g.S + grp * GRP, (unsigned)(GRP * sizeof(V)), &bar[slot]);
-  };
-  if (threadIdx.x == 0) {
-    issue(blockIdx.x, 0);
-    issue(blockIdx.x + gridDim.x, 1);
+#pragma unroll
+  for (int c = 0; c < NIN; ++c) {
+    const bool sine = (zin >> c) & 1;
+    V q[E];  // p_{N-m}
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      if constexpr (SH) {
+        q[s].x = __shfl_sync(0xffffffffu, in[c][E - 1 - s].x, partner);
+        q[s].y = __shfl_sync(0xffffffffu, in[c][E - 1 - s].y, partner);
+        if (t == 0) q[s] = in[c][(E - s) % E];
+      } else {
+        const T* X = Pl + 2 * c * g.S;
+        const int m = load_row<NZ, E>(t, s);
+        q[s] = m == 0 ? mk<V>(0, 0) : mk<V>(live0 ? X[NZ - m] : (T)0, live1 ? X[LD + NZ - m] : (T)0);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int m = load_row<NZ, E>(t, s);
+      const V p = in[c][s];
+      if (m == 0) in[c][s] = sine ? mk<V>(0, 0) : p;
+      else in[c][s] = mul(conjg(tq[m]), sine ? add_i<-1>(q[s], p) : add_i<-1>(p, q[s]));
+    }
   }
-  int k = 0;
-  for (long long grp = blockIdx.x; grp < ngroups; grp += gridDim.x, ++k) {
-    // slots alternate, so slot k & 1 completes its phase (k >> 1) & 1
-    const int slot = k & 1;
-    const uint32_t phase = (uint32_t)(k >> 1) & 1u;
-    const bool got = mbar_wait(&bar[slot], phase, err);
-    if (__syncthreads_or(!got)) {
-      // drain this group's copies and the next group's (other slot), each wait bounded
-      if (threadIdx.x == 0) {
-        mbar_wait(&bar[slot], phase, nullptr);
-        if (grp + (long long)gridDim.x < ngroups) mbar_wait(&bar[slot ^ 1], (uint32_t)((k + 1) >> 1) & 1u, nullptr);
-      }
-      return;
-    }
-    V in[NIN][E];
+  fft_regs_b<NZ, E, 1, NIN, WARP, 0, true, false>(in, t, xch, LDX, 1, 0, tw, 1);
 #pragma unroll
-    for (int c = 0; c < NIN; ++c) {
-      const V* X = inb + (slot * NIN + c) * GRP + l * H;
+  for (int f0 = 0; f0 < NOUT; f0 += NB) {
+    V p[NB][E];
+#pragma unroll
+    for (int s = 0; s < E; ++s)
+#pragma unroll
+      for (int f = 0; f < NB; ++f) {
+        V q[NIN];
+#pragma unroll
+        for (int c = 0; c < NIN; ++c) q[c] = in[c][s];
+        p[f][s] = z_product<FORM>(f0 + f, q);
+      }
+    fft_regs_b<NZ, E, -1, NB, WARP, 0, true, true>(p, t, xch, LDX, 1, 0, tw, 1);
+    if constexpr (!SH) {
+#pragma unroll
+      for (int f = 0; f < NB; ++f)
+#pragma unroll
+        for (int s = 0; s < E; ++s) xch[f * LDX + prow<true>(final_row<NZ, E, true>(t, s))] = p[f][s];
+      fft_sync<WARP>();
+    }
+#pragma unroll
+    for (int f = 0; f < NB; ++f) {
+      const bool sine = (zout >> (f0 + f)) & 1;
+      T* Xo = Pl + 2 * (f0 + f) * g.S;
 #pragma unroll
       for (int s = 0; s < E; ++s) {
-        // Z[k] = (X + Y) + i conj(w^k)(X - Y), Y = conj(X[M-k]); imag of X[0], X[M] dropped
-        const int kk = t + s * TPL;
-        V x = kk <= zkeep ? X[kk] : mk<V>(0, 0), b = M - kk <= zkeep ? conjg(X[M - kk]) : mk<V>(0, 0);
-        if (kk == 0) { x.y = 0; b.y = 0; }
-        in[c][s] = add(add(x, b), mul_i<1>(mul(conjg(tw[kk]), sub(x, b))));
-      }
-    }
-    // every thread has read this slot: refill it with the group after next
-    __syncthreads();
-    if (threadIdx.x == 0) issue(grp + 2 * (long long)gridDim.x, slot);
-#pragma unroll
-    for (int c = 0; c < NIN; ++c) fft_regs<M, E, 1, 0, true, false>(in[c], t, xch, 1, 0, tw, 2);
-    if (FORM == 1) {
-#pragma unroll
-      for (int s = 0; s < E; ++s) {
-        const V u1 = in[0][s], u2 = in[1][s], u3 = in[2][s], w1 = in[3][s], w2 = in[4][s], w3 = in[5][s];
-        in[0][s] = mk<V>(u2.x * w3.x - u3.x * w2.x, u2.y * w3.y - u3.y * w2.y);
-        in[1][s] = mk<V>(u3.x * w1.x - u1.x * w3.x, u3.y * w1.y - u1.y * w3.y);
-        in[2][s] = mk<V>(u1.x * w2.x - u2.x * w1.x, u1.y * w2.y - u2.y * w1.y);
-      }
-    }
-    const long long line = grp * LPB + l;
-#pragma unroll
-    for (int f = 0; f < NOUT; ++f) {
-      V p[E];
-#pragma unroll
-      for (int s = 0; s < E; ++s) {
-        if (FORM == 1) {
-          p[s] = in[f][s];
+        const int m = final_row<NZ, E, true>(t, s);
+        V zr;
+        if constexpr (SH) {
+          zr.x = __shfl_sync(0xffffffffu, p[f][E - 1 - s].x, partner);
+          zr.y = __shfl_sync(0xffffffffu, p[f][E - 1 - s].y, partner);
+          if (t == 0) zr = p[f][(E - s) % E];
         } else {
-          const int a = z_pa(f), b = z_pb(f);
-          p[s] = mk<V>(in[a][s].x * in[b][s].x, in[a][s].y * in[b][s].y);
+          zr = xch[f * LDX + prow<true>((NZ - m) % NZ)];
         }
+        const V w = tq[m], wz = mul(w, p[f][s]), wzr = mul(conjg(w), zr);
+        const V o = sine ? mul_i<1>(scale(sub(wz, wzr), scl)) : scale(add(wz, wzr), scl);
+        if (live0) Xo[m] = o.x;
+        if (live1) Xo[LD + m] = o.y;
       }
-      fft_regs<M, E, -1, 0, true, true>(p, t, xch, 1, 0, tw, 2);
-      // X[k] = 1/2 (Z + Z') - i/2 w^k (Z - Z'), Z' = conj(Z[M-k]), Z[M] = Z[0]; rows k = t + s*TPL
-      V* Xo = P + f * g.S + line * H;
-#pragma unroll
-      for (int s = 0; s < E; ++s) {
-        V zp;
-        zp.x = __shfl_sync(0xffffffffu, p[E - 1 - s].x, partner);
-        zp.y = __shfl_sync(0xffffffffu, p[E - 1 - s].y, partner);
-        if (t == 0) zp = p[(E - s) % E];
-        zp = conjg(zp);
-        const int kk = t + s * TPL;
-        const V z = p[s];
-        Xo[kk] = add(scale(add(z, zp), (T)0.5), mul_i<-1>(mul(tw[kk], scale(sub(z, zp), (T)0.5))));
-      }
-      if (t == 0) {
-        const V z = p[0], zp = conjg(p[0]);
-        Xo[M] = add(scale(add(z, zp), (T)0.5), mul_i<-1>(mul(tw[M], scale(sub(z, zp), (T)0.5))));
+      if (t < 2) {  // the two padding reals
+        if (live0) Xo[NZ + t] = (T)0;
+        if (live1) Xo[LD + NZ + t] = (T)0;
       }
     }
+    if constexpr (!SH) fft_sync<WARP>();  // the exchange lines are used again by the next group
   }
 }
 
@@ -1205,6 +1423,7 @@ constexpr int FLUX_MAX_BINS = 64;
 // Assembly of the stage's spectral vector from forward-transformed product f
 // (p already scaled by 1/(Nx Ny Nz)):
 //   FORM 0: N_i = sum_j i K_j F[u_i u_j]  (compute_diag_offdiag.cc:47-98)
+//   FORM 7: the same from d1, d2, u1u2, u2u3, u3u1 (N up to a gradient, for a step)
 //   FORM 1: N = -F[u x omega]
 //   FORM 3: A_i + (i K x B)_i  (adjoint; B = products 0-2, A = products 3-5)
 template <int FORM, typename V, typename S>
@@ -1216,6 +1435,14 @@ __device__ __forceinline__ void accum_product(int f, V p, S Kx, S Ky, S Kz, V& a
       case 2: a2 = add(a2, ik(Kz, p)); break;
       case 3: a0 = add(a0, ik(Ky, p)); a1 = add(a1, ik(Kx, p)); break;
       case 4: a1 = add(a1, ik(Kz, p)); a2 = add(a2, ik(Ky, p)); break;
+      default: a2 = add(a2, ik(Kx, p)); a0 = add(a0, ik(Kz, p)); break;
+    }
+  } else if (FORM == 7) {
+    switch (f) {
+      case 0: a0 = add(a0, ik(Kx, p)); break;
+      case 1: a1 = add(a1, ik(Ky, p)); break;
+      case 2: a0 = add(a0, ik(Ky, p)); a1 = add(a1, ik(Kx, p)); break;
+      case 3: a1 = add(a1, ik(Kz, p)); a2 = add(a2, ik(Ky, p)); break;
       default: a2 = add(a2, ik(Kx, p)); a0 = add(a0, ik(Kz, p)); break;
     }
   } else if (FORM == 3) {
@@ -1392,7 +1619,7 @@ __global__ void __launch_bounds__(CW * (L / E), 1)
     k_fwd_x(const __grid_constant__ CUtensorMap mP, const __grid_constant__ CUtensorMap mA,
             const __grid_constant__ CUtensorMap mB, Geo g, StageArgs a, const C<T>* __restrict__ tw) {
   typedef C<T> V;
-  constexpr int NF = FORM == 1 ? 3 : 6;
+  constexpr int NF = z_nout(FORM);
   constexpr int TILE = L * CW, BR = L < 256 ? L : 256, UNITS = (int)sizeof(V) / 8;
   constexpr int NST = MODE == MODE_NLIN ? 0 : 6;
   extern __shared__ __align__(128) unsigned char smraw_[];
@@ -1540,7 +1767,7 @@ __global__ void __launch_bounds__(CW * (L / E), 1)
 template <typename T, int FORM, int MODE>
 __global__ void __launch_bounds__(256) k_spec_epi(const C<T>* __restrict__ P, Geo g, StageArgs a) {
   typedef C<T> V;
-  constexpr int NF = FORM == 1 ? 3 : 6;
+  constexpr int NF = z_nout(FORM);
   double tb[MODE == MODE_FLUX ? FLUX_MAX_BINS : 1];  // MODE_FLUX: per-thread sphere partials
   if (MODE == MODE_FLUX)
     for (int i = 0; i <= a.nradii; ++i) tb[i] = 0.0;
@@ -1552,13 +1779,14 @@ __global__ void __launch_bounds__(256) k_spec_epi(const C<T>* __restrict__ P, Ge
   const bool ld1 = (MODE == MODE_STEP && a.stage > 1) || (MODE == MODE_ADJ && a.stage != 4);
   // two elements per thread and iteration (e and e + stride): every load of both is
   // issued before either is used, twice the loads in flight of one element at a time
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long e0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; e0 < g.S; e0 += 2 * stride) {
-    const bool has1 = e0 + stride < g.S;
+  // 32-bit index arithmetic (a component holds < 2^31 modes)
+  const unsigned n = (unsigned)g.S, stride = gridDim.x * blockDim.x;
+  for (unsigned e0 = blockIdx.x * blockDim.x + threadIdx.x; e0 < n; e0 += 2 * stride) {
+    const bool has1 = e0 + stride < n;
     V pv[2][NF], s0[2][3], s1[2][3];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const long long e = e0 + j * stride;
+      const unsigned e = e0 + j * stride;
       if (j == 0 || has1) {
 #pragma unroll
         for (int f = 0; f < NF; ++f) pv[j][f] = P[f * g.S + e];
@@ -1571,11 +1799,10 @@ __global__ void __launch_bounds__(256) k_spec_epi(const C<T>* __restrict__ P, Ge
     }
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const long long e = e0 + j * stride;
+      const unsigned e = e0 + j * stride;
       if (j == 1 && !has1) break;
-      const int lz = (int)(e % g.Hz);
-      const long long r = e / g.Hz;
-      const int ly = (int)(r % g.Ny), lx = (int)(r / g.Ny);
+      const unsigned r = e / (unsigned)g.Hz;
+      const int lz = (int)(e - r * g.Hz), lx = (int)(r / (unsigned)g.Ny), ly = (int)(r - (unsigned)lx * g.Ny);
       const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]), Ky = (T)(kfft(ly, g.Ny) * g.kf[1]), Kz = (T)(lz * g.kf[2]);
       V a0 = mk<V>(0, 0), a1 = mk<V>(0, 0), a2 = mk<V>(0, 0);
 #pragma unroll
@@ -1600,62 +1827,64 @@ namespace ts {
 // DIR=-1: real padded (Nx,Ny,Nz+2) -> spectral lines (Nx,Ny,Hz), unnormalised
 // DIR=+1: spectral lines -> real padded, unnormalised; pads written as 0
 // ---------------------------------------------------------------------------
-template <typename T, int NZ, int E, int DIR>
-__global__ void k_z_single(const C<T>* __restrict__ in, C<T>* __restrict__ out, Geo g, const C<T>* __restrict__ tw,
-                           int nl, int ncomp) {
+// Line pairs as in k_z_pair (two real lines a, b of component blockIdx.y as a + i b), one
+// transform of length N = Nz per pair, 16 elements per thread; the real points go through
+// the pair's exchange line so that their stores are contiguous.
+template <typename T, int NZ, int E, int DIR, int NTHR, int MINB>
+__global__ void __launch_bounds__(NTHR, MINB)
+    k_z_single(const C<T>* __restrict__ in, C<T>* __restrict__ out, Geo g, const C<T>* __restrict__ tw) {
   typedef C<T> V;
-  constexpr int M = NZ / 2, H = M + 1;
+  constexpr int M = NZ / 2, H = M + 1, LD = NZ + 2, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ);
+  constexpr bool WARP = TPL <= 32;
+  static_assert(NTHR % TPL == 0, "whole pairs per block");
   extern __shared__ __align__(16) unsigned char smraw[];
-  V* bufA = reinterpret_cast<V*>(smraw);
-  V* bufB = bufA + nl * H;
+  const int l = threadIdx.x / TPL, t = threadIdx.x % TPL;
   const long long nlines = (long long)g.Nx * g.Ny;
-  const long long line0 = (long long)blockIdx.x * nl;
-  const int nh = (int)((nlines - line0) < nl ? (nlines - line0) : nl);
-  const int comp = blockIdx.y;
-  // real line stride = Nz+2 reals = H complex: both layouts have H complex per line
-  const V* src = in + comp * g.S + line0 * H;
-  V* dst = out + comp * g.S + line0 * H;
-  for (int e = threadIdx.x; e < nh * H; e += blockDim.x) bufA[e] = src[e];
-  __syncthreads();
-  if (DIR > 0) {
-    for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
-      const int l = e / M, k = e % M;
-      if (l >= nh) continue;
-      const V* x = bufA + l * H;
-      V X = x[k], Y = conjg(x[M - k]);
-      if (k == 0) { X.y = 0; Y.y = 0; }
-      bufB[l * H + k] = add(add(X, Y), mul_i<1>(mul(conjg(tw[k]), sub(X, Y))));
+  const long long line = 2 * ((long long)blockIdx.x * PPB + l);
+  const bool live0 = line < nlines, live1 = line + 1 < nlines;
+  V* xch = reinterpret_cast<V*>(smraw) + l * LDX;
+  // both layouts have H complex (N + 2 reals) per line
+  const long long lo = blockIdx.y * g.S + (live0 ? line : 0) * H;
+  V v[1][E];
+  if constexpr (DIR > 0) {
+    const V* X = in + lo;
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int r = load_row<NZ, E>(t, s), k = r <= M ? r : NZ - r;
+      V a = live0 ? X[k] : mk<V>(0, 0), b = live1 ? X[H + k] : mk<V>(0, 0);
+      if (k == 0 || k == M) a.y = b.y = 0;
+      if (r > M) a.y = -a.y, b.y = -b.y;
+      v[0][s] = mk<V>(a.x - b.y, a.y + b.x);
     }
-    __syncthreads();
-    V* r = fft_smem_lines<M, E, 1>(bufB, bufA, nl, H, tw, 2);
-    for (int e = threadIdx.x; e < nh * H; e += blockDim.x) {
-      const int l = e / H, k = e % H;
-      dst[e] = k < M ? r[l * H + k] : mk<V>(0, 0);
+    fft_regs_b<NZ, E, 1, 1, WARP, 0, true, false>(v, t, xch, LDX, 1, 0, tw, 1);
+#pragma unroll
+    for (int s = 0; s < E; ++s) xch[prow<true>(final_row<NZ, E>(t, s))] = v[0][s];
+    fft_sync<WARP>();
+    // points 2 i, 2 i + 1 as one store; the pad is slot M
+    V* o = out + lo;
+    for (int i = t; i <= M; i += TPL) {
+      const V p = i < M ? xch[prow<true>(2 * i)] : mk<V>(0, 0), q = i < M ? xch[prow<true>(2 * i + 1)] : mk<V>(0, 0);
+      if (live0) o[i] = mk<V>(p.x, q.x);
+      if (live1) o[H + i] = mk<V>(p.y, q.y);
     }
   } else {
-    // padded real line: reals 0..NZ-1 = complex 0..M-1 of the line, pad = complex M
-    V* r = fft_smem_lines<M, E, -1>(bufA, bufB, nl, H, tw, 2);
-    V* o2 = (r == bufA) ? bufB : bufA;
-    for (int e = threadIdx.x; e < nl * H; e += blockDim.x) {
-      const int l = e / H, k = e % H;
-      if (l >= nh) continue;
-      const V* z = r + l * H;
-      const V Z = z[k == M ? 0 : k];
-      const V Zp = conjg(z[k == 0 ? 0 : M - k]);
-      const V s = scale(add(Z, Zp), (T)0.5);
-      const V d = mul_i<-1>(mul(tw[k], scale(sub(Z, Zp), (T)0.5)));
-      o2[e] = add(s, d);
+    const T* X = reinterpret_cast<const T*>(in + lo);
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int n = load_row<NZ, E>(t, s);
+      v[0][s] = mk<V>(live0 ? X[n] : (T)0, live1 ? X[LD + n] : (T)0);
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < nh * H; e += blockDim.x) dst[e] = o2[e];
+    fft_regs_b<NZ, E, -1, 1, WARP, 0, true, false>(v, t, xch, LDX, 1, 0, tw, 1);
+#pragma unroll
+    for (int s = 0; s < E; ++s) xch[prow<true>(final_row<NZ, E>(t, s))] = v[0][s];
+    fft_sync<WARP>();
+    V* o = out + lo;
+    for (int k = t; k <= M; k += TPL) {
+      const V z = xch[prow<true>(k)], zp = xch[prow<true>((NZ - k) % NZ)];
+      if (live0) o[k] = mk<V>((T)0.5 * (z.x + zp.x), (T)0.5 * (z.y - zp.y));
+      if (live1) o[H + k] = mk<V>((T)0.5 * (z.y + zp.y), (T)0.5 * (zp.x - z.x));
+    }
   }
 }
 
-template <typename T>
-__global__ void k_scale_range(C<T>* A, long long n, double s) {
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    C<T> a = A[e];
-    A[e] = mk<C<T>>((T)(a.x * s), (T)(a.y * s));
-  }
-}
 }  // namespace ts

@@ -1,5 +1,12 @@
-// Launcher definitions, included once per precision by ts_kern_f32.cu and
-// ts_kern_f64.cu with TS_REAL defined to float / double.
+// Launcher definitions, included by the ts_kern_<part>_<precision>.cu files with TS_REAL
+// defined to float / double and TS_PART to the group of launchers that the file
+// instantiates (one file per group and precision, so that they compile in parallel).
+#define TS_PART_STR 1   // strided-axis FFTs
+#define TS_PART_IX 2    // FFF inverse x pass
+#define TS_PART_Z 3     // z passes
+#define TS_PART_FX 4    // FFF forward x pass and epilogue
+#define TS_PART_SFF 5   // sin/cos x passes
+#define TS_PART_MISC 6  // elementwise, plane-sized and reduction kernels, tuning queries
 #include <type_traits>
 #include "ts_launch.h"
 #include "ts_misc.cuh"
@@ -83,15 +90,6 @@ inline unsigned grid1d(long long n, int threads) {
   return (unsigned)b;
 }
 
-// lines per block of the z kernels: about 96 KB of shared memory (two blocks per SM)
-inline int z_lines(int nbuf, int H) {
-  const long long per = 2LL * nbuf * H * (long long)sizeof(V);
-  long long nl = (96 * 1024) / per;
-  if (nl < 1) nl = 1;
-  if (nl > 16) nl = 16;
-  return (int)nl;
-}
-
 }  // namespace
 
 // strided passes at L = 1024 in FP32: 16 elements per thread and 8-column tiles
@@ -102,6 +100,40 @@ constexpr bool wide1024(int L) { return std::is_same<T, float>::value && L == 10
 constexpr int str_e(int L) { return wide1024(L) ? 16 : e_mixed(L, e_reg(L)); }
 constexpr int str_cw(int L) { return wide1024(L) ? 8 : cw_for(L, str_e(L)); }
 constexpr int str_nt(int L) { return wide1024(L) ? 2 : 3; }
+
+// sin/cos x kernel: elements per thread, tile columns, blocks per SM it is compiled for
+struct LdTile { int E, CW, MINB; };
+constexpr LdTile sc_tile(int L, int dir) {
+  return std::is_same<T, float>::value
+             ? (L == 16 ? LdTile{4, 16, 8} : L == 32 ? LdTile{8, 16, 16} : L == 64 ? LdTile{8, 16, 8}
+                : L == 128 ? LdTile{16, 16, dir > 0 ? 4 : 6} : L == 256 ? LdTile{16, 16, dir > 0 ? 2 : 4}
+                : L == 512 ? LdTile{16, 16, 1} : L == 96 ? LdTile{24, 16, 8} : LdTile{12, 16, 8})
+             : (L == 16 ? LdTile{4, 8, 16} : L == 32 ? LdTile{8, 8, 16} : L == 64 ? LdTile{8, 8, 8}
+                : L == 128 ? LdTile{16, 8, 4} : L == 256 ? LdTile{16, 8, 2} : L == 512 ? LdTile{16, 8, 1}
+                : LdTile{12, 8, 4});
+}
+
+// direct-load strided kernel: elements per thread, tile columns and blocks per SM the
+// kernel is compiled for
+constexpr LdTile ld_tile(int L) {
+  return std::is_same<T, float>::value
+             ? (L == 16 ? LdTile{4, 16, 8} : L == 32 ? LdTile{8, 16, 16} : L == 64 ? LdTile{8, 16, 8}
+                : L == 128 ? LdTile{16, 16, 6} : L == 256 ? LdTile{16, 16, 4} : L == 512 ? LdTile{32, 16, 2}
+                : L == 1024 ? LdTile{32, 8, 2} : L == 96 ? LdTile{24, 32, 4} : LdTile{12, 16, 8})
+             : (L == 16 ? LdTile{4, 8, 16} : L == 32 ? LdTile{8, 8, 16} : L == 64 ? LdTile{8, 8, 6}
+                : L == 128 ? LdTile{16, 8, 4} : L == 256 ? LdTile{16, 8, 2} : L == 512 ? LdTile{16, 8, 2}
+                : L == 1024 ? LdTile{16, 4, 2} : LdTile{12, 8, 4});
+}
+// inverse x kernel (one field per block)
+constexpr LdTile ix_tile(int L) {
+  return std::is_same<T, float>::value
+             ? (L == 16 ? LdTile{4, 16, 8} : L == 32 ? LdTile{8, 16, 16} : L == 64 ? LdTile{8, 16, 8}
+                : L == 128 ? LdTile{16, 16, 6} : L == 256 ? LdTile{16, 16, 3} : L == 512 ? LdTile{32, 16, 2}
+                : LdTile{32, 8, 2})
+             : (L == 16 ? LdTile{4, 8, 16} : L == 32 ? LdTile{8, 8, 16} : L == 64 ? LdTile{8, 8, 6}
+                : L == 128 ? LdTile{16, 8, 4} : L == 256 ? LdTile{16, 8, 2} : L == 512 ? LdTile{16, 8, 2}
+                : LdTile{16, 4, 2});
+}
 
 // ---------------------------------------------------------------------------
 // Launch-tuning candidates.  Candidate 0 of every pass class is the fixed rule;
@@ -137,73 +169,6 @@ constexpr bool str_valid(int L, int v) {
                     (v < 5 || !tile_eq(str_cand(L, v), str_cand(L, 4))));
 }
 
-template <int L, int VV, typename Fn> void with_str_tile(Fn&& fn) {
-  if constexpr (str_valid(L, VV)) fn(std::integral_constant<int, VV>{});
-  else fn(std::integral_constant<int, 0>{});
-}
-
-template <> cudaError_t Launch<T>::strided(const Geo& g, int axis, int dir, void* data, int nf, const void* tw,
-                                           cudaStream_t st, int per, long long mstride, int inner_eff,
-                                           int zero_hi) {
-  if (per <= 0) per = nf;
-  cudaError_t err = cudaErrorInvalidValue;
-  const int L = axis == 0 ? g.Nx : g.Ny;
-  if (L == 1) return cudaSuccess;  // a one-point transform is the identity (two-dimensional runs)
-  // the y passes follow the tuning of their class; x passes keep the rule
-  const int cls = axis == 1 ? (dir > 0 ? TUNE_Y_INV : TUNE_Y_FWD) : -1;
-  const int v = cls >= 0 ? g.tv[cls] : 0, bps = cls >= 0 ? g.tb[cls] : 0;
-  dispatch_L_sff(L, [&](auto Lc) {
-    constexpr int LL = decltype(Lc)::value;
-    auto run = [&](auto vc) {
-      constexpr Tile c = str_cand(LL, decltype(vc)::value);
-      constexpr int E = c.E, CW = c.CW, NT = c.NT;
-      const int inner = inner_eff > 0 ? inner_eff : (axis == 0 ? g.Ny * g.Hz : g.Hz);
-      const long long rstride = axis == 0 ? (long long)g.Ny * g.Hz : g.Hz;
-      const long long ostride = axis == 0 ? 0 : (long long)g.Ny * g.Hz;
-      const int nouter = axis == 0 ? 1 : g.Nx;
-      const long long nwork = (long long)nf * ((inner + CW - 1) / CW) * nouter;
-      const size_t sm = (size_t)str_tiles(NT) * LL * CW * sizeof(V);
-      // persistent grid: as many blocks as fit on the 148 SMs at once (or the tuned count)
-      const int cap = (CW * (LL / E)) <= 256 ? 2 : 1;
-      const int fit = (int)((227 * 1024) / sm);
-      const int per_sm = bps > 0 ? bps : (fit < cap ? fit : cap);
-      long long blocks = 148LL * (per_sm > 0 ? per_sm : 1);
-      if (blocks > nwork) blocks = nwork;
-      auto launch = [&](auto k) {
-        if ((err = smem_attr(k, sm)) != cudaSuccess) return;
-        k<<<(unsigned)blocks, CW * (LL / E), sm, st>>>((V*)data, nf, g.S, inner, rstride, ostride, nouter,
-                                                      (const V*)tw, per, mstride, zero_hi);
-        ++g_launches;
-        err = cudaGetLastError();
-      };
-      if (dir < 0) launch(k_strided_fft<T, LL, E, CW, -1, NT>);
-      else launch(k_strided_fft<T, LL, E, CW, 1, NT>);
-    };
-    // the y passes of 1024 points in FP32: the one-tile, 32-element form on 16-column
-    // tiles (tile 6) is the rule (on B200 at 1024^3: y inverse 9.9 ms against 10.4 for the
-    // two-tile, 16-element form on 8 columns; y forward 7.5 against 7.6 for 32 elements on
-    // 8 columns and 8.9 for the 16-element form); for the y forward pass candidate 5 is
-    // then the 16-element form
-    int vv = (wide1024(LL) && axis == 1) ? (v == 0 ? 6 : ((dir < 0 && v == 5) ? 0 : v)) : v;
-    // the x forward pass of 1024 points in FP32 (the split form's FFT): 16-column tiles,
-    // 128-byte row segments, 32 elements per thread, one staging tile (tile 6, not a tuning
-    // candidate).  An x row is Ny*Hz complex long (4.2 MB at 1024^3), so every row of a
-    // tile is a separate memory page; twice the bytes per row visit took the forward x
-    // FFT + epilogue from 20.4 to 17.0 ms per right-hand side at 1024^3 on B200
-    if (wide1024(LL) && axis == 0 && dir < 0) vv = 6;
-    switch (vv) {
-      case 6: with_str_tile<LL, 6>(run); break;
-      case 1: with_str_tile<LL, 1>(run); break;
-      case 2: with_str_tile<LL, 2>(run); break;
-      case 3: with_str_tile<LL, 3>(run); break;
-      case 4: with_str_tile<LL, 4>(run); break;
-      case 5: with_str_tile<LL, 5>(run); break;
-      default: run(std::integral_constant<int, 0>{});
-    }
-  });
-  return err;
-}
-
 // inverse x pass (FFF forms 0, 1): 8 elements per thread in FP32 (U held in
 // registers across the output fields; 16 at L = 1024 with per-field loads)
 constexpr int ix_e(int L) { return wide1024(L) ? 16 : (std::is_same<T, float>::value ? (8 < L ? 8 : L) : e_reg(L)); }
@@ -234,25 +199,187 @@ constexpr bool ix_valid(int L, int v) {
                     (v < 5 || !tile_eq(ix_cand(L, v), ix_cand(L, 4))));
 }
 
+// z candidates (forms 1, 2, 7): 1 = the slot kernel with 8 elements per thread
+// (12 with a factor 3), 2 = the slot kernel with 4 (power-of-two lines), 3 = the
+// FP32 register kernel with 4 elements per thread (lines of up to 256 points),
+// 4 = on 1024-point lines in FP32, the register kernel that loads each component just
+// before its transform (the rule there issues every load up front)
+template <int NZ, int FORM> constexpr bool z_rule_slots() {
+  constexpr int M = NZ / 2;
+  return !(std::is_same<T, float>::value && M <= 512) &&
+         !(!std::is_same<T, float>::value && M % 3 != 0 && M <= 128);
+}
+// line-pair kernel: elements per thread, threads per block and blocks per SM the kernel is
+// compiled for
+struct ZTile { int E, NTHR, MINB, NB; };
+constexpr ZTile zp_tile(int NZ, int form) {
+  const bool f32 = std::is_same<T, float>::value;
+  const int E = NZ % 3 == 0 ? 12 : 8;
+  const int tpl = NZ / E, thr = tpl > 64 ? tpl : 64;
+  return ZTile{E, thr, ((f32 && NZ % 3 != 0) || form == 3 ? 6 : 4) * 64 / thr, 1};
+}
+// FP32 lines of 48, 96 and 1024 points: single lines in registers (k_z_reg) are the rule
+template <int NZ, int FORM> constexpr bool zreg_rule() {
+  return std::is_same<T, float>::value && FORM != 3 && (NZ % 3 == 0 || NZ == 1024);
+}
+template <int NZ, int FORM> constexpr bool z_valid(int v) {
+  constexpr int M = NZ / 2;
+  return v == 0 || ((FORM == 1 || FORM == 2 || FORM == 7) && ((v == 1 && !z_rule_slots<NZ, FORM>()) ||
+                                  (v == 2 && M % 3 != 0 && M >= 8 && M / 4 <= 256) ||
+                                  (v == 3 && std::is_same<T, float>::value && M % 3 != 0 && M >= 8 && M / 4 <= 64) ||
+                                  (v == 4 && std::is_same<T, float>::value && M == 512)));
+}
+
+// forward x candidates (MODE_STEP): 1 = the split form (strided x FFT, then the
+// elementwise epilogue) where the rule is the fused TMA kernel; 2 = the fused
+// kernel with half-width column tiles (32-byte rows in FP32; where the rule
+// splits, the fused kernel at the rule's tile width); 3 = the fused kernel with
+// 8 elements per thread (half the threads)
+constexpr bool fx_rule_fused(int L) { return xcw(L) * sizeof(V) >= 64; }
+constexpr int fx_cw2(int L) { return fx_rule_fused(L) ? xcw(L) / 2 : xcw(L); }
+constexpr bool fx_valid(int L, int v) {
+  return v == 0 || (v == 1 && fx_rule_fused(L)) || (v == 2 && fx_cw2(L) * sizeof(V) >= 16 && fx_cw2(L) * (L / emin(E_ACC, L)) >= 32) ||
+         (v == 3 && fx_rule_fused(L) && emin(E_ACC_ALT, L) != emin(E_ACC, L));
+}
+
+
+// SFF x candidates. Inverse: 1 = 4 elements per thread (power-of-two lengths),
+// 2 = half-width column tiles. Forward: 1 = the other split choice (fused
+// epilogue from 64 points on, split below), 2 = half-width column tiles.
+constexpr int sx_e(int N, int dir) { return e_mixed(N, dir > 0 ? 8 : (std::is_same<T, float>::value ? 8 : 4)); }
+constexpr Tile sx_cand(int N, int dir, int v) {
+  return v == 0 ? Tile{sx_e(N, dir), cw_for(N, sx_e(N, dir)), 1}
+       : v == 1 ? (dir > 0 ? (N % 3 != 0 && sx_e(N, dir) > 4 ? Tile{4, cw_for(N, 4), 1} : Tile{0, 0, 0})
+                           : Tile{sx_e(N, dir), cw_for(N, sx_e(N, dir)), 2})
+       : v == 2 ? (cw_for(N, sx_e(N, dir)) > 1 ? Tile{sx_e(N, dir), cw_for(N, sx_e(N, dir)) / 2, 1} : Tile{0, 0, 0})
+                : Tile{0, 0, 0};
+}
+constexpr bool sx_valid(int N, int dir, int v) {
+  return v == 0 || (N <= 512 && v < 3 && tile_fits(N, sx_cand(N, dir, v), 3) &&
+                    !tile_eq(sx_cand(N, dir, v), sx_cand(N, dir, 0)));
+}
+
+#if TS_PART == TS_PART_STR
+template <int L, int VV, typename Fn> void with_str_tile(Fn&& fn) {
+  if constexpr (str_valid(L, VV)) fn(std::integral_constant<int, VV>{});
+  else fn(std::integral_constant<int, 0>{});
+}
+
+template <> cudaError_t Launch<T>::strided(const Geo& g, int axis, int dir, void* data, int nf, const void* tw,
+                                           cudaStream_t st, int per, long long mstride, int inner_eff,
+                                           int zero_hi, void* dst, double scl) {
+  if (per <= 0) per = nf;
+  cudaError_t err = cudaErrorInvalidValue;
+  const int L = axis == 0 ? g.Nx : g.Ny;
+  if (L == 1) return cudaSuccess;  // a one-point transform is the identity (two-dimensional runs)
+  // the y passes follow the tuning of their class; x passes keep the rule
+  const int cls = axis == 1 ? (dir > 0 ? TUNE_Y_INV : TUNE_Y_FWD) : -1;
+  const int v = cls >= 0 ? g.tv[cls] : 0, bps = cls >= 0 ? g.tb[cls] : 0;
+  // the rule is the direct-load kernel; a tuning candidate or a blocks-per-SM count of a y
+  // class launches the persistent kernel (in place, unscaled)
+  if (v == 0 && bps == 0) {
+    dispatch_L_sff(L, [&](auto Lc) {
+      constexpr int LL = decltype(Lc)::value;
+      constexpr LdTile c = ld_tile(LL);
+      const unsigned inner = inner_eff > 0 ? inner_eff : (axis == 0 ? g.Ny * g.Hz : g.Hz);
+      const long long rstride = axis == 0 ? (long long)g.Ny * g.Hz : g.Hz;
+      const unsigned nplane = axis == 0 ? inner : inner * (unsigned)g.Nx, ntot = nplane * (unsigned)nf;
+      constexpr size_t sm = (size_t)LL * c.CW * sizeof(V);
+      auto launch = [&](auto k) {
+        if ((err = smem_attr(k, sm)) != cudaSuccess) return;
+        k<<<(ntot + c.CW - 1) / c.CW, c.CW * (LL / c.E), sm, st>>>(
+            (const V*)data, (V*)(dst ? dst : data), ntot, nplane, inner, g.S, rstride, (long long)g.Ny * g.Hz,
+            (const V*)tw, (unsigned)per, mstride, zero_hi, (T)scl);
+        ++g_launches;
+        err = cudaGetLastError();
+      };
+      if (dir > 0) launch(k_strided_ld<T, LL, c.E, c.CW, 1, c.MINB, false>);
+      else if (scl == 1.0) launch(k_strided_ld<T, LL, c.E, c.CW, -1, c.MINB, false>);
+      else launch(k_strided_ld<T, LL, c.E, c.CW, -1, c.MINB, true>);
+    });
+    return err;
+  }
+  if ((dst && dst != data) || scl != 1.0) return err;
+  dispatch_L_sff(L, [&](auto Lc) {
+    constexpr int LL = decltype(Lc)::value;
+    auto run = [&](auto vc) {
+      constexpr Tile c = str_cand(LL, decltype(vc)::value);
+      constexpr int E = c.E, CW = c.CW, NT = c.NT;
+      const int inner = inner_eff > 0 ? inner_eff : (axis == 0 ? g.Ny * g.Hz : g.Hz);
+      const long long rstride = axis == 0 ? (long long)g.Ny * g.Hz : g.Hz;
+      const long long ostride = axis == 0 ? 0 : (long long)g.Ny * g.Hz;
+      const int nouter = axis == 0 ? 1 : g.Nx;
+      const long long nwork = (long long)nf * ((inner + CW - 1) / CW) * nouter;
+      const size_t sm = (size_t)str_tiles(NT) * LL * CW * sizeof(V);
+      // persistent grid: as many blocks as fit on the 148 SMs at once (or the tuned count)
+      const int cap = (CW * (LL / E)) <= 256 ? 2 : 1;
+      const int fit = (int)((227 * 1024) / sm);
+      const int per_sm = bps > 0 ? bps : (fit < cap ? fit : cap);
+      long long blocks = 148LL * (per_sm > 0 ? per_sm : 1);
+      if (blocks > nwork) blocks = nwork;
+      auto launch = [&](auto k) {
+        if ((err = smem_attr(k, sm)) != cudaSuccess) return;
+        k<<<(unsigned)blocks, CW * (LL / E), sm, st>>>((V*)data, nf, g.S, inner, rstride, ostride, nouter,
+                                                      (const V*)tw, per, mstride, zero_hi);
+        ++g_launches;
+        err = cudaGetLastError();
+      };
+      if (dir < 0) launch(k_strided_fft<T, LL, E, CW, -1, NT>);
+      else launch(k_strided_fft<T, LL, E, CW, 1, NT>);
+    };
+    // 1024 points in FP32: for the y forward pass candidate 5 is the two-tile, 16-element form
+    const int vv = wide1024(LL) && v == 0 ? 6 : (wide1024(LL) && dir < 0 && v == 5 ? 0 : v);
+    switch (vv) {
+      case 6: with_str_tile<LL, 6>(run); break;
+      case 1: with_str_tile<LL, 1>(run); break;
+      case 2: with_str_tile<LL, 2>(run); break;
+      case 3: with_str_tile<LL, 3>(run); break;
+      case 4: with_str_tile<LL, 4>(run); break;
+      case 5: with_str_tile<LL, 5>(run); break;
+      default: run(std::integral_constant<int, 0>{});
+    }
+  });
+  return err;
+}
+#endif  // TS_PART_STR
+
+#if TS_PART == TS_PART_IX
 template <> cudaError_t Launch<T>::inv_x(const Geo& g, int form, const void* U, void* W, const void* tw,
                                          const void* lam, double lsc, cudaStream_t st, int kept, double rad) {
   cudaError_t err_ = cudaErrorInvalidValue;
   // forms 0 and 1 follow the tuning; the adjoint forms keep the rule
   const int v = form <= 1 ? g.tv[TUNE_X_INV] : 0;
+  if (v == 0) {
+    dispatch_L(g.Nx, [&](auto Lc) {
+      constexpr int LL = decltype(Lc)::value;
+      constexpr LdTile c = ix_tile(LL);
+      const long long cols = kept ? (long long)(2 * (g.Ny / 3) + 1) * (g.Nz / 3 + 1) : (long long)g.Ny * g.Hz;
+      constexpr size_t sm = (size_t)LL * c.CW * sizeof(V);
+      auto run = [&](auto kern, int nf) {
+        if ((err_ = smem_attr(kern, sm)) != cudaSuccess) return;
+        kern<<<(unsigned)((cols + c.CW - 1) / c.CW) * nf, c.CW * (LL / c.E), sm, st>>>(
+            (const V*)U, (V*)W, g, (const V*)tw, (const V*)lam, (T)lsc, kept, rad);
+        ++g_launches;
+        err_ = cudaGetLastError();
+      };
+      if (form == 0) run(k_inv_x_f<T, LL, c.E, c.CW, 0, c.MINB>, 3);
+      else if (form == 1) run(k_inv_x_f<T, LL, c.E, c.CW, 1, c.MINB>, 6);
+      else if (form == 4) run(k_inv_x_f<T, LL, c.E, c.CW, 4, c.MINB>, 3);
+      else if (form == 5) run(k_inv_x_f<T, LL, c.E, c.CW, 5, c.MINB>, 6);
+    });
+    return err_;
+  }
   dispatch_L(g.Nx, [&](auto Lc) {
     constexpr int LL = decltype(Lc)::value;
-    // 1024 points in FP32 under two-thirds dealiasing: the staged kernel k_inv_x_st is the
-    // rule (on B200 7.0 against 10.1 ms per launch at 1024^3) and candidate 5 is then the
-    // direct-load kernel
-    const int vv = (ix_valid(LL, 5) && kept && form <= 1) ? (v == 0 ? 5 : (v == 5 ? 0 : v)) : v;
+    // 1024 points in FP32 under two-thirds dealiasing: candidate 5 is the direct-load kernel
+    const int vv = (ix_valid(LL, 5) && kept && v == 5) ? 0 : v;
     if constexpr (ix_valid(LL, 5)) {
       if (vv == 5 && kept) {
         // the kept U rows of a tile staged in shared memory (one load latency per tile)
         constexpr Tile c = ix_cand(LL, 5);
         constexpr int E = c.E, CW = c.CW;
         const size_t sm = ((size_t)LL + 3 * ix_kept_rows<LL>()) * CW * sizeof(V);
-        const int nzk = g.Nz / 3 + 1;
-        const unsigned blocks = (unsigned)((2 * (g.Ny / 3) + 1) * ((nzk + CW - 1) / CW));
+        const unsigned blocks = (unsigned)(((2 * (g.Ny / 3) + 1) * (g.Nz / 3 + 1) + CW - 1) / CW);
         auto run = [&](auto kern) {
           if ((err_ = smem_attr(kern, sm)) != cudaSuccess) return;
           kern<<<blocks, CW * (LL / E), sm, st>>>((const V*)U, (V*)W, g, (const V*)tw);
@@ -303,11 +430,6 @@ template <> cudaError_t Launch<T>::inv_x(const Geo& g, int form, const void* U, 
       };
       if (form == 0) run(k_inv_x_ld<T, LL, E, CW, 0>);
       else if (form == 1) run(k_inv_x_ld<T, LL, E, CW, 1>);
-      else if constexpr (decltype(vc)::value == 0) {
-        if (form == 3) run(k_inv_x_ld<T, LL, E, CW, 3>);
-        else if (form == 4) run(k_inv_x_ld<T, LL, E, CW, 4>);
-        else if (form == 5) run(k_inv_x_ld<T, LL, E, CW, 5>);
-      }
     };
     if (vv == 1 && ix_valid(LL, 1)) {
       if constexpr (ix_valid(LL, 1)) tile(std::integral_constant<int, 1>{});
@@ -321,7 +443,9 @@ template <> cudaError_t Launch<T>::inv_x(const Geo& g, int form, const void* U, 
   });
   return err_;
 }
+#endif  // TS_PART_IX
 
+#if TS_PART == TS_PART_Z
 // shared-memory slot variant of the z pass: E elements per thread, nl lines per
 // block within about 106 KB of shared memory
 template <int NZ, int FORM, int E>
@@ -343,30 +467,11 @@ static cudaError_t z_slots(const Geo& g, void* P, const void* tw, cudaStream_t s
   return cudaGetLastError();
 }
 
-// z candidates (forms 0, 1, 2): 1 = the slot kernel with 8 elements per thread
-// (12 with a factor 3), 2 = the slot kernel with 4 (power-of-two lines), 3 = the
-// FP32 register kernel with 4 elements per thread (lines of up to 256 points),
-// 4 = on 1024-point lines in FP32, the register kernel that loads each component just
-// before its transform (the rule there issues every load up front)
-template <int NZ, int FORM> constexpr bool z_rule_slots() {
-  constexpr int M = NZ / 2;
-  return !(std::is_same<T, float>::value && M <= 512) &&
-         !(!std::is_same<T, float>::value && FORM <= 2 && M % 3 != 0 && M / ztma_e<T>() <= 32);
-}
-template <int NZ, int FORM> constexpr bool z_valid(int v) {
-  constexpr int M = NZ / 2;
-  return v == 0 || (FORM <= 2 && ((v == 1 && !z_rule_slots<NZ, FORM>()) ||
-                                  (v == 2 && M % 3 != 0 && M >= 8 && M / 4 <= 256) ||
-                                  (v == 3 && std::is_same<T, float>::value && M % 3 != 0 && M >= 8 && M / 4 <= 64) ||
-                                  (v == 4 && std::is_same<T, float>::value && M == 512)));
-}
-
 template <int NZ, int FORM>
 static cudaError_t z_fused_impl(const Geo& g, void* P, const void* tw, int* zerr, cudaStream_t st, int nmem,
                                 long long msP, int zkeep, int v) {
   constexpr int M = NZ / 2;
   if (zkeep < 0) zkeep = M;
-  constexpr int NIN = z_nin(FORM);
   const long long nlines = (long long)g.Nx * g.Ny;
   cudaError_t err;
   if constexpr (z_valid<NZ, FORM>(1)) {
@@ -376,17 +481,20 @@ static cudaError_t z_fused_impl(const Geo& g, void* P, const void* tw, int* zerr
     if (v == 2) return z_slots<NZ, FORM, 4>(g, P, tw, st, nmem, msP, zkeep);
   }
   if constexpr (z_valid<NZ, FORM>(4)) {
-    // 1024-point z lines in FP32: the register kernel with every component's loads issued
-    // up front is the rule (on B200 13.0 against 15.8 ms per launch at 1024^3); candidate 4
-    // loads each component just before its transform
-    constexpr int NT = zreg_threads<FORM>(), LPB = NT / (M / 8);
-    const dim3 grid((unsigned)((nlines + LPB - 1) / LPB), nmem);
-    if (v == 4) k_z_reg<T, NZ, FORM, 0, false><<<grid, NT, 0, st>>>((V*)P, g, (const V*)tw, msP, zkeep);
-    else if (v == 0) k_z_reg<T, NZ, FORM, 0, true><<<grid, NT, 0, st>>>((V*)P, g, (const V*)tw, msP, zkeep);
-    if (v == 4 || v == 0) {
+    if (v == 4) {
+      constexpr int NT = zreg_threads<FORM>(), LPB = NT / (M / 8);
+      k_z_reg<T, NZ, FORM, 0, false><<<dim3((unsigned)((nlines + LPB - 1) / LPB), nmem), NT, 0, st>>>(
+          (V*)P, g, (const V*)tw, msP, zkeep);
       ++g_launches;
       return cudaGetLastError();
     }
+  }
+  if constexpr (zreg_rule<NZ, FORM>()) {
+    constexpr int E = M % 3 == 0 ? 12 : 8, NT = zreg_threads<FORM>(), LPB = NT / (M / E);
+    k_z_reg<T, NZ, FORM, 0, true><<<dim3((unsigned)((nlines + LPB - 1) / LPB), nmem), NT, 0, st>>>(
+        (V*)P, g, (const V*)tw, msP, zkeep);
+    ++g_launches;
+    return cudaGetLastError();
   }
   if constexpr (z_valid<NZ, FORM>(3)) {
     if (v == 3) {
@@ -397,41 +505,29 @@ static cudaError_t z_fused_impl(const Geo& g, void* P, const void* tw, int* zerr
       return cudaGetLastError();
     }
   }
-  if constexpr (FORM <= 2 && M % 3 != 0 && M / ztma_e<T>() <= 32 && !std::is_same<T, float>::value) {
-    // FP64: bulk-copy variant (whole groups, 16-byte aligned group starts)
-    constexpr int LPB = ztma_lpb<T, NZ>();
-    const size_t sm = 2ull * NIN * LPB * (M + 1) * sizeof(V) + (size_t)LPB * zslot<M>() * sizeof(V) + 128;
-    if (nlines % LPB == 0 && (LPB * (M + 1) * sizeof(V)) % 16 == 0 && sm <= 220 * 1024) {
-      const long long ngroups = nlines / LPB;
-      auto k = k_z_tma<T, NZ, FORM>;
-      if ((err = smem_attr(k, sm)) != cudaSuccess) return err;
-      k<<<dim3((unsigned)(ngroups < 148 ? ngroups : 148), nmem), 256, sm, st>>>((V*)P, g, (const V*)tw, zerr, msP,
-                                                                                 zkeep);
-      ++g_launches;
-      return cudaGetLastError();
-    }
-  }
-  if constexpr (FORM == 3 && !std::is_same<T, float>::value && M % 3 != 0 && M / 4 <= 32) {
-    // FP64 adjoint: register-resident with 4 elements per thread
-    constexpr int NT = zreg_threads<3>(), LPB = NT / (M / 4);
-    k_z_reg_adj<T, NZ><<<(unsigned)((nlines + LPB - 1) / LPB), NT, 0, st>>>((V*)P, g, (const V*)tw, zkeep);
+  if constexpr (FORM != 3) {
+    // the rule: line pairs
+    constexpr ZTile c = zp_tile(NZ, FORM);
+    constexpr int PPB = c.NTHR / (NZ / c.E);
+    constexpr size_t sm = (size_t)PPB * zpair_lines(z_nin(FORM), c.NB) * zpair_slot<T>(NZ) * sizeof(V);
+    const long long npairs = (nlines + 1) / 2;
+    auto k = k_z_pair<T, NZ, c.E, FORM, c.NTHR, c.MINB, c.NB>;
+    if ((err = smem_attr(k, sm)) != cudaSuccess) return err;
+    k<<<dim3((unsigned)((npairs + PPB - 1) / PPB), nmem), c.NTHR, sm, st>>>((V*)P, g, (const V*)tw, msP, zkeep);
     ++g_launches;
     return cudaGetLastError();
   }
-  if constexpr (M <= 512 && (M % 3 != 0 || FORM != 3) && std::is_same<T, float>::value) {
-    // FP32: register-resident variant, lines of M/E lanes (E = 8, or 12 with a factor 3;
-    // up to two warps per line)
-    constexpr int NT = zreg_threads<FORM>(), LPB = NT / (M / ((M % 3 == 0) ? 12 : 8));
-    if constexpr (FORM == 3)
-      k_z_reg_adj<T, NZ><<<(unsigned)((nlines + LPB - 1) / LPB), NT, 0, st>>>((V*)P, g, (const V*)tw, zkeep);
-    else
-      k_z_reg<T, NZ, FORM><<<dim3((unsigned)((nlines + LPB - 1) / LPB), nmem), NT, 0, st>>>((V*)P, g, (const V*)tw,
-                                                                                           msP, zkeep);
+  if constexpr (FORM == 3) {
+    constexpr ZTile c = zp_tile(NZ, FORM);
+    constexpr int PPB = c.NTHR / (NZ / c.E);
+    constexpr size_t sm = ((size_t)PPB * 3 * zpair_slot<T>(NZ) + 3ull * c.E * c.NTHR) * sizeof(V);
+    const long long npairs = (nlines + 1) / 2;
+    auto k = k_z_pair_adj<T, NZ, c.E, c.NTHR, c.MINB>;
+    if ((err = smem_attr(k, sm)) != cudaSuccess) return err;
+    k<<<(unsigned)((npairs + PPB - 1) / PPB), c.NTHR, sm, st>>>((V*)P, g, (const V*)tw, zkeep);
     ++g_launches;
     return cudaGetLastError();
   }
-  // shared-memory slot variant (large lines, and line lengths with a factor 3)
-  return z_slots<NZ, FORM, e_mixed(M, 8)>(g, P, tw, st, nmem, msP, zkeep);
 }
 
 template <> cudaError_t Launch<T>::z_fused(const Geo& g, int form, void* P, const void* tw, int* zerr,
@@ -441,7 +537,8 @@ template <> cudaError_t Launch<T>::z_fused(const Geo& g, int form, void* P, cons
   dispatch_L_sff(g.Nz, [&](auto Lc) {
     constexpr int NZ = decltype(Lc)::value;
     const int v = g.tv[TUNE_Z];
-    if (form == 0) err = z_fused_impl<NZ, 0>(g, P, tw, zerr, st, nmem, msP, zkeep, v);
+    if (form == 7) err = z_fused_impl<NZ, 7>(g, P, tw, zerr, st, nmem, msP, zkeep, v);
+    else if (form == 0) err = z_fused_impl<NZ, 0>(g, P, tw, zerr, st, nmem, msP, zkeep, 0);
     else if (form == 1) err = z_fused_impl<NZ, 1>(g, P, tw, zerr, st, nmem, msP, zkeep, v);
     else if (form == 2) err = z_fused_impl<NZ, 2>(g, P, tw, zerr, st, nmem, msP, zkeep, v);
     else if (form == 5) err = z_fused_impl<NZ, 5>(g, P, tw, zerr, st, nmem, msP, zkeep, 0);
@@ -451,26 +548,18 @@ template <> cudaError_t Launch<T>::z_fused(const Geo& g, int form, void* P, cons
   return err;
 }
 
-// SSS fused z pass (form 0 or 2): the slot layout of the FFF slot kernel with NIN
-// input slots and one work slot per line, lines per block within about 106 KB of
-// shared memory
+// SSS z pass (forms 0, 2, 6): line pairs, tiles as the Fourier z pass
 template <int NZ, int FORM>
-static cudaError_t sss_z_slots(const Geo& g, void* P, const void* tw, const void* tq, int zin, int zout,
+static cudaError_t sss_z_pairs(const Geo& g, void* P, const void* tw, const void* tq, int zin, int zout,
                                cudaStream_t st) {
-  constexpr int M = NZ / 2;
-  // 4 elements per thread: twice the threads per z line of the 8-element form, and half
-  // the shared memory per block, so more warps per SM for this latency-bound pass
-  constexpr int E = (M % 3 != 0 && M >= 8) ? 4 : e_mixed(M, 8);
-  constexpr int TPL = M / E;
-  constexpr int NSL = z_nin(FORM) + 1;
-  const long long nlines = (long long)g.Nx * g.Ny;
-  int nl = 256 / TPL;
-  while (nl > 1 && (size_t)NSL * nl * zslot<M>() * sizeof(V) > 106 * 1024) nl /= 2;
-  const size_t sm = (size_t)NSL * nl * zslot<M>() * sizeof(V);
+  constexpr ZTile c = zp_tile(NZ, FORM);
+  constexpr int PPB = c.NTHR / (NZ / c.E);
+  constexpr size_t sm = (size_t)PPB * zpair_lines(z_nin(FORM), c.NB) * zpair_slot<T>(NZ) * sizeof(V);
+  const long long npairs = ((long long)g.Nx * g.Ny + 1) / 2;
   cudaError_t err;
-  auto k = k_sss_z_fused<T, NZ, E, FORM>;
+  auto k = k_sss_z_pair<T, NZ, c.E, FORM, c.NTHR, c.MINB, c.NB>;
   if ((err = smem_attr(k, sm)) != cudaSuccess) return err;
-  k<<<(unsigned)((nlines + nl - 1) / nl), nl * TPL, sm, st>>>((V*)P, g, (const V*)tw, (const V*)tq, nl, zin, zout,
+  k<<<(unsigned)((npairs + PPB - 1) / PPB), c.NTHR, sm, st>>>((V*)P, g, (const V*)tw, (const V*)tq, zin, zout,
                                                               (T)(1.0 / (2.0 * NZ)));
   ++g_launches;
   return cudaGetLastError();
@@ -479,12 +568,12 @@ static cudaError_t sss_z_slots(const Geo& g, void* P, const void* tw, const void
 template <> cudaError_t Launch<T>::sss_z_fused(const Geo& g, int form, void* P, const void* tw, const void* tq, int zin,
                                                int zout, cudaStream_t st) {
   cudaError_t err = cudaErrorInvalidValue;
-  if (form != 0 && form != 2 && form != 6) return err;
+  if (form != 7 && form != 2 && form != 6) return err;
   dispatch_L(g.Nz, [&](auto Lc) {
     constexpr int NZ = decltype(Lc)::value;
-    err = form == 0 ? sss_z_slots<NZ, 0>(g, P, tw, tq, zin, zout, st)
-        : form == 2 ? sss_z_slots<NZ, 2>(g, P, tw, tq, zin, zout, st)
-                    : sss_z_slots<NZ, 6>(g, P, tw, tq, zin, zout, st);
+    err = form == 7 ? sss_z_pairs<NZ, 7>(g, P, tw, tq, zin, zout, st)
+        : form == 2 ? sss_z_pairs<NZ, 2>(g, P, tw, tq, zin, zout, st)
+                    : sss_z_pairs<NZ, 6>(g, P, tw, tq, zin, zout, st);
   });
   return err;
 }
@@ -494,42 +583,27 @@ template <> cudaError_t Launch<T>::z_single(const Geo& g, int dir, const void* i
   cudaError_t err = cudaErrorInvalidValue;
   dispatch_L(g.Nz, [&](auto Lc) {
     constexpr int NZ = decltype(Lc)::value;
-    constexpr int M = NZ / 2, H = M + 1;
-    constexpr int E = emin(E_REG, M);
-    const int nl = z_lines(1, H);
-    const size_t sm = 2ull * nl * H * sizeof(V);
-    const long long nlines = (long long)g.Nx * g.Ny;
-    dim3 grid((unsigned)((nlines + nl - 1) / nl), ncomp);
-    if (dir < 0) {
-      auto k = k_z_single<T, NZ, E, -1>;
+    constexpr int E = emin(16, NZ / 2), TPL = NZ / E, NT = TPL > 128 ? TPL : 128, PPB = NT / TPL;
+    constexpr size_t sm = (size_t)PPB * zpair_slot<T>(NZ) * sizeof(V);
+    const long long npairs = ((long long)g.Nx * g.Ny + 1) / 2;
+    const dim3 grid((unsigned)((npairs + PPB - 1) / PPB), ncomp);
+    auto run = [&](auto k) {
       if ((err = smem_attr(k, sm)) != cudaSuccess) return;
-      k<<<grid, 256, sm, st>>>((const V*)in, (V*)out, g, (const V*)tw, nl, ncomp);
-    } else {
-      auto k = k_z_single<T, NZ, E, 1>;
-      if ((err = smem_attr(k, sm)) != cudaSuccess) return;
-      k<<<grid, 256, sm, st>>>((const V*)in, (V*)out, g, (const V*)tw, nl, ncomp);
-    }
-    ++g_launches;
-    err = cudaGetLastError();
+      k<<<grid, NT, sm, st>>>((const V*)in, (V*)out, g, (const V*)tw);
+      ++g_launches;
+      err = cudaGetLastError();
+    };
+    constexpr int MINB = std::is_same<T, float>::value ? 6 : 3;
+    if (dir < 0) run(k_z_single<T, NZ, E, -1, NT, MINB>);
+    else run(k_z_single<T, NZ, E, 1, NT, MINB>);
   });
   return err;
 }
+#endif  // TS_PART_Z
 
+#if TS_PART == TS_PART_FX
 template <int FORM, int MODE, int LL, int E, int CW>
 static cudaError_t fwd_x_fused(const Geo& g, const void* P, const StageArgs& a, const void* tw, cudaStream_t st);
-
-// forward x candidates (MODE_STEP): 1 = the split form (strided x FFT, then the
-// elementwise epilogue) where the rule is the fused TMA kernel; 2 = the fused
-// kernel with half-width column tiles (32-byte rows in FP32; where the rule
-// splits, the fused kernel at the rule's tile width); 3 = the fused kernel with
-// 8 elements per thread (half the threads)
-constexpr bool fx_rule_fused(int L) { return xcw(L) * sizeof(V) >= 64; }
-constexpr int fx_cw2(int L) { return fx_rule_fused(L) ? xcw(L) / 2 : xcw(L); }
-constexpr bool fx_valid(int L, int v) {
-  return v == 0 || (v == 1 && fx_rule_fused(L)) || (v == 2 && fx_cw2(L) * sizeof(V) >= 16 && fx_cw2(L) * (L / emin(E_ACC, L)) >= 32) ||
-         (v == 3 && fx_rule_fused(L) && emin(E_ACC_ALT, L) != emin(E_ACC, L));
-}
-
 
 template <int FORM, int MODE, int LL>
 static cudaError_t fwd_x_impl(const Geo& g, const void* P, const StageArgs& a, const void* tw, cudaStream_t st) {
@@ -544,7 +618,7 @@ static cudaError_t fwd_x_impl(const Geo& g, const void* P, const StageArgs& a, c
   const bool split = CW * sizeof(V) < 64 || v == 1;
   if (split) {
     // tiles narrower than 64-byte rows: forward x FFT in place, then the elementwise epilogue
-    constexpr int NF = FORM == 1 ? 3 : 6;
+    constexpr int NF = z_nout(FORM);
     cudaError_t err = Launch<T>::strided(g, 0, -1, const_cast<void*>(P), NF, tw, st);
     if (err != cudaSuccess) return err;
     const unsigned blocks = grid1d(g.S, 256);
@@ -599,34 +673,60 @@ template <> cudaError_t Launch<T>::fwd_x(const Geo& g, int form, int mode, const
       else if (mode == MODE_FLUX) err = fwd_x_impl<1, MODE_FLUX, LL>(g, P, a, tw, st);
       else err = fwd_x_impl<1, MODE_NLIN, LL>(g, P, a, tw, st);
     } else {
-      if (mode == MODE_STEP) err = fwd_x_impl<0, MODE_STEP, LL>(g, P, a, tw, st);
+      if (mode == MODE_STEP) err = fwd_x_impl<7, MODE_STEP, LL>(g, P, a, tw, st);
       else if (mode == MODE_FLUX) err = fwd_x_impl<0, MODE_FLUX, LL>(g, P, a, tw, st);
       else err = fwd_x_impl<0, MODE_NLIN, LL>(g, P, a, tw, st);
     }
   });
   return err;
 }
+#endif  // TS_PART_FX
 
-// SFF x candidates. Inverse: 1 = 4 elements per thread (power-of-two lengths),
-// 2 = half-width column tiles. Forward: 1 = the other split choice (fused
-// epilogue from 64 points on, split below), 2 = half-width column tiles.
-constexpr int sx_e(int N, int dir) { return e_mixed(N, dir > 0 ? 8 : (std::is_same<T, float>::value ? 8 : 4)); }
-constexpr Tile sx_cand(int N, int dir, int v) {
-  return v == 0 ? Tile{sx_e(N, dir), cw_for(N, sx_e(N, dir)), 1}
-       : v == 1 ? (dir > 0 ? (N % 3 != 0 && sx_e(N, dir) > 4 ? Tile{4, cw_for(N, 4), 1} : Tile{0, 0, 0})
-                           : Tile{sx_e(N, dir), cw_for(N, sx_e(N, dir)), 2})
-       : v == 2 ? (cw_for(N, sx_e(N, dir)) > 1 ? Tile{sx_e(N, dir), cw_for(N, sx_e(N, dir)) / 2, 1} : Tile{0, 0, 0})
-                : Tile{0, 0, 0};
-}
-constexpr bool sx_valid(int N, int dir, int v) {
-  return v == 0 || (N <= 512 && v < 3 && tile_fits(N, sx_cand(N, dir, v), 3) &&
-                    !tile_eq(sx_cand(N, dir, v), sx_cand(N, dir, 0)));
+#if TS_PART == TS_PART_SFF
+template <> cudaError_t Launch<T>::sc_x(const Geo& g, int dir, const ScArgs& a, const void* tq, cudaStream_t st, int nf,
+                                        int nmem) {
+  cudaError_t err = cudaErrorInvalidValue;
+  dispatch_L_sff(g.Nx, [&](auto Lc) {
+    constexpr int NN = decltype(Lc)::value;
+    if constexpr (NN <= 512) {
+      constexpr LdTile c = sc_tile(NN, 1), cf = sc_tile(NN, -1);
+      static_assert(c.E == cf.E && c.CW == cf.CW, "one tile per length");
+      const long long cols = (long long)a.nplanes * g.Ny * g.Hz;
+      constexpr size_t sm = (size_t)NN * c.CW * sizeof(V);
+      const dim3 grid((unsigned)((cols + c.CW - 1) / c.CW), nmem, nf);
+      auto run = [&](auto k) {
+        if ((err = smem_attr(k, sm)) != cudaSuccess) return;
+        k<<<grid, c.CW * (NN / c.E), sm, st>>>(a, g, (const V*)tq);
+        ++g_launches;
+        err = cudaGetLastError();
+      };
+      if (dir < 0) run(k_sc_x<T, NN, c.E, c.CW, -1, cf.MINB>);
+      else run(k_sc_x<T, NN, c.E, c.CW, 1, c.MINB>);
+    }
+  });
+  return err;
 }
 
 template <> cudaError_t Launch<T>::sff_inv_x(const Geo& g, const void* U, const void* Tf, void* W, const void* tq,
                                              cudaStream_t st, int nmem, long long msU, long long msT, long long msW) {
   cudaError_t err = cudaErrorInvalidValue;
   const int v = g.tv[TUNE_X_INV];
+  if (v == 0) {
+    // the rule: one block per column tile and field
+    ScArgs a{};
+    a.s0 = U;
+    a.s3 = Tf;
+    a.d = W;
+    a.sF = a.dF = a.plane = g.S;
+    a.ms0 = msU;
+    a.ms3 = msT;
+    a.msd = msW;
+    a.nplanes = 1;
+    a.smask = 0x9;  // u1 and T sine series
+    a.scl = 1.0;
+    a.deal = g.dealias != 0;
+    return sc_x(g, +1, a, tq, st, 4, nmem);
+  }
   dispatch_L_sff(g.Nx, [&](auto Lc) {
     constexpr int NN = decltype(Lc)::value;
     if constexpr (NN <= 512) {
@@ -647,8 +747,6 @@ template <> cudaError_t Launch<T>::sff_inv_x(const Geo& g, const void* U, const 
         if constexpr (sx_valid(NN, 1, 1)) run(std::integral_constant<int, 1>{});
       } else if (v == 2 && sx_valid(NN, 1, 2)) {
         if constexpr (sx_valid(NN, 1, 2)) run(std::integral_constant<int, 2>{});
-      } else {
-        run(std::integral_constant<int, 0>{});
       }
     }
   });
@@ -659,6 +757,21 @@ template <> cudaError_t Launch<T>::sff_fwd_x(const Geo& g, const void* P, const 
                                              cudaStream_t st, int nmem) {
   cudaError_t err = cudaErrorInvalidValue;
   const int v = g.tv[TUNE_X_FWD];
+  if (v == 0) {
+    // the rule: the eight products transformed in place, then the elementwise epilogue
+    ScArgs s{};
+    s.s0 = P;
+    s.d = const_cast<void*>(P);
+    s.sF = s.dF = s.plane = g.S;
+    s.ms0 = s.msd = a.msP;
+    s.nplanes = 1;
+    for (int f = 0; f < 8; ++f) s.smask |= sff_prod_sine(f) << f;
+    s.scl = 1.0 / (2.0 * g.Nx * (double)g.Ny * g.Nz);
+    if ((err = sc_x(g, -1, s, tq, st, 8, nmem)) != cudaSuccess) return err;
+    k_sff_prod_epi<T><<<dim3(grid1d(g.S, 256), nmem), 256, 0, st>>>((const V*)P, g, a);
+    ++g_launches;
+    return cudaGetLastError();
+  }
   dispatch_L_sff(g.Nx, [&](auto Lc) {
     constexpr int NN = decltype(Lc)::value;
     if constexpr (NN <= 512) {
@@ -685,8 +798,6 @@ template <> cudaError_t Launch<T>::sff_fwd_x(const Geo& g, const void* P, const 
         if constexpr (sx_valid(NN, -1, 1)) run(std::integral_constant<int, 1>{});
       } else if (v == 2 && sx_valid(NN, -1, 2)) {
         if constexpr (sx_valid(NN, -1, 2)) run(std::integral_constant<int, 2>{});
-      } else {
-        run(std::integral_constant<int, 0>{});
       }
     }
   });
@@ -694,29 +805,22 @@ template <> cudaError_t Launch<T>::sff_fwd_x(const Geo& g, const void* P, const 
 }
 
 template <> cudaError_t Launch<T>::sff_x(const Geo& g, int dir, void* A, int ncomp, int sine, double scl,
-                                         const void* tq, cudaStream_t st, int nbatch, long long bstride) {
-  cudaError_t err = cudaErrorInvalidValue;
-  dispatch_L_sff(g.Nx, [&](auto Lc) {
-    constexpr int NN = decltype(Lc)::value;
-    if constexpr (NN <= 512) {
-      constexpr int E = e_mixed(NN, 8);
-      constexpr int CW = cw_for(NN, E);
-      const int inner = g.Ny * g.Hz;
-      const size_t sm = (size_t)NN * CW * sizeof(V);
-      const dim3 grid((unsigned)(((long long)ncomp * inner + CW - 1) / CW), 1, nbatch);
-      auto run = [&](auto k) {
-        if ((err = smem_attr(k, sm)) != cudaSuccess) return;
-        k<<<grid, CW * (NN / E), sm, st>>>((V*)A, g, (const V*)tq, sine, scl, bstride, ncomp);
-        ++g_launches;
-        err = cudaGetLastError();
-      };
-      if (dir < 0) run(k_sff_x<T, NN, E, CW, -1>);
-      else run(k_sff_x<T, NN, E, CW, 1>);
-    }
-  });
-  return err;
+                                         const void* tq, cudaStream_t st, int nbatch, long long bstride,
+                                         const void* src, int deal) {
+  ScArgs a{};
+  a.s0 = src ? src : A;
+  a.d = A;
+  a.sF = a.dF = bstride;
+  a.plane = g.S;
+  a.nplanes = ncomp;
+  a.smask = sine;
+  a.scl = scl;
+  a.deal = deal;
+  return sc_x(g, dir, a, tq, st, nbatch);
 }
+#endif  // TS_PART_SFF
 
+#if TS_PART == TS_PART_MISC
 template <> cudaError_t Launch<T>::reality(const Geo& g, void* A, int ncomp, cudaStream_t st) {
   const long long n = (long long)g.Nx * g.Ny * ncomp;
   k_reality<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>((V*)A, ncomp, g);
@@ -943,7 +1047,7 @@ template <> bool Launch<T>::tune_valid(const Geo& g, int form, int cls, int v) {
     case TUNE_Z:
       dispatch_L_sff(g.Nz, [&](auto Lc) {
         constexpr int NZ = decltype(Lc)::value;
-        ok = form == 0 ? z_valid<NZ, 0>(v) : form == 1 ? z_valid<NZ, 1>(v) : form == 2 ? z_valid<NZ, 2>(v) : false;
+        ok = form == 0 ? z_valid<NZ, 7>(v) : form == 1 ? z_valid<NZ, 1>(v) : form == 2 ? z_valid<NZ, 2>(v) : false;
       });
       break;
     default:
@@ -963,5 +1067,6 @@ template <> bool Launch<T>::tune_blocks(const Geo& g, int form, int cls) {
     });
   return ok;
 }
+#endif  // TS_PART_MISC
 
 }  // namespace ts

@@ -1,3 +1,3 @@
-// FP32 instantiation of the kernel launchers.
 #define TS_REAL float
+#define TS_PART TS_PART_MISC
 #include "ts_kern_impl.cuh"

@@ -1,0 +1,3 @@
+#define TS_REAL float
+#define TS_PART TS_PART_SFF
+#include "ts_kern_impl.cuh"

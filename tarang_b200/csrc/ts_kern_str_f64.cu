@@ -1,0 +1,3 @@
+#define TS_REAL double
+#define TS_PART TS_PART_STR
+#include "ts_kern_impl.cuh"

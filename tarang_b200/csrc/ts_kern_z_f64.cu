@@ -1,3 +1,3 @@
-// FP64 instantiation of the kernel launchers.
 #define TS_REAL double
+#define TS_PART TS_PART_Z
 #include "ts_kern_impl.cuh"

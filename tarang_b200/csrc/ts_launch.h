@@ -23,8 +23,10 @@ template <typename T> struct Launch {
   // per > 0: the nf fields are nf / per members of per fields each, members mstride complex apart
   // inner_eff > 0: transform only the first inner_eff columns (y axis: kz < inner_eff);
   // zero_hi: rows with 3|k| > L are zero and not read (two-thirds dealiased input)
+  // dst (x axis): write there instead of in place; scl (x axis, forward): multiply the outputs
   static cudaError_t strided(const Geo& g, int axis, int dir, void* data, int nf, const void* tw, cudaStream_t st,
-                             int per = 0, long long mstride = 0, int inner_eff = 0, int zero_hi = 0);
+                             int per = 0, long long mstride = 0, int inner_eff = 0, int zero_hi = 0,
+                             void* dst = nullptr, double scl = 1.0);
   // form 0 conservative (3 fields out), 1 rotational (6), 3 adjoint of the rotational form (9: also
   // lsc c^-1 P lam from the cotangent lam)
   // kept != 0 (forms 0, 1 with two-thirds dealiasing): write only the columns with 3|ky| <= Ny, 3 kz <= Nz
@@ -54,8 +56,12 @@ template <typename T> struct Launch {
                                int nmem = 1);
   // standalone sin/cos x transform of ncomp components in place (dir -1 forward with scale scl, +1 inverse);
   // nbatch > 1 repeats it on the fields at A + b * bstride (complex elements), field b with parity bit b of sine
+  // src: read the fields there instead (same strides); deal (inverse): dealias them on load (the plan's mode)
   static cudaError_t sff_x(const Geo& g, int dir, void* A, int ncomp, int sine, double scl, const void* tq,
-                           cudaStream_t st, int nbatch = 1, long long bstride = 0);
+                           cudaStream_t st, int nbatch = 1, long long bstride = 0, const void* src = nullptr,
+                           int deal = 0);
+  static cudaError_t sc_x(const Geo& g, int dir, const ScArgs& a, const void* tq, cudaStream_t st, int nf,
+                          int nmem = 1);
   // FFF passive scalar: elementwise epilogue of the nine x-transformed products in P
   static cudaError_t scalar_epi(const Geo& g, const void* P, const SffArgs& a, cudaStream_t st);
   // SSS z sin/cos helpers on nlines lines of N reals (padded to N + 2)

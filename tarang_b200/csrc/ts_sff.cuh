@@ -17,7 +17,8 @@
 //             V_0 = c_0 (C) or 0 (S), c_N = 0; v = inverse FFT_N(V) (unscaled);
 //             u_{2k} = v_k, u_{2k+1} = v_{N-1-k}, and u_n *= (-1)^n for S.
 // Parities (global/Global.cc:137-145, sincostr "SFF"): u1 S, u2 C, u3 C, T S;
-// products u1u1 u2u2 u3u3 C, u1u2 S, u2u3 C, u3u1 S, u1T C, u2T S, u3T S.
+// products (form 2 of the z pass) u1u1 - u3u3 and u2u2 - u3u3 C, u1u2 S, u2u3 C, u3u1 S,
+// u1T C, u2T S, u3T S.
 // x derivative of a C series is -Kx (result S), of an S series +Kx (result C)
 // (SFF_pencil_tr.cc:77-106).
 #pragma once
@@ -62,7 +63,7 @@ __host__ __device__ constexpr int sff_min_blocks(int threads, int e) {
 }
 
 // parity of product field f: true = sine
-__host__ __device__ constexpr bool sff_prod_sine(int f) { return f == 3 || f == 5 || f == 7 || f == 8; }
+__host__ __device__ constexpr bool sff_prod_sine(int f) { return f == 2 || f == 4 || f == 6 || f == 7; }
 
 // ---------------------------------------------------------------------------
 // inverse x pass: W_f = inverse sin/cos transform of D(field_f), f = u1,u2,u3,T.
@@ -225,6 +226,130 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
 }
 
 // ---------------------------------------------------------------------------
+// Sin/cos transform along x of several fields, one launch: grid x = column tiles of the
+// planes, y = batch members, z = fields (bit f of smask: field f is a sine series).
+// Every row a thread needs is loaded straight into its registers (the inverse reads the
+// mirrored rows N - m a second time: L1), one exchange tile of N x CW complex per block, so
+// that several blocks share an SM.  The planes (components, or the x-planes of a y pass)
+// are one run of columns, so no tile is cut at a plane's end.  Source and destination may
+// be the same: a block's columns are in registers before its first store.
+// DIR = +1: rows hold coefficients, the unscaled synthesis is written; deal: the rows that
+//           dealiasing clears are read as zero (basis and mode of g).
+// DIR = -1: rows hold points, the coefficients times 2N scl are written.
+// ---------------------------------------------------------------------------
+struct ScArgs {
+  const void* s0;             // source of field f < 3 (f sF), or of all fields where s3 is null
+  const void* s3;             // source of field 3 (the SFF temperature), or null
+  void* d;                    // destination of field f (f dF)
+  long long sF, dF;           // field strides
+  long long ms0, ms3, msd;    // member strides
+  long long plane;            // plane stride
+  unsigned nplanes;
+  int smask;
+  double scl;
+  int deal;
+};
+
+// rows q >= lim of the column (ly, lz) are cleared by dealiasing along a sin/cos x axis
+// (the conditions of dealias_zero, bases 1 and 2; sss: lz is the real index, the padding
+// reals cleared as well)
+__device__ __forceinline__ int sc_row_limit(int mode, int basis, int ly, int lz, int Nx, int Ny, int Nz) {
+  const bool sy = basis >= 2, sz = basis == 3;
+  if (sz && lz >= Nz) return 0;
+  if (mode == 1) {
+    const bool my = sy ? ly >= 2 * Ny / 3 + 1 : (ly >= Ny / 3 + 1 && ly <= 2 * Ny / 3 - 1);
+    const bool mz = sz ? lz >= Nz / 3 : lz >= Nz / 3 + 1;
+    return my && mz ? 2 * Nx / 3 + 1 : Nx;
+  }
+  if (mode == 2) {
+    const bool by = sy ? 3 * ly > 2 * Ny : 3 * abs(kfft(ly, Ny)) > Ny;
+    const bool bz = sz ? 3 * lz > 2 * Nz : 3 * lz > Nz;
+    return by || bz ? 0 : 2 * Nx / 3 + 1;
+  }
+  return Nx;
+}
+
+template <typename T, int N, int E, int CW, int DIR, int MINB>
+__global__ void __launch_bounds__(CW * (N / E), MINB)
+    k_sc_x(ScArgs a, Geo g, const C<T>* __restrict__ tq) {
+  typedef C<T> V;
+  constexpr int SWK = best_swk(N, E, CW, (int)sizeof(V));
+  extern __shared__ __align__(16) unsigned char smraw[];
+  V* xch = reinterpret_cast<V*>(smraw);
+  const int c = threadIdx.x % CW, t = threadIdx.x / CW;
+  const unsigned inner = g.Ny * g.Hz;
+  const unsigned col = blockIdx.x * CW + c;  // plane col / inner, column col % inner
+  const bool ok = col < a.nplanes * inner;
+  const unsigned pl = ok ? col / inner : 0, cc = ok ? col - pl * inner : 0;
+  const long long rstride = inner;
+  const int f = blockIdx.z;
+  const bool sine = (a.smask >> f) & 1;
+  const V* src = (f == 3 && a.s3) ? reinterpret_cast<const V*>(a.s3) + blockIdx.y * a.ms3
+                                  : reinterpret_cast<const V*>(a.s0) + f * a.sF + blockIdx.y * a.ms0;
+  V* dst = reinterpret_cast<V*>(a.d) + f * a.dF + blockIdx.y * a.msd;
+  const long long off = pl * a.plane + cc;
+  src += off;
+  dst += off;
+  V v[E];
+  if constexpr (DIR < 0) {
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int k = load_row<N, E>(t, s);
+      v[s] = ok ? src[(k < N / 2 ? 2 * k : 2 * (N - 1 - k) + 1) * rstride] : mk<V>(0, 0);
+    }
+#pragma unroll
+    for (int s = 0; s < E; ++s)
+      if (sine && load_row<N, E>(t, s) >= N / 2) v[s] = mk<V>(-v[s].x, -v[s].y);
+    fft_regs<N, E, -1, 0, false, false, SWK>(v, t, xch, CW, c, tq, 4);
+#pragma unroll
+    for (int s = 0; s < E; ++s) xch[final_row<N, E>(t, s) * CW + c] = v[s];
+    __syncthreads();
+    if (!ok) return;
+    const T scl = (T)a.scl;
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int m = final_row<N, E>(t, s);
+      const V zr = xch[((N - m) % N) * CW + c];
+      const V w = tq[m], wz = mul(w, v[s]), wzr = mul(conjg(w), zr);
+      dst[m * rstride] = sine ? mul_i<1>(scale(sub(wz, wzr), scl)) : scale(add(wz, wzr), scl);
+    }
+  } else {
+    const int ly = a.deal ? cc / g.Hz : 0, lz = a.deal ? cc - ly * g.Hz : 0;
+    // SSS: the two reals of a slot have limits of their own
+    const int lx0 = !a.deal ? N : sc_row_limit(g.dealias, g.basis, ly, g.basis == 3 ? 2 * lz : lz, N, g.Ny, g.Nz);
+    const int lx1 = (a.deal && g.basis == 3) ? sc_row_limit(g.dealias, 3, ly, 2 * lz + 1, N, g.Ny, g.Nz) : lx0;
+    V q[E];
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int m = load_row<N, E>(t, s), mr = (N - m) % N;
+      v[s] = (ok && (m < lx0 || m < lx1)) ? src[m * rstride] : mk<V>(0, 0);
+      q[s] = (ok && m > 0 && (mr < lx0 || mr < lx1)) ? src[mr * rstride] : mk<V>(0, 0);
+    }
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int m = load_row<N, E>(t, s), mr = (N - m) % N;
+      if (lx0 != lx1) {
+        if (m >= lx0) v[s].x = 0;
+        if (m >= lx1) v[s].y = 0;
+        if (mr >= lx0) q[s].x = 0;
+        if (mr >= lx1) q[s].y = 0;
+      }
+      // cosine: conj(w_m) (c_m - i c_{N-m}), V_0 = c_0; sine: conj(w_m) (s_{N-m} - i s_m), V_0 = 0
+      if (m == 0) v[s] = sine ? mk<V>(0, 0) : v[s];
+      else v[s] = mul(conjg(tq[m]), sine ? add_i<-1>(q[s], v[s]) : add_i<-1>(v[s], q[s]));
+    }
+    fft_regs<N, E, 1, 0, false, false, SWK>(v, t, xch, CW, c, tq, 4);
+    if (!ok) return;
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int k = final_row<N, E>(t, s);
+      const int n = k < N / 2 ? 2 * k : 2 * (N - 1 - k) + 1;
+      dst[n * rstride] = (sine && (n & 1)) ? mk<V>(-v[s].x, -v[s].y) : v[s];
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Boussinesq epilogue at spectral element (m, ly, lz) of batch member mb (offset
 // `off` in a component): force U.F1 = cu T, T.F = cT U.V1 of the stage input, SFF
 // projection, IF-RK4 stage update of U (nu) and T (kappa).  N1..N3, NT = the
@@ -241,6 +366,13 @@ __device__ __forceinline__ void sff_epilogue(const Geo& g, const SffArgs& a, lon
   const V* U1in = reinterpret_cast<const V*>(a.U1in) + mb * a.msU1in;
   const V* Tin = reinterpret_cast<const V*>(a.Tin) + mb * a.msTin;
   const long long tb = mb * a.mtab;
+  // the state, loaded ahead of the arithmetic
+  V u0v[4], ttv[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    u0v[i] = i < 3 ? U0[i * g.S + off] : T0[off];
+    if (a.stage > 1) ttv[i] = tot[i * g.S + off];
+  }
   const double Kxd = m * g.kf[0], Kyd = kfft(ly, g.Ny) * g.kf[1], Kzd = lz * g.kf[2];
   const T Kx = (T)Kxd, Ky = (T)Kyd, Kz = (T)Kzd;
   // force (compute_force_RBC.cc:104-150): U.F1 = cu T, T.F = cT U.V1 of the stage input
@@ -267,19 +399,19 @@ __device__ __forceinline__ void sff_epilogue(const Geo& g, const SffArgs& a, lon
     const Fac<T> Feh = i < 3 ? Fhu : Fht, Fe1 = i < 3 ? F1u : F1t;
     const long long o = i * g.S + off;
     const V R = Rv[i];
-    const V u0 = i < 3 ? U0[o] : T0[off];
+    const V u0 = u0v[i];
     V r;
     if (a.stage == 1) {
       Uc[o] = r = rk_u1_c(dz ? mk<V>(0, 0) : u0, R, Feh, Fc2);
       tot[o] = rk_t1_c(R, Fe1, Fc6);
     } else if (a.stage == 2) {
       Uc[o] = r = rk_u2_c(u0, R, Feh, Fc2);
-      tot[o] = rk_tacc_c(tot[o], R, Feh, Fc3);
+      tot[o] = rk_tacc_c(ttv[i], R, Feh, Fc3);
     } else if (a.stage == 3) {
       Uc[o] = r = rk_u3_c(u0, R, Feh, Fc1);
-      tot[o] = rk_tacc_c(tot[o], R, Feh, Fc3);
+      tot[o] = rk_tacc_c(ttv[i], R, Feh, Fc3);
     } else {
-      r = rk_u4_c(u0, tot[o], R, Fe1, Fc6);
+      r = rk_u4_c(u0, ttv[i], R, Fe1, Fc6);
       if (a.reality && lz == g.Nz / 2) r = mk<V>(0, 0);
       if (i < 3) const_cast<V*>(U0)[o] = r;
       else const_cast<V*>(T0)[off] = r;
@@ -358,24 +490,50 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_sff_epi(const C<T>* __restrict__ P, Geo g, SffArgs a) {
   const long long mb = blockIdx.y;
   P += mb * a.msP;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < g.S; e += stride) {
-    const int lz = (int)(e % g.Hz);
-    const long long r = e / g.Hz;
-    const int ly = (int)(r % g.Ny), m = (int)(r / g.Ny);
+  // 32-bit index arithmetic (a component holds < 2^31 modes)
+  const unsigned n = (unsigned)g.S, stride = gridDim.x * blockDim.x;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const unsigned r = e / (unsigned)g.Hz;
+    const int lz = (int)(e - r * g.Hz), m = (int)(r / (unsigned)g.Ny), ly = (int)(r - (unsigned)m * g.Ny);
     sff_epilogue<T>(g, a, mb, m, ly, lz, e, P[e], P[g.S + e], P[2 * g.S + e], P[3 * g.S + e]);
+  }
+}
+
+// Elementwise Boussinesq epilogue from the eight product spectra in P (after k_sc_x, sine
+// series where sff_prod_sine): assembly of N1..N3, NT (the terms of k_sff_fwd_x), then
+// sff_epilogue.  One thread per element, every array access coalesced.
+template <typename T>
+__global__ void __launch_bounds__(256) k_sff_prod_epi(const C<T>* __restrict__ P, Geo g, SffArgs a) {
+  typedef C<T> V;
+  const long long mb = blockIdx.y;
+  P += mb * a.msP;
+  // 32-bit index arithmetic (a component holds < 2^31 modes)
+  const unsigned n = (unsigned)g.S, stride = gridDim.x * blockDim.x;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const unsigned r = e / (unsigned)g.Hz;
+    const int lz = (int)(e - r * g.Hz), m = (int)(r / (unsigned)g.Ny), ly = (int)(r - (unsigned)m * g.Ny);
+    V q[8];
+#pragma unroll
+    for (int f = 0; f < 8; ++f) q[f] = P[f * g.S + e];
+    const T Kx = (T)(m * g.kf[0]), Ky = (T)(kfft(ly, g.Ny) * g.kf[1]), Kz = (T)(lz * g.kf[2]);
+    const V N1 = add(add(scale(q[0], -Kx), ik(Ky, q[2])), ik(Kz, q[4]));
+    const V N2 = add(add(ik(Ky, q[1]), scale(q[2], Kx)), ik(Kz, q[3]));
+    const V N3 = add(ik(Ky, q[3]), scale(q[4], Kx));
+    const V NT = add(add(scale(q[5], -Kx), ik(Ky, q[6])), ik(Kz, q[7]));
+    sff_epilogue<T>(g, a, mb, m, ly, lz, e, N1, N2, N3, NT);
   }
 }
 
 // ---------------------------------------------------------------------------
 // forward x pass + Boussinesq epilogue (PRLARGE / ULARGE):
-//   N1 = Dx(u1u1) + iKy F[u1u2] + iKz F[u3u1],  N2 = iKy F[u2u2] + Dx(u1u2) + iKz F[u2u3],
-//   N3 = iKz F[u3u3] + iKy F[u2u3] + Dx(u3u1),  NT = Dx(u1T) + iKy F[u2T] + iKz F[u3T]
+//   N1 = Dx(d1) + iKy F[u1u2] + iKz F[u3u1],  N2 = iKy F[d2] + Dx(u1u2) + iKz F[u2u3],
+//   N3 = iKy F[u2u3] + Dx(u3u1),  NT = Dx(u1T) + iKy F[u2T] + iKz F[u3T],
+//   d1 = u1u1 - u3u3, d2 = u2u2 - u3u3 (N up to a gradient, which the projection removes)
 //   (compute_diag_offdiag.cc:47-136); force U.F1 = cu T, T.F = cT U.V1 (compute_force_RBC.cc:104-150);
 //   N -= F; p = div(N)/K^2; N += grad p; R = -N, RT = -NT; IF-RK4 stage update of U (nu) and T (kappa)
 //   (RK_SF.cc:97-221, Tadvance_functions.cc:57-90,226-237,372-395,589-611).
 // ---------------------------------------------------------------------------
-// The nine product columns stream through two cp.async staging tiles (field
+// The eight product columns stream through two cp.async staging tiles (field
 // f+2 is in flight while f is transformed); each thread stages exactly the
 // elements it reads back, in FFT input order, so the reordering is done by the
 // copy and no barrier guards the staging tiles.
@@ -409,7 +567,7 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
   // field f's column into staging tile buf, row k of the tile = FFT input k
   // (even points, then odd points reversed)
   auto issue = [&](int f, int buf) {
-    if (f < 9 && ok) {
+    if (f < 8 && ok) {
       const V* src = P + f * g.S + col;
 #pragma unroll
       for (int s = 0; s < E; ++s) {
@@ -421,7 +579,7 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
   };
   issue(0, 0);
   issue(1, 1);
-  for (int f = 0; f < 9; ++f) {
+  for (int f = 0; f < 8; ++f) {
     const bool sine = sff_prod_sine(f);
     const int buf = f & 1;
     cp_async_wait<1>();
@@ -455,12 +613,11 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
       switch (f) {
         case 0: acc[0][s] = add(acc[0][s], scale(cm, -Kx)); break;
         case 1: acc[1][s] = add(acc[1][s], ik(Ky, cm)); break;
-        case 2: acc[2][s] = add(acc[2][s], ik(Kz, cm)); break;
-        case 3: acc[0][s] = add(acc[0][s], ik(Ky, cm)); acc[1][s] = add(acc[1][s], scale(cm, Kx)); break;
-        case 4: acc[1][s] = add(acc[1][s], ik(Kz, cm)); acc[2][s] = add(acc[2][s], ik(Ky, cm)); break;
-        case 5: acc[0][s] = add(acc[0][s], ik(Kz, cm)); acc[2][s] = add(acc[2][s], scale(cm, Kx)); break;
-        case 6: acc[3][s] = add(acc[3][s], scale(cm, -Kx)); break;
-        case 7: acc[3][s] = add(acc[3][s], ik(Ky, cm)); break;
+        case 2: acc[0][s] = add(acc[0][s], ik(Ky, cm)); acc[1][s] = add(acc[1][s], scale(cm, Kx)); break;
+        case 3: acc[1][s] = add(acc[1][s], ik(Kz, cm)); acc[2][s] = add(acc[2][s], ik(Ky, cm)); break;
+        case 4: acc[0][s] = add(acc[0][s], ik(Kz, cm)); acc[2][s] = add(acc[2][s], scale(cm, Kx)); break;
+        case 5: acc[3][s] = add(acc[3][s], scale(cm, -Kx)); break;
+        case 6: acc[3][s] = add(acc[3][s], ik(Ky, cm)); break;
         default: acc[3][s] = add(acc[3][s], ik(Kz, cm)); break;
       }
     }
@@ -498,21 +655,28 @@ __global__ void __launch_bounds__(256) k_scalar_epi(const C<T>* __restrict__ P, 
   const V* T0 = reinterpret_cast<const V*>(a.T0);
   V* Uc = reinterpret_cast<V*>(a.Ucur);
   V* tot = reinterpret_cast<V*>(a.tot);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < g.S; e += stride) {
-    const int lz = (int)(e % g.Hz);
-    const long long r = e / g.Hz;
-    const int ly = (int)(r % g.Ny), lx = (int)(r / g.Ny);
+  // 32-bit index arithmetic (a component holds < 2^31 modes)
+  const unsigned n = (unsigned)g.S, stride = gridDim.x * blockDim.x;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const unsigned r = e / (unsigned)g.Hz;
+    const int lz = (int)(e - r * g.Hz), lx = (int)(r / (unsigned)g.Ny), ly = (int)(r - (unsigned)lx * g.Ny);
     const double Kxd = kfft(lx, g.Nx) * g.kf[0], Kyd = kfft(ly, g.Ny) * g.kf[1], Kzd = lz * g.kf[2];
     const T Kx = (T)Kxd, Ky = (T)Kyd, Kz = (T)Kzd;
-    V p[9];
+    V p[8];
 #pragma unroll
-    for (int f = 0; f < 9; ++f) p[f] = scale(P[f * g.S + e], inv);
+    for (int f = 0; f < 8; ++f) p[f] = scale(P[f * g.S + e], inv);
+    // the state, loaded ahead of the arithmetic
+    V u0v[4], ttv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      u0v[i] = i < 3 ? U0[i * g.S + e] : T0[e];
+      if (a.stage > 1) ttv[i] = tot[i * g.S + e];
+    }
     // x, then y, then z derivative terms, as the reference accumulates them
-    V N1 = add(add(ik(Kx, p[0]), ik(Ky, p[3])), ik(Kz, p[5]));
-    V N2 = add(add(ik(Kx, p[3]), ik(Ky, p[1])), ik(Kz, p[4]));
-    V N3 = add(add(ik(Kx, p[5]), ik(Ky, p[4])), ik(Kz, p[2]));
-    const V NT = add(add(ik(Kx, p[6]), ik(Ky, p[7])), ik(Kz, p[8]));
+    V N1 = add(add(ik(Kx, p[0]), ik(Ky, p[2])), ik(Kz, p[4]));
+    V N2 = add(add(ik(Kx, p[2]), ik(Ky, p[1])), ik(Kz, p[3]));
+    V N3 = add(ik(Kx, p[4]), ik(Ky, p[3]));
+    const V NT = add(add(ik(Kx, p[5]), ik(Ky, p[6])), ik(Kz, p[7]));
     const double K2 = (Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd;
     const V div = add(add(ik(Kx, N1), ik(Ky, N2)), ik(Kz, N3));
     const V pr = (K2 > 0) ? mk<V>(div.x / (T)K2, div.y / (T)K2) : mk<V>(0, 0);
@@ -531,18 +695,18 @@ __global__ void __launch_bounds__(256) k_scalar_epi(const C<T>* __restrict__ P, 
       const Fac<T> Feh = i < 3 ? Fhu : Fht, Fe1 = i < 3 ? F1u : F1t;
       const long long o = i * g.S + e;
       const V R = Rv[i];
-      const V u0 = i < 3 ? U0[o] : T0[e];
+      const V u0 = u0v[i];
       if (a.stage == 1) {
         Uc[o] = rk_u1_c(dz ? mk<V>(0, 0) : u0, R, Feh, Fc2);
         tot[o] = rk_t1_c(R, Fe1, Fc6);
       } else if (a.stage == 2) {
         Uc[o] = rk_u2_c(u0, R, Feh, Fc2);
-        tot[o] = rk_tacc_c(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc_c(ttv[i], R, Feh, Fc3);
       } else if (a.stage == 3) {
         Uc[o] = rk_u3_c(u0, R, Feh, Fc1);
-        tot[o] = rk_tacc_c(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc_c(ttv[i], R, Feh, Fc3);
       } else {
-        V un = rk_u4_c(u0, tot[o], R, Fe1, Fc6);
+        V un = rk_u4_c(u0, ttv[i], R, Fe1, Fc6);
         if (a.reality && lz == g.Nz / 2) un = mk<V>(0, 0);
         if (i < 3) const_cast<V*>(U0)[o] = un;
         else const_cast<V*>(T0)[e] = un;
@@ -573,32 +737,29 @@ __global__ void __launch_bounds__(256, 3) k_mhd_epi(const C<T>* __restrict__ P, 
   const V* B0 = reinterpret_cast<const V*>(a.T0);
   V* Uc = reinterpret_cast<V*>(a.Ucur);
   V* tot = reinterpret_cast<V*>(a.tot);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < g.S; e += stride) {
-    const int lz = (int)(e % g.Hz);
-    const long long r = e / g.Hz;
-    const int ly = (int)(r % g.Ny), lx = (int)(r / g.Ny);
+  // 32-bit index arithmetic (a component holds < 2^31 modes)
+  const unsigned n = (unsigned)g.S, stride = gridDim.x * blockDim.x;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const unsigned r = e / (unsigned)g.Hz;
+    const int lz = (int)(e - r * g.Hz), lx = (int)(r / (unsigned)g.Ny), ly = (int)(r - (unsigned)lx * g.Ny);
     const double Kxd = kfft(lx, g.Nx) * g.kf[0], Kyd = kfft(ly, g.Ny) * g.kf[1], Kzd = lz * g.kf[2];
     const T K[3] = {(T)Kxd, (T)Kyd, (T)Kzd};
-    V q[9];
+    V q[8];
 #pragma unroll
-    for (int f = 0; f < 9; ++f) q[f] = scale(P[f * g.S + e], inv);
-    // Zp.nlin (np) and Zm.nlin (nm)
-    V np[3], nm[3];
+    for (int f = 0; f < 8; ++f) q[f] = scale(P[f * g.S + e], inv);
+    // the state, loaded ahead of the arithmetic
+    V u0v[6], ttv[6];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) np[i] = nm[i] = ik(K[i], q[4 * i]);
-    np[0] = add(np[0], ik(K[1], q[1])); nm[1] = add(nm[1], ik(K[0], q[1]));   // P01
-    nm[0] = add(nm[0], ik(K[1], q[3])); np[1] = add(np[1], ik(K[0], q[3]));   // P10
-    np[1] = add(np[1], ik(K[2], q[5])); nm[2] = add(nm[2], ik(K[1], q[5]));   // P12
-    nm[1] = add(nm[1], ik(K[2], q[7])); np[2] = add(np[2], ik(K[1], q[7]));   // P21
-    nm[0] = add(nm[0], ik(K[2], q[6])); np[2] = add(np[2], ik(K[0], q[6]));   // P20
-    np[0] = add(np[0], ik(K[2], q[2])); nm[2] = add(nm[2], ik(K[0], q[2]));   // P02
-    V NU[3], NB[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      NU[i] = scale(add(np[i], nm[i]), (T)0.5);
-      NB[i] = scale(sub(np[i], nm[i]), (T)0.5);
+    for (int i = 0; i < 6; ++i) {
+      u0v[i] = i < 3 ? U0[i * g.S + e] : B0[(i - 3) * g.S + e];
+      if (a.stage > 1) ttv[i] = tot[i * g.S + e];
     }
+    // U.nlin = sum_j D_j S_ij (up to a gradient), B.nlin = sum_j D_j A_ij
+    const V NU[3] = {add(add(ik(K[0], q[0]), ik(K[1], q[2])), ik(K[2], q[4])),
+                     add(add(ik(K[0], q[2]), ik(K[1], q[1])), ik(K[2], q[3])),
+                     add(ik(K[0], q[4]), ik(K[1], q[3]))};
+    const V NB[3] = {sub(ik(K[1], q[5]), ik(K[2], q[7])), sub(ik(K[2], q[6]), ik(K[0], q[5])),
+                     sub(ik(K[0], q[7]), ik(K[1], q[6]))};
     const double K2 = (Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd;
     const V div = add(add(ik(K[0], NU[0]), ik(K[1], NU[1])), ik(K[2], NU[2]));
     const V pr = (K2 > 0) ? mk<V>(div.x / (T)K2, div.y / (T)K2) : mk<V>(0, 0);
@@ -619,18 +780,18 @@ __global__ void __launch_bounds__(256, 3) k_mhd_epi(const C<T>* __restrict__ P, 
       const Fac<T> Feh = i < 3 ? Fhu : Fht, Fe1 = i < 3 ? F1u : F1t;
       const long long o = i * g.S + e;
       const V R = Rv[i];
-      const V u0 = i < 3 ? U0[o] : B0[(i - 3) * g.S + e];
+      const V u0 = u0v[i];
       if (a.stage == 1) {
         Uc[o] = rk_u1_c(dz ? mk<V>(0, 0) : u0, R, Feh, Fc2);
         tot[o] = rk_t1_c(R, Fe1, Fc6);
       } else if (a.stage == 2) {
         Uc[o] = rk_u2_c(u0, R, Feh, Fc2);
-        tot[o] = rk_tacc_c(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc_c(ttv[i], R, Feh, Fc3);
       } else if (a.stage == 3) {
         Uc[o] = rk_u3_c(u0, R, Feh, Fc1);
-        tot[o] = rk_tacc_c(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc_c(ttv[i], R, Feh, Fc3);
       } else {
-        V un = rk_u4_c(u0, tot[o], R, Fe1, Fc6);
+        V un = rk_u4_c(u0, ttv[i], R, Fe1, Fc6);
         if (a.reality && lz == g.Nz / 2) un = mk<V>(0, 0);
         if (i < 3) const_cast<V*>(U0)[o] = un;
         else const_cast<V*>(B0)[(i - 3) * g.S + e] = un;
@@ -657,22 +818,29 @@ __global__ void __launch_bounds__(256) k_ssf_epi(const C<T>* __restrict__ P, Geo
   V* Uc = reinterpret_cast<V*>(a.Ucur);
   V* tot = reinterpret_cast<V*>(a.tot);
   V* Uo = reinterpret_cast<V*>(a.Uout);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < g.S; e += stride) {
-    const int lz = (int)(e % g.Hz);
-    const long long r = e / g.Hz;
-    const int ly = (int)(r % g.Ny), lx = (int)(r / g.Ny);
+  // 32-bit index arithmetic (a component holds < 2^31 modes)
+  const unsigned n = (unsigned)g.S, stride = gridDim.x * blockDim.x;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const unsigned r = e / (unsigned)g.Hz;
+    const int lz = (int)(e - r * g.Hz), lx = (int)(r / (unsigned)g.Ny), ly = (int)(r - (unsigned)lx * g.Ny);
     const double Kxd = lx * g.kf[0], Kyd = ly * g.kf[1], Kzd = lz * g.kf[2];
     const T Kx = (T)Kxd, Ky = (T)Kyd, Kz = (T)Kzd;
-    V q[6];
+    V q[5];
 #pragma unroll
-    for (int f = 0; f < 6; ++f) q[f] = P[f * g.S + e];
+    for (int f = 0; f < 5; ++f) q[f] = P[f * g.S + e];
+    // the state, loaded ahead of the arithmetic
+    V u0v[3], ttv[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      u0v[i] = U0[i * g.S + e];
+      if (a.stage > 1) ttv[i] = tot[i * g.S + e];
+    }
     // x / y derivative of a sine (+K) or cosine (-K) series
     auto dS = [](T K, V A) { return scale(A, K); };
     auto dC = [](T K, V A) { return scale(A, -K); };
-    V N1 = add(add(dC(Kx, q[0]), dS(Ky, q[3])), ik(Kz, q[5]));
-    V N2 = add(add(dC(Ky, q[1]), dS(Kx, q[3])), ik(Kz, q[4]));
-    V N3 = add(add(ik(Kz, q[2]), dS(Ky, q[4])), dS(Kx, q[5]));
+    V N1 = add(add(dC(Kx, q[0]), dS(Ky, q[2])), ik(Kz, q[4]));
+    V N2 = add(add(dC(Ky, q[1]), dS(Kx, q[2])), ik(Kz, q[3]));
+    V N3 = add(dS(Ky, q[3]), dS(Kx, q[4]));
     const double K2 = (Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd;
     const V div = add(add(dS(Kx, N1), dS(Ky, N2)), ik(Kz, N3));
     const V pr = (K2 > 0) ? mk<V>(div.x / (T)K2, div.y / (T)K2) : mk<V>(0, 0);
@@ -689,18 +857,18 @@ __global__ void __launch_bounds__(256) k_ssf_epi(const C<T>* __restrict__ P, Geo
     for (int i = 0; i < 3; ++i) {
       const long long o = i * g.S + e;
       const V R = Rv[i];
-      const V u0 = U0[o];
+      const V u0 = u0v[i];
       if (a.stage == 1) {
         Uc[o] = rk_u1_c(dz ? mk<V>(0, 0) : u0, R, Feh, Fc2);
         tot[o] = rk_t1_c(R, Fe1, Fc6);
       } else if (a.stage == 2) {
         Uc[o] = rk_u2_c(u0, R, Feh, Fc2);
-        tot[o] = rk_tacc_c(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc_c(ttv[i], R, Feh, Fc3);
       } else if (a.stage == 3) {
         Uc[o] = rk_u3_c(u0, R, Feh, Fc1);
-        tot[o] = rk_tacc_c(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc_c(ttv[i], R, Feh, Fc3);
       } else {
-        const V un = rk_u4_c(u0, tot[o], R, Fe1, Fc6);
+        const V un = rk_u4_c(u0, ttv[i], R, Fe1, Fc6);
         Uo[o] = un;
         health_mark(nonfinite(un), a.err);
       }
@@ -742,19 +910,28 @@ __global__ void __launch_bounds__(256) k_sss_epi(const T* __restrict__ P, Geo g,
   T* Uc = reinterpret_cast<T*>(a.Ucur);
   T* tot = reinterpret_cast<T*>(a.tot);
   T* Uo = reinterpret_cast<T*>(a.Uout);
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < per; e += (long long)gridDim.x * blockDim.x) {
-    const int lzr = (int)(e % (g.Nz + 2));
+  // 32-bit index arithmetic (a component holds < 2^31 reals)
+  const unsigned n = (unsigned)per, stride = gridDim.x * blockDim.x;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const unsigned r = e / (unsigned)(g.Nz + 2);
+    const int lzr = (int)(e - r * (g.Nz + 2));
     if (lzr >= g.Nz) continue;  // padding
-    const long long r = e / (g.Nz + 2);
-    const int ly = (int)(r % g.Ny), lx = (int)(r / g.Ny);
+    const int lx = (int)(r / (unsigned)g.Ny), ly = (int)(r - (unsigned)lx * g.Ny);
     const double Kxd = lx * g.kf[0], Kyd = ly * g.kf[1], Kzd = lzr * g.kf[2];
     const T Kx = (T)Kxd, Ky = (T)Kyd, Kz = (T)Kzd;
-    T q[6];
+    T q[5];
 #pragma unroll
-    for (int f = 0; f < 6; ++f) q[f] = P[f * per + e];
-    T N1 = (-Kx * q[0] + Ky * q[3]) + Kz * q[5];
-    T N2 = (-Ky * q[1] + Kx * q[3]) + Kz * q[4];
-    T N3 = (-Kz * q[2] + Ky * q[4]) + Kx * q[5];
+    for (int f = 0; f < 5; ++f) q[f] = P[f * per + e];
+    // the state, loaded ahead of the arithmetic
+    T u0v[3], ttv[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      u0v[i] = U0[i * per + e];
+      if (a.stage > 1) ttv[i] = tot[i * per + e];
+    }
+    T N1 = (-Kx * q[0] + Ky * q[2]) + Kz * q[4];
+    T N2 = (-Ky * q[1] + Kx * q[2]) + Kz * q[3];
+    T N3 = Ky * q[3] + Kx * q[4];
     const double K2 = (Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd;
     const T div = (Kx * N1 + Ky * N2) + Kz * N3;
     const T pr = K2 > 0 ? div / (T)K2 : (T)0;
@@ -770,18 +947,18 @@ __global__ void __launch_bounds__(256) k_sss_epi(const T* __restrict__ P, Geo g,
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       const long long o = i * per + e;
-      const T R = Rv[i], u0 = U0[o];
+      const T R = Rv[i], u0 = u0v[i];
       if (a.stage == 1) {
         Uc[o] = rk_u1(dz ? (T)0 : u0, R, Feh, Fc2);
         tot[o] = rk_t1(R, Fe1, Fc6);
       } else if (a.stage == 2) {
         Uc[o] = rk_u2(u0, R, Feh, Fc2);
-        tot[o] = rk_tacc(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc(ttv[i], R, Feh, Fc3);
       } else if (a.stage == 3) {
         Uc[o] = rk_u3(u0, R, Feh, Fc1);
-        tot[o] = rk_tacc(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc(ttv[i], R, Feh, Fc3);
       } else {
-        const T un = rk_u4(u0, tot[o], R, Fe1, Fc6);
+        const T un = rk_u4(u0, ttv[i], R, Fe1, Fc6);
         Uo[o] = un;
         health_mark(!isfinite(un), a.err);
       }
@@ -811,22 +988,29 @@ __global__ void __launch_bounds__(256) k_ssf_rbc_epi(const C<T>* __restrict__ P,
   const V* Tin = reinterpret_cast<const V*>(a.Tin);
   V* Uc = reinterpret_cast<V*>(a.Ucur);
   V* tot = reinterpret_cast<V*>(a.tot);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < g.S; e += stride) {
-    const int lz = (int)(e % g.Hz);
-    const long long r = e / g.Hz;
-    const int ly = (int)(r % g.Ny), lx = (int)(r / g.Ny);
+  // 32-bit index arithmetic (a component holds < 2^31 modes)
+  const unsigned n = (unsigned)g.S, stride = gridDim.x * blockDim.x;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const unsigned r = e / (unsigned)g.Hz;
+    const int lz = (int)(e - r * g.Hz), lx = (int)(r / (unsigned)g.Ny), ly = (int)(r - (unsigned)lx * g.Ny);
     const double Kxd = lx * g.kf[0], Kyd = ly * g.kf[1], Kzd = lz * g.kf[2];
     const T Kx = (T)Kxd, Ky = (T)Kyd, Kz = (T)Kzd;
-    V q[9];
+    V q[8];
 #pragma unroll
-    for (int f = 0; f < 9; ++f) q[f] = P[f * g.S + e];
+    for (int f = 0; f < 8; ++f) q[f] = P[f * g.S + e];
+    // the state, loaded ahead of the arithmetic
+    V u0v[4], ttv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      u0v[i] = i < 3 ? U0[i * g.S + e] : T0[e];
+      if (a.stage > 1) ttv[i] = tot[i * g.S + e];
+    }
     auto dS = [](T K, V A) { return scale(A, K); };
     auto dC = [](T K, V A) { return scale(A, -K); };
-    V N1 = add(add(dC(Kx, q[0]), dS(Ky, q[3])), ik(Kz, q[5]));
-    V N2 = add(add(dC(Ky, q[1]), dS(Kx, q[3])), ik(Kz, q[4]));
-    V N3 = add(add(ik(Kz, q[2]), dS(Ky, q[4])), dS(Kx, q[5]));
-    V NT = add(add(dC(Kx, q[6]), dS(Ky, q[7])), ik(Kz, q[8]));
+    V N1 = add(add(dC(Kx, q[0]), dS(Ky, q[2])), ik(Kz, q[4]));
+    V N2 = add(add(dC(Ky, q[1]), dS(Kx, q[2])), ik(Kz, q[3]));
+    V N3 = add(dS(Ky, q[3]), dS(Kx, q[4]));
+    V NT = add(add(dC(Kx, q[5]), dS(Ky, q[6])), ik(Kz, q[7]));
     N1 = sub(N1, scale(Tin[e], (T)a.cu));
     NT = sub(NT, scale(U1in[e], (T)a.cT));
     const double K2 = (Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd;
@@ -847,18 +1031,18 @@ __global__ void __launch_bounds__(256) k_ssf_rbc_epi(const C<T>* __restrict__ P,
       const Fac<T> Feh = i < 3 ? Fhu : Fht, Fe1 = i < 3 ? F1u : F1t;
       const long long o = i * g.S + e;
       const V R = Rv[i];
-      const V u0 = i < 3 ? U0[o] : T0[e];
+      const V u0 = u0v[i];
       if (a.stage == 1) {
         Uc[o] = rk_u1_c(dz ? mk<V>(0, 0) : u0, R, Feh, Fc2);
         tot[o] = rk_t1_c(R, Fe1, Fc6);
       } else if (a.stage == 2) {
         Uc[o] = rk_u2_c(u0, R, Feh, Fc2);
-        tot[o] = rk_tacc_c(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc_c(ttv[i], R, Feh, Fc3);
       } else if (a.stage == 3) {
         Uc[o] = rk_u3_c(u0, R, Feh, Fc1);
-        tot[o] = rk_tacc_c(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc_c(ttv[i], R, Feh, Fc3);
       } else {
-        const V un = rk_u4_c(u0, tot[o], R, Fe1, Fc6);
+        const V un = rk_u4_c(u0, ttv[i], R, Fe1, Fc6);
         if (i < 3) U0[o] = un;
         else T0[e] = un;
         health_mark(nonfinite(un), a.health);
@@ -878,20 +1062,29 @@ __global__ void __launch_bounds__(256) k_sss_rbc_epi(const T* __restrict__ P, Ge
   const T* Tin = reinterpret_cast<const T*>(a.Tin);
   T* Uc = reinterpret_cast<T*>(a.Ucur);
   T* tot = reinterpret_cast<T*>(a.tot);
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < per; e += (long long)gridDim.x * blockDim.x) {
-    const int lzr = (int)(e % (g.Nz + 2));
+  // 32-bit index arithmetic (a component holds < 2^31 reals)
+  const unsigned n = (unsigned)per, stride = gridDim.x * blockDim.x;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const unsigned r = e / (unsigned)(g.Nz + 2);
+    const int lzr = (int)(e - r * (g.Nz + 2));
     if (lzr >= g.Nz) continue;  // padding
-    const long long r = e / (g.Nz + 2);
-    const int ly = (int)(r % g.Ny), lx = (int)(r / g.Ny);
+    const int lx = (int)(r / (unsigned)g.Ny), ly = (int)(r - (unsigned)lx * g.Ny);
     const double Kxd = lx * g.kf[0], Kyd = ly * g.kf[1], Kzd = lzr * g.kf[2];
     const T Kx = (T)Kxd, Ky = (T)Kyd, Kz = (T)Kzd;
-    T q[9];
+    T q[8];
 #pragma unroll
-    for (int f = 0; f < 9; ++f) q[f] = P[f * per + e];
-    T N1 = (-Kx * q[0] + Ky * q[3]) + Kz * q[5];
-    T N2 = (-Ky * q[1] + Kx * q[3]) + Kz * q[4];
-    T N3 = (-Kz * q[2] + Ky * q[4]) + Kx * q[5];
-    T NT = (-Kx * q[6] + Ky * q[7]) + Kz * q[8];
+    for (int f = 0; f < 8; ++f) q[f] = P[f * per + e];
+    // the state, loaded ahead of the arithmetic
+    T u0v[4], ttv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      u0v[i] = i < 3 ? U0[i * per + e] : T0[e];
+      if (a.stage > 1) ttv[i] = tot[i * per + e];
+    }
+    T N1 = (-Kx * q[0] + Ky * q[2]) + Kz * q[4];
+    T N2 = (-Ky * q[1] + Kx * q[2]) + Kz * q[3];
+    T N3 = Ky * q[3] + Kx * q[4];
+    T NT = (-Kx * q[5] + Ky * q[6]) + Kz * q[7];
     N1 -= (T)a.cu * Tin[e];
     NT -= (T)a.cT * U1in[e];
     const double K2 = (Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd;
@@ -911,18 +1104,18 @@ __global__ void __launch_bounds__(256) k_sss_rbc_epi(const T* __restrict__ P, Ge
     for (int i = 0; i < 4; ++i) {
       const Fac<T> Feh = i < 3 ? Fhu : Fht, Fe1 = i < 3 ? F1u : F1t;
       const long long o = i * per + e;
-      const T R = Rv[i], u0 = i < 3 ? U0[o] : T0[e];
+      const T R = Rv[i], u0 = u0v[i];
       if (a.stage == 1) {
         Uc[o] = rk_u1(dz ? (T)0 : u0, R, Feh, Fc2);
         tot[o] = rk_t1(R, Fe1, Fc6);
       } else if (a.stage == 2) {
         Uc[o] = rk_u2(u0, R, Feh, Fc2);
-        tot[o] = rk_tacc(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc(ttv[i], R, Feh, Fc3);
       } else if (a.stage == 3) {
         Uc[o] = rk_u3(u0, R, Feh, Fc1);
-        tot[o] = rk_tacc(tot[o], R, Feh, Fc3);
+        tot[o] = rk_tacc(ttv[i], R, Feh, Fc3);
       } else {
-        const T un = rk_u4(u0, tot[o], R, Fe1, Fc6);
+        const T un = rk_u4(u0, ttv[i], R, Fe1, Fc6);
         if (i < 3) U0[o] = un;
         else T0[e] = un;
         health_mark(!isfinite(un), a.health);
