@@ -1490,7 +1490,7 @@ static int flux_ssf(ts_plan* p, const void* U, const double* radii, int n_radii,
   const bool sff = g.basis == TS_BASIS_SFF;
   const long long nb = 1 + 148 * 16;
   CKS(ensure_work(p, p->nS, 9));
-  CKS(ensure_scratch(p, (size_t)n_radii * nb));
+  CKS(ensure_scratch(p, (size_t)n_radii * (nb + 1)));
   // x, y sine letters of u (SSF: Vx = SCF, Vy = CSF, Vz = CCF; SFF: Vx = SFF, Vy = Vz = CFF,
   // no y letters), the giver has the same; the product u_j G_i (field 3 j + i) is a sine
   // series along an axis when exactly one factor is
@@ -1520,8 +1520,9 @@ static int flux_ssf(ts_plan* p, const void* U, const double* radii, int n_radii,
     CK(LAUNCH(p, ssf_flux_outside, g, p->P, U, radii[r], mx_out, my_out, p->dscr + r * nb, p->st));
   }
   std::vector<double> h(n_radii);
-  for (int r = 0; r < n_radii; ++r)
-    CK(cudaMemcpyAsync(&h[r], p->dscr + r * nb, sizeof(double), cudaMemcpyDeviceToHost, p->st));
+  double* res = p->dscr + n_radii * nb;
+  CK(LAUNCH(p, flux_finish, g, p->dscr, nb, n_radii, res, p->st));
+  CK(cudaMemcpyAsync(h.data(), res, n_radii * sizeof(double), cudaMemcpyDeviceToHost, p->st));
   CK(cudaStreamSynchronize(p->st));
   for (int r = 0; r < n_radii; ++r) Pi[r] = -h[r];
   return TS_OK;
@@ -1537,7 +1538,7 @@ static int flux_sss(ts_plan* p, const void* U, const double* radii, int n_radii,
   const Geo gy = y_as_x(g);
   const long long nb = 1 + 148 * 16;
   CKS(ensure_work(p, p->nS, 9));
-  CKS(ensure_scratch(p, (size_t)n_radii * nb));
+  CKS(ensure_scratch(p, (size_t)n_radii * (nb + 1)));
   const int vx[3] = {1, 0, 0}, vy[3] = {0, 1, 0}, vz[3] = {0, 0, 1};
   int mx_in = 0, my_in = 0, mz_in = 0, mx_out = 0, my_out = 0, mz_out = 0;
   for (int c = 0; c < 3; ++c) {
@@ -1561,8 +1562,9 @@ static int flux_sss(ts_plan* p, const void* U, const double* radii, int n_radii,
     CK(LAUNCH(p, sss_flux_outside, g, p->P, U, radii[r], mx_out, my_out, mz_out, p->dscr + r * nb, p->st));
   }
   std::vector<double> h(n_radii);
-  for (int r = 0; r < n_radii; ++r)
-    CK(cudaMemcpyAsync(&h[r], p->dscr + r * nb, sizeof(double), cudaMemcpyDeviceToHost, p->st));
+  double* res = p->dscr + n_radii * nb;
+  CK(LAUNCH(p, flux_finish, g, p->dscr, nb, n_radii, res, p->st));
+  CK(cudaMemcpyAsync(h.data(), res, n_radii * sizeof(double), cudaMemcpyDeviceToHost, p->st));
   CK(cudaStreamSynchronize(p->st));
   for (int r = 0; r < n_radii; ++r) Pi[r] = -h[r];
   return TS_OK;
@@ -1621,17 +1623,21 @@ int ts_flux(ts_plan* p, const void* u_hat, const double* radii, int n_radii, dou
     // the giver nonlinear term N_i = sum_j D_j F[u_j G_i] (Compute_nlin(U, Giver)) and
     // Pi(R) = -sum_{|K| > R} 2 mult Re(N . conj(D U))
     CKS(ensure_work(p, p->nS, 9));
-    CKS(ensure_scratch(p, (size_t)n_radii * nb));
+    CKS(ensure_scratch(p, (size_t)n_radii * (nb + 1)));
+    // u is the same for every sphere: its x and y inverses once, into the stage field
+    CK(LAUNCH(p, inv_x, g, 0, U, p->Ucur, p->twx, nullptr, 0.0, p->st));
+    CK(LAUNCH(p, strided, g, 1, +1, p->Ucur, 3, p->twy, p->st));
     for (int i = 0; i < n_radii; ++i) {
       CK(LAUNCH(p, inv_x, g, 5, U, p->P, p->twx, nullptr, 0.0, p->st, 0, radii[i]));
-      CK(LAUNCH(p, strided, g, 1, +1, p->P, 6, p->twy, p->st));
-      CK(LAUNCH(p, z_fused, g, 6, p->P, p->twz, p->err_d, p->st));
+      CK(LAUNCH(p, strided, g, 1, +1, (char*)p->P + 3 * g.S * (long long)p->cb, 3, p->twy, p->st));
+      CK(LAUNCH(p, z_fused, g, 6, p->P, p->twz, p->err_d, p->st, 1, 0, -1, p->Ucur));
       CK(LAUNCH(p, strided, g, 1, -1, p->P, 9, p->twy, p->st));
       CK(LAUNCH(p, strided, g, 0, -1, p->P, 9, p->twx, p->st));
       CK(LAUNCH(p, flux_outside, g, p->P, U, radii[i], p->dscr + i * nb, p->st));
     }
-    for (int i = 0; i < n_radii; ++i)
-      CK(cudaMemcpyAsync(&h[i], p->dscr + i * nb, sizeof(double), cudaMemcpyDeviceToHost, p->st));
+    double* res = p->dscr + n_radii * nb;
+    CK(LAUNCH(p, flux_finish, g, p->dscr, nb, n_radii, res, p->st));
+    CK(cudaMemcpyAsync(h.data(), res, n_radii * sizeof(double), cudaMemcpyDeviceToHost, p->st));
     CK(cudaStreamSynchronize(p->st));
     for (int i = 0; i < n_radii; ++i) Pi[i] = -h[i];
     return (int)TS_OK;

@@ -273,14 +273,28 @@ __device__ __forceinline__ void pass_compute(V* v, int t, const V* __restrict__ 
   }
 }
 
-// padded shared-memory row index: one spare slot every 16 complex values keeps
-// the threads of a line (consecutive rows E apart) on distinct banks
-template <bool PAD> __device__ __forceinline__ int prow(int r) { return PAD ? r + (r >> 4) : r; }
-// exchange row of logical row r: padded (PAD), or with bit 0 flipped by bit SWK
-// (SWK > 0; a permutation of the rows) so that rows 2^SWK apart, which one
-// radix pass stores from neighbouring threads, land on different bank pairs
-template <bool PAD, int SWK> __device__ __forceinline__ int xrow(int r) {
-  return SWK > 0 ? (r ^ ((r >> SWK) & 1)) : prow<PAD>(r);
+// Shared-memory index of logical row r of an exchange.  PAD modes:
+//   0  r
+//   1  one spare slot every 16 complex values
+//   2  one spare slot every 8
+//   3  lines of 128 points and more, 8 elements per thread, FP32: the padding that leaves the
+//      exchange at hand without bank conflicts (KIND, all with offsets known at compile time):
+//      0 after the first pass: one spare slot every 16; 1 between later passes: two every 16;
+//      2 before a last pass of radix 2 or 4: one every 16 and four every 64.
+//      With mode 1 the stores of KIND 1 and 2 took twice the wavefronts, and the shared-memory
+//      pipe bounds the z pass (88 % busy at 256^3, B200)
+template <int PAD, int KIND = 0> __device__ __forceinline__ int prow(int r) {
+  return PAD == 0   ? r
+         : PAD == 2 ? r + (r >> 3)
+         : PAD == 3 && KIND == 1 ? r + 2 * (r >> 4)
+         : PAD == 3 && KIND == 2 ? r + (r >> 4) + 4 * (r >> 6)
+                                 : r + (r >> 4);
+}
+// the same with SWK > 0: bit 0 flipped by bit SWK (a permutation of the rows), so that rows
+// 2^SWK apart, which one radix pass stores from neighbouring threads, land on different
+// bank pairs
+template <int PAD, int SWK, int KIND = 0> __device__ __forceinline__ int xrow(int r) {
+  return SWK > 0 ? (r ^ ((r >> SWK) & 1)) : prow<PAD, KIND>(r);
 }
 
 // Full FFT of one line whose E-element slice per thread is in registers (loaded
@@ -288,7 +302,7 @@ template <bool PAD, int SWK> __device__ __forceinline__ int xrow(int r) {
 // `sm` addressed as sm[row*rs + cs] (caller supplies the per-thread column
 // offset cs and the row stride rs).  All threads of the block must call it.
 // On return v[s] holds output row final_row(t, s).
-template <int L, int E, int DIR, int P = 0, bool PAD = false, bool REV = false, int SWK = 0, typename V>
+template <int L, int E, int DIR, int P = 0, int PAD = 0, bool REV = false, int SWK = 0, typename V>
 __device__ __forceinline__ void fft_regs(V* v, int t, V* sm, int rs, int cs, const V* __restrict__ tw, int tws) {
   pass_compute<L, E, P, DIR, REV>(v, t, tw, tws);
   if constexpr (P + 1 < npasses(L, E)) {
@@ -332,21 +346,22 @@ __device__ __forceinline__ void pass_compute_b(V (&v)[NB][E], int t, const V* __
     for (int b = 0; b < NB; ++b) DFT<R, DIR, V>::run(v[b] + q * R);
   }
 }
-template <int L, int E, int DIR, int NB, bool WARP, int P = 0, bool PAD = false, bool REV = false, int SWK = 0,
+template <int L, int E, int DIR, int NB, bool WARP, int P = 0, int PAD = 0, bool REV = false, int SWK = 0,
           typename V>
 __device__ __forceinline__ void fft_regs_b(V (&v)[NB][E], int t, V* sm, int slot, int rs, int cs,
                                            const V* __restrict__ tw, int tws) {
   pass_compute_b<L, E, P, DIR, REV, NB>(v, t, tw, tws);
   if constexpr (P + 1 < npasses(L, E)) {
+    constexpr int KIND = P == 0 && npasses(L, E) > 2 ? 0 : (radix_sched(L, E, P + 1, REV) < E ? 2 : 1);
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
-      for (int s = 0; s < E; ++s) sm[b * slot + xrow<PAD, SWK>(Pass<L, E, P, REV>::out_row(t, s)) * rs + cs] = v[b][s];
+      for (int s = 0; s < E; ++s) sm[b * slot + xrow<PAD, SWK, KIND>(Pass<L, E, P, REV>::out_row(t, s)) * rs + cs] = v[b][s];
     fft_sync<WARP>();
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
-      for (int s = 0; s < E; ++s) v[b][s] = sm[b * slot + xrow<PAD, SWK>(Pass<L, E, P + 1, REV>::in_row(t, s)) * rs + cs];
+      for (int s = 0; s < E; ++s) v[b][s] = sm[b * slot + xrow<PAD, SWK, KIND>(Pass<L, E, P + 1, REV>::in_row(t, s)) * rs + cs];
     fft_sync<WARP>();
     fft_regs_b<L, E, DIR, NB, WARP, P + 1, PAD, REV, SWK>(v, t, sm, slot, rs, cs, tw, tws);
   }
@@ -368,6 +383,17 @@ template <typename V> __device__ __forceinline__ void cp_async16(V* dst, const V
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// Start of a kernel that may be launched while its predecessor in the stream is still running
+// (programmatic stream serialization, launch_chain): waits until the predecessor has ended
+// and its writes are visible, then lets the successor be launched.  Without the launch
+// attribute both instructions do nothing.  Data that a predecessor writes is read through
+// plain pointers in these kernels (not const __restrict__, whose loads the compiler may take
+// for invariant and move up).
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // ---------------------------------------------------------------------------
 // Index maps
@@ -431,13 +457,16 @@ __device__ __forceinline__ double block_sum(double v) {
   return v;
 }
 
-// out[i] = sum over b = 0..nblocks-1 of part[b * n + i], b in increasing order:
-// the fixed-order final sum of per-block partial bins
+// out[i] = sum over b = 0..nblocks-1 of part[b * n + i], one warp per bin: lane l adds the
+// blocks l, l + 32, ... in increasing order, then warp_sum; an order fixed by nblocks (one
+// thread per bin took 46 us for the 592 blocks of the shell sums, a serial chain of loads)
 static __global__ void k_bins_finish(const double* __restrict__ part, int nblocks, int n, double* __restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31, nw = gridDim.x * blockDim.x / 32;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) / 32; i < n; i += nw) {
     double s = 0;
-    for (int b = 0; b < nblocks; ++b) s += part[(long long)b * n + i];
-    out[i] = s;
+    for (int b = lane; b < nblocks; b += 32) s += part[(long long)b * n + i];
+    s = warp_sum(s);
+    if (lane == 0) out[i] = s;
   }
 }
 

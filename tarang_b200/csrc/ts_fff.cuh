@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(CW * (L / E), (CW * (L / E)) <= 256 ? 2 : 1)
     // each thread read back only what it staged itself; the barrier is for the
     // exchange writes into the consumed tile (NT = 2, 4)
     if (XC) __syncthreads();
-    fft_regs<L, E, DIR, 0, false, false, best_swk(L, E, CW, (int)sizeof(V))>(
+    fft_regs<L, E, DIR, 0, 0, false, best_swk(L, E, CW, (int)sizeof(V))>(
         v, t, XC ? stage + buf * L * CW : stage + 2 * L * CW, CW, c, tw, 1);
     if (ok) {
 #pragma unroll
@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(CW * (L / E), MINB)
     k_strided_ld(const C<T>* src, C<T>* dst, unsigned ntot, unsigned nplane, unsigned inner, long long fstride,
                  long long rstride, long long ostride, const C<T>* __restrict__ tw, unsigned per, long long mstride,
                  int zero_hi, T scl) {
+  chain_begin();
   typedef C<T> V;
   extern __shared__ __align__(16) unsigned char smraw[];
   V* xch = reinterpret_cast<V*>(smraw);
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(CW * (L / E), MINB)
     const int row = load_row<L, E>(t, s);
     v[s] = (ok && !(zero_hi && 3 * (row < L - row ? row : L - row) > L)) ? a[row * rstride] : mk<V>(0, 0);
   }
-  fft_regs<L, E, DIR, 0, false, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
+  fft_regs<L, E, DIR, 0, 0, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
   if (!ok) return;
   V* d = dst + off;
 #pragma unroll
@@ -162,122 +163,17 @@ __global__ void __launch_bounds__(CW * (L / E), MINB)
 }
 
 // ---------------------------------------------------------------------------
-// inverse x pass: W_i = IFFT_x(D(U_i)); rotational form also W_{3+i} = IFFT_x(D(omega_i)),
-// omega = i K x D(U).  col = ly*Hz + lz; row = lx.
-// Persistent over column tiles.  Thread 0 streams the three components of a
-// tile into shared memory with TMA (2-D boxes of CW columns x <=256 rows,
-// mbarrier completion), double buffered so tile k+1 loads while tile k is
-// transformed.  Shared memory: 2 x 3 staging tiles + 1 exchange tile.
+// inverse x pass, all output fields of a column tile in one block (tuning candidates; two
+// blocks of 256 threads per SM).
+// FORM 0: W_0..2 = D U.  FORM 1: also W_3..5 = D omega.
 // ---------------------------------------------------------------------------
-template <typename T, int L, int E, int CW, bool ROT>
-__global__ void __launch_bounds__(CW * (L / E), 1)
-    k_inv_x(const __grid_constant__ CUtensorMap mU, C<T>* __restrict__ W, Geo g, const C<T>* __restrict__ tw,
-            int* err) {
-  typedef C<T> V;
-  constexpr int TILE = L * CW, BR = L < 256 ? L : 256, UNITS = (int)sizeof(V) / 8;
-  extern __shared__ __align__(128) unsigned char smraw_[];
-  // TMA destinations: 128-byte aligned (the launcher adds 128 bytes of slack)
-  unsigned char* smraw = smraw_ + ((128 - (smem_u32(smraw_) & 127)) & 127);
-  V* stage = reinterpret_cast<V*>(smraw);  // [2][3][TILE]
-  V* xch = stage + 6 * TILE;
-  __shared__ __align__(8) uint64_t bar[2];
-  const int c = threadIdx.x % CW, t = threadIdx.x / CW;
-  const int inner = g.Ny * g.Hz;
-  const int ntiles = (inner + CW - 1) / CW;
-  const long long rstride = inner;
-  if (threadIdx.x == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  auto issue = [&](int tile, int slot) {
-    if (tile >= ntiles) return;
-    mbar_expect_tx(&bar[slot], 3u * TILE * (unsigned)sizeof(V));
-    for (int comp = 0; comp < 3; ++comp)
-      for (int r0 = 0; r0 < L; r0 += BR)
-        tma_load_2d(stage + (slot * 3 + comp) * TILE + r0 * CW, &mU, tile * CW * UNITS, comp * g.Nx + r0, &bar[slot]);
-  };
-  if (threadIdx.x == 0) {
-    issue(blockIdx.x, 0);
-    issue(blockIdx.x + gridDim.x, 1);
-  }
-  const int nout = ROT ? 6 : 3;
-  int k = 0;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++k) {
-    // slots alternate, so slot k & 1 completes its phase (k >> 1) & 1
-    const int slot = k & 1;
-    const uint32_t phase = (uint32_t)(k >> 1) & 1u;
-    const bool got = mbar_wait(&bar[slot], phase, err);
-    if (__syncthreads_or(!got)) {
-      // give every copy in flight (this tile's and the next tile's, issued into the
-      // other slot) a second bounded chance to land before the block's shared memory
-      // goes away, then leave
-      if (threadIdx.x == 0) {
-        mbar_wait(&bar[slot], phase, nullptr);
-        if (tile + (int)gridDim.x < ntiles) mbar_wait(&bar[slot ^ 1], (uint32_t)((k + 1) >> 1) & 1u, nullptr);
-      }
-      return;
-    }
-    const int col = tile * CW + c;
-    const bool ok = col < inner;
-    const int ly = ok ? col / g.Hz : 0, lz = ok ? col % g.Hz : 0;
-    const T Ky = (T)(kfft(ly, g.Ny) * g.kf[1]), Kz = (T)(lz * g.kf[2]);
-    const V* st = stage + slot * 3 * TILE + c;
-    for (int f = 0; f < nout; ++f) {
-      V v[E];
-#pragma unroll
-      for (int s = 0; s < E; ++s) {
-        const int lx = load_row<L, E>(t, s);
-        V a = mk<V>(0, 0);
-        if (ok && !dealias_zero(g.dealias, g.basis, lx, ly, lz, g.Nx, g.Ny, g.Nz)) {
-          if (f < 3) {
-            a = st[f * TILE + lx * CW];
-          } else {
-            // omega_i = i (K_{i+1} U_{i+2} - K_{i+2} U_{i+1})  (indices mod 3)
-            const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]);
-            const int i = f - 3, i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
-            const T Ka = i1 == 0 ? Kx : (i1 == 1 ? Ky : Kz);
-            const T Kb = i2 == 0 ? Kx : (i2 == 1 ? Ky : Kz);
-            const V ub = st[i2 * TILE + lx * CW], ua = st[i1 * TILE + lx * CW];
-            a = mul_i<1>(sub(scale(ub, Ka), scale(ua, Kb)));
-          }
-        }
-        v[s] = a;
-      }
-      if (f == nout - 1) {
-        // every thread has read this slot: refill it with the tile after next
-        __syncthreads();
-        if (threadIdx.x == 0) issue(tile + 2 * gridDim.x, slot);
-      }
-      fft_regs<L, E, 1, 0, false, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
-      if (ok) {
-        V* d = W + f * g.S + col;
-#pragma unroll
-        for (int s = 0; s < E; ++s) d[final_row<L, E>(t, s) * rstride] = v[s];
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// inverse x pass, direct-load variant (one column tile per block, loads straight
-// into registers; two blocks of 256 threads per SM).  Same result as k_inv_x.
-// FORM 0: W_0..2 = D U.  FORM 1: also W_3..5 = D omega.  FORM 3 (adjoint of the
-// rotational right-hand side): also W_6..8 = lsc c^-1 P Lam, the Leray-projected
-// cotangent divided by the C2R weight c (2 on the planes 0 < kz < Nz/2, else 1).
-// ---------------------------------------------------------------------------
-// FORM 4: the cotangent fields 6..8 of FORM 3 only (written at W + 6 S ...)
-// FORM 5 (the giver of the per-sphere energy flux): W_0..2 = D U and W_3..5 = D U
-// inside the sphere |K| <= rad (Fill_in_sphere, fill_space.cc:56-64), zero outside
-__host__ __device__ constexpr int inv_x_nout(int form) { return form == 0 ? 3 : ((form == 1 || form == 5) ? 6 : 9); }
-__host__ __device__ constexpr int inv_x_first(int form) { return form == 4 ? 6 : 0; }
+__host__ __device__ constexpr int inv_x_nout(int form) { return form == 0 ? 3 : 6; }
 
 template <typename T, int L, int E, int CW, int FORM>
 __global__ void __launch_bounds__(CW * (L / E), (CW * (L / E)) <= 256 ? 2 : 1)
-    k_inv_x_ld(const C<T>* __restrict__ U, C<T>* __restrict__ W, Geo g, const C<T>* __restrict__ tw,
-               const C<T>* __restrict__ Lam, T lsc, int kept, double rad) {
+    k_inv_x_ld(const C<T>* __restrict__ U, C<T>* __restrict__ W, Geo g, const C<T>* __restrict__ tw, int kept) {
   typedef C<T> V;
+  static_assert(FORM == 0 || FORM == 1, "the fluid forms");
   extern __shared__ __align__(16) unsigned char smraw[];
   V* sm = reinterpret_cast<V*>(smraw);
   const int c = threadIdx.x % CW, t = threadIdx.x / CW;
@@ -301,17 +197,10 @@ __global__ void __launch_bounds__(CW * (L / E), (CW * (L / E)) <= 256 ? 2 : 1)
   const T Ky = (T)(kfft(ly, g.Ny) * g.kf[1]), Kz = (T)(lz * g.kf[2]);
   const long long rstride = inner;
   constexpr int nout = inv_x_nout(FORM);
-  const T lw = (lz > 0 && 2 * lz < g.Nz) ? lsc * (T)0.5 : lsc;
-  // FORM 5: |K| <= rad with |K| = sqrt((Kx^2 + Ky^2) + Kz^2) in FP64 (Kmagnitude)
-  const double Kyd = kfft(ly, g.Ny) * g.kf[1], Kzd = lz * g.kf[2];
-  auto in_sphere = [&](int lx) {
-    const double Kxd = kfft(lx, g.Nx) * g.kf[0];
-    return sqrt((Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd) <= rad;
-  };
   // FP32 with up to 8 elements per thread: the three (dealiased) components of U
   // are loaded once, up front, and every output field is built from registers
   // (FP64 would spill them)
-  constexpr bool UPFRONT = E <= 8 && sizeof(T) == 4 && FORM != 4;
+  constexpr bool UPFRONT = E <= 8 && sizeof(T) == 4;
   V u[UPFRONT ? 3 : 1][UPFRONT ? E : 1];
   if constexpr (UPFRONT) {
 #pragma unroll
@@ -326,18 +215,16 @@ __global__ void __launch_bounds__(CW * (L / E), (CW * (L / E)) <= 256 ? 2 : 1)
   // unrolled (register path) so that the register-array indices below are compile-time constants
   constexpr int kUnroll = UPFRONT ? nout : 1;
 #pragma unroll kUnroll
-  for (int f = inv_x_first(FORM); f < nout; ++f) {
+  for (int f = 0; f < nout; ++f) {
     V v[E];
 #pragma unroll
     for (int s = 0; s < E; ++s) {
       const int lx = load_row<L, E>(t, s);
       const long long off = lx * rstride + col;
       V a = mk<V>(0, 0);
-      if (UPFRONT && f < 6) {
+      if (UPFRONT) {
         if (f < 3) {
           a = u[f][s];
-        } else if (FORM == 5) {
-          a = in_sphere(lx) ? u[f - 3][s] : mk<V>(0, 0);
         } else {
           const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]);
           const int i = f - 3, i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
@@ -345,23 +232,9 @@ __global__ void __launch_bounds__(CW * (L / E), (CW * (L / E)) <= 256 ? 2 : 1)
           const T Kb = i2 == 0 ? Kx : (i2 == 1 ? Ky : Kz);
           a = mul_i<1>(sub(scale(u[i2][s], Ka), scale(u[i1][s], Kb)));
         }
-      } else if ((FORM == 3 || FORM == 4) && f >= 6) {
-        if (ok) {
-          // (P Lam)_i = Lam_i - K_i (K . Lam) / K^2, identity at K = 0
-          const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]);
-          const V l0 = Lam[off], l1 = Lam[g.S + off], l2 = Lam[2 * g.S + off];
-          const T K2 = (Kx * Kx + Ky * Ky) + Kz * Kz;
-          const V d = add(add(scale(l0, Kx), scale(l1, Ky)), scale(l2, Kz));
-          const V q = K2 > (T)0 ? mk<V>(d.x / K2, d.y / K2) : mk<V>(0, 0);
-          const int i = f - 6;
-          const T Ki = i == 0 ? Kx : (i == 1 ? Ky : Kz);
-          a = scale(sub(i == 0 ? l0 : (i == 1 ? l1 : l2), scale(q, Ki)), lw);
-        }
       } else if (ok && !dealias_zero(g.dealias, g.basis, lx, ly, lz, g.Nx, g.Ny, g.Nz)) {
         if (f < 3) {
           a = U[f * g.S + off];
-        } else if (FORM == 5) {
-          a = in_sphere(lx) ? U[(f - 3) * g.S + off] : mk<V>(0, 0);
         } else {
           // omega_i = i (K_{i+1} U_{i+2} - K_{i+2} U_{i+1})  (indices mod 3)
           const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]);
@@ -374,7 +247,7 @@ __global__ void __launch_bounds__(CW * (L / E), (CW * (L / E)) <= 256 ? 2 : 1)
       }
       v[s] = a;
     }
-    fft_regs<L, E, 1, 0, false, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, sm, CW, c, tw, 1);
+    fft_regs<L, E, 1, 0, 0, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, sm, CW, c, tw, 1);
     if (ok) {
       V* d = W + f * g.S + col;
 #pragma unroll
@@ -386,13 +259,14 @@ __global__ void __launch_bounds__(CW * (L / E), (CW * (L / E)) <= 256 ? 2 : 1)
 
 // ---------------------------------------------------------------------------
 // inverse x pass, one output field per block: every row is loaded straight into registers
-// (as in k_strided_ld), a vorticity row is combined from the two components it needs, a
-// projected cotangent row from three.  The input components are read once per output field
+// (as in k_strided_ld), a vorticity row is combined from the two components it needs.  The input components are read once per output field
 // that needs them; the blocks of a column tile's fields are neighbours (field fastest), so
 // all but the first read hit L2.  16 elements per thread and one field keep it at 64-80
 // registers and 24-32 warps per SM, where the form with all fields of a tile in one block
 // (k_inv_x_ld) holds U in registers, 8 elements per thread and 16 warps.
-// Fields and FORMs as k_inv_x_ld (FORM 0, 1, 4, 5).
+// FORM 0: W_0..2 = D U.  FORM 1: also W_3..5 = D omega.  FORM 5 (the giver of the per-sphere
+// energy flux): W_3..5 = D U inside the sphere |K| <= R (Fill_in_sphere, fill_space.cc:56-64),
+// zero outside.
 // ---------------------------------------------------------------------------
 // rows [lo, hi) of the column (ly, lz) are cleared by dealiasing (dealias_zero, basis 0)
 __device__ __forceinline__ void fff_zero_rows(int mode, int ly, int lz, int Nx, int Ny, int Nz, int& lo, int& hi) {
@@ -408,11 +282,12 @@ __device__ __forceinline__ void fff_zero_rows(int mode, int ly, int lz, int Nx, 
 
 template <typename T, int L, int E, int CW, int FORM, int MINB>
 __global__ void __launch_bounds__(CW * (L / E), MINB)
-    k_inv_x_f(const C<T>* __restrict__ U, C<T>* __restrict__ W, Geo g, const C<T>* __restrict__ tw,
-              const C<T>* __restrict__ Lam, T lsc, int kept, double rad) {
+    k_inv_x_f(const C<T>* U, C<T>* W, Geo g, const C<T>* __restrict__ tw,
+              int kept, double K2max) {
+  chain_begin();
   typedef C<T> V;
-  static_assert(FORM == 0 || FORM == 1 || FORM == 4 || FORM == 5, "fluid forms, cotangent, flux giver");
-  constexpr unsigned NF = FORM == 1 || FORM == 5 ? 6 : 3;
+  static_assert(FORM == 0 || FORM == 1 || FORM == 5, "fluid forms, flux giver");
+  constexpr unsigned NF = FORM == 1 ? 6 : 3;
   extern __shared__ __align__(16) unsigned char smraw[];
   V* xch = reinterpret_cast<V*>(smraw);
   const int c = threadIdx.x % CW, t = threadIdx.x / CW;
@@ -437,136 +312,88 @@ __global__ void __launch_bounds__(CW * (L / E), MINB)
   const long long col = (long long)ly * g.Hz + lz, rstride = inner;
   const T Ky = (T)(kfft(ly, g.Ny) * g.kf[1]), Kz = (T)(lz * g.kf[2]);
   V v[E];
-  if constexpr (FORM == 4) {
-    // (P Lam)_i = Lam_i - K_i (K . Lam) / K^2, identity at K = 0
-    const T lw = (lz > 0 && 2 * (int)lz < g.Nz) ? lsc * (T)0.5 : lsc;
+  int zlo, zhi;
+  fff_zero_rows(g.dealias, ly, lz, g.Nx, g.Ny, g.Nz, zlo, zhi);
+  if (!ok) zlo = 0, zhi = L;
+  if (FORM != 1 || f < 3) {
+    const V* src = U + f * g.S + col;
 #pragma unroll
     for (int s = 0; s < E; ++s) {
       const int lx = load_row<L, E>(t, s);
-      const long long off = lx * rstride + col;
-      const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]);
-      v[s] = mk<V>(0, 0);
-      if (ok) {
-        const V l0 = Lam[off], l1 = Lam[g.S + off], l2 = Lam[2 * g.S + off];
-        const T K2 = (Kx * Kx + Ky * Ky) + Kz * Kz;
-        const V d = add(add(scale(l0, Kx), scale(l1, Ky)), scale(l2, Kz));
-        const V p = K2 > (T)0 ? mk<V>(d.x / K2, d.y / K2) : mk<V>(0, 0);
-        v[s] = scale(f == 0 ? sub(l0, scale(p, Kx)) : f == 1 ? sub(l1, scale(p, Ky)) : sub(l2, scale(p, Kz)), lw);
+      v[s] = (lx >= zlo && lx < zhi) ? mk<V>(0, 0) : src[lx * rstride];
+    }
+    if (FORM == 5) {
+      // inside |K| <= rad: (Kx^2 + Ky^2) + Kz^2 <= K2max in FP64 (Kmagnitude)
+      const double Kyd = kfft(ly, g.Ny) * g.kf[1], Kzd = lz * g.kf[2];
+#pragma unroll
+      for (int s = 0; s < E; ++s) {
+        const double Kxd = kfft(load_row<L, E>(t, s), g.Nx) * g.kf[0];
+        if (!((Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd <= K2max)) v[s] = mk<V>(0, 0);
       }
     }
   } else {
-    int zlo, zhi;
-    fff_zero_rows(g.dealias, ly, lz, g.Nx, g.Ny, g.Nz, zlo, zhi);
-    if (!ok) zlo = 0, zhi = L;
-    if (FORM == 0 || f < 3 || FORM == 5) {
-      const V* src = U + (f < 3 ? f : f - 3) * g.S + col;
+    // omega_i = i (K_{i+1} U_{i+2} - K_{i+2} U_{i+1})  (indices mod 3)
+    const int i = (int)f - 3, i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
+    const V *sa = U + i1 * g.S + col, *sb = U + i2 * g.S + col;
 #pragma unroll
-      for (int s = 0; s < E; ++s) {
-        const int lx = load_row<L, E>(t, s);
-        v[s] = (lx >= zlo && lx < zhi) ? mk<V>(0, 0) : src[lx * rstride];
-      }
-      if (FORM == 5 && f >= 3) {
-        // inside |K| <= rad with |K| = sqrt((Kx^2 + Ky^2) + Kz^2) in FP64 (Kmagnitude)
-        const double Kyd = kfft(ly, g.Ny) * g.kf[1], Kzd = lz * g.kf[2];
-#pragma unroll
-        for (int s = 0; s < E; ++s) {
-          const double Kxd = kfft(load_row<L, E>(t, s), g.Nx) * g.kf[0];
-          if (!(sqrt((Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd) <= rad)) v[s] = mk<V>(0, 0);
-        }
-      }
-    } else {
-      // omega_i = i (K_{i+1} U_{i+2} - K_{i+2} U_{i+1})  (indices mod 3)
-      const int i = (int)f - 3, i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
-      const V *sa = U + i1 * g.S + col, *sb = U + i2 * g.S + col;
-#pragma unroll
-      for (int s = 0; s < E; ++s) {
-        const int lx = load_row<L, E>(t, s);
-        const bool z = lx >= zlo && lx < zhi;
-        const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]);
-        const T Ka = i1 == 0 ? Kx : (i1 == 1 ? Ky : Kz), Kb = i2 == 0 ? Kx : (i2 == 1 ? Ky : Kz);
-        const V ua = z ? mk<V>(0, 0) : sa[lx * rstride], ub = z ? mk<V>(0, 0) : sb[lx * rstride];
-        v[s] = mul_i<1>(sub(scale(ub, Ka), scale(ua, Kb)));
-      }
+    for (int s = 0; s < E; ++s) {
+      const int lx = load_row<L, E>(t, s);
+      const bool z = lx >= zlo && lx < zhi;
+      const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]);
+      const T Ka = i1 == 0 ? Kx : (i1 == 1 ? Ky : Kz), Kb = i2 == 0 ? Kx : (i2 == 1 ? Ky : Kz);
+      const V ua = z ? mk<V>(0, 0) : sa[lx * rstride], ub = z ? mk<V>(0, 0) : sb[lx * rstride];
+      v[s] = mul_i<1>(sub(scale(ub, Ka), scale(ua, Kb)));
     }
   }
-  fft_regs<L, E, 1, 0, false, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
+  fft_regs<L, E, 1, 0, 0, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
   if (!ok) return;
-  V* d = W + (f + (FORM == 4 ? 6 : 0)) * g.S + col;
+  V* d = W + (f + (FORM == 5 ? 3 : 0)) * g.S + col;
 #pragma unroll
   for (int s = 0; s < E; ++s) d[final_row<L, E>(t, s) * rstride] = v[s];
 }
 
 // ---------------------------------------------------------------------------
-// inverse x pass with the tile's U staged in shared memory (two-thirds dealiasing,
-// FORM 0 / 1): one column tile per block (the kept-column mapping of k_inv_x_ld); every
-// thread stages the kept rows (3 |kx| <= Nx) of the three components that it will read
-// itself with cp.async, all in one group, so a tile pays one load latency instead of one
-// per output field; the output fields are then built from shared memory (the vorticity
-// from the staged components) and transformed through a separate exchange tile.
-// Shared memory: 3 x LK x CW staged complex (LK = 2 (L/3) + 1 kept rows) + L x CW exchange.
+// inverse x pass of the adjoint's cotangent: W_6..8 = IFFT_x(lsc c^-1 P Lam), the
+// Leray-projected cotangent divided by the C2R weight c (2 on the planes 0 < kz < Nz/2, else
+// 1).  The three components of a column stay in registers from the projection (one
+// division per mode) to their transforms, one after the other through one exchange tile.
 // ---------------------------------------------------------------------------
-template <int L> __host__ __device__ constexpr int ix_kept_rows() { return 2 * (L / 3) + 1; }
-template <typename T, int L, int E, int CW, int FORM, int MINB = 1>
+template <typename T, int L, int E, int CW, int MINB>
 __global__ void __launch_bounds__(CW * (L / E), MINB)
-    k_inv_x_st(const C<T>* __restrict__ U, C<T>* __restrict__ W, Geo g, const C<T>* __restrict__ tw) {
+    k_inv_x_cot(const C<T>* Lam, C<T>* W, Geo g, const C<T>* __restrict__ tw, T lsc) {
+  chain_begin();
   typedef C<T> V;
-  static_assert(FORM == 0 || FORM == 1, "the fluid forms");
-  constexpr int LK = ix_kept_rows<L>(), Q = L / 3;
   extern __shared__ __align__(16) unsigned char smraw[];
-  V* xch = reinterpret_cast<V*>(smraw);  // exchange tile, L x CW
-  V* stg = xch + L * CW;                  // staged kept rows, 3 x LK x CW
+  V* xch = reinterpret_cast<V*>(smraw);
   const int c = threadIdx.x % CW, t = threadIdx.x / CW;
-  const int inner = g.Ny * g.Hz;
-  const long long rstride = inner;
-  // the kept columns as one run, so no tile is cut at the end of a kept row
-  const unsigned qy = g.Ny / 3, nzk = g.Nz / 3 + 1, q0 = blockIdx.x * CW + c, iy0 = q0 / nzk;
-  const bool ok = iy0 <= 2 * qy;
-  const int iy = ok ? iy0 : 0, lz = ok ? q0 - iy0 * nzk : 0;
-  const int ky = iy <= (int)qy ? iy : iy - (int)(2 * qy + 1);
-  const int col = (ky < 0 ? ky + g.Ny : ky) * g.Hz + lz;
-  const T Ky = (T)(ky * g.kf[1]), Kz = (T)(lz * g.kf[2]);
-  // staged row of x row lx (kept rows only: lx <= Q or lx >= L - Q)
-  auto krow = [](int lx) { return lx <= Q ? lx : lx - (L - 2 * Q - 1); };
-  auto kept = [](int lx) { return lx <= Q || lx >= L - Q; };
-  if (ok) {
+  const unsigned inner = g.Ny * g.Hz, q = blockIdx.x * CW + c;
+  const bool ok = q < inner;
+  const unsigned ly = ok ? q / g.Hz : 0, lz = ok ? q - ly * g.Hz : 0;
+  const long long col = (long long)ly * g.Hz + lz, rstride = inner;
+  const T Ky = (T)(kfft(ly, g.Ny) * g.kf[1]), Kz = (T)(lz * g.kf[2]);
+  const T lw = (lz > 0 && 2 * (int)lz < g.Nz) ? lsc * (T)0.5 : lsc;
+  V v[3][E];
 #pragma unroll
-    for (int s = 0; s < E; ++s) {
-      const int lx = load_row<L, E>(t, s);
-      if (kept(lx))
+  for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int q = 0; q < 3; ++q) cp_async(stg + (q * LK + krow(lx)) * CW + c, U + q * g.S + lx * rstride + col);
-    }
+    for (int s = 0; s < E; ++s) v[i][s] = ok ? Lam[i * g.S + load_row<L, E>(t, s) * rstride + col] : mk<V>(0, 0);
+#pragma unroll
+  for (int s = 0; s < E; ++s) {
+    // (P Lam)_i = Lam_i - K_i (K . Lam) / K^2, identity at K = 0
+    const T Kx = (T)(kfft(load_row<L, E>(t, s), g.Nx) * g.kf[0]);
+    const T K2 = (Kx * Kx + Ky * Ky) + Kz * Kz, r = K2 > (T)0 ? (T)1 / K2 : (T)0;
+    const V d = scale(add(add(scale(v[0][s], Kx), scale(v[1][s], Ky)), scale(v[2][s], Kz)), r);
+    v[0][s] = scale(sub(v[0][s], scale(d, Kx)), lw);
+    v[1][s] = scale(sub(v[1][s], scale(d, Ky)), lw);
+    v[2][s] = scale(sub(v[2][s], scale(d, Kz)), lw);
   }
-  cp_async_commit();
-  cp_async_wait<0>();  // each thread reads back only the rows it staged itself
-  constexpr int nout = FORM == 0 ? 3 : 6;
-#pragma unroll 1
-  for (int f = 0; f < nout; ++f) {
-    V v[E];
 #pragma unroll
-    for (int s = 0; s < E; ++s) {
-      const int lx = load_row<L, E>(t, s);
-      V a = mk<V>(0, 0);
-      if (ok && kept(lx)) {
-        const V* st = stg + krow(lx) * CW + c;
-        if (f < 3) {
-          a = st[f * LK * CW];
-        } else {
-          // omega_i = i (K_{i+1} U_{i+2} - K_{i+2} U_{i+1})  (indices mod 3)
-          const T Kx = (T)(kfft(lx, g.Nx) * g.kf[0]);
-          const int i = f - 3, i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
-          const T Ka = i1 == 0 ? Kx : (i1 == 1 ? Ky : Kz);
-          const T Kb = i2 == 0 ? Kx : (i2 == 1 ? Ky : Kz);
-          a = mul_i<1>(sub(scale(st[i2 * LK * CW], Ka), scale(st[i1 * LK * CW], Kb)));
-        }
-      }
-      v[s] = a;
-    }
-    fft_regs<L, E, 1, 0, false, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
+  for (int i = 0; i < 3; ++i) {
+    fft_regs<L, E, 1, 0, 0, false, best_swk(L, E, CW, (int)sizeof(V))>(v[i], t, xch, CW, c, tw, 1);
     if (ok) {
-      V* d = W + f * g.S + col;
+      V* d = W + (6 + i) * g.S + col;
 #pragma unroll
-      for (int s = 0; s < E; ++s) d[final_row<L, E>(t, s) * rstride] = v[s];
+      for (int s = 0; s < E; ++s) d[final_row<L, E>(t, s) * rstride] = v[i][s];
     }
   }
 }
@@ -658,7 +485,7 @@ __global__ void __launch_bounds__(CW * (L / E), 1)
           v[s] = mul_i<1>(sub(scale(u[i2][s], Ka), scale(u[i1][s], Kb)));
         }
       }
-      fft_regs<L, E, 1, 0, false, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
+      fft_regs<L, E, 1, 0, 0, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
       if (ok) {
         V* d = W + f * g.S + col;
 #pragma unroll
@@ -770,14 +597,14 @@ __global__ void __launch_bounds__(256) k_z_fused(C<T>* __restrict__ P, Geo g, co
       v[s] = add(add(a, b), mul_i<1>(mul(conjg(tw[k]), sub(a, b))));
     }
     V* sl = slot(c, l < nl ? l : 0);
-    fft_regs<M, E, 1, 0, true>(v, t, sl, 1, 0, tw, 2);
+    fft_regs<M, E, 1, 0, 1>(v, t, sl, 1, 0, tw, 2);
 #pragma unroll
-    for (int s = 0; s < E; ++s) sl[prow<true>(final_row<M, E>(t, s))] = v[s];
+    for (int s = 0; s < E; ++s) sl[prow<1>(final_row<M, E>(t, s))] = v[s];
   }
   __syncthreads();
   // B. products, in place per real point pair
   for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
-    const int ll = e / M, m = prow<true>(e % M);
+    const int ll = e / M, m = prow<1>(e % M);
     V in[NIN];
 #pragma unroll
     for (int c = 0; c < NIN; ++c) in[c] = slot(c, ll)[m];
@@ -799,18 +626,18 @@ __global__ void __launch_bounds__(256) k_z_fused(C<T>* __restrict__ P, Geo g, co
     V* sl = slot(c, l < nl ? l : 0);
     V v[E];
 #pragma unroll
-    for (int s = 0; s < E; ++s) v[s] = sl[prow<true>(load_row<M, E>(t, s))];
+    for (int s = 0; s < E; ++s) v[s] = sl[prow<1>(load_row<M, E>(t, s))];
     __syncthreads();
-    fft_regs<M, E, -1, 0, true>(v, t, sl, 1, 0, tw, 2);
+    fft_regs<M, E, -1, 0, 1>(v, t, sl, 1, 0, tw, 2);
 #pragma unroll
-    for (int s = 0; s < E; ++s) sl[prow<true>(final_row<M, E>(t, s))] = v[s];
+    for (int s = 0; s < E; ++s) sl[prow<1>(final_row<M, E>(t, s))] = v[s];
     __syncthreads();
     V* dst = P + c * g.S + line0 * H;
     for (int e = threadIdx.x; e < nh * H; e += blockDim.x) {
       const int ll = e / H, k = e % H;
       const V* z = slot(c, ll);
-      const V Z = z[prow<true>(k == M ? 0 : k)];
-      const V Zp = conjg(z[prow<true>(k == 0 ? 0 : M - k)]);
+      const V Z = z[prow<1>(k == M ? 0 : k)];
+      const V Zp = conjg(z[prow<1>(k == 0 ? 0 : M - k)]);
       const V s = scale(add(Z, Zp), (T)0.5);
       const V d = mul_i<-1>(mul(tw[k], scale(sub(Z, Zp), (T)0.5)));
       dst[e] = add(s, d);
@@ -887,7 +714,7 @@ __device__ __forceinline__ void zreg_inverse_loaded(const C<T>* X, bool live, in
     if (k == 0) { x.y = 0; b.y = 0; }
     out[s] = add(add(x, b), mul_i<1>(mul(conjg(tw[k]), sub(x, b))));
   }
-  fft_regs<M, E, 1, 0, true, false>(out, t, xch, 1, 0, tw, 2);
+  fft_regs<M, E, 1, 0, 1, false>(out, t, xch, 1, 0, tw, 2);
 #pragma unroll
   for (int s = 0; s < E; ++s) a[s] = out[s];
 }
@@ -908,11 +735,11 @@ __device__ __forceinline__ void zreg_forward_store(C<T> (&p)[E], C<T>* Xo, bool 
                                                    const C<T>* __restrict__ tw, C<T>* xch) {
   typedef C<T> V;
   constexpr bool SH = zreg_shfl<M, E, TPL>();
-  fft_regs<M, E, -1, 0, true, true>(p, t, xch, 1, 0, tw, 2);
+  fft_regs<M, E, -1, 0, 1, true>(p, t, xch, 1, 0, tw, 2);
   // X[k] = 1/2 (Z + Z') - i/2 w^k (Z - Z'), Z' = conj(Z[M-k]), Z[M] = Z[0]
   if constexpr (!SH) {
 #pragma unroll
-    for (int s = 0; s < E; ++s) xch[prow<true>(final_row<M, E, true>(t, s))] = p[s];
+    for (int s = 0; s < E; ++s) xch[prow<1>(final_row<M, E, true>(t, s))] = p[s];
     __syncthreads();
   }
 #pragma unroll
@@ -924,7 +751,7 @@ __device__ __forceinline__ void zreg_forward_store(C<T> (&p)[E], C<T>* Xo, bool 
       zp.y = __shfl_sync(0xffffffffu, p[E - 1 - s].y, partner);
       if (t == 0) zp = p[(E - s) % E];
     } else {
-      zp = xch[prow<true>((M - k) % M)];
+      zp = xch[prow<1>((M - k) % M)];
     }
     zp = conjg(zp);
     const V z = p[s];
@@ -954,7 +781,8 @@ template <int NZ, int EZ = 0, int FORM = 0> __host__ __device__ constexpr int zr
 // transform (one load latency per line instead of one per component)
 template <typename T, int NZ, int FORM, int EZ = 0, bool BATCH = false>
 __global__ void __launch_bounds__(zreg_threads<FORM>(), zreg_min_blocks<NZ, EZ, FORM>())
-    k_z_reg(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw, long long msP, int zkeep) {
+    k_z_reg(C<T>* P, Geo g, const C<T>* __restrict__ tw, long long msP, int zkeep) {
+  chain_begin();
   typedef C<T> V;
   constexpr int M = NZ / 2, H = M + 1, E = EZ ? EZ : ((M % 3 == 0) ? 12 : 8), TPL = M / E, LDX = zslot<M>();
   static_assert(TPL >= 1 && TPL <= 64, "a line spans at most two warps");
@@ -1025,7 +853,11 @@ __global__ void __launch_bounds__(zreg_threads<FORM>(), zreg_min_blocks<NZ, EZ, 
 template <typename T, int NZ, int E> __host__ __device__ constexpr bool zpair_shfl() {
   return radix_at(NZ, E, 0) == E && NZ / E <= 32 && E >= 2;
 }
-template <typename T> __host__ __device__ constexpr int zpair_slot(int NZ) { return NZ + NZ / 16 + 1; }
+// exchange rows of a pair (prow modes) and the complex values they take
+template <typename T> __host__ __device__ constexpr int zpair_pad(int NZ) {
+  return sizeof(T) == 4 && NZ >= 128 && NZ % 3 != 0 ? 3 : 2;
+}
+template <typename T> __host__ __device__ constexpr int zpair_slot(int NZ) { return NZ + NZ / 8; }
 
 // lines of exchange space per pair: the inputs go through it together, the products NB at a time
 __host__ __device__ constexpr int zpair_lines(int nin, int nb) { return nin > nb ? nin : nb; }
@@ -1091,11 +923,12 @@ __device__ __forceinline__ void zpair_load(const C<T>* X, long long cs, bool liv
 // forward transform of NB packed line pairs and the store of their rows 0 .. M
 template <typename T, int NZ, int E, int NB>
 __device__ __forceinline__ void zpair_forward_store(C<T> (&p)[NB][E], C<T>* X, long long cs, bool live0, bool live1,
-                                                    int t, int partner, const C<T>* __restrict__ tw, C<T>* xch) {
+                                                    int t, int partner, const C<T>* __restrict__ tw, C<T>* xch,
+                                                    int slot) {
   typedef C<T> V;
-  constexpr int M = NZ / 2, H = M + 1, TPL = NZ / E, LDX = zpair_slot<T>(NZ);
+  constexpr int M = NZ / 2, H = M + 1, TPL = NZ / E;
   constexpr bool WARP = TPL <= 32;
-  fft_regs_b<NZ, E, -1, NB, WARP, 0, true, true>(p, t, xch, LDX, 1, 0, tw, 1);
+  fft_regs_b<NZ, E, -1, NB, WARP, 0, zpair_pad<T>(NZ), true>(p, t, xch, slot, 1, 0, tw, 1);
   if constexpr (zpair_shfl<T, NZ, E>()) {
 #pragma unroll
     for (int f = 0; f < NB; ++f) {
@@ -1120,14 +953,14 @@ __device__ __forceinline__ void zpair_forward_store(C<T> (&p)[NB][E], C<T>* X, l
 #pragma unroll
     for (int f = 0; f < NB; ++f)
 #pragma unroll
-      for (int s = 0; s < E; ++s) xch[f * LDX + prow<true>(final_row<NZ, E, true>(t, s))] = p[f][s];
+      for (int s = 0; s < E; ++s) xch[f * slot + prow<zpair_pad<T>(NZ)>(final_row<NZ, E, true>(t, s))] = p[f][s];
     fft_sync<WARP>();
 #pragma unroll
     for (int f = 0; f < NB; ++f) {
       V* Xo = X + f * cs;
-      const V* zl = xch + f * LDX;
+      const V* zl = xch + f * slot;
       for (int k = t; k <= M; k += TPL) {
-        const V z = zl[prow<true>(k)], zp = zl[prow<true>((NZ - k) % NZ)];
+        const V z = zl[prow<zpair_pad<T>(NZ)>(k)], zp = zl[prow<zpair_pad<T>(NZ)>((NZ - k) % NZ)];
         if (live0) Xo[k] = mk<V>((T)0.5 * (z.x + zp.x), (T)0.5 * (z.y - zp.y));
         if (live1) Xo[H + k] = mk<V>((T)0.5 * (z.y + zp.y), (T)0.5 * (zp.x - z.x));
       }
@@ -1138,9 +971,10 @@ __device__ __forceinline__ void zpair_forward_store(C<T> (&p)[NB][E], C<T>* X, l
 
 template <typename T, int NZ, int E, int FORM, int NTHR, int MINB, int NB>
 __global__ void __launch_bounds__(NTHR, MINB)
-    k_z_pair(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw, long long msP, int zkeep) {
+    k_z_pair(C<T>* P, Geo g, const C<T>* __restrict__ tw, long long msP, int zkeep, const C<T>* Q) {
+  chain_begin();
   typedef C<T> V;
-  constexpr int H = NZ / 2 + 1, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ);
+  constexpr int H = NZ / 2 + 1, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ), SLOT = PPB * LDX;
   constexpr int NIN = z_nin(FORM), NOUT = z_nout(FORM);
   constexpr bool WARP = TPL <= 32;
   static_assert(NOUT % NB == 0 && NTHR % TPL == 0 && (!WARP || 32 % TPL == 0), "whole pairs per warp or block");
@@ -1152,12 +986,27 @@ __global__ void __launch_bounds__(NTHR, MINB)
   const long long nlines = (long long)g.Nx * g.Ny;
   const long long line = 2 * ((long long)blockIdx.x * PPB + l);
   const bool live0 = line < nlines, live1 = line + 1 < nlines;
-  V* xch = reinterpret_cast<V*>(smraw) + l * (zpair_lines(NIN, NB) * LDX);
+  V* xch = reinterpret_cast<V*>(smraw) + l * LDX;  // line f of the pair at f * SLOT
   V* Pl = P + (live0 ? line : 0) * H;
 
   V in[NIN][E];
-  zpair_load<T, NZ, E, NIN>(Pl, g.S, live0, live1, t, partner, zkeep, in);
-  fft_regs_b<NZ, E, 1, NIN, WARP, 0, true, false>(in, t, xch, LDX, 1, 0, tw, 1);
+  if constexpr (FORM == 6) {
+    // u from Q (transformed once for all spheres), the giver from P
+    const V* Ql = Q + (live0 ? line : 0) * H;
+    V a[3][E], b[3][E];
+    zpair_load<T, NZ, E, 3>(Ql, g.S, live0, live1, t, partner, zkeep, a);
+    zpair_load<T, NZ, E, 3>(Pl + 3 * g.S, g.S, live0, live1, t, partner, zkeep, b);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int s = 0; s < E; ++s) {
+        in[c][s] = a[c][s];
+        in[c + 3][s] = b[c][s];
+      }
+  } else {
+    zpair_load<T, NZ, E, NIN>(Pl, g.S, live0, live1, t, partner, zkeep, in);
+  }
+  fft_regs_b<NZ, E, 1, NIN, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
 #pragma unroll
   for (int f0 = 0; f0 < NOUT; f0 += NB) {
     V p[NB][E];
@@ -1170,57 +1019,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
         for (int c = 0; c < NIN; ++c) q[c] = in[c][s];
         p[f][s] = z_product<FORM>(f0 + f, q);
       }
-    zpair_forward_store<T, NZ, E, NB>(p, Pl + f0 * g.S, g.S, live0, live1, t, partner, tw, xch);
-  }
-}
-
-// line pairs, the points of the components in shared memory: component c is transformed
-// while the rows of component c + 1 are on their way, its points wait in slots that only
-// their own thread reads, and each product is formed from them as it is transformed.  One
-// component and one product are in registers at a time, so twice the warps of k_z_pair fit.
-template <typename T, int NZ, int E, int FORM, int NTHR, int MINB>
-__global__ void __launch_bounds__(NTHR, MINB)
-    k_z_pair_s(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw, long long msP, int zkeep) {
-  typedef C<T> V;
-  constexpr int H = NZ / 2 + 1, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ);
-  constexpr int NIN = z_nin(FORM), NOUT = z_nout(FORM);
-  constexpr bool WARP = TPL <= 32;
-  static_assert(NTHR % TPL == 0 && (!WARP || 32 % TPL == 0), "whole pairs per warp or block");
-  extern __shared__ __align__(16) unsigned char smraw[];
-  P += blockIdx.y * msP;  // member blockIdx.y
-  const int l = threadIdx.x / TPL, t = threadIdx.x % TPL;
-  const int lane = threadIdx.x & 31;
-  const int partner = (lane - t) + (TPL - t) % TPL;  // lane holding the rows N - k
-  const long long nlines = (long long)g.Nx * g.Ny;
-  const long long line = 2 * ((long long)blockIdx.x * PPB + l);
-  const bool live0 = line < nlines, live1 = line + 1 < nlines;
-  V* xch = reinterpret_cast<V*>(smraw) + l * LDX;
-  V* pts = reinterpret_cast<V*>(smraw) + PPB * LDX + threadIdx.x;  // point s of component c at (c E + s) NTHR
-  V* Pl = P + (live0 ? line : 0) * H;
-  V in[1][E], nx[1][E];
-  zpair_load<T, NZ, E, 1>(Pl, g.S, live0, live1, t, partner, zkeep, in);
-#pragma unroll
-  for (int c = 0; c < NIN; ++c) {
-    if (c + 1 < NIN) zpair_load<T, NZ, E, 1>(Pl + (c + 1) * g.S, g.S, live0, live1, t, partner, zkeep, nx);
-    fft_regs_b<NZ, E, 1, 1, WARP, 0, true, false>(in, t, xch, LDX, 1, 0, tw, 1);
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-      pts[(c * E + s) * NTHR] = in[0][s];
-      in[0][s] = nx[0][s];
-    }
-  }
-  if constexpr (!WARP) __syncthreads();  // outputs overwrite rows that other threads of the pair have read
-#pragma unroll
-  for (int f = 0; f < NOUT; ++f) {
-    V p[1][E];
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-      V q[NIN];
-#pragma unroll
-      for (int c = 0; c < NIN; ++c) q[c] = pts[(c * E + s) * NTHR];
-      p[0][s] = z_product<FORM>(f, q);
-    }
-    zpair_forward_store<T, NZ, E, 1>(p, Pl + f * g.S, g.S, live0, live1, t, partner, tw, xch);
+    zpair_forward_store<T, NZ, E, NB>(p, Pl + f0 * g.S, g.S, live0, live1, t, partner, tw, xch, SLOT);
   }
 }
 
@@ -1230,9 +1029,10 @@ __global__ void __launch_bounds__(NTHR, MINB)
 // registers at a time.
 template <typename T, int NZ, int E, int NTHR, int MINB>
 __global__ void __launch_bounds__(NTHR, MINB)
-    k_z_pair_adj(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw, int zkeep) {
+    k_z_pair_adj(C<T>* P, Geo g, const C<T>* __restrict__ tw, int zkeep) {
+  chain_begin();
   typedef C<T> V;
-  constexpr int M = NZ / 2, H = M + 1, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ);
+  constexpr int M = NZ / 2, H = M + 1, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ), SLOT = PPB * LDX;
   constexpr bool WARP = TPL <= 32;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int l = threadIdx.x / TPL, t = threadIdx.x % TPL;
@@ -1241,12 +1041,12 @@ __global__ void __launch_bounds__(NTHR, MINB)
   const long long nlines = (long long)g.Nx * g.Ny;
   const long long line = 2 * ((long long)blockIdx.x * PPB + l);
   const bool live0 = line < nlines, live1 = line + 1 < nlines;
-  V* xch = reinterpret_cast<V*>(smraw) + l * (3 * LDX);
+  V* xch = reinterpret_cast<V*>(smraw) + l * LDX;  // line f of the pair at f * SLOT
   V* mus = reinterpret_cast<V*>(smraw) + PPB * (3 * LDX) + threadIdx.x;  // slot (f, s) at (f E + s) NTHR
   V* Pl = P + (live0 ? line : 0) * H;
   V in[3][E];
   zpair_load<T, NZ, E, 3>(Pl + 6 * g.S, g.S, live0, live1, t, partner, M, in);
-  fft_regs_b<NZ, E, 1, 3, WARP, 0, true, false>(in, t, xch, LDX, 1, 0, tw, 1);
+  fft_regs_b<NZ, E, 1, 3, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
 #pragma unroll
   for (int f = 0; f < 3; ++f)
 #pragma unroll
@@ -1254,7 +1054,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     zpair_load<T, NZ, E, 3>(Pl + 3 * h * g.S, g.S, live0, live1, t, partner, zkeep, in);
-    fft_regs_b<NZ, E, 1, 3, WARP, 0, true, false>(in, t, xch, LDX, 1, 0, tw, 1);
+    fft_regs_b<NZ, E, 1, 3, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       V p[1][E];
@@ -1265,7 +1065,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
         const V c = h == 0 ? mus[(j * E + s) * NTHR] : in[j][s], d = h == 0 ? in[i][s] : mus[(i * E + s) * NTHR];
         p[0][s] = mk<V>(a.x * b.x - c.x * d.x, a.y * b.y - c.y * d.y);
       }
-      zpair_forward_store<T, NZ, E, 1>(p, Pl + (3 * h + f) * g.S, g.S, live0, live1, t, partner, tw, xch);
+      zpair_forward_store<T, NZ, E, 1>(p, Pl + (3 * h + f) * g.S, g.S, live0, live1, t, partner, tw, xch, SLOT);
     }
   }
 }
@@ -1287,10 +1087,11 @@ __global__ void __launch_bounds__(NTHR, MINB)
 // ---------------------------------------------------------------------------
 template <typename T, int NZ, int E, int FORM, int NTHR, int MINB, int NB>
 __global__ void __launch_bounds__(NTHR, MINB)
-    k_sss_z_pair(C<T>* __restrict__ P, Geo g, const C<T>* __restrict__ tw, const C<T>* __restrict__ tq, int zin,
+    k_sss_z_pair(C<T>* P, Geo g, const C<T>* __restrict__ tw, const C<T>* __restrict__ tq, int zin,
                  int zout, T scl) {
+  chain_begin();
   typedef C<T> V;
-  constexpr int H = NZ / 2 + 1, LD = NZ + 2, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ);
+  constexpr int H = NZ / 2 + 1, LD = NZ + 2, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ), SLOT = PPB * LDX;
   constexpr int NIN = z_nin(FORM), NOUT = z_nout(FORM);
   constexpr bool WARP = TPL <= 32, SH = zpair_shfl<T, NZ, E>();
   static_assert(FORM == 7 || FORM == 2 || FORM == 6, "conservative products, with or without T, or the flux giver's");
@@ -1302,7 +1103,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
   const long long nlines = (long long)g.Nx * g.Ny;
   const long long line = 2 * ((long long)blockIdx.x * PPB + l);
   const bool live0 = line < nlines, live1 = line + 1 < nlines;
-  V* xch = reinterpret_cast<V*>(smraw) + l * (zpair_lines(NIN, NB) * LDX);
+  V* xch = reinterpret_cast<V*>(smraw) + l * LDX;  // line f of the pair at f * SLOT
   T* Pl = reinterpret_cast<T*>(P + (live0 ? line : 0) * H);  // line a; line b follows at Pl + LD
 
   V in[NIN][E];
@@ -1339,7 +1140,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
       else in[c][s] = mul(conjg(tq[m]), sine ? add_i<-1>(q[s], p) : add_i<-1>(p, q[s]));
     }
   }
-  fft_regs_b<NZ, E, 1, NIN, WARP, 0, true, false>(in, t, xch, LDX, 1, 0, tw, 1);
+  fft_regs_b<NZ, E, 1, NIN, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
 #pragma unroll
   for (int f0 = 0; f0 < NOUT; f0 += NB) {
     V p[NB][E];
@@ -1352,12 +1153,12 @@ __global__ void __launch_bounds__(NTHR, MINB)
         for (int c = 0; c < NIN; ++c) q[c] = in[c][s];
         p[f][s] = z_product<FORM>(f0 + f, q);
       }
-    fft_regs_b<NZ, E, -1, NB, WARP, 0, true, true>(p, t, xch, LDX, 1, 0, tw, 1);
+    fft_regs_b<NZ, E, -1, NB, WARP, 0, zpair_pad<T>(NZ), true>(p, t, xch, SLOT, 1, 0, tw, 1);
     if constexpr (!SH) {
 #pragma unroll
       for (int f = 0; f < NB; ++f)
 #pragma unroll
-        for (int s = 0; s < E; ++s) xch[f * LDX + prow<true>(final_row<NZ, E, true>(t, s))] = p[f][s];
+        for (int s = 0; s < E; ++s) xch[f * SLOT + prow<zpair_pad<T>(NZ)>(final_row<NZ, E, true>(t, s))] = p[f][s];
       fft_sync<WARP>();
     }
 #pragma unroll
@@ -1373,7 +1174,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
           zr.y = __shfl_sync(0xffffffffu, p[f][E - 1 - s].y, partner);
           if (t == 0) zr = p[f][(E - s) % E];
         } else {
-          zr = xch[f * LDX + prow<true>((NZ - m) % NZ)];
+          zr = xch[f * SLOT + prow<zpair_pad<T>(NZ)>((NZ - m) % NZ)];
         }
         const V w = tq[m], wz = mul(w, p[f][s]), wzr = mul(conjg(w), zr);
         const V o = sine ? mul_i<1>(scale(sub(wz, wzr), scl)) : scale(add(wz, wzr), scl);
@@ -1618,6 +1419,7 @@ template <typename T, int L, int E, int CW, int FORM, int MODE>
 __global__ void __launch_bounds__(CW * (L / E), 1)
     k_fwd_x(const __grid_constant__ CUtensorMap mP, const __grid_constant__ CUtensorMap mA,
             const __grid_constant__ CUtensorMap mB, Geo g, StageArgs a, const C<T>* __restrict__ tw) {
+  chain_begin();
   typedef C<T> V;
   constexpr int NF = z_nout(FORM);
   constexpr int TILE = L * CW, BR = L < 256 ? L : 256, UNITS = (int)sizeof(V) / 8;
@@ -1717,7 +1519,7 @@ __global__ void __launch_bounds__(CW * (L / E), 1)
       // elements and 8 columns: bit 0 flipped by bit 2, since the first pass stores
       // rows 4 apart from neighbouring threads; 1.0x the minimum wavefronts against
       // 2.0x with the earlier padded pitch CW + 1)
-      fft_regs<L, E, -1, 0, false, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
+      fft_regs<L, E, -1, 0, 0, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
 #pragma unroll
       for (int s = 0; s < E; ++s) {
         const int lx = final_row<L, E>(t, s);
@@ -1757,6 +1559,247 @@ __global__ void __launch_bounds__(CW * (L / E), 1)
   }
 }
 
+// Stage update of one mode of an IF-RK4 step from its unscaled transforms p (FORM 1, 7), the
+// arithmetic of spec_epilogue with the projection folded into the assembly:
+//   FORM 1: N = -inv p,        R = -(N - K (K.N) / K^2) = inv (p - K (K.p) / K^2)
+//   FORM 7: N = i inv m, m_i = sum_j K_j p_ij,        R = -i inv (m - K (K.m) / K^2)
+// (inv is a power of two: every FFF axis is).  STAGE is known at compile time, rK2 = 1 / K^2
+// (0 at K = 0), fc the force of the mode (zero outside the band).
+template <typename T, int FORM, int STAGE>
+__device__ __forceinline__ void step_mode(const C<T>* p, const T (&K)[3], T rK2, T inv, const C<T>* fc, bool dz,
+                                          bool clear, Fac<T> Feh, Fac<T> Fe1, const Fac<T> (&Fc)[4], const C<T>* u0,
+                                          const C<T>* tt, C<T>* Uc, C<T>* tot, C<T>* Uo, long long off, long long S,
+                                          int* err) {
+  typedef C<T> V;
+  V m[3];
+  if constexpr (FORM == 1) {
+    m[0] = p[0]; m[1] = p[1]; m[2] = p[2];
+  } else {
+    m[0] = add(add(scale(p[0], K[0]), scale(p[2], K[1])), scale(p[4], K[2]));
+    m[1] = add(add(scale(p[2], K[0]), scale(p[1], K[1])), scale(p[3], K[2]));
+    m[2] = add(scale(p[4], K[0]), scale(p[3], K[1]));
+  }
+  if (fc) {
+    // N - F: with N = -inv m (FORM 1) m + F / inv, with N = i inv m (FORM 7) m + i F / inv
+    const T w = (T)1 / inv;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) m[i] = FORM == 1 ? add(m[i], scale(fc[i], w)) : add_i<1>(m[i], scale(fc[i], w));
+  }
+  V d = mk<V>(K[0] * m[0].x + K[1] * m[1].x + K[2] * m[2].x, K[0] * m[0].y + K[1] * m[1].y + K[2] * m[2].y);
+  d = scale(d, rK2);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const V r = mk<V>((m[i].x - K[i] * d.x) * inv, (m[i].y - K[i] * d.y) * inv);
+    const V R = FORM == 1 ? r : mk<V>(r.y, -r.x);
+    const long long o = off + i * S;
+    if constexpr (STAGE == 1) {
+      Uc[o] = rk_u1_c(dz ? mk<V>(0, 0) : u0[i], R, Feh, Fc[1]);
+      tot[o] = rk_t1_c(R, Fe1, Fc[3]);
+    } else if constexpr (STAGE == 2) {
+      Uc[o] = rk_u2_c(u0[i], R, Feh, Fc[1]);
+      tot[o] = rk_tacc_c(tt[i], R, Feh, Fc[2]);
+    } else if constexpr (STAGE == 3) {
+      Uc[o] = rk_u3_c(u0[i], R, Feh, Fc[0]);
+      tot[o] = rk_tacc_c(tt[i], R, Feh, Fc[2]);
+    } else {
+      const V un = rk_u4_c(u0[i], tt[i], R, Fe1, Fc[3]);
+      Uo[o] = clear ? mk<V>(0, 0) : un;
+      health_mark(nonfinite(un), err);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// forward x pass + epilogue of a step, pipelined form: persistent over column tiles of L x CW.
+// The NF product fields of a tile sit in shared memory; NF groups of CW * (L / E) threads
+// transform one field each (in registers, the field's own tile as the exchange tile) and
+// leave the spectra there, then all threads sweep the tile's modes (assembly, projection,
+// stage update), each thread down one column, so everything that depends on the column is
+// formed once per tile; what depends on the row comes from shared-memory tables.  While
+// tile k is transformed and swept, the products of the block's next tile stream into the
+// other buffer (16-byte cp.async, NBUF = 2) and the state its sweep will read is prefetched
+// into L2 (PF).  FORM 3: the adjoint's stage.
+// ---------------------------------------------------------------------------
+__host__ __device__ constexpr size_t pipe_row_bytes() { return 3 * sizeof(double); }
+// Mode of the adjoint (FORM 3): W = D c (A + i K x B) and the transposed stage update (see
+// k_fwd_x).
+template <typename T, int STAGE>
+__device__ __forceinline__ void adj_mode(const C<T>* p, const T (&K)[3], T inv, T cw, double eh, double dt, const C<T>* Lv,
+                                         const C<T>* Acc, C<T>* lam, C<T>* Ac, C<T>* Lm, long long off, long long S) {
+  typedef C<T> V;
+  V a[3] = {mk<V>(0, 0), mk<V>(0, 0), mk<V>(0, 0)};
+#pragma unroll
+  for (int f = 0; f < 6; ++f) accum_product<3>(f, scale(p[f], inv), K[0], K[1], K[2], a[0], a[1], a[2]);
+  const double e1 = eh * eh;
+  const T Eh = (T)eh, E1 = (T)e1;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const long long o = off + i * S;
+    const V W = scale(a[i], cw);
+    if constexpr (STAGE == 4) {
+      Ac[o] = add(scale(Lv[i], E1), scale(W, E1));
+      lam[o] = add(scale(Lv[i], (T)(dt / 3 * eh)), scale(W, (T)(dt * eh)));
+    } else if constexpr (STAGE == 1) {
+      Lm[o] = add(Acc[i], W);
+    } else {
+      Ac[o] = add(Acc[i], scale(W, Eh));
+      lam[o] = STAGE == 3 ? add(scale(Lv[i], (T)(dt / 3 * eh)), scale(W, (T)(0.5 * dt)))
+                          : add(scale(Lv[i], (T)(dt / 6 * e1)), scale(W, (T)(0.5 * dt * eh)));
+    }
+  }
+}
+
+template <typename T, int L, int E, int CW, int FORM, int STAGE, int NBUF, bool PF>
+__global__ void __launch_bounds__(z_nout(FORM) * CW * (L / E), 1)
+    k_fwd_x_pipe(const C<T>* P, Geo g, StageArgs a, const C<T>* __restrict__ tw) {
+  chain_begin();
+  typedef C<T> V;
+  constexpr bool ADJ = FORM == 3, F32 = sizeof(T) == 4 && !ADJ;
+  // the state fields the sweep reads at this stage
+  constexpr bool LD0 = !(ADJ && STAGE == 1), LD1 = ADJ ? STAGE != 4 : STAGE > 1;
+  constexpr int NF = z_nout(FORM), GT = CW * (L / E), NT = NF * GT, TILE = L * CW;
+  constexpr int VEC = 16 / (int)sizeof(V), SWK = best_swk(L, E, CW, (int)sizeof(V));
+  static_assert(NT % CW == 0 && TILE % VEC == 0, "a thread sweeps one column; 16-byte copies");
+  extern __shared__ __align__(16) unsigned char smraw[];
+  V* buf0 = reinterpret_cast<V*>(smraw);
+  // per row: Kx^2, the x integrating factor (FP32: (hi, lo) pair), Kx
+  double* tk2 = reinterpret_cast<double*>(buf0 + NBUF * NF * TILE);
+  double* tex = tk2 + L;
+  T* tkx = reinterpret_cast<T*>(tex + L);
+  const int grp = threadIdx.x / GT, gt = threadIdx.x % GT, c = gt % CW, t = gt / CW;
+  const unsigned inner = g.Ny * g.Hz;  // a multiple of CW (Ny is a multiple of 16)
+  const unsigned ntiles = inner / CW;
+  const T inv = (T)(1.0 / ((double)g.Nx * g.Ny * g.Nz));
+  const V* st0 = reinterpret_cast<const V*>(a.U0);
+  V* tot = reinterpret_cast<V*>(a.tot);
+  V* Uc = reinterpret_cast<V*>(a.Ucur);
+  V* Uo = reinterpret_cast<V*>(a.Uout);
+  for (int i = threadIdx.x; i < L; i += NT) {
+    const double K = kfft(i, g.Nx) * g.kf[0];
+    tk2[i] = K * K;
+    if constexpr (F32) reinterpret_cast<float2*>(tex)[i] = a.exf[i];
+    else tex[i] = a.ex[i];
+    tkx[i] = (T)K;
+  }
+  auto issue = [&](unsigned tile, int b) {
+    if (tile < ntiles) {
+      V* d = buf0 + b * (NF * TILE);
+      for (int i = threadIdx.x; i < NF * TILE / VEC; i += NT) {
+        const int f = i / (TILE / VEC), r = (i % (TILE / VEC)) / (CW / VEC), cc = (i % (CW / VEC)) * VEC;
+        cp_async16(d + f * TILE + r * CW + cc, P + f * g.S + (long long)r * inner + tile * CW + cc);
+      }
+      if constexpr (PF) {
+        for (int r = threadIdx.x; r < 3 * L; r += NT) {
+          const long long off = (r / L) * g.S + (long long)(r % L) * inner + tile * CW;
+          if (LD0) asm volatile("prefetch.global.L2 [%0];" ::"l"(st0 + off));
+          if (LD1) asm volatile("prefetch.global.L2 [%0];" ::"l"(tot + off));
+        }
+      }
+    }
+    cp_async_commit();
+  };
+  issue(blockIdx.x, 0);
+  const Fac<T> Fc[4] = {fac<T>(a.dt), fac<T>(0.5 * a.dt), fac<T>((1.0 / 3) * a.dt), fac<T>((1.0 / 6) * a.dt)};
+  const int sc = threadIdx.x % CW, sr0 = threadIdx.x / CW;  // the sweep's column and first row
+  constexpr int SR = NT / CW;
+  int b = 0;
+  for (unsigned tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    V* buf = buf0 + b * (NF * TILE);
+    cp_async_wait<0>();
+    __syncthreads();  // the tile has arrived, and the sweep of the previous one is over
+    if (NBUF == 2) issue(tile + gridDim.x, b ^ 1);
+    {
+      V* ft = buf + grp * TILE;
+      V v[E];
+#pragma unroll
+      for (int s = 0; s < E; ++s) v[s] = ft[load_row<L, E>(t, s) * CW + c];
+      __syncthreads();  // every row of the tile is in registers: it is the exchange tile now
+      fft_regs<L, E, -1, 0, 0, false, SWK>(v, t, ft, CW, c, tw, 1);
+#pragma unroll
+      for (int s = 0; s < E; ++s) ft[final_row<L, E>(t, s) * CW + c] = v[s];
+    }
+    __syncthreads();
+    // column constants
+    const unsigned col = tile * CW + sc;
+    const int ly = col / (unsigned)g.Hz, lz = col - ly * g.Hz, ky = kfft(ly, g.Ny);
+    const double Kyd = ky * g.kf[1], Kzd = lz * g.kf[2], c2 = Kyd * Kyd + Kzd * Kzd;
+    const T Ky = (T)Kyd, Kz = (T)Kzd;
+    const double ecol64 = F32 ? 0.0 : a.ey[ly] * a.ez[lz];
+    Fac<T> ecol;
+    if constexpr (F32) ecol = pair_mul(a.eyf[ly], a.ezf[lz]);
+    else ecol = fac<T>(ecol64);
+    int zlo = L, zhi = L;
+    if (ADJ || STAGE == 1) fff_zero_rows(g.dealias, ly, lz, g.Nx, g.Ny, g.Nz, zlo, zhi);
+    const bool clear = STAGE == 4 && a.reality && lz == g.Nz / 2;
+    const bool band = a.fcube && abs(ky) <= a.fkm && lz <= a.fkm;
+    const V* fcol = reinterpret_cast<const V*>(a.fcube) + ((long long)a.fkm * (2 * a.fkm + 1) + ky + a.fkm) * (a.fkm + 1) + lz;
+    const V *u0p = st0 + col, *ttp = tot + col;
+    auto load = [&](int r, V* u0, V* tt) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        if (LD0) u0[i] = u0p[i * g.S + (long long)r * inner];
+        if (LD1) tt[i] = ttp[i * g.S + (long long)r * inner];
+      }
+    };
+    auto mode = [&](int r, const V* u0, const V* tt) {
+      V p[NF];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) p[f] = buf[f * TILE + r * CW + sc];
+      const T K[3] = {tkx[r], Ky, Kz};
+      if constexpr (ADJ) {
+        const T cw = (r >= zlo && r < zhi) ? (T)0 : ((lz > 0 && 2 * lz < g.Nz) ? (T)2 : (T)1);
+        adj_mode<T, STAGE>(p, K, inv, cw, tex[r] * ecol64, a.dt, u0, tt, Uc, tot, const_cast<V*>(st0),
+                           (long long)r * inner + col, g.S);
+        return;
+      }
+      const T K2 = (T)(tk2[r] + c2);
+      const T rK2 = K2 > (T)0 ? (T)1 / K2 : (T)0;
+      Fac<T> Feh, Fe1;
+      if constexpr (F32) {
+        Feh = pair_mul(reinterpret_cast<const float2*>(tex)[r], ecol);
+        if (STAGE == 1 || STAGE == 4) Fe1 = pair_mul(Feh, Feh);
+      } else {
+        const double eh = tex[r] * ecol64;
+        Feh = fac<T>(eh);
+        Fe1 = fac<T>(eh * eh);
+      }
+      V fcv[3];
+      bool forced = false;
+      if (band) {
+        const int kx = kfft(r, g.Nx);
+        if (abs(kx) <= a.fkm) {
+          forced = true;
+          const long long n = 2 * a.fkm + 1, fs = n * n * (a.fkm + 1);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) fcv[i] = fcol[i * fs + (long long)kx * n * (a.fkm + 1)];
+        }
+      }
+      step_mode<T, FORM, STAGE>(p, K, rK2, inv, forced ? fcv : nullptr, r >= zlo && r < zhi, clear, Feh, Fe1, Fc, u0, tt,
+                                Uc, tot, Uo, (long long)r * inner + col, g.S, a.err);
+    };
+    // the state of the next row is on its way while a row is updated
+    V u0[3], tt[3];
+    if (sr0 < L) load(sr0, u0, tt);
+    for (int r = sr0; r < L; r += SR) {
+      V u1[3], t1[3];
+      if (r + SR < L) load(r + SR, u1, t1);
+      mode(r, u0, tt);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        u0[i] = u1[i];
+        tt[i] = t1[i];
+      }
+    }
+    if (NBUF == 1) {
+      __syncthreads();
+      issue(tile + gridDim.x, 0);
+    } else {
+      b ^= 1;
+    }
+  }
+  cp_async_wait<0>();
+}
+
 // ---------------------------------------------------------------------------
 // Elementwise spectral epilogue, used where the fused x kernel's column tiles
 // would have rows narrower than 64 bytes (FP32 and FP64 at Nx >= 512): the NF
@@ -1765,7 +1808,8 @@ __global__ void __launch_bounds__(CW * (L / E), 1)
 // coalesced.  Same arithmetic as k_fwd_x's epilogue (spec_epilogue).
 // ---------------------------------------------------------------------------
 template <typename T, int FORM, int MODE>
-__global__ void __launch_bounds__(256) k_spec_epi(const C<T>* __restrict__ P, Geo g, StageArgs a) {
+__global__ void __launch_bounds__(256) k_spec_epi(const C<T>* P, Geo g, StageArgs a) {
+  chain_begin();
   typedef C<T> V;
   constexpr int NF = z_nout(FORM);
   double tb[MODE == MODE_FLUX ? FLUX_MAX_BINS : 1];  // MODE_FLUX: per-thread sphere partials
@@ -1856,14 +1900,14 @@ __global__ void __launch_bounds__(NTHR, MINB)
       if (r > M) a.y = -a.y, b.y = -b.y;
       v[0][s] = mk<V>(a.x - b.y, a.y + b.x);
     }
-    fft_regs_b<NZ, E, 1, 1, WARP, 0, true, false>(v, t, xch, LDX, 1, 0, tw, 1);
+    fft_regs_b<NZ, E, 1, 1, WARP, 0, 1, false>(v, t, xch, LDX, 1, 0, tw, 1);
 #pragma unroll
-    for (int s = 0; s < E; ++s) xch[prow<true>(final_row<NZ, E>(t, s))] = v[0][s];
+    for (int s = 0; s < E; ++s) xch[prow<1>(final_row<NZ, E>(t, s))] = v[0][s];
     fft_sync<WARP>();
     // points 2 i, 2 i + 1 as one store; the pad is slot M
     V* o = out + lo;
     for (int i = t; i <= M; i += TPL) {
-      const V p = i < M ? xch[prow<true>(2 * i)] : mk<V>(0, 0), q = i < M ? xch[prow<true>(2 * i + 1)] : mk<V>(0, 0);
+      const V p = i < M ? xch[prow<1>(2 * i)] : mk<V>(0, 0), q = i < M ? xch[prow<1>(2 * i + 1)] : mk<V>(0, 0);
       if (live0) o[i] = mk<V>(p.x, q.x);
       if (live1) o[H + i] = mk<V>(p.y, q.y);
     }
@@ -1874,13 +1918,13 @@ __global__ void __launch_bounds__(NTHR, MINB)
       const int n = load_row<NZ, E>(t, s);
       v[0][s] = mk<V>(live0 ? X[n] : (T)0, live1 ? X[LD + n] : (T)0);
     }
-    fft_regs_b<NZ, E, -1, 1, WARP, 0, true, false>(v, t, xch, LDX, 1, 0, tw, 1);
+    fft_regs_b<NZ, E, -1, 1, WARP, 0, 1, false>(v, t, xch, LDX, 1, 0, tw, 1);
 #pragma unroll
-    for (int s = 0; s < E; ++s) xch[prow<true>(final_row<NZ, E>(t, s))] = v[0][s];
+    for (int s = 0; s < E; ++s) xch[prow<1>(final_row<NZ, E>(t, s))] = v[0][s];
     fft_sync<WARP>();
     V* o = out + lo;
     for (int k = t; k <= M; k += TPL) {
-      const V z = xch[prow<true>(k)], zp = xch[prow<true>((NZ - k) % NZ)];
+      const V z = xch[prow<1>(k)], zp = xch[prow<1>((NZ - k) % NZ)];
       if (live0) o[k] = mk<V>((T)0.5 * (z.x + zp.x), (T)0.5 * (z.y - zp.y));
       if (live1) o[H + k] = mk<V>((T)0.5 * (z.y + zp.y), (T)0.5 * (zp.x - z.x));
     }

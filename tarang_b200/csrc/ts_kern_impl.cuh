@@ -7,6 +7,7 @@
 #define TS_PART_FX 4    // FFF forward x pass and epilogue
 #define TS_PART_SFF 5   // sin/cos x passes
 #define TS_PART_MISC 6  // elementwise, plane-sized and reduction kernels, tuning queries
+#include <math.h>
 #include <type_traits>
 #include "ts_launch.h"
 #include "ts_misc.cuh"
@@ -74,6 +75,14 @@ template <typename Fn> bool dispatch_L_sff(int L, Fn&& fn) {
 // holds four accumulators per element and spilled at 12)
 constexpr int e_mixed(int L, int e_pow2) { return L % 3 == 0 ? (e_pow2 >= 8 ? 12 : 6) : (e_pow2 < L ? e_pow2 : L); }
 
+// the largest x with sqrt(x) <= R, so that |K| > R is K^2 > x without a square root per mode
+inline double k2_limit(double R) {
+  double x = R * R;
+  while (sqrt(x) > R) x = nextafter(x, 0.0);
+  while (sqrt(nextafter(x, HUGE_VAL)) <= R) x = nextafter(x, HUGE_VAL);
+  return x;
+}
+
 template <typename K> cudaError_t smem_attr(K kernel, size_t bytes) {
   if (bytes > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -81,6 +90,31 @@ template <typename K> cudaError_t smem_attr(K kernel, size_t bytes) {
     return e;
   }
   return cudaSuccess;
+}
+
+// Launch of a kernel that begins with chain_begin().  Kernels on small fields are launched
+// while the preceding kernel of the stream still runs: a pass takes 2-4 us there and the gap
+// between two plain launches another 2 us.  Large grids are launched plainly: their early
+// blocks would take the slots of the running grid's last waves.  B200, plain -> chained: 32^3
+// FP32 step 126 -> 77 us, 64^3 FP64 172 -> 161, SSF 96^3 (3.6 MB per component) 329 -> 281, SSS
+// 128^3 FP32 (8.5 MB) 653 -> 616, 18-sphere flux 128^3 3278 -> 3084; FP64 adjoint 128^3 (17 MB)
+// 12750 -> 13080, 256^3 2711 -> 2715, MHD 256^3 4908 -> 5008.
+constexpr long long CHAIN_BYTES = 10000000;
+inline bool chained(const Geo& g, int nmem = 1) { return nmem == 1 && g.S * (long long)sizeof(V) <= CHAIN_BYTES; }
+template <typename... P, typename... A>
+cudaError_t launch_chain(bool chain, void (*k)(P...), dim3 grid, unsigned block, size_t sm, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = sm;
+  c.stream = st;
+  c.attrs = at;
+  c.numAttrs = chain ? 1 : 0;
+  ++g_launches;
+  return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
 }
 
 inline unsigned grid1d(long long n, int threads) {
@@ -180,8 +214,7 @@ constexpr int ix_e_alt(int L) {
 // (the three components of U held in registers), staging + exchange tiles (NT = 4 tiles);
 // candidate 4 (FP32, 1024-point lines): 32 elements per thread over 8-column tiles
 // (256-thread blocks, two per SM; radix 32 x 32, one exchange per field);
-// candidate 5 (FP32, 1024-point lines, two-thirds dealiasing): k_inv_x_st, the tile's
-// kept U rows staged in shared memory in one cp.async group (the rule elsewhere)
+// candidate 5 (FP32, 1024-point lines): 16 elements per thread over 8-column tiles
 constexpr Tile ix_cand(int L, int v) {
   return v == 0 ? Tile{ix_e(L), ix_cw(L), 1}
        : v == 1 ? (ix_e_alt(L) > 0 ? Tile{ix_e_alt(L), cw_for(L, ix_e_alt(L)), 1} : Tile{0, 0, 0})
@@ -214,13 +247,14 @@ template <int NZ, int FORM> constexpr bool z_rule_slots() {
 struct ZTile { int E, NTHR, MINB, NB; };
 constexpr ZTile zp_tile(int NZ, int form) {
   const bool f32 = std::is_same<T, float>::value;
-  const int E = NZ % 3 == 0 ? 12 : 8;
+  // FP64 with six inputs at 128 points: 4 elements per thread (187 us against 195; 8 spill)
+  const int E = NZ % 3 == 0 ? 12 : (!f32 && form == 1 && NZ == 128 ? 4 : 8);
   const int tpl = NZ / E, thr = tpl > 64 ? tpl : 64;
-  return ZTile{E, thr, ((f32 && NZ % 3 != 0) || form == 3 ? 6 : 4) * 64 / thr, 1};
+  return ZTile{E, thr, ((f32 && NZ % 3 != 0) || E == 4 ? 6 : 4) * 64 / thr, 1};
 }
 // FP32 lines of 48, 96 and 1024 points: single lines in registers (k_z_reg) are the rule
 template <int NZ, int FORM> constexpr bool zreg_rule() {
-  return std::is_same<T, float>::value && FORM != 3 && (NZ % 3 == 0 || NZ == 1024);
+  return std::is_same<T, float>::value && FORM != 3 && FORM != 6 && (NZ % 3 == 0 || NZ == 1024);
 }
 template <int NZ, int FORM> constexpr bool z_valid(int v) {
   constexpr int M = NZ / 2;
@@ -229,6 +263,28 @@ template <int NZ, int FORM> constexpr bool z_valid(int v) {
                                   (v == 3 && std::is_same<T, float>::value && M % 3 != 0 && M >= 8 && M / 4 <= 64) ||
                                   (v == 4 && std::is_same<T, float>::value && M == 512)));
 }
+
+// pipelined forward x kernel of a step or an adjoint step (CW = 0: not used): elements per
+// thread, tile columns, buffers, state prefetch into L2.  B200, the four stages' average, us:
+// 256x256x256 FP32 rotational 197 (203 without the prefetch, 240 with two buffers; fused TMA
+// kernel 235, split 76 + 157), conservative 239 (split 117 + 176); 128x256x256 FP32 91 (99 with
+// the prefetch) and 118 (split 35 + 83, 58 + 94); FP64 at 128^3 56 (fused 58, split 18 + 41),
+// adjoint 67 (fused 80, split 35 + 51).  FP32 at 512 points (234 against 82 + 160) and FP64 at
+// 256 (113 against 36 + 77) gain nothing.
+struct PipeTile { int E, CW, NBUF; bool PF; };
+constexpr PipeTile pipe_tile(int L, int form) {
+  return !std::is_same<T, float>::value
+             ? (L == 128 ? (form == 1 ? PipeTile{16, 16, 1, false} : form == 3 ? PipeTile{16, 8, 2, true} : PipeTile{0, 0, 0, false})
+                         : PipeTile{0, 0, 0, false})
+         : form == 3 ? PipeTile{0, 0, 0, false}
+         : L == 256  ? (form == 1 ? PipeTile{16, 16, 1, true} : PipeTile{32, 16, 1, true})
+         : L == 128  ? (form == 1 ? PipeTile{16, 32, 2, false} : PipeTile{16, 16, 2, false})
+                     : PipeTile{0, 0, 0, false};
+}
+// lengths whose step takes the split form although the fused kernel's tiles fit: short lines,
+// where a fused launch is a serial chain of loads, transforms and updates on few blocks (64^3
+// FP64 15 us against 5 + 6, 32^3 FP32 8 against 2 + 2), and FP64 above 128
+constexpr bool fx_rule_split(int L) { return L <= 64 || std::is_same<T, float>::value || L > 128; }
 
 // forward x candidates (MODE_STEP): 1 = the split form (strided x FFT, then the
 // elementwise epilogue) where the rule is the fused TMA kernel; 2 = the fused
@@ -287,11 +343,9 @@ template <> cudaError_t Launch<T>::strided(const Geo& g, int axis, int dir, void
       constexpr size_t sm = (size_t)LL * c.CW * sizeof(V);
       auto launch = [&](auto k) {
         if ((err = smem_attr(k, sm)) != cudaSuccess) return;
-        k<<<(ntot + c.CW - 1) / c.CW, c.CW * (LL / c.E), sm, st>>>(
-            (const V*)data, (V*)(dst ? dst : data), ntot, nplane, inner, g.S, rstride, (long long)g.Ny * g.Hz,
-            (const V*)tw, (unsigned)per, mstride, zero_hi, (T)scl);
-        ++g_launches;
-        err = cudaGetLastError();
+        err = launch_chain(chained(g, per == nf ? 1 : nf / per), k, (ntot + c.CW - 1) / c.CW, c.CW * (LL / c.E), sm, st,
+                           (const V*)data, (V*)(dst ? dst : data), ntot, nplane, inner, g.S, rstride,
+                           (long long)g.Ny * g.Hz, (const V*)tw, (unsigned)per, mstride, zero_hi, (T)scl);
       };
       if (dir > 0) launch(k_strided_ld<T, LL, c.E, c.CW, 1, c.MINB, false>);
       else if (scl == 1.0) launch(k_strided_ld<T, LL, c.E, c.CW, -1, c.MINB, false>);
@@ -357,39 +411,28 @@ template <> cudaError_t Launch<T>::inv_x(const Geo& g, int form, const void* U, 
       constexpr size_t sm = (size_t)LL * c.CW * sizeof(V);
       auto run = [&](auto kern, int nf) {
         if ((err_ = smem_attr(kern, sm)) != cudaSuccess) return;
-        kern<<<(unsigned)((cols + c.CW - 1) / c.CW) * nf, c.CW * (LL / c.E), sm, st>>>(
-            (const V*)U, (V*)W, g, (const V*)tw, (const V*)lam, (T)lsc, kept, rad);
-        ++g_launches;
-        err_ = cudaGetLastError();
+        err_ = launch_chain(chained(g), kern, (unsigned)((cols + c.CW - 1) / c.CW) * nf, c.CW * (LL / c.E), sm, st,
+                            (const V*)U, (V*)W, g, (const V*)tw, kept, form == 5 ? k2_limit(rad) : 0.0);
       };
       if (form == 0) run(k_inv_x_f<T, LL, c.E, c.CW, 0, c.MINB>, 3);
       else if (form == 1) run(k_inv_x_f<T, LL, c.E, c.CW, 1, c.MINB>, 6);
-      else if (form == 4) run(k_inv_x_f<T, LL, c.E, c.CW, 4, c.MINB>, 3);
-      else if (form == 5) run(k_inv_x_f<T, LL, c.E, c.CW, 5, c.MINB>, 6);
+      else if (form == 5) run(k_inv_x_f<T, LL, c.E, c.CW, 5, c.MINB>, 3);
+      else if (form == 4) {
+        // three components in registers: 8 elements per thread
+        constexpr int E = 8 < LL ? 8 : 4, CW = cw_for(LL, E), NT = CW * (LL / E);
+        constexpr size_t sm4 = (size_t)LL * CW * sizeof(V);
+        auto k = k_inv_x_cot<T, LL, E, CW, NT <= 256 ? 256 / NT * (std::is_same<T, float>::value ? 2 : 1) : 1>;
+        if ((err_ = smem_attr(k, sm4)) != cudaSuccess) return;
+        err_ = launch_chain(chained(g), k, (unsigned)((cols + CW - 1) / CW), NT, sm4, st, (const V*)lam, (V*)W, g,
+                            (const V*)tw, (T)lsc);
+      }
     });
     return err_;
   }
   dispatch_L(g.Nx, [&](auto Lc) {
     constexpr int LL = decltype(Lc)::value;
-    // 1024 points in FP32 under two-thirds dealiasing: candidate 5 is the direct-load kernel
-    const int vv = (ix_valid(LL, 5) && kept && v == 5) ? 0 : v;
-    if constexpr (ix_valid(LL, 5)) {
-      if (vv == 5 && kept) {
-        // the kept U rows of a tile staged in shared memory (one load latency per tile)
-        constexpr Tile c = ix_cand(LL, 5);
-        constexpr int E = c.E, CW = c.CW;
-        const size_t sm = ((size_t)LL + 3 * ix_kept_rows<LL>()) * CW * sizeof(V);
-        const unsigned blocks = (unsigned)(((2 * (g.Ny / 3) + 1) * (g.Nz / 3 + 1) + CW - 1) / CW);
-        auto run = [&](auto kern) {
-          if ((err_ = smem_attr(kern, sm)) != cudaSuccess) return;
-          kern<<<blocks, CW * (LL / E), sm, st>>>((const V*)U, (V*)W, g, (const V*)tw);
-          ++g_launches;
-          err_ = cudaGetLastError();
-        };
-        if (form == 0) { run(k_inv_x_st<T, LL, E, CW, 0>); return; }
-        if (form == 1) { run(k_inv_x_st<T, LL, E, CW, 1>); return; }
-      }
-    }
+    // candidate 5 (1024 points in FP32): tile 0
+    const int vv = v == 5 ? 0 : v;
     if constexpr (ix_valid(LL, 3)) {
       if (vv == 3) {
         // persistent, prefetching form: one block per SM
@@ -411,8 +454,6 @@ template <> cudaError_t Launch<T>::inv_x(const Geo& g, int form, const void* U, 
         return;
       }
     }
-    // the direct-load kernel measured faster than the TMA-staged k_inv_x on B200
-    // (0.19 vs 0.28 ms at 256^3 FP32, rotational); k_inv_x stays available
     auto tile = [&](auto vc) {
       constexpr Tile c = ix_cand(LL, decltype(vc)::value);
       constexpr int E = c.E, CW = c.CW;
@@ -423,8 +464,7 @@ template <> cudaError_t Launch<T>::inv_x(const Geo& g, int form, const void* U, 
                                    : (unsigned)((inner + CW - 1) / CW);
       auto run = [&](auto kern) {
         if ((err_ = smem_attr(kern, sm)) != cudaSuccess) return;
-        kern<<<blocks, CW * (LL / E), sm, st>>>((const V*)U, (V*)W, g, (const V*)tw, (const V*)lam, (T)lsc, kept,
-                                                 rad);
+        kern<<<blocks, CW * (LL / E), sm, st>>>((const V*)U, (V*)W, g, (const V*)tw, kept);
         ++g_launches;
         err_ = cudaGetLastError();
       };
@@ -469,7 +509,7 @@ static cudaError_t z_slots(const Geo& g, void* P, const void* tw, cudaStream_t s
 
 template <int NZ, int FORM>
 static cudaError_t z_fused_impl(const Geo& g, void* P, const void* tw, int* zerr, cudaStream_t st, int nmem,
-                                long long msP, int zkeep, int v) {
+                                long long msP, int zkeep, int v, const void* q = nullptr) {
   constexpr int M = NZ / 2;
   if (zkeep < 0) zkeep = M;
   const long long nlines = (long long)g.Nx * g.Ny;
@@ -491,10 +531,8 @@ static cudaError_t z_fused_impl(const Geo& g, void* P, const void* tw, int* zerr
   }
   if constexpr (zreg_rule<NZ, FORM>()) {
     constexpr int E = M % 3 == 0 ? 12 : 8, NT = zreg_threads<FORM>(), LPB = NT / (M / E);
-    k_z_reg<T, NZ, FORM, 0, true><<<dim3((unsigned)((nlines + LPB - 1) / LPB), nmem), NT, 0, st>>>(
-        (V*)P, g, (const V*)tw, msP, zkeep);
-    ++g_launches;
-    return cudaGetLastError();
+    return launch_chain(chained(g, nmem), k_z_reg<T, NZ, FORM, 0, true>, dim3((unsigned)((nlines + LPB - 1) / LPB), nmem),
+                        NT, 0, st, (V*)P, g, (const V*)tw, msP, zkeep);
   }
   if constexpr (z_valid<NZ, FORM>(3)) {
     if (v == 3) {
@@ -513,9 +551,8 @@ static cudaError_t z_fused_impl(const Geo& g, void* P, const void* tw, int* zerr
     const long long npairs = (nlines + 1) / 2;
     auto k = k_z_pair<T, NZ, c.E, FORM, c.NTHR, c.MINB, c.NB>;
     if ((err = smem_attr(k, sm)) != cudaSuccess) return err;
-    k<<<dim3((unsigned)((npairs + PPB - 1) / PPB), nmem), c.NTHR, sm, st>>>((V*)P, g, (const V*)tw, msP, zkeep);
-    ++g_launches;
-    return cudaGetLastError();
+    return launch_chain(chained(g, nmem), k, dim3((unsigned)((npairs + PPB - 1) / PPB), nmem), c.NTHR, sm, st, (V*)P, g,
+                        (const V*)tw, msP, zkeep, (const V*)(q ? q : P));
   }
   if constexpr (FORM == 3) {
     constexpr ZTile c = zp_tile(NZ, FORM);
@@ -524,14 +561,12 @@ static cudaError_t z_fused_impl(const Geo& g, void* P, const void* tw, int* zerr
     const long long npairs = (nlines + 1) / 2;
     auto k = k_z_pair_adj<T, NZ, c.E, c.NTHR, c.MINB>;
     if ((err = smem_attr(k, sm)) != cudaSuccess) return err;
-    k<<<(unsigned)((npairs + PPB - 1) / PPB), c.NTHR, sm, st>>>((V*)P, g, (const V*)tw, zkeep);
-    ++g_launches;
-    return cudaGetLastError();
+    return launch_chain(chained(g), k, (unsigned)((npairs + PPB - 1) / PPB), c.NTHR, sm, st, (V*)P, g, (const V*)tw, zkeep);
   }
 }
 
 template <> cudaError_t Launch<T>::z_fused(const Geo& g, int form, void* P, const void* tw, int* zerr,
-                                           cudaStream_t st, int nmem, long long msP, int zkeep) {
+                                           cudaStream_t st, int nmem, long long msP, int zkeep, const void* q) {
   cudaError_t err = cudaErrorInvalidValue;
   if (form == 3 && nmem != 1) return err;  // the adjoint z pass has no member batching
   dispatch_L_sff(g.Nz, [&](auto Lc) {
@@ -542,7 +577,7 @@ template <> cudaError_t Launch<T>::z_fused(const Geo& g, int form, void* P, cons
     else if (form == 1) err = z_fused_impl<NZ, 1>(g, P, tw, zerr, st, nmem, msP, zkeep, v);
     else if (form == 2) err = z_fused_impl<NZ, 2>(g, P, tw, zerr, st, nmem, msP, zkeep, v);
     else if (form == 5) err = z_fused_impl<NZ, 5>(g, P, tw, zerr, st, nmem, msP, zkeep, 0);
-    else if (form == 6) err = z_fused_impl<NZ, 6>(g, P, tw, zerr, st, nmem, msP, zkeep, 0);
+    else if (form == 6) err = z_fused_impl<NZ, 6>(g, P, tw, zerr, st, nmem, msP, zkeep, 0, q);
     else if constexpr (NZ % 3 != 0) err = z_fused_impl<NZ, 3>(g, P, tw, zerr, st, 1, 0, zkeep, 0);
   });
   return err;
@@ -559,10 +594,8 @@ static cudaError_t sss_z_pairs(const Geo& g, void* P, const void* tw, const void
   cudaError_t err;
   auto k = k_sss_z_pair<T, NZ, c.E, FORM, c.NTHR, c.MINB, c.NB>;
   if ((err = smem_attr(k, sm)) != cudaSuccess) return err;
-  k<<<(unsigned)((npairs + PPB - 1) / PPB), c.NTHR, sm, st>>>((V*)P, g, (const V*)tw, (const V*)tq, zin, zout,
-                                                              (T)(1.0 / (2.0 * NZ)));
-  ++g_launches;
-  return cudaGetLastError();
+  return launch_chain(chained(g), k, (unsigned)((npairs + PPB - 1) / PPB), c.NTHR, sm, st, (V*)P, g, (const V*)tw,
+                      (const V*)tq, zin, zout, (T)(1.0 / (2.0 * NZ)));
 }
 
 template <> cudaError_t Launch<T>::sss_z_fused(const Geo& g, int form, void* P, const void* tw, const void* tq, int zin,
@@ -605,6 +638,24 @@ template <> cudaError_t Launch<T>::z_single(const Geo& g, int dir, const void* i
 template <int FORM, int MODE, int LL, int E, int CW>
 static cudaError_t fwd_x_fused(const Geo& g, const void* P, const StageArgs& a, const void* tw, cudaStream_t st);
 
+// pipelined forward x kernel of a step
+template <int FORM, int LL>
+static cudaError_t fwd_x_pipe(const Geo& g, const void* P, const StageArgs& a, const void* tw, cudaStream_t st) {
+  constexpr PipeTile c = pipe_tile(LL, FORM);
+  constexpr size_t sm = (size_t)c.NBUF * z_nout(FORM) * LL * c.CW * sizeof(V) + LL * pipe_row_bytes();
+  const unsigned ntiles = (unsigned)(g.Ny * g.Hz / c.CW), blocks = ntiles < 148u ? ntiles : 148u;
+  cudaError_t err = cudaErrorInvalidValue;
+  auto run = [&](auto k) {
+    if ((err = smem_attr(k, sm)) != cudaSuccess) return;
+    err = launch_chain(chained(g), k, blocks, z_nout(FORM) * c.CW * (LL / c.E), sm, st, (const V*)P, g, a, (const V*)tw);
+  };
+  if (a.stage == 1) run(k_fwd_x_pipe<T, LL, c.E, c.CW, FORM, 1, c.NBUF, c.PF>);
+  else if (a.stage == 2) run(k_fwd_x_pipe<T, LL, c.E, c.CW, FORM, 2, c.NBUF, c.PF>);
+  else if (a.stage == 3) run(k_fwd_x_pipe<T, LL, c.E, c.CW, FORM, 3, c.NBUF, c.PF>);
+  else run(k_fwd_x_pipe<T, LL, c.E, c.CW, FORM, 4, c.NBUF, c.PF>);
+  return err;
+}
+
 template <int FORM, int MODE, int LL>
 static cudaError_t fwd_x_impl(const Geo& g, const void* P, const StageArgs& a, const void* tw, cudaStream_t st) {
   constexpr int CW = xcw(LL);
@@ -615,17 +666,29 @@ static cudaError_t fwd_x_impl(const Geo& g, const void* P, const StageArgs& a, c
   if constexpr (fx_valid(LL, 3)) {
     if (v == 3) return fwd_x_fused<FORM, MODE, LL, emin(E_ACC_ALT, LL), CW>(g, P, a, tw, st);
   }
-  const bool split = CW * sizeof(V) < 64 || v == 1;
+  // the rule (a blocks-per-SM count of the tuning launches the fused TMA kernel): the
+  // pipelined kernel where it has a tile and the tiles divide the columns, otherwise the split
+  // form of a step (fx_rule_split) and the fused kernel of the other modes
+  const bool rule = v == 0 && !(MODE == MODE_STEP && g.tb[TUNE_X_FWD] > 0);
+  // state pointers as the fused kernel's tensor maps take them
+  const void* sA = MODE == MODE_FLUX ? a.Ud : ((MODE == MODE_STEP || MODE == MODE_ADJ) ? a.U0 : P);
+  const void* sB = (MODE == MODE_STEP || MODE == MODE_ADJ) ? a.tot : P;
+  const bool fused16 = fx_rule_fused(LL) && (((uintptr_t)sA | (uintptr_t)sB) & 15);
+  if (fused16 && !(MODE == MODE_STEP && v == 1)) return cudaErrorInvalidValue;
+  if constexpr ((MODE == MODE_STEP || MODE == MODE_ADJ) && pipe_tile(LL, FORM).CW > 0) {
+    if (rule && g.Ny * g.Hz % pipe_tile(LL, FORM).CW == 0) return fwd_x_pipe<FORM, LL>(g, P, a, tw, st);
+  }
+  const bool split = CW * sizeof(V) < 64 || v == 1 || (rule && MODE == MODE_STEP && fx_rule_split(LL));
   if (split) {
     // tiles narrower than 64-byte rows: forward x FFT in place, then the elementwise epilogue
     constexpr int NF = z_nout(FORM);
     cudaError_t err = Launch<T>::strided(g, 0, -1, const_cast<void*>(P), NF, tw, st);
     if (err != cudaSuccess) return err;
     const unsigned blocks = grid1d(g.S, 256);
-    k_spec_epi<T, FORM, MODE><<<blocks, 256, 0, st>>>((const V*)P, g, a);
-    ++g_launches;
+    if ((err = launch_chain(chained(g), k_spec_epi<T, FORM, MODE>, blocks, 256, 0, st, (const V*)P, g, a)) != cudaSuccess)
+      return err;
     if (MODE == MODE_FLUX) {
-      k_bins_finish<<<1, 64, 0, st>>>(a.bins + (a.nradii + 1), (int)blocks, a.nradii + 1, a.bins);
+      k_bins_finish<<<8, 256, 0, st>>>(a.bins + (a.nradii + 1), (int)blocks, a.nradii + 1, a.bins);
       ++g_launches;
     }
     return cudaGetLastError();
@@ -652,10 +715,10 @@ static cudaError_t fwd_x_fused(const Geo& g, const void* P, const StageArgs& a, 
   if ((err = make_field_map(&mB, B, inner, 3LL * g.Nx, UNITS, CW, br)) != cudaSuccess) return err;
   auto k = k_fwd_x<T, LL, E, CW, FORM, MODE>;
   if ((err = smem_attr(k, sm)) != cudaSuccess) return err;
-  k<<<blocks, CW * (LL / E), sm, st>>>(mP, mA, mB, g, a, (const V*)tw);
-  ++g_launches;
+  if ((err = launch_chain(chained(g), k, blocks, CW * (LL / E), sm, st, mP, mA, mB, g, a, (const V*)tw)) != cudaSuccess)
+    return err;
   if (MODE == MODE_FLUX) {
-    k_bins_finish<<<1, 64, 0, st>>>(a.bins + (a.nradii + 1), blocks, a.nradii + 1, a.bins);
+    k_bins_finish<<<8, 256, 0, st>>>(a.bins + (a.nradii + 1), blocks, a.nradii + 1, a.bins);
     ++g_launches;
   }
   return cudaGetLastError();
@@ -696,9 +759,7 @@ template <> cudaError_t Launch<T>::sc_x(const Geo& g, int dir, const ScArgs& a, 
       const dim3 grid((unsigned)((cols + c.CW - 1) / c.CW), nmem, nf);
       auto run = [&](auto k) {
         if ((err = smem_attr(k, sm)) != cudaSuccess) return;
-        k<<<grid, c.CW * (NN / c.E), sm, st>>>(a, g, (const V*)tq);
-        ++g_launches;
-        err = cudaGetLastError();
+        err = launch_chain(chained(g, nmem), k, grid, c.CW * (NN / c.E), sm, st, a, g, (const V*)tq);
       };
       if (dir < 0) run(k_sc_x<T, NN, c.E, c.CW, -1, cf.MINB>);
       else run(k_sc_x<T, NN, c.E, c.CW, 1, c.MINB>);
@@ -768,9 +829,7 @@ template <> cudaError_t Launch<T>::sff_fwd_x(const Geo& g, const void* P, const 
     for (int f = 0; f < 8; ++f) s.smask |= sff_prod_sine(f) << f;
     s.scl = 1.0 / (2.0 * g.Nx * (double)g.Ny * g.Nz);
     if ((err = sc_x(g, -1, s, tq, st, 8, nmem)) != cudaSuccess) return err;
-    k_sff_prod_epi<T><<<dim3(grid1d(g.S, 256), nmem), 256, 0, st>>>((const V*)P, g, a);
-    ++g_launches;
-    return cudaGetLastError();
+    return launch_chain(chained(g, nmem), k_sff_prod_epi<T>, dim3(grid1d(g.S, 256), nmem), 256, 0, st, (const V*)P, g, a);
   }
   dispatch_L_sff(g.Nx, [&](auto Lc) {
     constexpr int NN = decltype(Lc)::value;
@@ -823,9 +882,7 @@ template <> cudaError_t Launch<T>::sff_x(const Geo& g, int dir, void* A, int nco
 #if TS_PART == TS_PART_MISC
 template <> cudaError_t Launch<T>::reality(const Geo& g, void* A, int ncomp, cudaStream_t st) {
   const long long n = (long long)g.Nx * g.Ny * ncomp;
-  k_reality<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>((V*)A, ncomp, g);
-  ++g_launches;
-  return cudaGetLastError();
+  return launch_chain(chained(g, (ncomp + 2) / 3), k_reality<T>, (unsigned)((n + 255) / 256), 256, 0, st, (V*)A, ncomp, g);
 }
 
 template <> cudaError_t Launch<T>::rbc_slave(const Geo& g, void* U, void* Tf, int slave, double vs, cudaStream_t st) {
@@ -844,9 +901,7 @@ template <> cudaError_t Launch<T>::reality_adj(const Geo& g, void* A, int ncomp,
 template <> cudaError_t Launch<T>::carati(const Geo& g, const void* U, void* fc, int km, double rin, double rout,
                                           const double* es, const double* hs, const double* mis, int nsup,
                                           cudaStream_t st) {
-  k_carati<T><<<1, 256, 0, st>>>((const V*)U, (V*)fc, g, km, rin, rout, es, hs, mis, nsup);
-  ++g_launches;
-  return cudaGetLastError();
+  return launch_chain(chained(g), k_carati<T>, 1, 256, 0, st, (const V*)U, (V*)fc, g, km, rin, rout, es, hs, mis, nsup);
 }
 
 template <> cudaError_t Launch<T>::energy(const Geo& g, const void* A, const void* B, int ncomp, double* out,
@@ -873,7 +928,7 @@ template <> cudaError_t Launch<T>::shell(const Geo& g, const void* A, int ncomp,
   if (err != cudaSuccess) return err;
   const unsigned blocks = shell_blocks(g, cap);
   k_shell<T><<<blocks, 32 * SHELL_WARPS, sm, st>>>((const V*)A, (const V*)B, ncomp, g, nbins, bins + 2 * nbins);
-  k_bins_finish<<<(2 * nbins + 255) / 256, 256, 0, st>>>(bins + 2 * nbins, (int)blocks, 2 * nbins, bins);
+  k_bins_finish<<<(2 * nbins + 7) / 8, 256, 0, st>>>(bins + 2 * nbins, (int)blocks, 2 * nbins, bins);
   g_launches += 2;
   return cudaGetLastError();
 }
@@ -884,12 +939,18 @@ template <> cudaError_t Launch<T>::expire_wait(int* err, int polls, cudaStream_t
   return cudaGetLastError();
 }
 
+template <> cudaError_t Launch<T>::flux_finish(const Geo& g, const double* part, long long pitch, int n_radii, double* res,
+                                               cudaStream_t st) {
+  k_sum_partials_many<<<n_radii, 256, 0, st>>>(part, pitch, (int)grid1d((g.basis == 3 ? 2 : 1) * g.S, 256), res);
+  ++g_launches;
+  return cudaGetLastError();
+}
+
 template <> cudaError_t Launch<T>::flux_outside(const Geo& g, const void* P, const void* U, double R, double* out,
                                                 cudaStream_t st) {
   const unsigned blocks = grid1d(g.S, 256);
-  k_flux_outside<T><<<blocks, 256, 0, st>>>((const V*)P, (const V*)U, g, R, out);
-  k_sum_partials<<<1, 256, 0, st>>>(out, (int)blocks);
-  g_launches += 2;
+  k_flux_outside<T><<<blocks, 256, 0, st>>>((const V*)P, (const V*)U, g, k2_limit(R), out);
+  ++g_launches;
   return cudaGetLastError();
 }
 
@@ -903,8 +964,7 @@ template <> cudaError_t Launch<T>::ssf_flux_outside(const Geo& g, const void* P,
                                                     int qy, double* out, cudaStream_t st) {
   const unsigned blocks = grid1d(g.S, 256);
   k_ssf_flux_outside<T><<<blocks, 256, 0, st>>>((const V*)P, (const V*)U, g, R, qx, qy, out);
-  k_sum_partials<<<1, 256, 0, st>>>(out, (int)blocks);
-  g_launches += 2;
+  ++g_launches;
   return cudaGetLastError();
 }
 
@@ -918,8 +978,7 @@ template <> cudaError_t Launch<T>::sss_flux_outside(const Geo& g, const void* P,
                                                     int qy, int qz, double* out, cudaStream_t st) {
   const unsigned blocks = grid1d(2 * g.S, 256);
   k_sss_flux_outside<T><<<blocks, 256, 0, st>>>((const T*)P, (const T*)U, g, R, qx, qy, qz, out);
-  k_sum_partials<<<1, 256, 0, st>>>(out, (int)blocks);
-  g_launches += 2;
+  ++g_launches;
   return cudaGetLastError();
 }
 
@@ -951,9 +1010,7 @@ template <> cudaError_t Launch<T>::scale(void* A, long long n, double s, cudaStr
 }
 
 template <> cudaError_t Launch<T>::scalar_epi(const Geo& g, const void* P, const SffArgs& a, cudaStream_t st) {
-  k_scalar_epi<T><<<grid1d(g.S, 256), 256, 0, st>>>((const V*)P, g, a);
-  ++g_launches;
-  return cudaGetLastError();
+  return launch_chain(chained(g), k_scalar_epi<T>, grid1d(g.S, 256), 256, 0, st, (const V*)P, g, a);
 }
 
 template <> cudaError_t Launch<T>::sss_zperm_fwd(const void* u, void* v, long long nlines, int N, int sine,
@@ -990,34 +1047,24 @@ template <> cudaError_t Launch<T>::sss_dealias_copy(const Geo& g, const void* A,
   return cudaGetLastError();
 }
 template <> cudaError_t Launch<T>::sss_epi(const Geo& g, const void* P, const StageArgs& a, cudaStream_t st) {
-  k_sss_epi<T><<<grid1d(2 * g.S, 256), 256, 0, st>>>((const T*)P, g, a);
-  ++g_launches;
-  return cudaGetLastError();
+  return launch_chain(chained(g), k_sss_epi<T>, grid1d(2 * g.S, 256), 256, 0, st, (const T*)P, g, a);
 }
 
 
 template <> cudaError_t Launch<T>::ssf_epi(const Geo& g, const void* P, const StageArgs& a, cudaStream_t st) {
-  k_ssf_epi<T><<<grid1d(g.S, 256), 256, 0, st>>>((const V*)P, g, a);
-  ++g_launches;
-  return cudaGetLastError();
+  return launch_chain(chained(g), k_ssf_epi<T>, grid1d(g.S, 256), 256, 0, st, (const V*)P, g, a);
 }
 
 template <> cudaError_t Launch<T>::ssf_rbc_epi(const Geo& g, const void* P, const SffArgs& a, cudaStream_t st) {
-  k_ssf_rbc_epi<T><<<grid1d(g.S, 256), 256, 0, st>>>((const V*)P, g, a);
-  ++g_launches;
-  return cudaGetLastError();
+  return launch_chain(chained(g), k_ssf_rbc_epi<T>, grid1d(g.S, 256), 256, 0, st, (const V*)P, g, a);
 }
 
 template <> cudaError_t Launch<T>::sss_rbc_epi(const Geo& g, const void* P, const SffArgs& a, cudaStream_t st) {
-  k_sss_rbc_epi<T><<<grid1d(2 * g.S, 256), 256, 0, st>>>((const T*)P, g, a);
-  ++g_launches;
-  return cudaGetLastError();
+  return launch_chain(chained(g), k_sss_rbc_epi<T>, grid1d(2 * g.S, 256), 256, 0, st, (const T*)P, g, a);
 }
 
 template <> cudaError_t Launch<T>::mhd_epi(const Geo& g, const void* P, const SffArgs& a, cudaStream_t st) {
-  k_mhd_epi<T><<<grid1d(g.S, 256), 256, 0, st>>>((const V*)P, g, a);
-  ++g_launches;
-  return cudaGetLastError();
+  return launch_chain(chained(g), k_mhd_epi<T>, grid1d(g.S, 256), 256, 0, st, (const V*)P, g, a);
 }
 
 template <> cudaError_t Launch<T>::dealias_copy(const Geo& g, const void* A, void* B, int ncomp, cudaStream_t st) {

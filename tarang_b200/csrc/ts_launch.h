@@ -30,15 +30,17 @@ template <typename T> struct Launch {
   // form 0 conservative (3 fields out), 1 rotational (6), 3 adjoint of the rotational form (9: also
   // lsc c^-1 P lam from the cotangent lam)
   // kept != 0 (forms 0, 1 with two-thirds dealiasing): write only the columns with 3|ky| <= Ny, 3 kz <= Nz
-  // form 5: u and the giver u inside |K| <= rad (6 fields) for the per-sphere energy flux
+  // form 4: the adjoint's cotangent fields 6-8; form 5: the giver, u inside |K| <= rad, into
+  // fields 3-5 for the per-sphere energy flux
   static cudaError_t inv_x(const Geo& g, int form, const void* U, void* W, const void* tw, const void* lam,
                            double lsc, cudaStream_t st, int kept = 0, double rad = 0.0);
   // form 0 conservative, 1 rotational, 2 Boussinesq (u, T), 3 adjoint of the rotational form,
   // 5 MHD (Elsasser products), 6 flux giver (u_i g_j)
   // nmem members, member fields msP complex apart
   // zkeep >= 0: input rows kz > zkeep are zero and not read
+  // q (form 6): u is read there (three components) instead of from P
   static cudaError_t z_fused(const Geo& g, int form, void* P, const void* tw, int* err, cudaStream_t st,
-                             int nmem = 1, long long msP = 0, int zkeep = -1);
+                             int nmem = 1, long long msP = 0, int zkeep = -1, const void* q = nullptr);
   static cudaError_t z_single(const Geo& g, int dir, const void* in, void* out, int ncomp, const void* tw, cudaStream_t st);
   // SSS: the fused z pass on real coefficients (form 0 / 2 products; zin / zout sine masks)
   static cudaError_t sss_z_fused(const Geo& g, int form, void* P, const void* tw, const void* tq, int zin, int zout,
@@ -93,13 +95,16 @@ template <typename T> struct Launch {
   // doubles (the per-block partials follow the result); the sums are reproducible bit for bit
   static cudaError_t shell(const Geo& g, const void* A, int ncomp, int nbins, double* bins, cudaStream_t st,
                            const void* B = nullptr, unsigned cap = SHELL_MAX_BLOCKS);
-  // per-sphere energy flux: out[0] = sum over |K| > R of 2 mult Re(N . conj(D U)), N from the
-  // nine x-forward-transformed giver products in P; out must hold 1 + 148 * 16 doubles
+  // per-sphere energy flux: out[1 ...] = per-block sums over |K| > R of 2 mult Re(N . conj(D U)), N
+  // from the nine x-forward-transformed giver products in P; out must hold 1 + 148 * 16 doubles
   static cudaError_t ssf_giver(const Geo& g, const void* U, void* P, double R, cudaStream_t st);
   static cudaError_t ssf_flux_outside(const Geo& g, const void* P, const void* U, double R, int qx, int qy,
                                       double* out, cudaStream_t st);
   static cudaError_t flux_outside(const Geo& g, const void* P, const void* U, double R, double* out,
                                   cudaStream_t st);
+  // the fixed-order sums of the partials of n_radii such launches (out = part + r * pitch) into res
+  static cudaError_t flux_finish(const Geo& g, const double* part, long long pitch, int n_radii, double* res,
+                                 cudaStream_t st);
   // the same on SSS (real coefficients, sine letters along x, y and z)
   static cudaError_t sss_giver(const Geo& g, const void* U, void* P, double R, cudaStream_t st);
   static cudaError_t sss_flux_outside(const Geo& g, const void* P, const void* U, double R, int qx, int qy, int qz,

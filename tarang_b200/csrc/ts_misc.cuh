@@ -13,6 +13,7 @@ namespace ts {
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void k_reality(C<T>* A, int ncomp, Geo g) {
+  chain_begin();
   typedef C<T> V;
   const long long plane = (long long)g.Nx * g.Ny;
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -86,9 +87,10 @@ __global__ void k_force_scatter(const C<T>* __restrict__ fc, C<T>* __restrict__ 
 // One block.  fc: 3 comps of (2km+1)(2km+1)(km+1).
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void k_carati(const C<T>* __restrict__ U, C<T>* fc, Geo g, int km, double r_in, double r_out,
+__global__ void k_carati(const C<T>* U, C<T>* fc, Geo g, int km, double r_in, double r_out,
                          const double* __restrict__ esup, const double* __restrict__ hsup,
                          const double* __restrict__ mis, int nsup) {
+  chain_begin();
   typedef C<T> V;
   const int n = 2 * km + 1;
   const int ncube = n * n * (km + 1);
@@ -226,6 +228,14 @@ __global__ void k_energy(const C<T>* __restrict__ A, const C<T>* __restrict__ B,
 // out[0] = sum of the n partial sums out[1..n], in an order that does not depend
 // on scheduling (one block), so energies and the normalised initial condition are
 // reproducible bit for bit
+// res[r] = the sum of the n partials at out + r * pitch + 1 (block r; the order of k_sum_partials)
+static __global__ void k_sum_partials_many(const double* out, long long pitch, int n, double* res) {
+  const double* o = out + blockIdx.x * pitch;
+  double s = 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s += o[1 + i];
+  s = block_sum(s);
+  if (threadIdx.x == 0) res[blockIdx.x] = s;
+}
 static __global__ void k_sum_partials(double* out, int n) {
   double s = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += out[1 + i];
@@ -374,31 +384,34 @@ __global__ void __launch_bounds__(32 * SHELL_WARPS)
 // (Prod_out_sphere_nlinV prod_nlinV.cc:61-69, Local_shell_mult_single universal_ET.cc:51-70),
 // D = the dealias mask; k_sum_partials adds the blocks in a fixed order.
 template <typename T>
-__global__ void k_flux_outside(const C<T>* __restrict__ P, const C<T>* __restrict__ U, Geo g, double R,
-                               double* __restrict__ out) {
-  const long long n = g.S;
+__global__ void __launch_bounds__(256) k_flux_outside(const C<T>* __restrict__ P, const C<T>* __restrict__ U, Geo g,
+                                                      double K2max, double* __restrict__ out) {
+  typedef C<T> V;
+  // 32-bit index arithmetic (a component holds < 2^31 modes); K2max: |K| > R as K^2 > K2max
+  const unsigned n = (unsigned)g.S;
   const double inv = 1.0 / ((double)g.Nx * g.Ny * g.Nz);
   double s = 0;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int lz = (int)(e % g.Hz);
-    const int ly = (int)((e / g.Hz) % g.Ny);
-    const int lx = (int)(e / ((long long)g.Ny * g.Hz));
-    if (dealias_zero(g.dealias, 0, lx, ly, lz, g.Nx, g.Ny, g.Nz)) continue;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const unsigned r = e / (unsigned)g.Hz;
+    const int lz = (int)(e - r * g.Hz), lx = (int)(r / (unsigned)g.Ny), ly = (int)(r - (unsigned)lx * g.Ny);
     const double K[3] = {kfft(lx, g.Nx) * g.kf[0], kfft(ly, g.Ny) * g.kf[1], lz * g.kf[2]};
-    const double Kmag = sqrt((K[0] * K[0] + K[1] * K[1]) + K[2] * K[2]);
-    if (!(Kmag > R)) continue;
+    if (!((K[0] * K[0] + K[1] * K[1]) + K[2] * K[2] > K2max)) continue;
+    if (dealias_zero(g.dealias, 0, lx, ly, lz, g.Nx, g.Ny, g.Nz)) continue;
+    V q[9], u[3];
+#pragma unroll
+    for (int f = 0; f < 9; ++f) q[f] = P[f * g.S + e];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) u[i] = U[i * g.S + e];
     double re = 0;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       double nr = 0, ni = 0;
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
-        const C<T> q = P[(3 * j + i) * n + e];
-        nr -= K[j] * (double)q.y;
-        ni += K[j] * (double)q.x;
+        nr -= K[j] * (double)q[3 * j + i].y;
+        ni += K[j] * (double)q[3 * j + i].x;
       }
-      const C<T> u = U[i * n + e];
-      re += (nr * inv) * (double)u.x + (ni * inv) * (double)u.y;
+      re += (nr * inv) * (double)u[i].x + (ni * inv) * (double)u[i].y;
     }
     s += 2.0 * multiplicity(0, lx, ly, lz, g.Nx, g.Ny) * re;
   }

@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
     }
     __syncthreads();  // every thread has read tile buf: field f + 2 may overwrite it
     issue(f + 2, buf);
-    fft_regs<N, E, 1, 0, false, false, best_swk(N, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tq, 4);
+    fft_regs<N, E, 1, 0, 0, false, best_swk(N, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tq, 4);
     if (ok) {
       V* d = W + f * g.S + col;
 #pragma unroll
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
       if (sine && k >= N / 2) x = scale(x, (T)-1);
       v[s] = x;
     }
-    fft_regs<N, E, -1, 0, false, false, best_swk(N, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tq, 4);
+    fft_regs<N, E, -1, 0, 0, false, best_swk(N, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tq, 4);
 #pragma unroll
     for (int s = 0; s < E; ++s) xch[final_row<N, E>(t, s) * CW + c] = v[s];
     __syncthreads();
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
       }
       v[s] = z;
     }
-    fft_regs<N, E, 1, 0, false, false, best_swk(N, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tq, 4);
+    fft_regs<N, E, 1, 0, 0, false, best_swk(N, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tq, 4);
     if (ok) {
 #pragma unroll
       for (int s = 0; s < E; ++s) {
@@ -272,6 +272,7 @@ __device__ __forceinline__ int sc_row_limit(int mode, int basis, int ly, int lz,
 template <typename T, int N, int E, int CW, int DIR, int MINB>
 __global__ void __launch_bounds__(CW * (N / E), MINB)
     k_sc_x(ScArgs a, Geo g, const C<T>* __restrict__ tq) {
+  chain_begin();
   typedef C<T> V;
   constexpr int SWK = best_swk(N, E, CW, (int)sizeof(V));
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(CW * (N / E), MINB)
 #pragma unroll
     for (int s = 0; s < E; ++s)
       if (sine && load_row<N, E>(t, s) >= N / 2) v[s] = mk<V>(-v[s].x, -v[s].y);
-    fft_regs<N, E, -1, 0, false, false, SWK>(v, t, xch, CW, c, tq, 4);
+    fft_regs<N, E, -1, 0, 0, false, SWK>(v, t, xch, CW, c, tq, 4);
 #pragma unroll
     for (int s = 0; s < E; ++s) xch[final_row<N, E>(t, s) * CW + c] = v[s];
     __syncthreads();
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(CW * (N / E), MINB)
       if (m == 0) v[s] = sine ? mk<V>(0, 0) : v[s];
       else v[s] = mul(conjg(tq[m]), sine ? add_i<-1>(q[s], v[s]) : add_i<-1>(v[s], q[s]));
     }
-    fft_regs<N, E, 1, 0, false, false, SWK>(v, t, xch, CW, c, tq, 4);
+    fft_regs<N, E, 1, 0, 0, false, SWK>(v, t, xch, CW, c, tq, 4);
     if (!ok) return;
 #pragma unroll
     for (int s = 0; s < E; ++s) {
@@ -503,7 +504,8 @@ __global__ void __launch_bounds__(256) k_sff_epi(const C<T>* __restrict__ P, Geo
 // series where sff_prod_sine): assembly of N1..N3, NT (the terms of k_sff_fwd_x), then
 // sff_epilogue.  One thread per element, every array access coalesced.
 template <typename T>
-__global__ void __launch_bounds__(256) k_sff_prod_epi(const C<T>* __restrict__ P, Geo g, SffArgs a) {
+__global__ void __launch_bounds__(256) k_sff_prod_epi(const C<T>* P, Geo g, SffArgs a) {
+  chain_begin();
   typedef C<T> V;
   const long long mb = blockIdx.y;
   P += mb * a.msP;
@@ -595,7 +597,7 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
       v[s] = x;
     }
     issue(f + 2, buf);
-    fft_regs<N, E, -1, 0, false, false, best_swk(N, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tq, 4);
+    fft_regs<N, E, -1, 0, 0, false, best_swk(N, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tq, 4);
     // pair terms Z_{N-m} through the exchange tile
 #pragma unroll
     for (int s = 0; s < E; ++s) xch[final_row<N, E>(t, s) * CW + c] = v[s];
@@ -648,7 +650,8 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
 //   epilogue (RK_SF.cc:97-221).  One thread per element, every access coalesced.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256) k_scalar_epi(const C<T>* __restrict__ P, Geo g, SffArgs a) {
+__global__ void __launch_bounds__(256) k_scalar_epi(const C<T>* P, Geo g, SffArgs a) {
+  chain_begin();
   typedef C<T> V;
   const T inv = (T)(1.0 / ((double)g.Nx * g.Ny * g.Nz));
   const V* U0 = reinterpret_cast<const V*>(a.U0);
@@ -730,7 +733,8 @@ __global__ void __launch_bounds__(256) k_scalar_epi(const C<T>* __restrict__ P, 
 //   Compiled for three blocks per SM (66 registers): with 123 it ran 20 % slower.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256, 3) k_mhd_epi(const C<T>* __restrict__ P, Geo g, SffArgs a) {
+__global__ void __launch_bounds__(256, 3) k_mhd_epi(const C<T>* P, Geo g, SffArgs a) {
+  chain_begin();
   typedef C<T> V;
   const T inv = (T)(1.0 / ((double)g.Nx * g.Ny * g.Nz));
   const V* U0 = reinterpret_cast<const V*>(a.U0);
@@ -812,7 +816,8 @@ __global__ void __launch_bounds__(256, 3) k_mhd_epi(const C<T>* __restrict__ P, 
 //   IF-RK4 stage update as the FFF step (RK.cc:91-170); no reality condition.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256) k_ssf_epi(const C<T>* __restrict__ P, Geo g, StageArgs a) {
+__global__ void __launch_bounds__(256) k_ssf_epi(const C<T>* P, Geo g, StageArgs a) {
+  chain_begin();
   typedef C<T> V;
   const V* U0 = reinterpret_cast<const V*>(a.U0);
   V* Uc = reinterpret_cast<V*>(a.Ucur);
@@ -904,7 +909,8 @@ __global__ void __launch_bounds__(256) k_sss_dealias_copy(const T* __restrict__ 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_sss_epi(const T* __restrict__ P, Geo g, StageArgs a) {
+__global__ void __launch_bounds__(256) k_sss_epi(const T* P, Geo g, StageArgs a) {
+  chain_begin();
   const long long per = 2 * g.S;
   const T* U0 = reinterpret_cast<const T*>(a.U0);
   T* Uc = reinterpret_cast<T*>(a.Ucur);
@@ -980,7 +986,8 @@ __global__ void __launch_bounds__(256) k_sss_epi(const T* __restrict__ P, Geo g,
 // SSF: x and y derivatives of a sine series +K, of a cosine series -K; z: i Kz.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256) k_ssf_rbc_epi(const C<T>* __restrict__ P, Geo g, SffArgs a) {
+__global__ void __launch_bounds__(256) k_ssf_rbc_epi(const C<T>* P, Geo g, SffArgs a) {
+  chain_begin();
   typedef C<T> V;
   V* U0 = const_cast<V*>(reinterpret_cast<const V*>(a.U0));
   V* T0 = const_cast<V*>(reinterpret_cast<const V*>(a.T0));
@@ -1054,7 +1061,8 @@ __global__ void __launch_bounds__(256) k_ssf_rbc_epi(const C<T>* __restrict__ P,
 // SSS: real coefficients in the padded real layout; every axis sine +K, cosine -K.
 // Parities: u1u1..u3u3 CCC, u1u2 SSC, u2u3 CSS, u3u1 SCS, u1T CCC, u2T SSC, u3T SCS.
 template <typename T>
-__global__ void __launch_bounds__(256) k_sss_rbc_epi(const T* __restrict__ P, Geo g, SffArgs a) {
+__global__ void __launch_bounds__(256) k_sss_rbc_epi(const T* P, Geo g, SffArgs a) {
+  chain_begin();
   const long long per = 2 * g.S;
   T* U0 = const_cast<T*>(reinterpret_cast<const T*>(a.U0));
   T* T0 = const_cast<T*>(reinterpret_cast<const T*>(a.T0));

@@ -1,0 +1,125 @@
+"""Transforms and steps at the edges of the line kernels' ranges: the shortest and longest
+lines of every axis, lengths with a factor 3, planes whose columns end inside a column tile.
+
+The transforms are compared with numpy / scipy in FP64; an FFT of n points of unit-variance
+data loses about eps * log2(n) in relative L2 norm, so the bounds are 4 eps log2(points).
+The steps are compared with the FP64 oracle: the state moves by a few per cent, FP32
+states are rounded to 2^-24 each stage, so 1e-6 holds for FP32 and 1e-13 for FP64."""
+import math
+
+import numpy as np
+import pytest
+
+from oracle import tarang_ref as R
+
+pytestmark = pytest.mark.gpu
+
+EPS = {"f32": 2.0 ** -23, "f64": 2.0 ** -52}
+
+
+def rel(a, b):
+    return float(np.linalg.norm((np.asarray(a) - b).ravel()) / np.linalg.norm(np.asarray(b).ravel()))
+
+
+TRANSFORMS = [("FFF", "FFF", N) for N in ((16, 16, 16), (1024, 16, 16), (16, 1024, 32), (32, 16, 1024), (512, 32, 16),
+                                          (16, 512, 64), (32, 16, 512))]
+TRANSFORMS += [("SFF", p, N) for p in ("SFF", "CFF") for N in ((16, 48, 16), (96, 16, 32), (512, 16, 16), (48, 96, 64))]
+TRANSFORMS += [("SSF", p, N) for p in ("SCF", "CSF") for N in ((16, 512, 16), (48, 96, 32), (256, 16, 128))]
+TRANSFORMS += [("SSS", p, N) for p in ("SCC", "CSS") for N in ((16, 16, 16), (96, 48, 1024), (512, 16, 32))]
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("basis,parity,N", TRANSFORMS)
+def test_transforms_at_line_edges(cuda, basis, parity, N, prec):
+    import torch
+    import tarang_b200 as tb
+    g = R.Grid(N, (1.0, 1.0, 1.0), basis)
+    plan = tb.Plan(N, basis=basis, precision=prec)
+    rt = torch.float32 if prec == "f32" else torch.float64
+    rng = np.random.default_rng(7)
+    u = rng.standard_normal((2,) + N)
+    par = {"FFF": "F", "SFF": parity[0]}.get(basis, parity)
+    want = np.stack([R.forward(g, u[i], par) for i in range(2)])
+    real = torch.zeros((2,) + N[:2] + (N[2] + 2,), dtype=rt, device=cuda)
+    real[..., : N[2]] = torch.from_numpy(u).to(rt)
+    real[..., N[2]:] = float("nan")  # the padding is not read
+    spec = torch.empty((2,) + plan.spec_shape, dtype=plan.torch_dtype(), device=cuda)
+    plan.forward(real, spec, parity)
+    got = spec.cpu().numpy()
+    if basis == "SSS":
+        got = got.view(got.real.dtype)
+        assert np.all(got[..., N[2]:] == 0)
+        got = got[..., : N[2]]
+    tol = 4 * EPS[prec] * math.log2(np.prod(N))
+    assert rel(got, want) < tol
+    back = torch.full_like(real, float("nan"))
+    plan.inverse(spec, back, parity)
+    out = back.cpu().numpy()
+    assert np.all(out[..., N[2]:] == 0)
+    u0 = np.stack([R.inverse(g, want[i], par) for i in range(2)])
+    assert rel(out[..., : N[2]], u0) < 2 * tol
+
+
+STEPS = [("rotational", "two_thirds", N) for N in ((16, 16, 16), (1024, 16, 32), (16, 1024, 16), (16, 32, 1024),
+                                                   (512, 16, 16), (32, 16, 512), (128, 32, 16), (256, 16, 32))]
+STEPS += [("conservative", "reference", N) for N in ((16, 16, 16), (1024, 16, 16), (16, 512, 32), (16, 16, 1024), (64, 32, 256),
+                                                     (128, 16, 16), (256, 16, 16))]
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("form,dealias,N", STEPS)
+def test_forced_step_at_line_edges(cuda, form, dealias, N, prec):
+    import torch
+    import tarang_b200 as tb
+    g = R.Grid(N)
+    es = np.zeros(g.n_shells())
+    es[3] = 0.1
+    V = R.init_energy_spectrum(g, R.spectrum_k4_gauss(g.n_shells(), 4.0), 0, 0.5)
+    mode = {"reference": 1, "two_thirds": 2}[dealias]
+    want = R.rk4_step(R.FluidConfig(g, 0.01, 1e-2, mode, form, True, R.CaratiForcing(2.0, 3.0, es)), V)
+    plan = tb.Plan(N, precision=prec, nlin_form=form, dealias=dealias, nu=0.01, dt=1e-2,
+                   forcing=tb.Forcing(2.0, 3.0, es))
+    u = torch.from_numpy(V).to(plan.torch_dtype()).to(cuda)
+    plan.rk4_step(u, 1)
+    assert rel(u.cpu().numpy(), want) < {"f32": 1e-6, "f64": 1e-13}[prec]
+
+
+RBC = [("SFF", (16, 16, 48)), ("SFF", (96, 48, 16)), ("SFF", (16, 1, 96)), ("SFF", (512, 16, 16)), ("SSF", (48, 96, 16)),
+       ("SSF", (16, 16, 96)), ("SSF", (512, 16, 16)), ("SSS", (16, 96, 16)), ("SSS", (96, 16, 512)), ("SSS", (16, 16, 1024))]
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("basis,N", RBC)
+def test_convection_step_at_line_edges(cuda, basis, N, prec):
+    import torch
+    import tarang_b200 as tb
+    kf = (math.pi, 2 * math.pi, 2 * math.pi) if basis == "SFF" else (math.pi,) * 3
+    g = R.Grid(N, kf, basis)
+    rng = np.random.default_rng(3)
+    par = {"SFF": ("S", "C", "C", "S"), "SSF": ("SCF", "CSF", "CCF", "SCF"), "SSS": ("SCC", "CSC", "CCS", "SCC")}[basis]
+    # random fields inside the dealiased range, without Nyquist planes, U solenoidal
+    F = np.stack([R.reality_fix(g, R.forward(g, 0.3 * rng.standard_normal(N), p)) for p in par])
+    F[..., R.dealias_mask(g, 2)] = 0
+    U, T = -R.project_rhs(g, F[:3]), F[3]
+    cfg = R.RBCConfig(grid=g, Ra=1e4, Pr=1.0, dt=1e-3, dealias_mode=1)
+    wu, wt = R.rbc_rk4_step(cfg, U, T)
+    plan = tb.Plan(N, basis=basis, precision=prec, kfactor=kf, dealias="reference", nu=cfg.nu, kappa=cfg.kappa, Ra=1e4,
+                   Pr=1.0, dt=1e-3)
+
+    def pack(a):
+        if basis == "SSS":
+            p = np.zeros(a.shape[:-1] + (a.shape[-1] + 2,))
+            p[..., : a.shape[-1]] = a
+            a = p.view(np.complex128)
+        return torch.from_numpy(np.ascontiguousarray(a)).to(plan.torch_dtype()).to(cuda)
+
+    u, t = pack(U), pack(T[None])
+    plan.rk4_step_rbc(u, t, 1)
+
+    def unpack(x):
+        x = x.cpu().numpy().astype(np.complex128)
+        return x.view(np.float64)[..., : N[2]] if basis == "SSS" else x
+
+    tol = {"f32": 1e-6, "f64": 1e-13}[prec]
+    assert rel(unpack(u), wu) < tol
+    assert rel(unpack(t)[0], wt) < tol
