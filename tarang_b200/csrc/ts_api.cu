@@ -48,6 +48,7 @@ struct ts_plan {
   void* Ucur = nullptr;
   void* tot = nullptr;
   void* P = nullptr;  // nP components of transform / product work fields
+  long long P_elems = 0, P_asked = 0;  // complex elements that P holds, and the most that were asked for
   int nP = 0;
   int nS = 0;         // components of the stage field Ucur and the accumulator tot
   void* twx = nullptr;
@@ -271,6 +272,53 @@ static void compute_modes_in_shell(ts_plan* p) {
       }
 }
 
+// line pitch of the compact inverse-transformed fields of product form `form`, 0: in place
+static int compact_pitch(const ts_plan* p, const Geo& g, int form) {
+  const int h = p->prec ? Launch<float>::inverse_pitch(g, form) : Launch<double>::inverse_pitch(g, form);
+  return h != g.Hz ? h : 0;
+}
+
+// Work fields for nprod components in place, or for nin compact inverse-transformed fields
+// followed by nout products where a step of product form `form` takes that layout.  The second,
+// larger size is a wish: without the memory for it the step runs in place.
+static int alloc_work(ts_plan* p, int nprod, int form, int nin, int nout) {
+  Geo g = p->g;
+  for (int c = 0; c < TUNE_NCLASS; ++c) g.tv[c] = g.tb[c] = 0;
+  const long long base = nprod * g.S, h = compact_pitch(p, g, form);
+  const long long want = std::max(base, h ? nin * (long long)g.Nx * g.Ny * h + nout * g.S : 0);
+  if (want <= p->P_asked && p->nP >= nprod) return TS_OK;
+  CK(cudaStreamSynchronize(p->st));
+  CK(cudaFree(p->P));
+  p->P = nullptr;
+  p->nP = 0;
+  p->P_elems = 0;
+  const long long most = std::max(want, p->P_asked);
+  long long got = most;
+  if (cudaMalloc(&p->P, most * p->cb) != cudaSuccess) {
+    cudaGetLastError();
+    got = base;
+    CK(cudaMalloc(&p->P, base * p->cb));
+  }
+  p->P_asked = most;
+  p->P_elems = got;
+  p->nP = nprod;
+  return TS_OK;
+}
+
+// The geometry of a right-hand side of product form `form` (nin fields in, nout products out) and
+// where its products go: after the compact inverse-transformed fields, or over them.
+static Geo step_geo(const ts_plan* p, int form, int nin, int nout, bool kept, char** prod) {
+  Geo g = p->g;
+  *prod = (char*)p->P;
+  const long long h = kept ? compact_pitch(p, g, form) : 0, sp = (long long)g.Nx * g.Ny * h;
+  if (h && nin * sp + nout * g.S <= p->P_elems) {
+    g.Hp = (int)h;
+    g.Sp = sp;
+    *prod += nin * sp * (long long)p->cb;
+  }
+  return g;
+}
+
 static int ensure_scratch(ts_plan* p, size_t n) {
   if (p->dscr_n >= n) return TS_OK;
   if (p->dscr) cudaFree(p->dscr);
@@ -418,6 +466,8 @@ int ts_plan_create(const ts_config* cfg, ts_plan** out) {
   g.Nz = cfg->N[2];
   g.Hz = g.Nz / 2 + 1;
   g.S = (long long)g.Nx * g.Ny * g.Hz;
+  g.Hp = g.Hz;
+  g.Sp = g.S;
   for (int i = 0; i < 3; ++i) g.kf[i] = cfg->kfactor[i];
   g.basis = cfg->basis;
   g.dealias = cfg->dealias_mode;
@@ -437,7 +487,7 @@ int ts_plan_create(const ts_config* cfg, ts_plan** out) {
     return TS_OK;
   };
   // SFF (Boussinesq): stage / accumulator fields carry T as a fourth component,
-  // and the z pass makes nine products
+  // and the z pass makes eight products (the flux giver nine)
   const int ncs = cfg->basis == TS_BASIS_SFF ? 4 : 3,
             nps = cfg->basis == TS_BASIS_SFF ? 9 : (cfg->basis == TS_BASIS_SSS ? 12 : 6);
   if (cfg->basis == TS_BASIS_SFF && g.Nx > 512) {
@@ -447,8 +497,8 @@ int ts_plan_create(const ts_config* cfg, ts_plan** out) {
   }
   CKP(alloc(&p->Ucur, ncs * g.S * p->cb));
   CKP(alloc(&p->tot, ncs * g.S * p->cb));
-  CKP(alloc(&p->P, nps * g.S * p->cb));
-  p->nP = nps;
+  const bool rot = cfg->nlin_form == TS_NLIN_ROTATIONAL;
+  CKP(alloc_work(p, nps, rot ? 1 : 7, rot ? 6 : 3, rot ? 3 : 5));
   p->nS = ncs;
   if (p->prec) {
     CKP(upload_twiddles<float>(g.Nx, &p->twx));
@@ -650,7 +700,6 @@ static double fff_pass_bytes(const ts_plan* p, int cls, int nin, int nout, int k
 }
 
 static int rhs_fff(ts_plan* p, const void* Uin, int mode, const StageArgs& a_in) {
-  const Geo& g = p->g;
   StageArgs a = a_in;
   a.err = p->err_d;
   a.ex = p->eax[0];
@@ -668,7 +717,10 @@ static int rhs_fff(ts_plan* p, const void* Uin, int mode, const StageArgs& a_in)
   // 3 kz <= Nz can be nonzero, so the inverse x pass writes only those, the y
   // inverse transforms only kz <= Nz/3 and reads only the 3|ky| <= Ny rows, and the
   // z pass reads only kz <= Nz/3 (the skipped memory is never read)
-  const int kept = g.dealias == TS_DEALIAS_TWO_THIRDS;
+  const int kept = p->g.dealias == TS_DEALIAS_TWO_THIRDS;
+  char* prod;
+  const Geo g = step_geo(p, zform, nin, nout, kept, &prod), gw = work_geo(g);
+  const bool compact = g.Hp != g.Hz;
   auto by = [&](int cls) { return p->prof ? fff_pass_bytes(p, cls, nin, nout, kept, mode, a.stage) : -1.0; };
   {
     ProfScope ps(p, TS_KCLASS_INV_X, by(TS_KCLASS_INV_X));
@@ -676,14 +728,15 @@ static int rhs_fff(ts_plan* p, const void* Uin, int mode, const StageArgs& a_in)
   }
   {
     ProfScope ps(p, TS_KCLASS_Y_INV, by(TS_KCLASS_Y_INV));
-    CK(LAUNCH(p, strided, g, 1, +1, p->P, nin, p->twy, p->st, 0, 0, kept ? g.Nz / 3 + 1 : 0, kept));
+    CK(LAUNCH(p, strided, gw, 1, +1, p->P, nin, p->twy, p->st, 0, 0, compact ? g.Hp : kept ? g.Nz / 3 + 1 : 0, kept));
   }
   {
     ProfScope ps(p, TS_KCLASS_Z, by(TS_KCLASS_Z));
-    CK(LAUNCH(p, z_fused, g, zform, p->P, p->twz, p->err_d, p->st, 1, 0, kept ? g.Nz / 3 : -1));
+    CK(LAUNCH(p, z_fused, g, zform, prod, p->twz, p->err_d, p->st, 1, 0, kept ? g.Nz / 3 : -1, nullptr,
+              compact ? p->P : nullptr));
   }
-  { ProfScope ps(p, TS_KCLASS_Y_FWD, by(TS_KCLASS_Y_FWD)); CK(LAUNCH(p, strided, g, 1, -1, p->P, nout, p->twy, p->st)); }
-  { ProfScope ps(p, TS_KCLASS_FWD_X, by(TS_KCLASS_FWD_X)); CK(LAUNCH(p, fwd_x, g, zform, mode, p->P, a, p->twx, p->st)); }
+  { ProfScope ps(p, TS_KCLASS_Y_FWD, by(TS_KCLASS_Y_FWD)); CK(LAUNCH(p, strided, g, 1, -1, prod, nout, p->twy, p->st)); }
+  { ProfScope ps(p, TS_KCLASS_FWD_X, by(TS_KCLASS_FWD_X)); CK(LAUNCH(p, fwd_x, g, zform, mode, prod, a, p->twx, p->st)); }
   return TS_OK;
 }
 
@@ -732,15 +785,8 @@ static int adjoint_supported(ts_plan* p) {
     g_last_error = "the adjoint step is implemented for FFF, rotational form, unforced plans";
     return TS_ERR_UNSUPPORTED;
   }
-  if (p->nP < 9) {
-    // the adjoint right-hand side transforms nine fields (u, w, and the projected cotangent)
-    CK(cudaStreamSynchronize(p->st));
-    CK(cudaFree(p->P));
-    p->P = nullptr;
-    p->nP = 0;
-    CK(cudaMalloc(&p->P, 9 * p->g.S * p->cb));
-    p->nP = 9;
-  }
+  // the adjoint right-hand side transforms nine fields (u, w, and the projected cotangent)
+  CKS(alloc_work(p, std::max(p->nP, 9), 1, 6, 3));
   return TS_OK;
 }
 
@@ -838,7 +884,7 @@ static int step_rbc(ts_plan* p, void* U0, void* T0) {
 // ---------------------------------------------------------------------------
 // FFF passive scalar (program.kind SCALAR_INCOMPRESS): RK4(U,T,P,F) with no force
 // ---------------------------------------------------------------------------
-static int ensure_work(ts_plan* p, int nstage, int nprod);
+static int ensure_work(ts_plan* p, int nstage, int nprod, int form = -1, int nin = 0, int nout = 0);
 
 static int scalar_supported(ts_plan* p) {
   if (p->cfg.basis != TS_BASIS_FFF || p->cfg.force_type != TS_FORCE_NONE ||
@@ -846,14 +892,14 @@ static int scalar_supported(ts_plan* p) {
     g_last_error = "the passive-scalar step is implemented for FFF, conservative form, unforced plans";
     return TS_ERR_UNSUPPORTED;
   }
-  // stage and accumulator fields carry T as a fourth component; the z pass makes nine products
+  // stage and accumulator fields carry T as a fourth component; the z pass makes eight products
   return ensure_work(p, 4, 9);
 }
 
 // one IF-RK4 step of U and the passive scalar T on the FFF basis (RK_SF.cc:97-221 with
 // Compute_force_TO_rhs_scalar, Tadvance_functions.cc:464-474, and Compute_nlin_scalar,
-// compute_nlin_SF.cc:75-112): dealiased u, T to real space, the nine products u_i u_j and
-// u_i T (z pass form 2), forward transforms, then N, NT, the projection and the stage update
+// compute_nlin_SF.cc:75-112): dealiased u, T to real space, the products u_i u_j (without the
+// trace, five) and u_i T (z pass form 2), forward transforms, then N, NT, the projection and the stage update
 static int step_scalar_fff(ts_plan* p, void* U0, void* T0) {
   const Geo& g = p->g;
   SffArgs a;
@@ -904,10 +950,9 @@ static int step_scalar_fff(ts_plan* p, void* U0, void* T0) {
 // ---------------------------------------------------------------------------
 // FFF incompressible MHD: RK4(U, W, P, F) with W = B, no force
 // ---------------------------------------------------------------------------
-static int ensure_work(ts_plan* p, int nstage, int nprod) {
-  if (p->nS >= nstage && p->nP >= nprod) return TS_OK;
-  CK(cudaStreamSynchronize(p->st));
+static int ensure_work(ts_plan* p, int nstage, int nprod, int form, int nin, int nout) {
   if (p->nS < nstage) {
+    CK(cudaStreamSynchronize(p->st));
     CK(cudaFree(p->Ucur));
     CK(cudaFree(p->tot));
     p->Ucur = p->tot = nullptr;
@@ -916,13 +961,7 @@ static int ensure_work(ts_plan* p, int nstage, int nprod) {
     CK(cudaMalloc(&p->tot, nstage * p->g.S * p->cb));
     p->nS = nstage;
   }
-  if (p->nP < nprod) {
-    CK(cudaFree(p->P));
-    p->P = nullptr;
-    p->nP = 0;
-    CK(cudaMalloc(&p->P, nprod * p->g.S * p->cb));
-    p->nP = nprod;
-  }
+  CKS(alloc_work(p, std::max(p->nP, nprod), form, nin, nout));
   return TS_OK;
 }
 
@@ -931,16 +970,20 @@ static int mhd_supported(ts_plan* p) {
     g_last_error = "the MHD step is implemented for FFF, unforced plans";
     return TS_ERR_UNSUPPORTED;
   }
-  // stage and accumulator fields carry U and B (6 components); nine Elsasser products
-  return ensure_work(p, 6, 9);
+  // stage and accumulator fields carry U and B (6 components); eight products
+  return ensure_work(p, 6, 9, 5, 6, 8);
 }
 
 // one IF-RK4 step of U (nu) and B (eta = the plan's kappa) (RK_VF_MHD.cc:126-186,
 // Compute_force_TO_rhs Tadvance_functions.cc:506-517, Compute_nlin(U, W)
-// compute_nlin_VF_MHD.cc:40-95): dealiased u, b to real space, the nine Elsasser
-// products Zp_i Zm_j (z pass form 5), forward transforms, then the MHD epilogue
+// compute_nlin_VF_MHD.cc:40-95): dealiased u, b to real space, the symmetric (without its
+// trace, five) and the antisymmetric (three) part of the Elsasser products Zp_i Zm_j (z pass
+// form 5), forward transforms, then the MHD epilogue
 static int step_mhd_fff(ts_plan* p, void* U0, void* B0) {
-  const Geo& g = p->g;
+  const int kept = p->g.dealias == TS_DEALIAS_TWO_THIRDS;
+  char* prod;
+  const Geo g = step_geo(p, 5, 6, 8, kept, &prod), gw = work_geo(g);
+  const bool compact = g.Hp != g.Hz;
   SffArgs a;
   memset(&a, 0, sizeof(a));
   a.health = p->err_d;
@@ -955,8 +998,7 @@ static int step_mhd_fff(ts_plan* p, void* U0, void* B0) {
     a.et[i] = p->eaxT[i];
   }
   const long long cs = 3 * g.S * (long long)p->cb;
-  const int kept = g.dealias == TS_DEALIAS_TWO_THIRDS;
-  void* P3 = (char*)p->P + cs;
+  void* P3 = (char*)p->P + 3 * g.Sp * (long long)p->cb;
   for (int stage = 1; stage <= 4; ++stage) {
     const void* Uin = stage == 1 ? U0 : p->Ucur;
     const void* Bin = stage == 1 ? B0 : (const void*)((const char*)p->Ucur + cs);
@@ -966,13 +1008,14 @@ static int step_mhd_fff(ts_plan* p, void* U0, void* B0) {
       CK(LAUNCH(p, inv_x, g, 0, Uin, p->P, p->twx, nullptr, 0.0, p->st, kept));
       CK(LAUNCH(p, inv_x, g, 0, Bin, P3, p->twx, nullptr, 0.0, p->st, kept));
     }
-    { ProfScope ps(p, TS_KCLASS_Y_INV); CK(LAUNCH(p, strided, g, 1, +1, p->P, 6, p->twy, p->st, 0, 0, kept ? g.Nz / 3 + 1 : 0, kept)); }
-    { ProfScope ps(p, TS_KCLASS_Z); CK(LAUNCH(p, z_fused, g, 5, p->P, p->twz, p->err_d, p->st, 1, 0, kept ? g.Nz / 3 : -1)); }
-    { ProfScope ps(p, TS_KCLASS_Y_FWD); CK(LAUNCH(p, strided, g, 1, -1, p->P, 8, p->twy, p->st)); }
+    { ProfScope ps(p, TS_KCLASS_Y_INV); CK(LAUNCH(p, strided, gw, 1, +1, p->P, 6, p->twy, p->st, 0, 0, compact ? g.Hp : kept ? g.Nz / 3 + 1 : 0, kept)); }
+    { ProfScope ps(p, TS_KCLASS_Z); CK(LAUNCH(p, z_fused, g, 5, prod, p->twz, p->err_d, p->st, 1, 0, kept ? g.Nz / 3 : -1, nullptr,
+              compact ? p->P : nullptr)); }
+    { ProfScope ps(p, TS_KCLASS_Y_FWD); CK(LAUNCH(p, strided, g, 1, -1, prod, 8, p->twy, p->st)); }
     {
       ProfScope ps(p, TS_KCLASS_FWD_X);
-      CK(LAUNCH(p, strided, g, 0, -1, p->P, 8, p->twx, p->st));
-      CK(LAUNCH(p, mhd_epi, g, p->P, a, p->st));
+      CK(LAUNCH(p, strided, g, 0, -1, prod, 8, p->twx, p->st));
+      CK(LAUNCH(p, mhd_epi, g, prod, a, p->st));
     }
   }
   if (p->cfg.reality_fix) {
@@ -1866,8 +1909,8 @@ int ts_profile_read(ts_plan* p, int kclass, double* total_ms, long long* launche
     const int rot = p->cfg.nlin_form == TS_NLIN_ROTATIONAL;
     double b = 0;
     if (p->cfg.basis == TS_BASIS_SFF) {
-      // u1, u2, u3, T in; nine products out; the epilogue's state traffic averages 16 fields over a step
-      const double sff[TS_KCLASS_COUNT] = {8 * f, 8 * f, 13 * f, 18 * f, 25 * f, 0};
+      // u1, u2, u3, T in; eight products out; the epilogue's state traffic averages 16 fields over a step
+      const double sff[TS_KCLASS_COUNT] = {8 * f, 8 * f, 12 * f, 16 * f, 24 * f, 0};
       *bytes_per_launch = kclass < TS_KCLASS_COUNT ? sff[kclass] : 0;
       return TS_OK;
     }

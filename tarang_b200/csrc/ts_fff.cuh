@@ -23,6 +23,10 @@ enum { TUNE_X_INV = 0, TUNE_Y_INV = 1, TUNE_Z = 2, TUNE_Y_FWD = 3, TUNE_X_FWD = 
 struct Geo {
   int Nx, Ny, Nz, Hz;
   long long S;          // complex elements per component
+  // inverse-transformed fields of a right-hand side: complex elements per z line and per
+  // component (Hz and S, or the compact lines of Launch::inverse_pitch)
+  int Hp;
+  long long Sp;
   double kf[3];         // kfactor (reference kfactor[1..3])
   int basis;            // 0 FFF, 1 SFF
   int dealias;          // 0 none, 1 reference corner, 2 two thirds
@@ -31,6 +35,14 @@ struct Geo {
   signed char tv[TUNE_NCLASS] = {0, 0, 0, 0, 0};
   signed char tb[TUNE_NCLASS] = {0, 0, 0, 0, 0};
 };
+
+// the geometry as the strided passes see the inverse-transformed fields
+inline Geo work_geo(const Geo& g) {
+  Geo w = g;
+  w.Hz = g.Hp;
+  w.S = g.Sp;
+  return w;
+}
 
 // warps per block of the shell-sum kernel k_shell (each warp walks whole z lines)
 constexpr int SHELL_WARPS = 4;
@@ -299,9 +311,10 @@ __global__ void __launch_bounds__(CW * (L / E), MINB)
     // two-thirds dealiasing: only the columns with 3|ky| <= Ny and 3 kz <= Nz can be
     // nonzero; they are one run of columns here, the others are not written, and the y and
     // z passes treat them as zero without reading them
-    const unsigned qy = g.Ny / 3, nzk = g.Nz / 3 + 1, iy = q / nzk;
-    lz = q - iy * nzk;
-    ok = iy <= 2 * qy;
+    // (kept == 2: compact lines of whole tiles)
+    const unsigned qy = g.Ny / 3, nzk = g.Nz / 3 + 1, nzt = kept == 2 ? g.Hp : nzk, iy = q / nzt;
+    lz = q - iy * nzt;
+    ok = iy <= 2 * qy && lz < nzk;
     ly = iy <= qy ? iy : iy + g.Ny - (2 * qy + 1);
   } else {
     ok = q < inner;
@@ -347,9 +360,10 @@ __global__ void __launch_bounds__(CW * (L / E), MINB)
   }
   fft_regs<L, E, 1, 0, 0, false, best_swk(L, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tw, 1);
   if (!ok) return;
-  V* d = W + (f + (FORM == 5 ? 3 : 0)) * g.S + col;
+  V* d = W + (f + (FORM == 5 ? 3 : 0)) * g.Sp + (long long)ly * g.Hp + lz;
+  const long long wstride = (long long)g.Ny * g.Hp;
 #pragma unroll
-  for (int s = 0; s < E; ++s) d[final_row<L, E>(t, s) * rstride] = v[s];
+  for (int s = 0; s < E; ++s) d[final_row<L, E>(t, s) * wstride] = v[s];
 }
 
 // ---------------------------------------------------------------------------
@@ -719,15 +733,6 @@ __device__ __forceinline__ void zreg_inverse_loaded(const C<T>* X, bool live, in
   for (int s = 0; s < E; ++s) a[s] = out[s];
 }
 
-template <typename T, int M, int E, int TPL>
-__device__ __forceinline__ void zreg_inverse(const C<T>* X, bool live, int t, int partner,
-                                             const C<T>* __restrict__ tw, C<T>* xch, C<T> (&out)[E]) {
-  typedef C<T> V;
-  V XM;
-  zreg_load<T, M, E, TPL>(X, live, t, out, XM, M);
-  zreg_inverse_loaded<T, M, E, TPL>(X, live, t, partner, tw, xch, out, XM, M);
-}
-
 // R2C of one packed real line in registers (reversed radix schedule, so the
 // inverse's output order is its input order) and the store of its M+1 rows
 template <typename T, int M, int E, int TPL>
@@ -770,7 +775,7 @@ __device__ __forceinline__ void zreg_forward_store(C<T> (&p)[E], C<T>* Xo, bool 
 // the 12-element radix-3 lines (which would spill at 170), 4 for 512-point lines
 // (two warps per line, the pair terms through the exchange line; spilled at 170)
 // (8 for the 4-element variant)
-// (4 for the MHD and flux-giver forms, which hold six lines while they make nine products)
+// (4 for the MHD and flux-giver forms, which hold six lines while they make eight or nine products)
 template <int NZ, int EZ = 0, int FORM = 0> __host__ __device__ constexpr int zreg_min_blocks() {
   return EZ == 4 ? 8 : ((NZ / 2) % 3 == 0 ? 3 : ((NZ >= 1024 || FORM == 5 || FORM == 6) ? 4 : 6));
 }
@@ -787,7 +792,7 @@ __global__ void __launch_bounds__(zreg_threads<FORM>(), zreg_min_blocks<NZ, EZ, 
   constexpr int M = NZ / 2, H = M + 1, E = EZ ? EZ : ((M % 3 == 0) ? 12 : 8), TPL = M / E, LDX = zslot<M>();
   static_assert(TPL >= 1 && TPL <= 64, "a line spans at most two warps");
   constexpr int NIN = z_nin(FORM), NOUT = z_nout(FORM);
-  static_assert(NIN <= 6, "the adjoint form runs in k_z_reg_adj");
+  static_assert(NIN <= 6, "the adjoint form runs in k_z_pair_adj");
   constexpr int LPB = zreg_threads<FORM>() / TPL;
   __shared__ __align__(16) V xch_all[LPB * LDX];
   P += blockIdx.y * msP;  // member blockIdx.y
@@ -862,13 +867,13 @@ template <typename T> __host__ __device__ constexpr int zpair_slot(int NZ) { ret
 // lines of exchange space per pair: the inputs go through it together, the products NB at a time
 __host__ __device__ constexpr int zpair_lines(int nin, int nb) { return nin > nb ? nin : nb; }
 
-// the two lines X, X + H of NC components (stride cs) as Z rows in registers, rows above zkeep
+// the two lines X, X + H (H: line pitch) of NC components (stride cs) as Z rows in registers, rows above zkeep
 // zero and not read; every load is issued before any of them is used
 template <typename T, int NZ, int E, int NC>
-__device__ __forceinline__ void zpair_load(const C<T>* X, long long cs, bool live0, bool live1, int t, int partner,
+__device__ __forceinline__ void zpair_load(const C<T>* X, int H, long long cs, bool live0, bool live1, int t, int partner,
                                            int zkeep, C<T> (&in)[NC][E]) {
   typedef C<T> V;
-  constexpr int M = NZ / 2, H = M + 1, TPL = NZ / E;
+  constexpr int M = NZ / 2, TPL = NZ / E;
   if constexpr (zpair_shfl<T, NZ, E>()) {
     // slots s < E/2 hold rows t + s TPL < M, slot E/2 of lane 0 row M
     V a[NC][E / 2], b[NC][E / 2], aM[NC], bM[NC];
@@ -971,7 +976,8 @@ __device__ __forceinline__ void zpair_forward_store(C<T> (&p)[NB][E], C<T>* X, l
 
 template <typename T, int NZ, int E, int FORM, int NTHR, int MINB, int NB>
 __global__ void __launch_bounds__(NTHR, MINB)
-    k_z_pair(C<T>* P, Geo g, const C<T>* __restrict__ tw, long long msP, int zkeep, const C<T>* Q) {
+    k_z_pair(C<T>* P, Geo g, const C<T>* __restrict__ tw, long long msP, int zkeep, const C<T>* Q,
+             const C<T>* X) {
   chain_begin();
   typedef C<T> V;
   constexpr int H = NZ / 2 + 1, TPL = NZ / E, PPB = NTHR / TPL, LDX = zpair_slot<T>(NZ), SLOT = PPB * LDX;
@@ -980,6 +986,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
   static_assert(NOUT % NB == 0 && NTHR % TPL == 0 && (!WARP || 32 % TPL == 0), "whole pairs per warp or block");
   extern __shared__ __align__(16) unsigned char smraw[];
   P += blockIdx.y * msP;  // member blockIdx.y
+  if (X == nullptr) X = P;
   const int l = threadIdx.x / TPL, t = threadIdx.x % TPL;
   const int lane = threadIdx.x & 31;
   const int partner = (lane - t) + (TPL - t) % TPL;  // lane holding the rows N - k
@@ -994,8 +1001,8 @@ __global__ void __launch_bounds__(NTHR, MINB)
     // u from Q (transformed once for all spheres), the giver from P
     const V* Ql = Q + (live0 ? line : 0) * H;
     V a[3][E], b[3][E];
-    zpair_load<T, NZ, E, 3>(Ql, g.S, live0, live1, t, partner, zkeep, a);
-    zpair_load<T, NZ, E, 3>(Pl + 3 * g.S, g.S, live0, live1, t, partner, zkeep, b);
+    zpair_load<T, NZ, E, 3>(Ql, H, g.S, live0, live1, t, partner, zkeep, a);
+    zpair_load<T, NZ, E, 3>(Pl + 3 * g.S, H, g.S, live0, live1, t, partner, zkeep, b);
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -1004,7 +1011,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
         in[c + 3][s] = b[c][s];
       }
   } else {
-    zpair_load<T, NZ, E, NIN>(Pl, g.S, live0, live1, t, partner, zkeep, in);
+    zpair_load<T, NZ, E, NIN>(X + (live0 ? line : 0) * g.Hp, g.Hp, g.Sp, live0, live1, t, partner, zkeep, in);
   }
   fft_regs_b<NZ, E, 1, NIN, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
 #pragma unroll
@@ -1045,7 +1052,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
   V* mus = reinterpret_cast<V*>(smraw) + PPB * (3 * LDX) + threadIdx.x;  // slot (f, s) at (f E + s) NTHR
   V* Pl = P + (live0 ? line : 0) * H;
   V in[3][E];
-  zpair_load<T, NZ, E, 3>(Pl + 6 * g.S, g.S, live0, live1, t, partner, M, in);
+  zpair_load<T, NZ, E, 3>(Pl + 6 * g.S, H, g.S, live0, live1, t, partner, M, in);
   fft_regs_b<NZ, E, 1, 3, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
 #pragma unroll
   for (int f = 0; f < 3; ++f)
@@ -1053,7 +1060,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
     for (int s = 0; s < E; ++s) mus[(f * E + s) * NTHR] = in[f][s];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    zpair_load<T, NZ, E, 3>(Pl + 3 * h * g.S, g.S, live0, live1, t, partner, zkeep, in);
+    zpair_load<T, NZ, E, 3>(Pl + 3 * h * g.S, H, g.S, live0, live1, t, partner, zkeep, in);
     fft_regs_b<NZ, E, 1, 3, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
 #pragma unroll
     for (int f = 0; f < 3; ++f) {

@@ -158,6 +158,14 @@ constexpr LdTile ld_tile(int L) {
                 : L == 128 ? LdTile{16, 8, 4} : L == 256 ? LdTile{16, 8, 2} : L == 512 ? LdTile{16, 8, 2}
                 : L == 1024 ? LdTile{16, 4, 2} : LdTile{12, 8, 4});
 }
+// the same for lines whose rows lie FAR_ROW_BYTES or more apart (the x axis of large grids), 0: no
+// other tile.  1024 points in FP32: with a page or so per row, 128-byte row segments beat the
+// second block per SM (512 x 512 planes, rows 1 MB apart: 1838 -> 1609 us); with nearer rows they
+// do not (256 x 256 planes, rows 264 KB apart: 364 -> 420 us).
+constexpr long long FAR_ROW_BYTES = 1 << 19;
+constexpr LdTile far_tile(int L) {
+  return std::is_same<T, float>::value && L == 1024 ? LdTile{32, 16, 1} : LdTile{0, 0, 0};
+}
 // inverse x kernel (one field per block)
 constexpr LdTile ix_tile(int L) {
   return std::is_same<T, float>::value
@@ -336,20 +344,26 @@ template <> cudaError_t Launch<T>::strided(const Geo& g, int axis, int dir, void
   if (v == 0 && bps == 0) {
     dispatch_L_sff(L, [&](auto Lc) {
       constexpr int LL = decltype(Lc)::value;
-      constexpr LdTile c = ld_tile(LL);
       const unsigned inner = inner_eff > 0 ? inner_eff : (axis == 0 ? g.Ny * g.Hz : g.Hz);
       const long long rstride = axis == 0 ? (long long)g.Ny * g.Hz : g.Hz;
       const unsigned nplane = axis == 0 ? inner : inner * (unsigned)g.Nx, ntot = nplane * (unsigned)nf;
-      constexpr size_t sm = (size_t)LL * c.CW * sizeof(V);
-      auto launch = [&](auto k) {
-        if ((err = smem_attr(k, sm)) != cudaSuccess) return;
-        err = launch_chain(chained(g, per == nf ? 1 : nf / per), k, (ntot + c.CW - 1) / c.CW, c.CW * (LL / c.E), sm, st,
-                           (const V*)data, (V*)(dst ? dst : data), ntot, nplane, inner, g.S, rstride,
-                           (long long)g.Ny * g.Hz, (const V*)tw, (unsigned)per, mstride, zero_hi, (T)scl);
+      auto tile = [&](auto far) {
+        constexpr LdTile c = decltype(far)::value ? far_tile(LL) : ld_tile(LL);
+        constexpr size_t sm = (size_t)LL * c.CW * sizeof(V);
+        auto launch = [&](auto k) {
+          if ((err = smem_attr(k, sm)) != cudaSuccess) return;
+          err = launch_chain(chained(g, per == nf ? 1 : nf / per), k, (ntot + c.CW - 1) / c.CW, c.CW * (LL / c.E), sm, st,
+                             (const V*)data, (V*)(dst ? dst : data), ntot, nplane, inner, g.S, rstride,
+                             (long long)g.Ny * g.Hz, (const V*)tw, (unsigned)per, mstride, zero_hi, (T)scl);
+        };
+        if (dir > 0) launch(k_strided_ld<T, LL, c.E, c.CW, 1, c.MINB, false>);
+        else if (scl == 1.0) launch(k_strided_ld<T, LL, c.E, c.CW, -1, c.MINB, false>);
+        else launch(k_strided_ld<T, LL, c.E, c.CW, -1, c.MINB, true>);
       };
-      if (dir > 0) launch(k_strided_ld<T, LL, c.E, c.CW, 1, c.MINB, false>);
-      else if (scl == 1.0) launch(k_strided_ld<T, LL, c.E, c.CW, -1, c.MINB, false>);
-      else launch(k_strided_ld<T, LL, c.E, c.CW, -1, c.MINB, true>);
+      if constexpr (far_tile(LL).CW > 0) {
+        if (rstride * (long long)sizeof(V) >= FAR_ROW_BYTES) return tile(std::true_type{});
+      }
+      tile(std::false_type{});
     });
     return err;
   }
@@ -407,7 +421,9 @@ template <> cudaError_t Launch<T>::inv_x(const Geo& g, int form, const void* U, 
     dispatch_L(g.Nx, [&](auto Lc) {
       constexpr int LL = decltype(Lc)::value;
       constexpr LdTile c = ix_tile(LL);
-      const long long cols = kept ? (long long)(2 * (g.Ny / 3) + 1) * (g.Nz / 3 + 1) : (long long)g.Ny * g.Hz;
+      const int nzt = g.Hp != g.Hz ? g.Hp : g.Nz / 3 + 1;  // columns of a kept line
+      const long long cols = kept ? (long long)(2 * (g.Ny / 3) + 1) * nzt : (long long)g.Ny * g.Hz;
+      if (kept) kept = g.Hp != g.Hz ? 2 : 1;
       constexpr size_t sm = (size_t)LL * c.CW * sizeof(V);
       auto run = [&](auto kern, int nf) {
         if ((err_ = smem_attr(kern, sm)) != cudaSuccess) return;
@@ -509,7 +525,7 @@ static cudaError_t z_slots(const Geo& g, void* P, const void* tw, cudaStream_t s
 
 template <int NZ, int FORM>
 static cudaError_t z_fused_impl(const Geo& g, void* P, const void* tw, int* zerr, cudaStream_t st, int nmem,
-                                long long msP, int zkeep, int v, const void* q = nullptr) {
+                                long long msP, int zkeep, int v, const void* q = nullptr, const void* x = nullptr) {
   constexpr int M = NZ / 2;
   if (zkeep < 0) zkeep = M;
   const long long nlines = (long long)g.Nx * g.Ny;
@@ -552,7 +568,7 @@ static cudaError_t z_fused_impl(const Geo& g, void* P, const void* tw, int* zerr
     auto k = k_z_pair<T, NZ, c.E, FORM, c.NTHR, c.MINB, c.NB>;
     if ((err = smem_attr(k, sm)) != cudaSuccess) return err;
     return launch_chain(chained(g, nmem), k, dim3((unsigned)((npairs + PPB - 1) / PPB), nmem), c.NTHR, sm, st, (V*)P, g,
-                        (const V*)tw, msP, zkeep, (const V*)(q ? q : P));
+                        (const V*)tw, msP, zkeep, (const V*)(q ? q : P), (const V*)x);
   }
   if constexpr (FORM == 3) {
     constexpr ZTile c = zp_tile(NZ, FORM);
@@ -566,17 +582,19 @@ static cudaError_t z_fused_impl(const Geo& g, void* P, const void* tw, int* zerr
 }
 
 template <> cudaError_t Launch<T>::z_fused(const Geo& g, int form, void* P, const void* tw, int* zerr,
-                                           cudaStream_t st, int nmem, long long msP, int zkeep, const void* q) {
+                                           cudaStream_t st, int nmem, long long msP, int zkeep, const void* q,
+                                           const void* x) {
   cudaError_t err = cudaErrorInvalidValue;
   if (form == 3 && nmem != 1) return err;  // the adjoint z pass has no member batching
+  if (x && nmem != 1) return err;
   dispatch_L_sff(g.Nz, [&](auto Lc) {
     constexpr int NZ = decltype(Lc)::value;
     const int v = g.tv[TUNE_Z];
-    if (form == 7) err = z_fused_impl<NZ, 7>(g, P, tw, zerr, st, nmem, msP, zkeep, v);
-    else if (form == 0) err = z_fused_impl<NZ, 0>(g, P, tw, zerr, st, nmem, msP, zkeep, 0);
-    else if (form == 1) err = z_fused_impl<NZ, 1>(g, P, tw, zerr, st, nmem, msP, zkeep, v);
+    if (form == 7) err = z_fused_impl<NZ, 7>(g, P, tw, zerr, st, nmem, msP, zkeep, v, nullptr, x);
+    else if (form == 0) err = z_fused_impl<NZ, 0>(g, P, tw, zerr, st, nmem, msP, zkeep, 0, nullptr, x);
+    else if (form == 1) err = z_fused_impl<NZ, 1>(g, P, tw, zerr, st, nmem, msP, zkeep, v, nullptr, x);
     else if (form == 2) err = z_fused_impl<NZ, 2>(g, P, tw, zerr, st, nmem, msP, zkeep, v);
-    else if (form == 5) err = z_fused_impl<NZ, 5>(g, P, tw, zerr, st, nmem, msP, zkeep, 0);
+    else if (form == 5) err = z_fused_impl<NZ, 5>(g, P, tw, zerr, st, nmem, msP, zkeep, 0, nullptr, x);
     else if (form == 6) err = z_fused_impl<NZ, 6>(g, P, tw, zerr, st, nmem, msP, zkeep, 0, q);
     else if constexpr (NZ % 3 != 0) err = z_fused_impl<NZ, 3>(g, P, tw, zerr, st, 1, 0, zkeep, 0);
   });
@@ -722,6 +740,26 @@ static cudaError_t fwd_x_fused(const Geo& g, const void* P, const StageArgs& a, 
     ++g_launches;
   }
   return cudaGetLastError();
+}
+
+// Line pitch of the inverse-transformed fields of a two-thirds dealiased FFF step of product
+// form `form`.  Only the nzk = Nz / 3 + 1 columns kz <= Nz / 3 are ever written there.  In lines
+// of Hz = Nz / 2 + 1 elements (odd) they start at any element, a column tile straddles lines,
+// and its 128-byte row segments cost five or six sectors of two cache lines each; in compact
+// lines of whole 16-column tiles every segment is one aligned cache line, and the z pass writes
+// the products elsewhere in lines of Hz.  B200, 256^3 FP32 rotational: inverse x 100 -> 72 us,
+// y inverse 112 -> 92.  Lines up to an eighth longer than nzk only (128 points and more: 43 of
+// 48, 86 of 96, 171 of 176 columns; at 64 points 22 of 32, and the fields sit in L2), FP32 only
+// (in FP64 a segment of unaligned columns costs one sector more of five: 22.1 and 21.9 us), and
+// with the rule's kernels in the three inverse passes.
+template <> int Launch<T>::inverse_pitch(const Geo& g, int form) {
+  if (!std::is_same<T, float>::value || g.basis != 0 || g.dealias != 2) return g.Hz;
+  if (form != 0 && form != 1 && form != 5 && form != 7) return g.Hz;
+  for (int c : {TUNE_X_INV, TUNE_Y_INV, TUNE_Z})
+    if (g.tv[c] || g.tb[c]) return g.Hz;
+  if (g.Nz % 3 == 0 || g.Nz == 1024) return g.Hz;  // zreg_rule: in place
+  const int nzk = g.Nz / 3 + 1, p = (nzk + 15) / 16 * 16;
+  return 8 * p <= 9 * nzk && p < g.Hz ? p : g.Hz;
 }
 
 template <> cudaError_t Launch<T>::fwd_x(const Geo& g, int form, int mode, const void* P, const StageArgs& a,
@@ -953,7 +991,6 @@ template <> cudaError_t Launch<T>::flux_outside(const Geo& g, const void* P, con
   ++g_launches;
   return cudaGetLastError();
 }
-
 template <> cudaError_t Launch<T>::ssf_giver(const Geo& g, const void* U, void* P, double R, cudaStream_t st) {
   k_ssf_giver<T><<<grid1d(g.S, 256), 256, 0, st>>>((const V*)U, (V*)P, g, R);
   ++g_launches;

@@ -29,6 +29,7 @@ template <typename T> struct Launch {
                              void* dst = nullptr, double scl = 1.0);
   // form 0 conservative (3 fields out), 1 rotational (6), 3 adjoint of the rotational form (9: also
   // lsc c^-1 P lam from the cotangent lam)
+  // forms 0, 1, 5: W has lines of g.Hp and components of g.Sp elements
   // kept != 0 (forms 0, 1 with two-thirds dealiasing): write only the columns with 3|ky| <= Ny, 3 kz <= Nz
   // form 4: the adjoint's cotangent fields 6-8; form 5: the giver, u inside |K| <= rad, into
   // fields 3-5 for the per-sphere energy flux
@@ -39,12 +40,17 @@ template <typename T> struct Launch {
   // nmem members, member fields msP complex apart
   // zkeep >= 0: input rows kz > zkeep are zero and not read
   // q (form 6): u is read there (three components) instead of from P
+  // x: the inputs are read there, lines of g.Hp and components of g.Sp elements (one member)
   static cudaError_t z_fused(const Geo& g, int form, void* P, const void* tw, int* err, cudaStream_t st,
-                             int nmem = 1, long long msP = 0, int zkeep = -1, const void* q = nullptr);
+                             int nmem = 1, long long msP = 0, int zkeep = -1, const void* q = nullptr,
+                             const void* x = nullptr);
   static cudaError_t z_single(const Geo& g, int dir, const void* in, void* out, int ncomp, const void* tw, cudaStream_t st);
   // SSS: the fused z pass on real coefficients (form 0 / 2 products; zin / zout sine masks)
   static cudaError_t sss_z_fused(const Geo& g, int form, void* P, const void* tw, const void* tq, int zin, int zout,
                                  cudaStream_t st);
+  // line pitch of the inverse-transformed fields for a right-hand side of product form `form`
+  // (g.Hz: the fields' own, and the products go in place)
+  static int inverse_pitch(const Geo& g, int form);
   // a.U0 / a.Ud / a.tot must be 16-byte aligned (TMA)
   // form 0 / 1 / 3 as inv_x; mode MODE_STEP, MODE_FLUX, MODE_NLIN (forms 0, 1) or MODE_ADJ (form 3)
   static cudaError_t fwd_x(const Geo& g, int form, int mode, const void* P, const StageArgs& a, const void* tw,

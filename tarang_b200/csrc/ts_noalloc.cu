@@ -110,6 +110,8 @@ extern "C" int ts_shell_spectrum_noalloc(int basis, int precision, const int N[3
   g.Nx = N[0]; g.Ny = N[1]; g.Nz = N[2];
   g.Hz = g.Nz / 2 + 1;
   g.S = (long long)g.Nx * g.Ny * g.Hz;
+  g.Hp = g.Hz;
+  g.Sp = g.S;
   for (int i = 0; i < 3; ++i) g.kf[i] = kfactor[i];
   g.basis = basis;
   g.dealias = 0;

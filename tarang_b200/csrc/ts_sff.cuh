@@ -145,87 +145,6 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
 }
 
 // ---------------------------------------------------------------------------
-// Standalone sin/cos transform along x, in place on component blockIdx.y of A
-// (spectral layout: rows lx, columns ly*Hz + lz): the x part of
-// SFF_PENCIL::Forward_transform / Inverse_transform (SFF_pencil_tr.cc:43-68)
-// for one parity (sine != 0: S, else C).
-// DIR = -1: rows hold real-space x points (after the z and y transforms); the
-//           coefficients c_m * (2N * scl) replace them (scl carries the y, z
-//           normalisation as well).
-// DIR = +1: rows hold coefficients; the unscaled synthesis replaces them.
-// Every thread loads its rows before the first barrier inside the FFT and
-// stores after the last one, so the in-place update needs no extra buffer.
-// ---------------------------------------------------------------------------
-// Planes: the nplanes planes of g.S elements (components, or the x-planes of a y pass)
-// are one run of nplanes * Ny * Hz columns, so no column tile straddles idle columns
-// at a plane's end.  Batches: blockIdx.z = b runs the pass on the planes at
-// A + b * bstride, whose parity is bit b of smask (one batch: b = 0, smask = 0 or 1).
-template <typename T, int N, int E, int CW, int DIR>
-__global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
-    k_sff_x(C<T>* __restrict__ A, Geo g, const C<T>* __restrict__ tq, int smask, double scl, long long bstride,
-            int nplanes) {
-  typedef C<T> V;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  V* xch = reinterpret_cast<V*>(smraw);
-  const int c = threadIdx.x % CW, t = threadIdx.x / CW;
-  const int inner = g.Ny * g.Hz;
-  const int col = blockIdx.x * CW + c;  // plane col / inner, column col % inner
-  const bool ok = col < nplanes * inner;
-  const long long rstride = inner;
-  const int sine = (smask >> blockIdx.z) & 1;
-  const int pl = ok ? col / inner : 0, cc = ok ? col % inner : 0;
-  V* a = A + (long long)pl * g.S + blockIdx.z * bstride + cc;
-  V v[E];
-  if (DIR < 0) {
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-      const int k = load_row<N, E>(t, s);
-      V x = ok ? a[(k < N / 2 ? 2 * k : 2 * (N - 1 - k) + 1) * rstride] : mk<V>(0, 0);
-      if (sine && k >= N / 2) x = scale(x, (T)-1);
-      v[s] = x;
-    }
-    fft_regs<N, E, -1, 0, 0, false, best_swk(N, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tq, 4);
-#pragma unroll
-    for (int s = 0; s < E; ++s) xch[final_row<N, E>(t, s) * CW + c] = v[s];
-    __syncthreads();
-    V zr[E];
-#pragma unroll
-    for (int s = 0; s < E; ++s) zr[s] = xch[((N - final_row<N, E>(t, s)) % N) * CW + c];
-    if (ok) {
-#pragma unroll
-      for (int s = 0; s < E; ++s) {
-        const int m = final_row<N, E>(t, s);
-        const V wz = mul(tq[m], v[s]), wzr = mul(conjg(tq[m]), zr[s]);
-        a[m * rstride] = sine ? mul_i<1>(scale(sub(wz, wzr), (T)scl)) : scale(add(wz, wzr), (T)scl);
-      }
-    }
-  } else {
-    auto coef = [&](int q) -> V { return (ok && q > 0 && q < N) ? a[q * rstride] : mk<V>(0, 0); };
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-      const int m = load_row<N, E>(t, s);
-      V z;
-      if (m == 0) {
-        z = (!sine && ok) ? a[0] : mk<V>(0, 0);
-      } else {
-        const V p = sine ? coef(N - m) : coef(m), q = sine ? coef(m) : coef(N - m);
-        z = mul(conjg(tq[m]), sub(p, mul_i<1>(q)));
-      }
-      v[s] = z;
-    }
-    fft_regs<N, E, 1, 0, 0, false, best_swk(N, E, CW, (int)sizeof(V))>(v, t, xch, CW, c, tq, 4);
-    if (ok) {
-#pragma unroll
-      for (int s = 0; s < E; ++s) {
-        const int k = final_row<N, E>(t, s);
-        const int n = k < N / 2 ? 2 * k : 2 * (N - 1 - k) + 1;
-        a[n * rstride] = (sine && (n & 1)) ? scale(v[s], (T)-1) : v[s];
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Sin/cos transform along x of several fields, one launch: grid x = column tiles of the
 // planes, y = batch members, z = fields (bit f of smask: field f is a sine series).
 // Every row a thread needs is loaded straight into its registers (the inverse reads the
@@ -641,9 +560,10 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
 
 // ---------------------------------------------------------------------------
 // FFF passive scalar (program.kind SCALAR_INCOMPRESS), elementwise epilogue after the
-// forward x FFT of the nine products of form 2 (u1u1, u2u2, u3u3, u1u2, u2u3,
-// u3u1, u1T, u2T, u3T; unnormalised):
-//   N_i = sum_j i K_j F[u_j u_i]  (compute_diag_offdiag.cc:47-98, conservative)
+// forward x FFT of the eight products of form 2 (u1u1 - u3u3, u2u2 - u3u3, u1u2,
+// u2u3, u3u1, u1T, u2T, u3T; unnormalised):
+//   N_i = sum_j i K_j F[u_j u_i]  (compute_diag_offdiag.cc:47-98, conservative) less the
+//   gradient of u3u3, which the projection removes
 //   NT  = sum_j i K_j F[u_j T]    (compute_diag_offdiag.cc:116-136)
 //   no force (Add_force with F = 0); p = (i K . N)/K^2, N <- N + i K p; R = -N,
 //   RT = -NT; IF-RK4 stage update of U (nu) and T (kappa) as the Boussinesq
@@ -721,12 +641,12 @@ __global__ void __launch_bounds__(256) k_scalar_epi(const C<T>* P, Geo g, SffArg
 
 // ---------------------------------------------------------------------------
 // FFF incompressible MHD (RK4(U, W, P, F) with W = B, no force), elementwise
-// epilogue after the forward x FFT of the nine products P_ij = F[Zp_i Zm_j]
-// (f = 3 i + j, unnormalised) of the z pass form 5:
-//   Zp.nlin_i = sum_j D_j P_ij, Zm.nlin_i = sum_j D_j P_ji, accumulated as the
-//   reference does (diagonal term, then the off-diagonal products in the order of
-//   compute_diag_offdiag.cc:202-258); U.nlin = (Zp.nlin + Zm.nlin)/2,
-//   B.nlin = (Zp.nlin - Zm.nlin)/2 (MHD.cc:150-161); pressure from U.nlin;
+// epilogue after the forward x FFT of the eight products of the z pass form 5: with
+// P_ij = F[Zp_i Zm_j], S_ij = (P_ij + P_ji)/2 and A_ij = (P_ij - P_ji)/2, the products are
+// S11 - S33, S22 - S33, S12, S23, S13, A12, A23, A31 (unnormalised).  Zp.nlin_i = sum_j D_j P_ij,
+//   Zm.nlin_i = sum_j D_j P_ji (compute_diag_offdiag.cc:202-258), so
+//   U.nlin = (Zp.nlin + Zm.nlin)/2 = sum_j D_j S_ij, here less the gradient of S33, which the
+//   pressure removes; B.nlin = (Zp.nlin - Zm.nlin)/2 = sum_j D_j A_ij (MHD.cc:150-161);
 //   R_U = -(U.nlin + i K p), R_B = -B.nlin (Tadvance_functions.cc:259-267); IF-RK4
 //   stage update of U (nu, tables eu) and B (eta, tables et), RK_VF_MHD.cc:126-186.
 //   a.U0 = U (3 components), a.T0 = B (3), Ucur and tot carry 6 components.
@@ -976,8 +896,8 @@ __global__ void __launch_bounds__(256) k_sss_epi(const T* P, Geo g, StageArgs a)
 // Boussinesq RBC (PRLARGE, ULARGE) on the SSF and SSS bases: the temperature takes
 // the Vx parity and the products u_x T, u_y T, u_z T take Vi2, VxVy and VxVz
 // (Global_process_basic_vars.cc:108, 114-116).  Epilogues after the forward
-// transforms of the nine products (u1u1, u2u2, u3u3, u1u2, u2u3, u3u1, u1T, u2T,
-// u3T; normalised):
+// transforms of the eight products (u1u1 - u3u3, u2u2 - u3u3, u1u2, u2u3, u3u1, u1T,
+// u2T, u3T; normalised):
 //   N as the fluid step; NT = Dx(u1T) + Dy(u2T) + Dz(u3T) (compute_diag_offdiag.cc:116-136);
 //   force (compute_force_RBC.cc:104-150): U.F1 = cu T, T.F = cT U.V1, both from the
 //   un-dealiased stage input; N1 -= T, NT -= u1 (Add_force); pressure from N;

@@ -123,3 +123,63 @@ def test_convection_step_at_line_edges(cuda, basis, N, prec):
     tol = {"f32": 1e-6, "f64": 1e-13}[prec]
     assert rel(unpack(u), wu) < tol
     assert rel(unpack(t)[0], wt) < tol
+
+
+def in_place():
+    """A tuning whose y passes take a blocks-per-SM count: the inverse-transformed fields then keep
+    their lines of Nz / 2 + 1 and the products go over them."""
+    return {"variant": [0] * 5, "blocks_per_sm": [0, 1, 0, 1, 0]}
+
+
+COMPACT = [((16, 16, 128), "rotational"), ((32, 16, 128), "conservative"), ((128, 16, 256), "conservative"),
+           ((256, 32, 128), "rotational"), ((16, 64, 512), "rotational"), ((512, 16, 256), "conservative"),
+           ((32, 16, 512), "mhd"), ((256, 16, 128), "mhd"), ((128, 32, 128), "adjoint"), ((64, 32, 64), "rotational")]
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("N,kind", COMPACT)
+def test_compact_inverse_lines_match_in_place(cuda, N, kind, prec):
+    """Two-thirds dealiased right-hand sides on compact inverse-transformed lines (FP32, 128 points
+    along z and more) against the same steps in place.  The arithmetic of a mode is the same but
+    for the order of the y butterflies' rounding, so the two agree to a few roundings of the state."""
+    import torch
+    import tarang_b200 as tb
+    g = R.Grid(N)
+    V = R.init_energy_spectrum(g, R.spectrum_k4_gauss(g.n_shells(), 4.0), 0, 0.5)
+    B = R.init_energy_spectrum(g, R.spectrum_k4_gauss(g.n_shells(), 3.0), 1, 0.3)
+    form = {"adjoint": "rotational", "mhd": "conservative"}.get(kind, kind)
+    got = []
+    for tuning in (None, in_place()):
+        plan = tb.Plan(N, precision=prec, nlin_form=form, dealias="two_thirds", nu=0.01, kappa=0.02, dt=1e-2)
+        if tuning:
+            plan.set_tuning(tuning)
+        u, b = (torch.from_numpy(a).to(plan.torch_dtype()).to(cuda) for a in (V, B))
+        if kind == "mhd":
+            plan.rk4_step_mhd(u, b, 2)
+        elif kind == "adjoint":
+            work = torch.empty(plan.adjoint_work_bytes(2), dtype=torch.uint8, device=cuda)
+            plan.adjoint_window(u, 2, b, work)
+        else:
+            plan.rk4_step(u, 2)
+        plan.status()
+        got.append((u.cpu().numpy(), b.cpu().numpy()))
+    tol = 16 * math.log2(np.prod(N)) * EPS[prec]
+    for x, y in zip(*got):
+        assert rel(x, y) < tol
+
+
+@pytest.mark.parametrize("prec,tol", [("f64", 1e-12), ("f32", 2e-6)])
+@pytest.mark.parametrize("N", [(16, 16, 16), (1024, 16, 16), (512, 16, 32), (64, 32, 16), (256, 16, 16), (128, 16, 64)])
+def test_flux_at_line_edges(cuda, N, prec, tol):
+    """The per-sphere flux at the edges of its x lines, and the same bits twice."""
+    import torch
+    import tarang_b200 as tb
+    g = R.Grid(N)
+    V = R.init_energy_spectrum(g, R.spectrum_k4_gauss(g.n_shells(), 6.0), 3, 0.5)
+    radii = [0.0, 2.0, 5.0, 5.0, 1e9]
+    ref = R.flux_per_sphere(g, V, radii, 1)
+    plan = tb.Plan(N, precision=prec, dealias="reference")
+    u = torch.from_numpy(V).to(plan.torch_dtype()).to(cuda)
+    Pi = plan.flux(u, radii)
+    assert np.max(np.abs(Pi - ref)) < tol * np.max(np.abs(ref))
+    assert np.array_equal(Pi, plan.flux(u, radii))
