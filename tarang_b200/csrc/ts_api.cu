@@ -241,6 +241,36 @@ static int upload_twiddles(int L, void** dst) {
   return TS_OK;
 }
 
+// the z axis: the plain table, then the tables of the batched register transforms (ct_table)
+template <typename T>
+static int upload_z_twiddles(int L, void** dst) {
+  std::vector<T> h(2 * (size_t)L * (1 + CT_TABLES), (T)0);
+  for (int m = 0; m < L; ++m) {
+    const double a = -2.0 * M_PI * (double)m / (double)L;
+    h[2 * m] = (T)cos(a);
+    h[2 * m + 1] = (T)sin(a);
+  }
+  for (int E : {4, 8, 12, 16})
+    for (int rev = 0; rev < 2; ++rev) {
+      if (L % E) continue;
+      T* tab = h.data() + 2 * (size_t)L * (1 + 2 * ct_slot(E) + rev);
+      int ns = 1;
+      for (int q = 0; q < npasses(L, E); ++q) {
+        const int R = radix_sched(L, E, q, rev != 0);
+        for (int r = 1; r < R; ++r)
+          for (int k = 0; k < ns; ++k) {
+            const int m = r * k * (L / (ns * R));
+            tab[2 * (r * ns + k)] = h[2 * m];
+            tab[2 * (r * ns + k) + 1] = h[2 * m + 1];
+          }
+        ns *= R;
+      }
+    }
+  CK(cudaMalloc(dst, sizeof(T) * h.size()));
+  CK(cudaMemcpy(*dst, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
+  return TS_OK;
+}
+
 static void compute_modes_in_shell(ts_plan* p) {
   // Compute_modes_in_shell_array (universal_basic.cc:104-143): full box count
   const int Nx = p->g.Nx, Ny = p->g.Ny, Nz = p->g.Nz;
@@ -503,11 +533,11 @@ int ts_plan_create(const ts_config* cfg, ts_plan** out) {
   if (p->prec) {
     CKP(upload_twiddles<float>(g.Nx, &p->twx));
     CKP(upload_twiddles<float>(g.Ny, &p->twy));
-    CKP(upload_twiddles<float>(g.Nz, &p->twz));
+    CKP(upload_z_twiddles<float>(g.Nz, &p->twz));
   } else {
     CKP(upload_twiddles<double>(g.Nx, &p->twx));
     CKP(upload_twiddles<double>(g.Ny, &p->twy));
-    CKP(upload_twiddles<double>(g.Nz, &p->twz));
+    CKP(upload_z_twiddles<double>(g.Nz, &p->twz));
   }
   compute_modes_in_shell(p);
   CKP(alloc((void**)&p->mis_d, p->mis.size() * sizeof(double)));

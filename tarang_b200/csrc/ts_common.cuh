@@ -325,32 +325,57 @@ template <bool WARP> __device__ __forceinline__ void fft_sync() {
   if (WARP) __syncwarp();
   else __syncthreads();
 }
+// Twiddle tables of fft_regs_b, one per number of elements per thread and schedule direction,
+// behind the plain table of the axis: pass P keeps its factors exp(-2 pi i r k / (NS R)) at
+// r NS + k (r = 1 .. R - 1, k < NS; the passes fill the L entries between them), so the lanes of a
+// warp (neighbouring k) read neighbouring entries.  From the plain table the reads of factor r
+// are r entries apart, up to 14 cache lines an instruction, and made up 29 % of the z pass's
+// shared-memory pipe wavefronts.
+__host__ __device__ constexpr int ct_slot(int E) { return E == 4 ? 0 : E == 8 ? 1 : E == 12 ? 2 : E == 16 ? 3 : -1; }
+constexpr int CT_TABLES = 8;  // 4 element counts, 2 directions
+template <int L, int E, bool REV, typename V> __device__ __forceinline__ const V* ct_table(const V* tw) {
+  static_assert(ct_slot(E) >= 0, "no table");
+  return tw + L * (1 + 2 * ct_slot(E) + (REV ? 1 : 0));
+}
 template <int L, int E, int P, int DIR, bool REV, int NB, typename V>
-__device__ __forceinline__ void pass_compute_b(V (&v)[NB][E], int t, const V* __restrict__ tw, int tws) {
+__device__ __forceinline__ void pass_compute_b(V (&v)[NB][E], int t, const V* __restrict__ ct) {
   typedef Pass<L, E, P, REV> PP;
   constexpr int R = PP::R, NS = PP::NS;
+  // two butterflies' factors in one 16-byte load where they are neighbours (FP32)
+  constexpr int Q = sizeof(V) == 8 && PP::B % 2 == 0 && NS % 2 == 0 ? 2 : 1;
 #pragma unroll
-  for (int q = 0; q < PP::B; ++q) {
+  for (int q0 = 0; q0 < PP::B; q0 += Q) {
     if (NS > 1) {
-      const int j = t * PP::B + q;
-      const int k = j % NS;
+      const V* tk = ct + (t * PP::B + q0) % NS;
 #pragma unroll
       for (int r = 1; r < R; ++r) {
-        V w = tw[(r * k * (L / (NS * R))) * tws];
-        if (DIR > 0) w.y = -w.y;
+        V w[Q];
+        if constexpr (Q == 2) {
+          const float4 x = *reinterpret_cast<const float4*>(tk + r * NS);
+          w[0] = mk<V>(x.x, x.y);
+          w[1] = mk<V>(x.z, x.w);
+        } else {
+          w[0] = tk[r * NS];
+        }
 #pragma unroll
-        for (int b = 0; b < NB; ++b) v[b][q * R + r] = mul(v[b][q * R + r], w);
+        for (int q = 0; q < Q; ++q) {
+          if (DIR > 0) w[q].y = -w[q].y;
+#pragma unroll
+          for (int b = 0; b < NB; ++b) v[b][(q0 + q) * R + r] = mul(v[b][(q0 + q) * R + r], w[q]);
+        }
       }
     }
 #pragma unroll
-    for (int b = 0; b < NB; ++b) DFT<R, DIR, V>::run(v[b] + q * R);
+    for (int q = q0; q < q0 + Q; ++q)
+#pragma unroll
+      for (int b = 0; b < NB; ++b) DFT<R, DIR, V>::run(v[b] + q * R);
   }
 }
 template <int L, int E, int DIR, int NB, bool WARP, int P = 0, int PAD = 0, bool REV = false, int SWK = 0,
           typename V>
 __device__ __forceinline__ void fft_regs_b(V (&v)[NB][E], int t, V* sm, int slot, int rs, int cs,
-                                           const V* __restrict__ tw, int tws) {
-  pass_compute_b<L, E, P, DIR, REV, NB>(v, t, tw, tws);
+                                           const V* __restrict__ ct) {
+  pass_compute_b<L, E, P, DIR, REV, NB>(v, t, ct);
   if constexpr (P + 1 < npasses(L, E)) {
     constexpr int KIND = P == 0 && npasses(L, E) > 2 ? 0 : (radix_sched(L, E, P + 1, REV) < E ? 2 : 1);
 #pragma unroll
@@ -363,7 +388,7 @@ __device__ __forceinline__ void fft_regs_b(V (&v)[NB][E], int t, V* sm, int slot
 #pragma unroll
       for (int s = 0; s < E; ++s) v[b][s] = sm[b * slot + xrow<PAD, SWK, KIND>(Pass<L, E, P + 1, REV>::in_row(t, s)) * rs + cs];
     fft_sync<WARP>();
-    fft_regs_b<L, E, DIR, NB, WARP, P + 1, PAD, REV, SWK>(v, t, sm, slot, rs, cs, tw, tws);
+    fft_regs_b<L, E, DIR, NB, WARP, P + 1, PAD, REV, SWK>(v, t, sm, slot, rs, cs, ct);
   }
 }
 

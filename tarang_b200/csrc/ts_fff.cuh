@@ -933,7 +933,7 @@ __device__ __forceinline__ void zpair_forward_store(C<T> (&p)[NB][E], C<T>* X, l
   typedef C<T> V;
   constexpr int M = NZ / 2, H = M + 1, TPL = NZ / E;
   constexpr bool WARP = TPL <= 32;
-  fft_regs_b<NZ, E, -1, NB, WARP, 0, zpair_pad<T>(NZ), true>(p, t, xch, slot, 1, 0, tw, 1);
+  fft_regs_b<NZ, E, -1, NB, WARP, 0, zpair_pad<T>(NZ), true>(p, t, xch, slot, 1, 0, ct_table<NZ, E, true>(tw));
   if constexpr (zpair_shfl<T, NZ, E>()) {
 #pragma unroll
     for (int f = 0; f < NB; ++f) {
@@ -1013,7 +1013,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
   } else {
     zpair_load<T, NZ, E, NIN>(X + (live0 ? line : 0) * g.Hp, g.Hp, g.Sp, live0, live1, t, partner, zkeep, in);
   }
-  fft_regs_b<NZ, E, 1, NIN, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
+  fft_regs_b<NZ, E, 1, NIN, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, ct_table<NZ, E, false>(tw));
 #pragma unroll
   for (int f0 = 0; f0 < NOUT; f0 += NB) {
     V p[NB][E];
@@ -1053,7 +1053,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
   V* Pl = P + (live0 ? line : 0) * H;
   V in[3][E];
   zpair_load<T, NZ, E, 3>(Pl + 6 * g.S, H, g.S, live0, live1, t, partner, M, in);
-  fft_regs_b<NZ, E, 1, 3, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
+  fft_regs_b<NZ, E, 1, 3, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, ct_table<NZ, E, false>(tw));
 #pragma unroll
   for (int f = 0; f < 3; ++f)
 #pragma unroll
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     zpair_load<T, NZ, E, 3>(Pl + 3 * h * g.S, H, g.S, live0, live1, t, partner, zkeep, in);
-    fft_regs_b<NZ, E, 1, 3, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
+    fft_regs_b<NZ, E, 1, 3, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, ct_table<NZ, E, false>(tw));
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       V p[1][E];
@@ -1147,7 +1147,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
       else in[c][s] = mul(conjg(tq[m]), sine ? add_i<-1>(q[s], p) : add_i<-1>(p, q[s]));
     }
   }
-  fft_regs_b<NZ, E, 1, NIN, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, tw, 1);
+  fft_regs_b<NZ, E, 1, NIN, WARP, 0, zpair_pad<T>(NZ), false>(in, t, xch, SLOT, 1, 0, ct_table<NZ, E, false>(tw));
 #pragma unroll
   for (int f0 = 0; f0 < NOUT; f0 += NB) {
     V p[NB][E];
@@ -1160,7 +1160,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
         for (int c = 0; c < NIN; ++c) q[c] = in[c][s];
         p[f][s] = z_product<FORM>(f0 + f, q);
       }
-    fft_regs_b<NZ, E, -1, NB, WARP, 0, zpair_pad<T>(NZ), true>(p, t, xch, SLOT, 1, 0, tw, 1);
+    fft_regs_b<NZ, E, -1, NB, WARP, 0, zpair_pad<T>(NZ), true>(p, t, xch, SLOT, 1, 0, ct_table<NZ, E, true>(tw));
     if constexpr (!SH) {
 #pragma unroll
       for (int f = 0; f < NB; ++f)
@@ -1907,7 +1907,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
       if (r > M) a.y = -a.y, b.y = -b.y;
       v[0][s] = mk<V>(a.x - b.y, a.y + b.x);
     }
-    fft_regs_b<NZ, E, 1, 1, WARP, 0, 1, false>(v, t, xch, LDX, 1, 0, tw, 1);
+    fft_regs_b<NZ, E, 1, 1, WARP, 0, 1, false>(v, t, xch, LDX, 1, 0, ct_table<NZ, E, false>(tw));
 #pragma unroll
     for (int s = 0; s < E; ++s) xch[prow<1>(final_row<NZ, E>(t, s))] = v[0][s];
     fft_sync<WARP>();
@@ -1925,7 +1925,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
       const int n = load_row<NZ, E>(t, s);
       v[0][s] = mk<V>(live0 ? X[n] : (T)0, live1 ? X[LD + n] : (T)0);
     }
-    fft_regs_b<NZ, E, -1, 1, WARP, 0, 1, false>(v, t, xch, LDX, 1, 0, tw, 1);
+    fft_regs_b<NZ, E, -1, 1, WARP, 0, 1, false>(v, t, xch, LDX, 1, 0, ct_table<NZ, E, false>(tw));
 #pragma unroll
     for (int s = 0; s < E; ++s) xch[prow<1>(final_row<NZ, E>(t, s))] = v[0][s];
     fft_sync<WARP>();
