@@ -140,7 +140,7 @@ struct LdTile { int E, CW, MINB; };
 constexpr LdTile sc_tile(int L, int dir) {
   return std::is_same<T, float>::value
              ? (L == 16 ? LdTile{4, 16, 8} : L == 32 ? LdTile{8, 16, 16} : L == 64 ? LdTile{8, 16, 8}
-                : L == 128 ? LdTile{16, 16, dir > 0 ? 4 : 6} : L == 256 ? LdTile{16, 16, dir > 0 ? 2 : 4}
+                : L == 128 ? LdTile{16, 16, 6} : L == 256 ? LdTile{16, 16, dir > 0 ? 3 : 4}
                 : L == 512 ? LdTile{16, 16, 1} : L == 96 ? LdTile{24, 16, 8} : LdTile{12, 16, 8})
              : (L == 16 ? LdTile{4, 8, 16} : L == 32 ? LdTile{8, 8, 16} : L == 64 ? LdTile{8, 8, 8}
                 : L == 128 ? LdTile{16, 8, 4} : L == 256 ? LdTile{16, 8, 2} : L == 512 ? LdTile{16, 8, 1}
