@@ -7,10 +7,11 @@
 // One right-hand-side evaluation is five launches:
 //   inv_x  : dealias on load (+ vorticity for the rotational form), inverse FFT along x
 //   y      : inverse FFT along y (in place)
-//   z      : C2R along z -> real-space products -> R2C along z (one kernel, smem resident)
+//   z      : C2R along z -> real-space products -> R2C along z (one kernel, lines in registers)
 //   y      : forward FFT along y (in place)
 //   fwd_x  : forward FFT along x + N_i assembly + force + Leray projection
-//            + the IF-RK4 stage update (or a flux reduction / plain N output)
+//            + the IF-RK4 stage update (or a flux reduction / plain N output); one kernel, or an
+//            in-place FFT and an elementwise epilogue
 #pragma once
 #include "ts_common.cuh"
 #include "ts_tma.cuh"

@@ -135,12 +135,16 @@ constexpr int str_e(int L) { return wide1024(L) ? 16 : e_mixed(L, e_reg(L)); }
 constexpr int str_cw(int L) { return wide1024(L) ? 8 : cw_for(L, str_e(L)); }
 constexpr int str_nt(int L) { return wide1024(L) ? 2 : 3; }
 
-// sin/cos x kernel: elements per thread, tile columns, blocks per SM it is compiled for
+// sin/cos x kernel: elements per thread, tile columns, blocks per SM it is compiled for.  Bound by
+// DRAM latency: rows of whole 128-byte lines, as many elements per thread as leave two radix
+// passes (one exchange), and the blocks per SM at which the registers just do not spill.  B200,
+// FP32 forward, us: 128 points 27 (8 elements 35; 8 columns 36; four blocks 31), 256 points 57
+// (three blocks 62, 8 elements 117), 96 points with 24 elements 15.1 (12: 17.0, 6: 23.3)
 struct LdTile { int E, CW, MINB; };
 constexpr LdTile sc_tile(int L, int dir) {
   return std::is_same<T, float>::value
              ? (L == 16 ? LdTile{4, 16, 8} : L == 32 ? LdTile{8, 16, 16} : L == 64 ? LdTile{8, 16, 8}
-                : L == 128 ? LdTile{16, 16, 6} : L == 256 ? LdTile{16, 16, dir > 0 ? 3 : 4}
+                : L == 128 ? LdTile{16, 16, 6} : L == 256 ? LdTile{16, 16, dir > 0 ? 2 : 4}
                 : L == 512 ? LdTile{16, 16, 1} : L == 96 ? LdTile{24, 16, 8} : LdTile{12, 16, 8})
              : (L == 16 ? LdTile{4, 8, 16} : L == 32 ? LdTile{8, 8, 16} : L == 64 ? LdTile{8, 8, 8}
                 : L == 128 ? LdTile{16, 8, 4} : L == 256 ? LdTile{16, 8, 2} : L == 512 ? LdTile{16, 8, 1}
@@ -148,7 +152,14 @@ constexpr LdTile sc_tile(int L, int dir) {
 }
 
 // direct-load strided kernel: elements per thread, tile columns and blocks per SM the
-// kernel is compiled for
+// kernel is compiled for, chosen as for sc_tile.  B200, FP32, us: 256 points forward, three
+// fields of 256^3, 72 (8 columns 81, 32 columns 79, 8 elements 101, two blocks 79; the persistent
+// cp.async kernel 89-101); 128 points 25 (8 elements 31; persistent 40); 64 points 25 (persistent
+// 70); 96 points with 24 elements on 32 columns 49 (16 columns 54, 12 elements 55-60; persistent
+// 93); 512 points with 32 elements 165 (16: 189; three blocks 172); 1024 points with 32 elements
+// on 8 columns 391 (16 columns 416, 16 elements 455).  FP64: 256 points with 16 elements 72 (8:
+// 80; persistent 93), 128 points 35 (8 elements 36), 512 points 83 (32 elements 90, three blocks
+// 101), 1024 points on 4 columns 204 (16 elements on 8 columns 220)
 constexpr LdTile ld_tile(int L) {
   return std::is_same<T, float>::value
              ? (L == 16 ? LdTile{4, 16, 8} : L == 32 ? LdTile{8, 16, 16} : L == 64 ? LdTile{8, 16, 8}
@@ -166,7 +177,10 @@ constexpr long long FAR_ROW_BYTES = 1 << 19;
 constexpr LdTile far_tile(int L) {
   return std::is_same<T, float>::value && L == 1024 ? LdTile{32, 16, 1} : LdTile{0, 0, 0};
 }
-// inverse x kernel (one field per block)
+// inverse x kernel (one field per block): the tiles of the strided kernel; three blocks per SM
+// at 256 points, where the vorticity's second operand takes registers.  The three fields of a
+// group in one block read U once but need 128 registers at 8 elements per thread: 115 us against
+// 102 (256^3 rotational)
 constexpr LdTile ix_tile(int L) {
   return std::is_same<T, float>::value
              ? (L == 16 ? LdTile{4, 16, 8} : L == 32 ? LdTile{8, 16, 16} : L == 64 ? LdTile{8, 16, 8}

@@ -195,9 +195,10 @@ __global__ void __launch_bounds__(CW * (N / E), MINB)
   typedef C<T> V;
   constexpr int SWK = best_swk(N, E, CW, (int)sizeof(V));
   // inverse: the mirrored rows come from shared memory (QX) or are read again.  FP32, 128 points,
-  // 256 x 256 columns, four fields: 57 us against 60 (64 us when it was read again at four blocks
-  // per SM); 256 points: 36 against 39; 96 points: 31 against 30; 64: 33 against 31; FP64: 36, 36
-  constexpr bool QX = sizeof(T) == 4 && (N == 128 || N == 256);
+  // 256 x 256 columns, four fields, dealiased: 57 us through shared memory at six blocks per SM
+  // against 60-64 us read again at four to six; 256 points (128 x 128 columns): 36 against 34 (two
+  // blocks per SM); 96 points 31 against 30, 64 points 33 against 31, FP64 36 against 36
+  constexpr bool QX = sizeof(T) == 4 && N == 128;
   extern __shared__ __align__(16) unsigned char smraw[];
   V* xch = reinterpret_cast<V*>(smraw);
   const int c = threadIdx.x % CW, t = threadIdx.x / CW;
