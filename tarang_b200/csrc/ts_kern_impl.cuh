@@ -287,15 +287,23 @@ template <int NZ, int FORM> constexpr bool z_valid(int v) {
                                   (v == 4 && std::is_same<T, float>::value && M == 512)));
 }
 
-// pipelined forward x kernel of a step or an adjoint step (CW = 0: not used): elements per
+// pipelined forward x kernel of a step or of an adjoint step (CW = 0: not used): elements per
 // thread, tile columns, buffers, state prefetch into L2.  B200, the four stages' average, us:
 // 256x256x256 FP32 rotational 197 (203 without the prefetch, 240 with two buffers; fused TMA
 // kernel 235, split 76 + 157), conservative 239 (split 117 + 176); 128x256x256 FP32 91 (99 with
 // the prefetch) and 118 (split 35 + 83, 58 + 94); FP64 at 128^3 56 (fused 58, split 18 + 41),
 // adjoint 67 (fused 80, split 35 + 51).  FP32 at 512 points (234 against 82 + 160) and FP64 at
 // 256 (113 against 36 + 77) gain nothing.
+// 32 (FP32) and 64 points: on fields of at most PIPE_SMALL_BYTES, where it saves a launch and the
+// products sit in L2.  Steps, us, split -> pipelined, conservative / rotational: FP32 32^3 66 ->
+// 64 / 68 -> 65, 64^3 (1 MB per component) 109 -> 93 / 115 -> 102, 32x128x128 (2 MB) 146 -> 127 /
+// 147 -> 138; 64x128x128 (4 MB) 196 -> 189 / 193 -> 195, 32x256x256 (9 MB) 328 -> 332 / 326 -> 348;
+// FP64 64^3 127 -> 126 / 153 -> 138, but 32^3 75 -> 73 / 92 -> 99
+constexpr long long PIPE_SMALL_BYTES = 3000000;
 struct PipeTile { int E, CW, NBUF; bool PF; };
 constexpr PipeTile pipe_tile(int L, int form) {
+  if (form != 3 && L == 64) return PipeTile{8, std::is_same<T, float>::value ? 16 : 8, 1, false};
+  if (form != 3 && L == 32 && std::is_same<T, float>::value) return PipeTile{8, 16, 1, false};
   return !std::is_same<T, float>::value
              ? (L == 128 ? (form == 1 ? PipeTile{16, 16, 1, false} : form == 3 ? PipeTile{16, 8, 2, true} : PipeTile{0, 0, 0, false})
                          : PipeTile{0, 0, 0, false})
@@ -676,7 +684,7 @@ template <int FORM, int LL>
 static cudaError_t fwd_x_pipe(const Geo& g, const void* P, const StageArgs& a, const void* tw, cudaStream_t st) {
   constexpr PipeTile c = pipe_tile(LL, FORM);
   constexpr size_t sm = (size_t)c.NBUF * z_nout(FORM) * LL * c.CW * sizeof(V) + LL * pipe_row_bytes();
-  const unsigned ntiles = (unsigned)(g.Ny * g.Hz / c.CW), blocks = ntiles < 148u ? ntiles : 148u;
+  const unsigned ntiles = (unsigned)(g.Ny * g.Hz / c.CW), most = LL <= 64 ? 2 * 148u : 148u, blocks = ntiles < most ? ntiles : most;
   cudaError_t err = cudaErrorInvalidValue;
   auto run = [&](auto k) {
     if ((err = smem_attr(k, sm)) != cudaSuccess) return;
@@ -709,7 +717,8 @@ static cudaError_t fwd_x_impl(const Geo& g, const void* P, const StageArgs& a, c
   const bool fused16 = fx_rule_fused(LL) && (((uintptr_t)sA | (uintptr_t)sB) & 15);
   if (fused16 && !(MODE == MODE_STEP && v == 1)) return cudaErrorInvalidValue;
   if constexpr ((MODE == MODE_STEP || MODE == MODE_ADJ) && pipe_tile(LL, FORM).CW > 0) {
-    if (rule && g.Ny * g.Hz % pipe_tile(LL, FORM).CW == 0) return fwd_x_pipe<FORM, LL>(g, P, a, tw, st);
+    const bool fits = LL > 64 || g.S * (long long)sizeof(V) <= PIPE_SMALL_BYTES;
+    if (rule && fits && g.Ny * g.Hz % pipe_tile(LL, FORM).CW == 0) return fwd_x_pipe<FORM, LL>(g, P, a, tw, st);
   }
   const bool split = CW * sizeof(V) < 64 || v == 1 || (rule && MODE == MODE_STEP && fx_rule_split(LL));
   if (split) {

@@ -64,6 +64,10 @@ STEPS = [("rotational", "two_thirds", N) for N in ((16, 16, 16), (1024, 16, 32),
                                                    (512, 16, 16), (32, 16, 512), (128, 32, 16), (256, 16, 32))]
 STEPS += [("conservative", "reference", N) for N in ((16, 16, 16), (1024, 16, 16), (16, 512, 32), (16, 16, 1024), (64, 32, 256),
                                                      (128, 16, 16), (256, 16, 16))]
+# 32 and 64 points along x: the pipelined forward x pass on small fields, the split one above (FP64
+# 64 x 128 x 64: 4.3 MB a component)
+STEPS += [(f, d, N) for f, d in (("rotational", "two_thirds"), ("conservative", "reference"))
+          for N in ((32, 16, 16), (32, 64, 32), (64, 16, 16), (64, 128, 64))]
 
 
 @pytest.mark.parametrize("prec", ["f32", "f64"])
