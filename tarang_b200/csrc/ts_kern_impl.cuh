@@ -11,6 +11,7 @@
 #include <type_traits>
 #include "ts_launch.h"
 #include "ts_misc.cuh"
+#include "ts_radius.h"
 
 namespace ts {
 
@@ -74,14 +75,6 @@ template <typename Fn> bool dispatch_L_sff(int L, Fn&& fn) {
 // (6 where the power-of-two choice is 4 or less: the FP64 SFF forward x kernel
 // holds four accumulators per element and spilled at 12)
 constexpr int e_mixed(int L, int e_pow2) { return L % 3 == 0 ? (e_pow2 >= 8 ? 12 : 6) : (e_pow2 < L ? e_pow2 : L); }
-
-// the largest x with sqrt(x) <= R, so that |K| > R is K^2 > x without a square root per mode
-inline double k2_limit(double R) {
-  double x = R * R;
-  while (sqrt(x) > R) x = nextafter(x, 0.0);
-  while (sqrt(nextafter(x, HUGE_VAL)) <= R) x = nextafter(x, HUGE_VAL);
-  return x;
-}
 
 template <typename K> cudaError_t smem_attr(K kernel, size_t bytes) {
   if (bytes > 48 * 1024) {

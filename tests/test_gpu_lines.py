@@ -187,3 +187,21 @@ def test_flux_at_line_edges(cuda, N, prec, tol):
     Pi = plan.flux(u, radii)
     assert np.max(np.abs(Pi - ref)) < tol * np.max(np.abs(ref))
     assert np.array_equal(Pi, plan.flux(u, radii))
+
+
+@pytest.mark.parametrize("prec,tol", [("f64", 1e-12), ("f32", 2e-6)])
+@pytest.mark.parametrize("dealias", ["none", "reference", "two_thirds"])
+def test_flux_takes_every_radius(cuda, dealias, prec, tol):
+    """Radii that do not ascend (the per-sphere form on every dealias mode), among them the sphere
+    that holds no mode, the one that holds all and one whose square overflows."""
+    import torch
+    import tarang_b200 as tb
+    N = (32, 16, 16)
+    g = R.Grid(N)
+    V = R.init_energy_spectrum(g, R.spectrum_k4_gauss(g.n_shells(), 6.0), 3, 0.5)
+    radii = [3.0, math.inf, -1.0, 1e200, 0.0, -math.inf]
+    ref = R.flux_per_sphere(g, V, radii, {"none": 0, "reference": 1, "two_thirds": 2}[dealias])
+    plan = tb.Plan(N, precision=prec, dealias=dealias)
+    Pi = plan.flux(torch.from_numpy(V).to(plan.torch_dtype()).to(cuda), radii)
+    assert np.max(np.abs(Pi - ref)) < tol * np.max(np.abs(ref))
+    assert np.all(Pi[[1, 2, 3, 5]] == 0)
