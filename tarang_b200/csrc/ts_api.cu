@@ -1877,7 +1877,12 @@ int ts_fft_inverse(ts_plan* p, const char* parity, const void* spec_in, void* re
   if (!is_device_ptr(spec_in) || !is_device_ptr(real_out)) return TS_ERR_ARG;
   const Geo& g = p->g;
   // the reference copies the input to X_transform first (FFF_pencil_tr.cc:59); here the x
-  // pass reads the input and writes the work fields
+  // pass reads the input and writes the work fields.  It reads whole complex values: an input
+  // that is not aligned to them is copied first, the work fields then transformed in place
+  if ((uintptr_t)spec_in % p->cb) {
+    CK(cudaMemcpyAsync(p->P, spec_in, ncomp * g.S * p->cb, cudaMemcpyDeviceToDevice, p->st));
+    spec_in = p->P;
+  }
   if (zp) {
     const long long cs = g.S * (long long)p->cb, nl = (long long)ncomp * g.Nx * g.Ny;
     char* P = (char*)p->P;

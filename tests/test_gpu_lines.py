@@ -205,3 +205,27 @@ def test_flux_takes_every_radius(cuda, dealias, prec, tol):
     Pi = plan.flux(torch.from_numpy(V).to(plan.torch_dtype()).to(cuda), radii)
     assert np.max(np.abs(Pi - ref)) < tol * np.max(np.abs(ref))
     assert np.all(Pi[[1, 2, 3, 5]] == 0)
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("basis,parity", [("FFF", "FFF"), ("SFF", "CFF"), ("SSF", "SCF"), ("SSS", "SCC")])
+def test_inverse_takes_inputs_aligned_to_a_real(cuda, basis, parity, prec):
+    """A spectrum that starts between two complex values (a C program's pointer into its own
+    buffer): the same bits as from an aligned one, and the input untouched."""
+    import ctypes
+    import torch
+    import tarang_b200 as tb
+    N = (32, 16, 64)
+    plan = tb.Plan(N, basis=basis, precision=prec)
+    rt = torch.float32 if prec == "f32" else torch.float64
+    spec = torch.randn((2,) + plan.spec_shape, dtype=plan.torch_dtype(), device=cuda)
+    want = torch.zeros((2,) + N[:2] + (N[2] + 2,), dtype=rt, device=cuda)
+    plan.inverse(spec, want, parity)
+    flat = torch.view_as_real(spec).reshape(-1)
+    buf = torch.zeros(flat.numel() + 1, dtype=rt, device=cuda)
+    buf[1:] = flat
+    got = torch.zeros_like(want)
+    rc = plan.lib.ts_fft_inverse(plan.h, parity.encode(), ctypes.c_void_p(buf[1:].data_ptr()),
+                                 ctypes.c_void_p(got.data_ptr()), 2)
+    torch.cuda.synchronize()
+    assert rc == 0 and torch.equal(got, want) and torch.equal(buf[1:], flat)
