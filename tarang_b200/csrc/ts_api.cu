@@ -1063,7 +1063,8 @@ static int ssf_transforms_only() {
 }
 
 // the geometry that makes the x-axis sin/cos kernel transform along y: every
-// x-plane of every component is one "component" of Ny rows x Hz columns
+// x-plane of every component is one "component" of Ny rows x Hz columns (Sp stays the whole
+// component, S < Sp tells the launcher that this is a y pass)
 static Geo y_as_x(const Geo& g) {
   Geo h = g;
   h.Nx = g.Ny;

@@ -87,13 +87,19 @@ template <typename K> cudaError_t smem_attr(K kernel, size_t bytes) {
 
 // Launch of a kernel that begins with chain_begin().  Kernels on small fields are launched
 // while the preceding kernel of the stream still runs: a pass takes 2-4 us there and the gap
-// between two plain launches another 2 us.  Large grids are launched plainly: their early
-// blocks would take the slots of the running grid's last waves.  B200, plain -> chained: 32^3
+// between two plain launches another 2 us.  Large grids are launched plainly (but for chained_sc):
+// their early blocks would take the slots of the running grid's last waves.  B200, plain -> chained: 32^3
 // FP32 step 126 -> 77 us, 64^3 FP64 172 -> 161, SSF 96^3 (3.6 MB per component) 329 -> 281, SSS
 // 128^3 FP32 (8.5 MB) 653 -> 616, 18-sphere flux 128^3 3278 -> 3084; FP64 adjoint 128^3 (17 MB)
 // 12750 -> 13080, 256^3 2711 -> 2715, MHD 256^3 4908 -> 5008.
 constexpr long long CHAIN_BYTES = 10000000;
 inline bool chained(const Geo& g, int nmem = 1) { return nmem == 1 && g.S * (long long)sizeof(V) <= CHAIN_BYTES; }
+// The sin/cos passes: along y (y_as_x: S is one x plane, Sp the component) fields of any size are
+// chained.  B200, step, us, plain -> chained: FP32 SSS Boussinesq 64x64x1024 1345 -> 1311,
+// 128x256x256 2462 -> 2413, 256^3 4848 -> 4763, SSF fluid 64x64x1024 799 -> 785, 256^3 2988 -> 2973;
+// FP64 SSF fluid 128^3 (17 MB) 790 -> 775, 64x64x1024 (34 MB) 1546 -> 1529, 128x256x256 (135 MB) 2969 ->
+// 2944, SSF Boussinesq 128x256x256 4391 -> 4415, SSS 256^3 9205 -> 9270.
+inline bool chained_sc(const Geo& g, int nmem) { return g.S < g.Sp ? nmem == 1 : chained(g, nmem); }
 template <typename... P, typename... A>
 cudaError_t launch_chain(bool chain, void (*k)(P...), dim3 grid, unsigned block, size_t sm, cudaStream_t st, A&&... args) {
   cudaLaunchAttribute at[1];
@@ -814,7 +820,7 @@ template <> cudaError_t Launch<T>::sc_x(const Geo& g, int dir, const ScArgs& a, 
       const dim3 grid((unsigned)((cols + c.CW - 1) / c.CW), nmem, nf);
       auto run = [&](auto k) {
         if ((err = smem_attr(k, sm)) != cudaSuccess) return;
-        err = launch_chain(chained(g, nmem), k, grid, c.CW * (NN / c.E), sm, st, a, g, (const V*)tq);
+        err = launch_chain(chained_sc(g, nmem), k, grid, c.CW * (NN / c.E), sm, st, a, g, (const V*)tq);
       };
       if (dir < 0) run(k_sc_x<T, NN, c.E, c.CW, -1, cf.MINB>);
       else run(k_sc_x<T, NN, c.E, c.CW, 1, c.MINB>);
