@@ -26,6 +26,11 @@ _DEALIAS = {"none": L.TS_DEALIAS_NONE, "reference": L.TS_DEALIAS_REFERENCE_CORNE
             "two_thirds": L.TS_DEALIAS_TWO_THIRDS}
 _FORM = {"conservative": L.TS_NLIN_CONSERVATIVE, "rotational": L.TS_NLIN_ROTATIONAL}
 
+# Numbering of the library's kernel candidates (candidate 0, the rule, among them), part of the
+# autotune cache's key: raised whenever a rule or a candidate of the library changes, so that
+# timings of other kernels are not applied.
+TUNING_SET = 2
+
 
 @dataclass
 class Forcing:
@@ -204,19 +209,24 @@ class Plan:
         dev = torch.cuda.get_device_name() if torch.cuda.is_available() else "cpu"
         c = self.cfg
         return (f"{dev}|{self.basis}|{'x'.join(map(str, self.N))}|{self.precision}|form{c.nlin_form}"
-                f"|dealias{c.dealias_mode}|force{c.force_type}")
+                f"|dealias{c.dealias_mode}|force{c.force_type}|set{TUNING_SET}")
 
     def autotune(self, reps: int = 3, cache: str | None = None) -> dict:
         """Pick the fastest kernel candidate of every pass class on this GPU (ts_plan_autotune) and
-        return the timing report.  cache: a JSON file of earlier results keyed by device and plan
-        configuration; a hit applies the stored tuning without timing anything."""
+        return the timing report.  cache: a JSON file of earlier results keyed by device, plan
+        configuration and candidate numbering; a hit applies the stored tuning without timing
+        anything, one that the plan rejects is timed again."""
         key = self.tuning_key()
         if cache and os.path.exists(cache):
             with open(cache) as f:
                 hit = json.load(f).get(key)
             if hit is not None:
-                self.set_tuning(hit)
-                return {"cached": True, "tuning": hit}
+                try:
+                    self.set_tuning(hit)
+                    return {"cached": True, "tuning": hit}
+                except L.TsError as e:
+                    if e.status != L.TS_ERR_ARG:  # a candidate that this plan does not have: a miss
+                        raise
         buf = ctypes.create_string_buffer(1 << 16)
         L.check(self.lib.ts_plan_autotune(self.h, reps, buf, len(buf)), "ts_plan_autotune")
         report = json.loads(buf.value.decode())
