@@ -48,6 +48,14 @@ template <> __device__ __forceinline__ float2 scale<float2, float>(float2 a, flo
   return r;
 }
 #undef TS_F32X2
+// component by component product, rounded by itself (not contracted into an fma with a later add,
+// as the packed mul is): a difference of two equal products is exactly zero
+__device__ __forceinline__ float2 mul_rn(float2 a, float2 b) {
+  return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+}
+__device__ __forceinline__ double2 mul_rn(double2 a, double2 b) {
+  return make_double2(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y));
+}
 // multiply by +i (SIGN=+1) or -i (SIGN=-1)
 template <int SIGN, typename V> __device__ __forceinline__ V mul_i(V a) {
   return SIGN > 0 ? mk<V>(-a.y, a.x) : mk<V>(a.y, -a.x);

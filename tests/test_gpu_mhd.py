@@ -69,3 +69,29 @@ def test_mhd_step_rejects_other_plans(cuda):
     sff = tb.Plan(32, basis="SFF", kfactor=(math.pi, 2 * math.pi, 2 * math.pi))
     with pytest.raises(tb.TsError):
         sff.rk4_step_mhd(sff.field(3), sff.field(3), 1)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("sign", [1, -1])
+@pytest.mark.parametrize("N,dealias", [((32, 16, 16), "reference"), ((16, 32, 128), "two_thirds"),
+                                       ((16, 16, 1024), "two_thirds")])
+def test_aligned_states_only_decay(cuda, N, dealias, sign, prec):
+    """u = b or u = -b with nu = eta: one Elsasser field is zero, every product with it too, so the
+    fields stay aligned to the last bit and decay by exp(-nu K^2 t): two roundings of the stored
+    state a step (stage 4 reads U0 only)."""
+    import torch
+    import tarang_b200 as tb
+    g, U0, _ = state(N)
+    nu, dt, steps = 0.01, 1e-2, 3
+    plan = tb.Plan(N, precision=prec, nu=nu, kappa=nu, dt=dt, dealias=dealias)
+    u = torch.from_numpy(U0).to(cuda).to(plan.torch_dtype())
+    b = sign * u
+    start = u.cpu().numpy().astype(np.complex128)
+    plan.rk4_step_mhd(u, b, steps)
+    plan.status()
+    assert torch.equal(u, sign * b)
+    Kx, Ky, Kz = np.meshgrid(np.fft.fftfreq(N[0], 1 / N[0]), np.fft.fftfreq(N[1], 1 / N[1]), np.arange(N[2] // 2 + 1),
+                             indexing="ij")
+    want = start * np.exp(-nu * dt * steps * (Kx ** 2 + Ky ** 2 + Kz ** 2))
+    eps = 2.0 ** -52 if prec == "f64" else 2.0 ** -23
+    assert rel(u.cpu().numpy().astype(np.complex128), want) < 2 * steps * eps
