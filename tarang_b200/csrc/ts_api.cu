@@ -1132,7 +1132,7 @@ static int step_ssf(ts_plan* p, void* U0, void* T0 = nullptr) {
   a.ez = p->eax[2];
   SffArgs b = ssf_rbc_args(p, U0, T0);
   // x, y sine (1) / cosine (0) letters of Vx = SCF, Vy = CSF, Vz = CCF, T = SCF and of the
-  // products u1u1, u2u2, u3u3 (Vi2 = CCF), u1u2 (VxVy = SSF), u2u3 (VyVz = CSF),
+  // products u2u2 - u1u1, u3u3 - u1u1 (Vi2 = CCF), u1u2 (VxVy = SSF), u2u3 (VyVz = CSF),
   // u3u1 (VxVz = SCF), u1T (CCF), u2T (SSF), u3T (SCF)
   const int vx[4] = {1, 0, 0, 1}, vy[4] = {0, 1, 0, 0};
   const int qx[8] = {0, 0, 1, 0, 1, 0, 1, 1}, qy[8] = {0, 0, 1, 1, 0, 0, 1, 0};
@@ -1209,8 +1209,8 @@ static int step_sss(ts_plan* p, void* U0, void* T0 = nullptr) {
   a.ey = p->eax[1];
   a.ez = p->eax[2];
   SffArgs b = ssf_rbc_args(p, U0, T0);
-  // sine (1) / cosine (0) letters: Vx = SCC, Vy = CSC, Vz = CCS, T = SCC; products u1u1,
-  // u2u2, u3u3 (CCC), u1u2 (SSC), u2u3 (CSS), u3u1 (SCS), u1T (CCC), u2T (SSC), u3T (SCS)
+  // sine (1) / cosine (0) letters: Vx = SCC, Vy = CSC, Vz = CCS, T = SCC; products
+  // u2u2 - u1u1, u3u3 - u1u1 (CCC), u1u2 (SSC), u2u3 (CSS), u3u1 (SCS), u1T (CCC), u2T (SSC), u3T (SCS)
   const int vx[4] = {1, 0, 0, 1}, vy[4] = {0, 1, 0, 0}, vz[4] = {0, 0, 1, 0};
   const int qx[8] = {0, 0, 1, 0, 1, 0, 1, 1}, qy[8] = {0, 0, 1, 1, 0, 0, 1, 0};
   const int qz[8] = {0, 0, 0, 1, 1, 0, 0, 1};

@@ -530,15 +530,20 @@ template <int M> __host__ __device__ constexpr int zslot() { return M + M / 16 +
 
 // Real-space product forms of the z pass.
 // FORM 0 (conservative, whole tensor): in u1,u2,u3 -> u1u1,u2u2,u3u3,u1u2,u2u3,u3u1
-// FORM 7 (conservative step): in u1,u2,u3 -> d1,d2,u1u2,u2u3,u3u1 with d1 = u1u1 - u3u3,
-//         d2 = u2u2 - u3u3: taking u3u3 off the diagonal changes N by the gradient of u3u3,
-//         which the projection removes, so a step needs one transform less
+// FORM 7 (conservative step): in u1,u2,u3 -> d2,d3,u1u2,u2u3,u3u1 with d2 = u2u2 - u1u1,
+//         d3 = u3u3 - u1u1: taking u1u1 off the diagonal changes N by the gradient of u1u1,
+//         which the projection removes, so a step needs one transform less.  It removes it to
+//         rounding only: N carries an error of the size of eps |K| u1u1 in the modes with kx = 0,
+//         where the whole tensor has none (the other modes have it either way).  u1u1 because x
+//         is the bounded axis of SFF and SSF, along which no flow or mean wind is uniform: shear
+//         flows and winds along z keep a nonlinear term of exactly zero (with u3u3 taken off, one
+//         of 1e-6 at a wind of 10 in FP32); on FFF a flow along x has that error
 // FORM 1 (rotational):    in u1..3,w1..3    -> u x w
 // FORM 2 (scalar, Boussinesq): in u1,u2,u3,T -> the five of FORM 7, then u1T,u2T,u3T
 //                         (compute_diag_offdiag.cc:47-136)
 // FORM 3 (adjoint of the rotational form): in u, w, mu -> mu x u, then w x mu
 // FORM 5 (MHD):           in u1..3, b1..3 -> the symmetric part S_ij = u_i u_j - b_i b_j of
-//         Zp_i Zm_j, Zp = u + b, Zm = u - b, as S11 - S33, S22 - S33, S12, S23, S31, and the
+//         Zp_i Zm_j, Zp = u + b, Zm = u - b, as S22 - S11, S33 - S11, S12, S23, S31, and the
 //         antisymmetric part A_ij = b_i u_j - u_i b_j as A12, A23, A31: U.nlin is the
 //         divergence of S and B.nlin that of A (compute_nlin_VF_MHD.cc:40-95, MHD.cc:75-84,150-161).
 //         Every product is rounded by itself (mul_rn), so that the products of an aligned state,
@@ -574,11 +579,11 @@ template <int FORM, typename V> __device__ __forceinline__ V z_product(int f, co
     return prod_pk(in[f / 3], in[3 + f % 3]);
   } else if constexpr (FORM == 5) {
     auto dif = [&](int a, int c, int b, int d) { return sub(mul_rn(in[a], in[c]), mul_rn(in[b], in[d])); };
-    if (f < 2) return sub(dif(f, f, 3 + f, 3 + f), dif(2, 2, 5, 5));
+    if (f < 2) return sub(dif(f + 1, f + 1, f + 4, f + 4), dif(0, 0, 3, 3));
     const int i = (f - 2) % 3, j = (i + 1) % 3;
     return f < 5 ? dif(i, j, 3 + i, 3 + j) : dif(3 + i, j, i, 3 + j);
   } else {
-    if (f < 2) return diff_pk(in[f], in[f], in[2], in[2]);
+    if (f < 2) return diff_pk(in[f + 1], in[f + 1], in[0], in[0]);
     return f < 5 ? prod_pk(in[f - 2], in[(f - 1) % 3]) : prod_pk(in[f - 5], in[3]);
   }
 }
@@ -1237,7 +1242,7 @@ constexpr int FLUX_MAX_BINS = 64;
 // Assembly of the stage's spectral vector from forward-transformed product f
 // (p already scaled by 1/(Nx Ny Nz)):
 //   FORM 0: N_i = sum_j i K_j F[u_i u_j]  (compute_diag_offdiag.cc:47-98)
-//   FORM 7: the same from d1, d2, u1u2, u2u3, u3u1 (N up to a gradient, for a step)
+//   FORM 7: the same from d2, d3, u1u2, u2u3, u3u1 (N up to a gradient, for a step)
 //   FORM 1: N = -F[u x omega]
 //   FORM 3: A_i + (i K x B)_i  (adjoint; B = products 0-2, A = products 3-5)
 template <int FORM, typename V, typename S>
@@ -1253,8 +1258,8 @@ __device__ __forceinline__ void accum_product(int f, V p, S Kx, S Ky, S Kz, V& a
     }
   } else if (FORM == 7) {
     switch (f) {
-      case 0: a0 = add(a0, ik(Kx, p)); break;
-      case 1: a1 = add(a1, ik(Ky, p)); break;
+      case 0: a1 = add(a1, ik(Ky, p)); break;
+      case 1: a2 = add(a2, ik(Kz, p)); break;
       case 2: a0 = add(a0, ik(Ky, p)); a1 = add(a1, ik(Kx, p)); break;
       case 3: a1 = add(a1, ik(Kz, p)); a2 = add(a2, ik(Ky, p)); break;
       default: a2 = add(a2, ik(Kx, p)); a0 = add(a0, ik(Kz, p)); break;
@@ -1588,9 +1593,9 @@ __device__ __forceinline__ void step_mode(const C<T>* p, const T (&K)[3], T rK2,
   if constexpr (FORM == 1) {
     m[0] = p[0]; m[1] = p[1]; m[2] = p[2];
   } else {
-    m[0] = add(add(scale(p[0], K[0]), scale(p[2], K[1])), scale(p[4], K[2]));
-    m[1] = add(add(scale(p[2], K[0]), scale(p[1], K[1])), scale(p[3], K[2]));
-    m[2] = add(scale(p[4], K[0]), scale(p[3], K[1]));
+    m[0] = add(scale(p[2], K[1]), scale(p[4], K[2]));
+    m[1] = add(add(scale(p[2], K[0]), scale(p[0], K[1])), scale(p[3], K[2]));
+    m[2] = add(add(scale(p[4], K[0]), scale(p[3], K[1])), scale(p[1], K[2]));
   }
   if (fc) {
     // N - F: with N = -inv m (FORM 1) m + F / inv, with N = i inv m (FORM 7) m + i F / inv

@@ -17,7 +17,7 @@
 //             V_0 = c_0 (C) or 0 (S), c_N = 0; v = inverse FFT_N(V) (unscaled);
 //             u_{2k} = v_k, u_{2k+1} = v_{N-1-k}, and u_n *= (-1)^n for S.
 // Parities (global/Global.cc:137-145, sincostr "SFF"): u1 S, u2 C, u3 C, T S;
-// products (form 2 of the z pass) u1u1 - u3u3 and u2u2 - u3u3 C, u1u2 S, u2u3 C, u3u1 S,
+// products (form 2 of the z pass) u2u2 - u1u1 and u3u3 - u1u1 C, u1u2 S, u2u3 C, u3u1 S,
 // u1T C, u2T S, u3T S.
 // x derivative of a C series is -Kx (result S), of an S series +Kx (result C)
 // (SFF_pencil_tr.cc:77-106).
@@ -450,9 +450,9 @@ __global__ void __launch_bounds__(256) k_sff_prod_epi(const C<T>* P, Geo g, SffA
 #pragma unroll
     for (int f = 0; f < 8; ++f) q[f] = P[f * g.S + e];
     const T Kx = (T)(m * g.kf[0]), Ky = (T)(kfft(ly, g.Ny) * g.kf[1]), Kz = (T)(lz * g.kf[2]);
-    const V N1 = add(add(scale(q[0], -Kx), ik(Ky, q[2])), ik(Kz, q[4]));
-    const V N2 = add(add(ik(Ky, q[1]), scale(q[2], Kx)), ik(Kz, q[3]));
-    const V N3 = add(ik(Ky, q[3]), scale(q[4], Kx));
+    const V N1 = add(ik(Ky, q[2]), ik(Kz, q[4]));
+    const V N2 = add(add(ik(Ky, q[0]), scale(q[2], Kx)), ik(Kz, q[3]));
+    const V N3 = add(add(ik(Kz, q[1]), ik(Ky, q[3])), scale(q[4], Kx));
     const V NT = add(add(scale(q[5], -Kx), ik(Ky, q[6])), ik(Kz, q[7]));
     sff_epilogue<T>(g, a, mb, m, ly, lz, e, N1, N2, N3, NT);
   }
@@ -460,9 +460,9 @@ __global__ void __launch_bounds__(256) k_sff_prod_epi(const C<T>* P, Geo g, SffA
 
 // ---------------------------------------------------------------------------
 // forward x pass + Boussinesq epilogue (PRLARGE / ULARGE):
-//   N1 = Dx(d1) + iKy F[u1u2] + iKz F[u3u1],  N2 = iKy F[d2] + Dx(u1u2) + iKz F[u2u3],
-//   N3 = iKy F[u2u3] + Dx(u3u1),  NT = Dx(u1T) + iKy F[u2T] + iKz F[u3T],
-//   d1 = u1u1 - u3u3, d2 = u2u2 - u3u3 (N up to a gradient, which the projection removes)
+//   N1 = iKy F[u1u2] + iKz F[u3u1],  N2 = iKy F[d2] + Dx(u1u2) + iKz F[u2u3],
+//   N3 = iKz F[d3] + iKy F[u2u3] + Dx(u3u1),  NT = Dx(u1T) + iKy F[u2T] + iKz F[u3T],
+//   d2 = u2u2 - u1u1, d3 = u3u3 - u1u1 (N up to a gradient, which the projection removes)
 //   (compute_diag_offdiag.cc:47-136); force U.F1 = cu T, T.F = cT U.V1 (compute_force_RBC.cc:104-150);
 //   N -= F; p = div(N)/K^2; N += grad p; R = -N, RT = -NT; IF-RK4 stage update of U (nu) and T (kappa)
 //   (RK_SF.cc:97-221, Tadvance_functions.cc:57-90,226-237,372-395,589-611).
@@ -545,8 +545,8 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
       const V cm = sine ? mul_i<1>(scale(sub(wz, wzr), (T)scl)) : scale(add(wz, wzr), (T)scl);
       const T Kx = (T)(m * g.kf[0]);
       switch (f) {
-        case 0: acc[0][s] = add(acc[0][s], scale(cm, -Kx)); break;
-        case 1: acc[1][s] = add(acc[1][s], ik(Ky, cm)); break;
+        case 0: acc[1][s] = add(acc[1][s], ik(Ky, cm)); break;
+        case 1: acc[2][s] = add(acc[2][s], ik(Kz, cm)); break;
         case 2: acc[0][s] = add(acc[0][s], ik(Ky, cm)); acc[1][s] = add(acc[1][s], scale(cm, Kx)); break;
         case 3: acc[1][s] = add(acc[1][s], ik(Kz, cm)); acc[2][s] = add(acc[2][s], ik(Ky, cm)); break;
         case 4: acc[0][s] = add(acc[0][s], ik(Kz, cm)); acc[2][s] = add(acc[2][s], scale(cm, Kx)); break;
@@ -573,10 +573,10 @@ __global__ void __launch_bounds__(CW * (N / E), sff_min_blocks(CW * (N / E), E))
 
 // ---------------------------------------------------------------------------
 // FFF passive scalar (program.kind SCALAR_INCOMPRESS), elementwise epilogue after the
-// forward x FFT of the eight products of form 2 (u1u1 - u3u3, u2u2 - u3u3, u1u2,
+// forward x FFT of the eight products of form 2 (u2u2 - u1u1, u3u3 - u1u1, u1u2,
 // u2u3, u3u1, u1T, u2T, u3T; unnormalised):
 //   N_i = sum_j i K_j F[u_j u_i]  (compute_diag_offdiag.cc:47-98, conservative) less the
-//   gradient of u3u3, which the projection removes
+//   gradient of u1u1, which the projection removes
 //   NT  = sum_j i K_j F[u_j T]    (compute_diag_offdiag.cc:116-136)
 //   no force (Add_force with F = 0); p = (i K . N)/K^2, N <- N + i K p; R = -N,
 //   RT = -NT; IF-RK4 stage update of U (nu) and T (kappa) as the Boussinesq
@@ -609,9 +609,9 @@ __global__ void __launch_bounds__(256) k_scalar_epi(const C<T>* P, Geo g, SffArg
       if (a.stage > 1) ttv[i] = tot[i * g.S + e];
     }
     // x, then y, then z derivative terms, as the reference accumulates them
-    V N1 = add(add(ik(Kx, p[0]), ik(Ky, p[2])), ik(Kz, p[4]));
-    V N2 = add(add(ik(Kx, p[2]), ik(Ky, p[1])), ik(Kz, p[3]));
-    V N3 = add(ik(Kx, p[4]), ik(Ky, p[3]));
+    V N1 = add(ik(Ky, p[2]), ik(Kz, p[4]));
+    V N2 = add(add(ik(Kx, p[2]), ik(Ky, p[0])), ik(Kz, p[3]));
+    V N3 = add(add(ik(Kx, p[4]), ik(Ky, p[3])), ik(Kz, p[1]));
     const V NT = add(add(ik(Kx, p[5]), ik(Ky, p[6])), ik(Kz, p[7]));
     const double K2 = (Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd;
     const V div = add(add(ik(Kx, N1), ik(Ky, N2)), ik(Kz, N3));
@@ -656,9 +656,9 @@ __global__ void __launch_bounds__(256) k_scalar_epi(const C<T>* P, Geo g, SffArg
 // FFF incompressible MHD (RK4(U, W, P, F) with W = B, no force), elementwise
 // epilogue after the forward x FFT of the eight products of the z pass form 5: with
 // P_ij = F[Zp_i Zm_j], S_ij = (P_ij + P_ji)/2 and A_ij = (P_ij - P_ji)/2, the products are
-// S11 - S33, S22 - S33, S12, S23, S13, A12, A23, A31 (unnormalised).  Zp.nlin_i = sum_j D_j P_ij,
+// S22 - S11, S33 - S11, S12, S23, S13, A12, A23, A31 (unnormalised).  Zp.nlin_i = sum_j D_j P_ij,
 //   Zm.nlin_i = sum_j D_j P_ji (compute_diag_offdiag.cc:202-258), so
-//   U.nlin = (Zp.nlin + Zm.nlin)/2 = sum_j D_j S_ij, here less the gradient of S33, which the
+//   U.nlin = (Zp.nlin + Zm.nlin)/2 = sum_j D_j S_ij, here less the gradient of S11, which the
 //   pressure removes; B.nlin = (Zp.nlin - Zm.nlin)/2 = sum_j D_j A_ij (MHD.cc:150-161);
 //   R_U = -(U.nlin + i K p), R_B = -B.nlin (Tadvance_functions.cc:259-267); IF-RK4
 //   stage update of U (nu, tables eu) and B (eta, tables et), RK_VF_MHD.cc:126-186.
@@ -692,9 +692,9 @@ __global__ void __launch_bounds__(256, 3) k_mhd_epi(const C<T>* P, Geo g, SffArg
       if (a.stage > 1) ttv[i] = tot[i * g.S + e];
     }
     // U.nlin = sum_j D_j S_ij (up to a gradient), B.nlin = sum_j D_j A_ij
-    const V NU[3] = {add(add(ik(K[0], q[0]), ik(K[1], q[2])), ik(K[2], q[4])),
-                     add(add(ik(K[0], q[2]), ik(K[1], q[1])), ik(K[2], q[3])),
-                     add(ik(K[0], q[4]), ik(K[1], q[3]))};
+    const V NU[3] = {add(ik(K[1], q[2]), ik(K[2], q[4])),
+                     add(add(ik(K[0], q[2]), ik(K[1], q[0])), ik(K[2], q[3])),
+                     add(add(ik(K[0], q[4]), ik(K[1], q[3])), ik(K[2], q[1]))};
     const V NB[3] = {sub(ik(K[1], q[5]), ik(K[2], q[7])), sub(ik(K[2], q[6]), ik(K[0], q[5])),
                      sub(ik(K[0], q[7]), ik(K[1], q[6]))};
     const double K2 = (Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd;
@@ -740,11 +740,12 @@ __global__ void __launch_bounds__(256, 3) k_mhd_epi(const C<T>* P, Geo g, SffArg
 
 // ---------------------------------------------------------------------------
 // SSF fluid step (sincostr_switch "SCF": Vx = SCF, Vy = CSF, Vz = CCF), elementwise
-// epilogue after the forward transforms of the six products (normalised; parities
-// Vi2 = CCF for u_i u_i, VxVy = SSF, VyVz = CSF, VxVz = SCF; Global.cc:184-191).
+// epilogue after the forward transforms of the five products of form 7 (normalised;
+// parities Vi2 = CCF for d2 = u2u2 - u1u1 and d3 = u3u3 - u1u1, VxVy = SSF, VyVz = CSF,
+// VxVz = SCF; Global.cc:184-191).
 // Derivatives (SSF_pencil_tr.cc): x and y parity S -> +K, C -> -K; z -> i Kz.
-//   N1 = Dx(u1u1) + Dy(u1u2) + Dz(u3u1), N2 = Dy(u2u2) + Dx(u1u2) + Dz(u2u3),
-//   N3 = Dz(u3u3) + Dy(u2u3) + Dx(u3u1)  (compute_diag_offdiag.cc:47-98)
+//   N1 = Dy(u1u2) + Dz(u3u1), N2 = Dy(d2) + Dx(u1u2) + Dz(u2u3), N3 = Dz(d3) + Dy(u2u3) +
+//   Dx(u3u1)  (compute_diag_offdiag.cc:47-98, less the gradient of u1u1)
 //   div = Dx^Vx N1 + Dy^Vy N2 + Dz N3, p = div/K^2, N += (Dx^div p, Dy^div p, Dz p), R = -N;
 //   IF-RK4 stage update as the FFF step (RK.cc:91-170); no reality condition.
 // ---------------------------------------------------------------------------
@@ -776,9 +777,9 @@ __global__ void __launch_bounds__(256) k_ssf_epi(const C<T>* P, Geo g, StageArgs
     // x / y derivative of a sine (+K) or cosine (-K) series
     auto dS = [](T K, V A) { return scale(A, K); };
     auto dC = [](T K, V A) { return scale(A, -K); };
-    V N1 = add(add(dC(Kx, q[0]), dS(Ky, q[2])), ik(Kz, q[4]));
-    V N2 = add(add(dC(Ky, q[1]), dS(Kx, q[2])), ik(Kz, q[3]));
-    V N3 = add(dS(Ky, q[3]), dS(Kx, q[4]));
+    V N1 = add(dS(Ky, q[2]), ik(Kz, q[4]));
+    V N2 = add(add(dC(Ky, q[0]), dS(Kx, q[2])), ik(Kz, q[3]));
+    V N3 = add(add(ik(Kz, q[1]), dS(Ky, q[3])), dS(Kx, q[4]));
     const double K2 = (Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd;
     const V div = add(add(dS(Kx, N1), dS(Ky, N2)), ik(Kz, N3));
     const V pr = (K2 > 0) ? mk<V>(div.x / (T)K2, div.y / (T)K2) : mk<V>(0, 0);
@@ -818,7 +819,7 @@ __global__ void __launch_bounds__(256) k_ssf_epi(const C<T>* P, Geo g, StageArgs
 // SSS fluid step (sincostr_switch "SCC": Vx = SCC, Vy = CSC, Vz = CCS), on real
 // coefficients in the padded real layout (Nz + 2 reals per line, lzr < Nz used):
 // dealiased copy, and the elementwise epilogue after the forward transforms of the
-// six products (Vi2 = CCC, VxVy = SSC, VyVz = CSS, VxVz = SCS; Global.cc:221-228).
+// five products of form 7 (Vi2 = CCC, VxVy = SSC, VyVz = CSS, VxVz = SCS; Global.cc:221-228).
 // Derivatives along every axis: parity S -> +K, C -> -K (SSS_pencil_tr.cc).
 // ---------------------------------------------------------------------------
 template <typename T>
@@ -868,9 +869,9 @@ __global__ void __launch_bounds__(256) k_sss_epi(const T* P, Geo g, StageArgs a)
       u0v[i] = U0[i * per + e];
       if (a.stage > 1) ttv[i] = tot[i * per + e];
     }
-    T N1 = (-Kx * q[0] + Ky * q[2]) + Kz * q[4];
-    T N2 = (-Ky * q[1] + Kx * q[2]) + Kz * q[3];
-    T N3 = Ky * q[3] + Kx * q[4];
+    T N1 = Ky * q[2] + Kz * q[4];
+    T N2 = (-Ky * q[0] + Kx * q[2]) + Kz * q[3];
+    T N3 = (-Kz * q[1] + Ky * q[3]) + Kx * q[4];
     const double K2 = (Kxd * Kxd + Kyd * Kyd) + Kzd * Kzd;
     const T div = (Kx * N1 + Ky * N2) + Kz * N3;
     const T pr = K2 > 0 ? div / (T)K2 : (T)0;
@@ -909,7 +910,7 @@ __global__ void __launch_bounds__(256) k_sss_epi(const T* P, Geo g, StageArgs a)
 // Boussinesq RBC (PRLARGE, ULARGE) on the SSF and SSS bases: the temperature takes
 // the Vx parity and the products u_x T, u_y T, u_z T take Vi2, VxVy and VxVz
 // (Global_process_basic_vars.cc:108, 114-116).  Epilogues after the forward
-// transforms of the eight products (u1u1 - u3u3, u2u2 - u3u3, u1u2, u2u3, u3u1, u1T,
+// transforms of the eight products (u2u2 - u1u1, u3u3 - u1u1, u1u2, u2u3, u3u1, u1T,
 // u2T, u3T; normalised):
 //   N as the fluid step; NT = Dx(u1T) + Dy(u2T) + Dz(u3T) (compute_diag_offdiag.cc:116-136);
 //   force (compute_force_RBC.cc:104-150): U.F1 = cu T, T.F = cT U.V1, both from the
@@ -947,9 +948,9 @@ __global__ void __launch_bounds__(256) k_ssf_rbc_epi(const C<T>* P, Geo g, SffAr
     }
     auto dS = [](T K, V A) { return scale(A, K); };
     auto dC = [](T K, V A) { return scale(A, -K); };
-    V N1 = add(add(dC(Kx, q[0]), dS(Ky, q[2])), ik(Kz, q[4]));
-    V N2 = add(add(dC(Ky, q[1]), dS(Kx, q[2])), ik(Kz, q[3]));
-    V N3 = add(dS(Ky, q[3]), dS(Kx, q[4]));
+    V N1 = add(dS(Ky, q[2]), ik(Kz, q[4]));
+    V N2 = add(add(dC(Ky, q[0]), dS(Kx, q[2])), ik(Kz, q[3]));
+    V N3 = add(add(ik(Kz, q[1]), dS(Ky, q[3])), dS(Kx, q[4]));
     V NT = add(add(dC(Kx, q[5]), dS(Ky, q[6])), ik(Kz, q[7]));
     N1 = sub(N1, scale(Tin[e], (T)a.cu));
     NT = sub(NT, scale(U1in[e], (T)a.cT));
@@ -1022,9 +1023,9 @@ __global__ void __launch_bounds__(256) k_sss_rbc_epi(const T* P, Geo g, SffArgs 
       u0v[i] = i < 3 ? U0[i * per + e] : T0[e];
       if (a.stage > 1) ttv[i] = tot[i * per + e];
     }
-    T N1 = (-Kx * q[0] + Ky * q[2]) + Kz * q[4];
-    T N2 = (-Ky * q[1] + Kx * q[2]) + Kz * q[3];
-    T N3 = Ky * q[3] + Kx * q[4];
+    T N1 = Ky * q[2] + Kz * q[4];
+    T N2 = (-Ky * q[0] + Kx * q[2]) + Kz * q[3];
+    T N3 = (-Kz * q[1] + Ky * q[3]) + Kx * q[4];
     T NT = (-Kx * q[5] + Ky * q[6]) + Kz * q[7];
     N1 -= (T)a.cu * Tin[e];
     NT -= (T)a.cT * U1in[e];
