@@ -400,6 +400,19 @@ __device__ __forceinline__ void fft_regs_b(V (&v)[NB][E], int t, V* sm, int slot
   }
 }
 
+// Division of several x by one d > 0 (0 for d = 0): the reciprocal as a pair hi + lo (lo: its
+// rounding, from the exact remainder), applied in one fma chain, so that a quotient has the one
+// rounding of a division at two operations
+template <typename S> struct Recip { S hi, lo; };
+template <typename S> __host__ __device__ __forceinline__ Recip<S> recip(S d) {
+  const S h = d > (S)0 ? (S)1 / d : (S)0;
+  return {h, h > (S)0 ? h * fma(-h, d, (S)1) : (S)0};
+}
+template <typename S> __host__ __device__ __forceinline__ S quot1(S x, Recip<S> r) { return fma(x, r.hi, x * r.lo); }
+template <typename V, typename S> __device__ __forceinline__ V quot(V x, Recip<S> r) {
+  return mk<V>(quot1(x.x, r), quot1(x.y, r));
+}
+
 // ---------------------------------------------------------------------------
 // asynchronous global -> shared copies (cp.async): each thread stages the
 // elements it will read itself, so a per-thread wait_group is enough.

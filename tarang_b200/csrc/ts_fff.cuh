@@ -370,8 +370,7 @@ __global__ void __launch_bounds__(CW * (L / E), MINB)
 // ---------------------------------------------------------------------------
 // inverse x pass of the adjoint's cotangent: W_6..8 = IFFT_x(lsc c^-1 P Lam), the
 // Leray-projected cotangent divided by the C2R weight c (2 on the planes 0 < kz < Nz/2, else
-// 1).  The three components of a column stay in registers from the projection (one
-// division per mode) to their transforms, one after the other through one exchange tile.
+// 1).  The three components of a column stay in registers from the projection to their transforms, one after the other through one exchange tile.
 // ---------------------------------------------------------------------------
 template <typename T, int L, int E, int CW, int MINB>
 __global__ void __launch_bounds__(CW * (L / E), MINB)
@@ -396,8 +395,9 @@ __global__ void __launch_bounds__(CW * (L / E), MINB)
   for (int s = 0; s < E; ++s) {
     // (P Lam)_i = Lam_i - K_i (K . Lam) / K^2, identity at K = 0
     const T Kx = (T)(kfft(load_row<L, E>(t, s), g.Nx) * g.kf[0]);
-    const T K2 = (Kx * Kx + Ky * Ky) + Kz * Kz, r = K2 > (T)0 ? (T)1 / K2 : (T)0;
-    const V d = scale(add(add(scale(v[0][s], Kx), scale(v[1][s], Ky)), scale(v[2][s], Kz)), r);
+    const T K2 = (Kx * Kx + Ky * Ky) + Kz * Kz;
+    const V n = add(add(scale(v[0][s], Kx), scale(v[1][s], Ky)), scale(v[2][s], Kz));
+    const V d = quot(n, recip(K2));
     v[0][s] = scale(sub(v[0][s], scale(d, Kx)), lw);
     v[1][s] = scale(sub(v[1][s], scale(d, Ky)), lw);
     v[2][s] = scale(sub(v[2][s], scale(d, Kz)), lw);
@@ -1584,7 +1584,7 @@ __global__ void __launch_bounds__(CW * (L / E), 1)
 // (inv is a power of two: every FFF axis is).  STAGE is known at compile time, rK2 = 1 / K^2
 // (0 at K = 0), fc the force of the mode (zero outside the band).
 template <typename T, int FORM, int STAGE>
-__device__ __forceinline__ void step_mode(const C<T>* p, const T (&K)[3], T rK2, T inv, const C<T>* fc, bool dz,
+__device__ __forceinline__ void step_mode(const C<T>* p, const T (&K)[3], Recip<T> rK2, T inv, const C<T>* fc, bool dz,
                                           bool clear, Fac<T> Feh, Fac<T> Fe1, const Fac<T> (&Fc)[4], const C<T>* u0,
                                           const C<T>* tt, C<T>* Uc, C<T>* tot, C<T>* Uo, long long off, long long S,
                                           int* err) {
@@ -1604,7 +1604,7 @@ __device__ __forceinline__ void step_mode(const C<T>* p, const T (&K)[3], T rK2,
     for (int i = 0; i < 3; ++i) m[i] = FORM == 1 ? add(m[i], scale(fc[i], w)) : add_i<1>(m[i], scale(fc[i], w));
   }
   V d = mk<V>(K[0] * m[0].x + K[1] * m[1].x + K[2] * m[2].x, K[0] * m[0].y + K[1] * m[1].y + K[2] * m[2].y);
-  d = scale(d, rK2);
+  d = quot(d, rK2);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const V r = mk<V>((m[i].x - K[i] * d.x) * inv, (m[i].y - K[i] * d.y) * inv);
@@ -1770,8 +1770,7 @@ __global__ void __launch_bounds__(z_nout(FORM) * CW * (L / E), 1)
                            (long long)r * inner + col, g.S);
         return;
       }
-      const T K2 = (T)(tk2[r] + c2);
-      const T rK2 = K2 > (T)0 ? (T)1 / K2 : (T)0;
+      const Recip<T> rK2 = recip((T)(tk2[r] + c2));
       Fac<T> Feh, Fe1;
       if constexpr (F32) {
         Feh = pair_mul(reinterpret_cast<const float2*>(tex)[r], ecol);
