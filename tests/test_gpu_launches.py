@@ -3,6 +3,8 @@ ones only the sin/cos y passes (two in each of the four stages).  Read from the 
 a step, whose edges say whether a kernel may start before its predecessor has ended."""
 import pytest
 
+from capture import captured
+
 pytestmark = pytest.mark.gpu
 
 # (basis, precision, sizes, launches that overlap; None: most of them)
@@ -13,25 +15,11 @@ CASES += [("FFF", "f32", (128, 128, 256), 0), ("FFF", "f64", (128, 128, 128), 0)
 
 @pytest.mark.parametrize("basis,prec,N,count", CASES)
 def test_overlapped_launches_of_a_step(cuda, basis, prec, N, count):
-    import torch
     import tarang_b200 as tb
-    rt = pytest.importorskip("cuda.bindings.runtime")
-
-    def ok(r):
-        assert r[0] == rt.cudaError_t.cudaSuccess, r[0]
-        return r[1:]
-
     plan = tb.Plan(N, basis=basis, precision=prec, dealias="two_thirds", nu=0.01, kappa=0.01, dt=1e-4, Ra=1e4, Pr=1.0)
     u, T = plan.field(3), plan.field(1)
-    stream = torch.cuda.Stream()
-    plan.set_stream(stream)
     step = (lambda: plan.rk4_step(u, 1)) if basis == "FFF" else (lambda: plan.rk4_step_rbc(u, T, 1))
-    step()  # work fields are allocated by the first step
-    plan.status()
-    ok(rt.cudaStreamBeginCapture(stream.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeRelaxed))
     step()
-    (graph,) = ok(rt.cudaStreamEndCapture(stream.cuda_stream))
-    _, _, edges, n = ok(rt.cudaGraphGetEdges_v2(graph, 1024))
-    overlapped = sum(e.type == int(rt.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic) for e in edges[:n])
-    ok(rt.cudaGraphDestroy(graph))
-    assert n > 16 and (overlapped > n // 2 if count is None else overlapped == count)
+    types = captured(plan, step)[1]
+    overlapped = types.count(1)
+    assert len(types) > 16 and (overlapped > len(types) // 2 if count is None else overlapped == count)

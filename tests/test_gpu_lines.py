@@ -3,18 +3,38 @@ lines of every axis, lengths with a factor 3, planes whose columns end inside a 
 
 The transforms are compared with numpy / scipy in FP64; an FFT of n points of unit-variance
 data loses about eps * log2(n) in relative L2 norm, so the bounds are 4 eps log2(points).
-The steps are compared with the FP64 oracle: the state moves by a few per cent, FP32
-states are rounded to 2^-24 each stage, so 1e-6 holds for FP32 and 1e-13 for FP64."""
+The steps are compared with the FP64 oracle from states with energy in every mode, so that a
+lost or wrongly dealiased row shows.  The time step is such that a step moves the state by at
+most CHANGE = 5 %: its error is the rounding of the stored state (half an ulp in FP32, where one
+fma chain ends it; three roundings in FP64) plus CHANGE times that of the transforms (step_tol)."""
 import math
 
 import numpy as np
 import pytest
 
+from capture import captured
 from oracle import tarang_ref as R
 
 pytestmark = pytest.mark.gpu
 
 EPS = {"f32": 2.0 ** -23, "f64": 2.0 ** -52}
+CHANGE = 0.05
+
+
+def step_tol(prec, N):
+    return EPS[prec] * ({"f32": 0.5, "f64": 1.5}[prec] + CHANGE * math.log2(np.prod(N)))
+
+
+def lively(g, seed):
+    """A solenoidal field: the benchmark's spectrum plus noise of the same energy in every mode."""
+    rng = np.random.default_rng(seed)
+    F = np.stack([R.reality_fix(g, R.forward(g, 0.3 * rng.standard_normal(g.rshape))) for _ in range(3)])
+    return R.init_energy_spectrum(g, R.spectrum_k4_gauss(g.n_shells(), 4.0), seed, 0.5) - R.project_rhs(g, F)
+
+
+def small_dt(N):
+    """CHANGE / (largest wavenumber times largest speed, 5)"""
+    return CHANGE / (5 * max(N) / 2)
 
 
 def rel(a, b):
@@ -70,6 +90,13 @@ STEPS += [(f, d, N) for f, d in (("rotational", "two_thirds"), ("conservative", 
           for N in ((32, 16, 16), (32, 64, 32), (64, 16, 16), (64, 128, 64))]
 
 
+# more column tiles than blocks of the persistent pipelined kernel (148, or 296 at 32 and 64 points; no
+# field of its size has more at 64): a block's buffers are used again
+STEPS += [("conservative", "reference", (32, 128, 128)), ("rotational", "two_thirds", (128, 64, 256)),
+          ("conservative", "two_thirds", (128, 64, 128)), ("rotational", "reference", (256, 64, 128)),
+          ("conservative", "reference", (256, 64, 128))]
+
+
 @pytest.mark.parametrize("prec", ["f32", "f64"])
 @pytest.mark.parametrize("form,dealias,N", STEPS)
 def test_forced_step_at_line_edges(cuda, form, dealias, N, prec):
@@ -78,14 +105,62 @@ def test_forced_step_at_line_edges(cuda, form, dealias, N, prec):
     g = R.Grid(N)
     es = np.zeros(g.n_shells())
     es[3] = 0.1
-    V = R.init_energy_spectrum(g, R.spectrum_k4_gauss(g.n_shells(), 4.0), 0, 0.5)
+    V, dt = lively(g, 0), small_dt(N)
     mode = {"reference": 1, "two_thirds": 2}[dealias]
-    want = R.rk4_step(R.FluidConfig(g, 0.01, 1e-2, mode, form, True, R.CaratiForcing(2.0, 3.0, es)), V)
-    plan = tb.Plan(N, precision=prec, nlin_form=form, dealias=dealias, nu=0.01, dt=1e-2,
-                   forcing=tb.Forcing(2.0, 3.0, es))
+    plan = tb.Plan(N, precision=prec, nlin_form=form, dealias=dealias, nu=0.01, dt=dt, forcing=tb.Forcing(2.0, 3.0, es))
     u = torch.from_numpy(V).to(plan.torch_dtype()).to(cuda)
+    V = u.cpu().numpy().astype(np.complex128)
+    want = R.rk4_step(R.FluidConfig(g, 0.01, dt, mode, form, True, R.CaratiForcing(2.0, 3.0, es)), V)
     plan.rk4_step(u, 1)
-    assert rel(u.cpu().numpy(), want) < {"f32": 1e-6, "f64": 1e-13}[prec]
+    assert rel(u.cpu().numpy(), want) < step_tol(prec, N)
+
+
+MORE = [(N, d) for N in ((16, 16, 16), (1024, 16, 16), (16, 1024, 16), (16, 32, 1024), (512, 16, 32), (16, 512, 64), (32, 16, 512),
+                         (128, 64, 64), (256, 16, 128)) for d in ("reference", "two_thirds")]
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("kind", ["scalar", "mhd"])
+@pytest.mark.parametrize("N,dealias", MORE)
+def test_scalar_and_mhd_step_at_line_edges(cuda, N, dealias, kind, prec):
+    import torch
+    import tarang_b200 as tb
+    g = R.Grid(N)
+    dt, mode = small_dt(N), {"reference": 1, "two_thirds": 2}[dealias]
+    U, B = lively(g, 0), lively(g, 1)
+    if kind == "scalar":
+        B = B[:1]
+    plan = tb.Plan(N, precision=prec, dealias=dealias, nu=0.01, kappa=0.02, dt=dt)
+    u, b = (torch.from_numpy(a).to(plan.torch_dtype()).to(cuda) for a in (U, B))
+    U, B = (x.cpu().numpy().astype(np.complex128) for x in (u, b))
+    if kind == "scalar":
+        wu, wb = R.rbc_rk4_step(R.ScalarConfig(g, nu=0.01, kappa=0.02, dt=dt, dealias_mode=mode), U, B[0])
+        plan.rk4_step_scalar(u, b, 1)
+        wb = wb[None]
+    else:
+        wu, wb = R.mhd_rk4_step(R.MHDConfig(g, nu=0.01, eta=0.02, dt=dt, dealias_mode=mode), U, B)
+        plan.rk4_step_mhd(u, b, 1)
+    assert rel(u.cpu().numpy(), wu) < step_tol(prec, N)
+    assert rel(b.cpu().numpy(), wb) < step_tol(prec, N)
+
+
+@pytest.mark.parametrize("N", [(128, 64, 64), (128, 16, 256), (256, 16, 32), (64, 32, 128)])
+def test_adjoint_step_at_line_edges(cuda, N):
+    """FP64, the bound of the oracle comparisons of the adjoint; 128 x 64 x 64 has more column tiles
+    than the pipelined kernel has blocks."""
+    import torch
+    import tarang_b200 as tb
+    g, dt = R.Grid(N), small_dt(N)
+    V = lively(g, 0)
+    rng = np.random.default_rng(5)
+    Lam = rng.standard_normal((3,) + g.shape) + 1j * rng.standard_normal((3,) + g.shape)
+    plan = tb.Plan(N, precision="f64", nlin_form="rotational", dealias="two_thirds", nu=0.01, dt=dt)
+    u = torch.from_numpy(V).to(cuda)
+    lam = torch.from_numpy(Lam.copy()).to(cuda)
+    work = torch.empty(plan.adjoint_work_bytes(1), dtype=torch.uint8, device=cuda)
+    plan.adjoint_window(u, 1, lam, work)
+    cfg = R.FluidConfig(g, nu=0.01, dt=dt, dealias_mode=2, nlin_form="rotational", reality_fix=True)
+    assert rel(lam.cpu().numpy(), R.rk4_step_adjoint(cfg, V, Lam)) < 1e-11
 
 
 RBC = [("SFF", (16, 16, 48)), ("SFF", (96, 48, 16)), ("SFF", (16, 1, 96)), ("SFF", (512, 16, 16)), ("SSF", (48, 96, 16)),
@@ -93,22 +168,27 @@ RBC = [("SFF", (16, 16, 48)), ("SFF", (96, 48, 16)), ("SFF", (16, 1, 96)), ("SFF
 
 
 @pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("dealias", ["reference", "two_thirds"])
 @pytest.mark.parametrize("basis,N", RBC)
-def test_convection_step_at_line_edges(cuda, basis, N, prec):
+def test_convection_step_at_line_edges(cuda, basis, N, dealias, prec):
     import torch
     import tarang_b200 as tb
     kf = (math.pi, 2 * math.pi, 2 * math.pi) if basis == "SFF" else (math.pi,) * 3
     g = R.Grid(N, kf, basis)
     rng = np.random.default_rng(3)
     par = {"SFF": ("S", "C", "C", "S"), "SSF": ("SCF", "CSF", "CCF", "SCF"), "SSS": ("SCC", "CSC", "CCS", "SCC")}[basis]
-    # random fields inside the dealiased range, without Nyquist planes, U solenoidal
+    # random fields with energy in every mode but the Nyquist planes, U solenoidal
     F = np.stack([R.reality_fix(g, R.forward(g, 0.3 * rng.standard_normal(N), p)) for p in par])
-    F[..., R.dealias_mask(g, 2)] = 0
+    if basis == "SFF" and N[1] > 1:
+        F[:, :, N[1] // 2] = 0
+    if basis != "SSS":
+        F[..., N[2] // 2] = 0
     U, T = -R.project_rhs(g, F[:3]), F[3]
-    cfg = R.RBCConfig(grid=g, Ra=1e4, Pr=1.0, dt=1e-3, dealias_mode=1)
-    wu, wt = R.rbc_rk4_step(cfg, U, T)
-    plan = tb.Plan(N, basis=basis, precision=prec, kfactor=kf, dealias="reference", nu=cfg.nu, kappa=cfg.kappa, Ra=1e4,
-                   Pr=1.0, dt=1e-3)
+    kmax = max(f * n / (1 if b == "S" else 2) for f, n, b in zip(kf, N, basis))
+    dt = CHANGE / (2 * kmax)  # speeds stay below 2
+    cfg = R.RBCConfig(grid=g, Ra=1e4, Pr=1.0, dt=dt, dealias_mode={"reference": 1, "two_thirds": 2}[dealias])
+    plan = tb.Plan(N, basis=basis, precision=prec, kfactor=kf, dealias=dealias, nu=cfg.nu, kappa=cfg.kappa, Ra=1e4,
+                   Pr=1.0, dt=dt)
 
     def pack(a):
         if basis == "SSS":
@@ -117,16 +197,15 @@ def test_convection_step_at_line_edges(cuda, basis, N, prec):
             a = p.view(np.complex128)
         return torch.from_numpy(np.ascontiguousarray(a)).to(plan.torch_dtype()).to(cuda)
 
-    u, t = pack(U), pack(T[None])
-    plan.rk4_step_rbc(u, t, 1)
-
     def unpack(x):
         x = x.cpu().numpy().astype(np.complex128)
         return x.view(np.float64)[..., : N[2]] if basis == "SSS" else x
 
-    tol = {"f32": 1e-6, "f64": 1e-13}[prec]
-    assert rel(unpack(u), wu) < tol
-    assert rel(unpack(t)[0], wt) < tol
+    u, t = pack(U), pack(T[None])
+    wu, wt = R.rbc_rk4_step(cfg, unpack(u), unpack(t)[0])
+    plan.rk4_step_rbc(u, t, 1)
+    assert rel(unpack(u), wu) < step_tol(prec, N)
+    assert rel(unpack(t)[0], wt) < step_tol(prec, N)
 
 
 def in_place():
@@ -145,7 +224,8 @@ COMPACT = [((16, 16, 128), "rotational"), ((32, 16, 128), "conservative"), ((128
 def test_compact_inverse_lines_match_in_place(cuda, N, kind, prec):
     """Two-thirds dealiased right-hand sides on compact inverse-transformed lines (FP32, 128 points
     along z and more) against the same steps in place.  The arithmetic of a mode is the same but
-    for the order of the y butterflies' rounding, so the two agree to a few roundings of the state."""
+    for the order of the y butterflies' rounding, so the two agree to a few roundings of the state.
+    The layout shows in the y inverse's grid: tiles of 16 columns over whole compact lines."""
     import torch
     import tarang_b200 as tb
     g = R.Grid(N)
@@ -159,14 +239,18 @@ def test_compact_inverse_lines_match_in_place(cuda, N, kind, prec):
             plan.set_tuning(tuning)
         u, b = (torch.from_numpy(a).to(plan.torch_dtype()).to(cuda) for a in (V, B))
         if kind == "mhd":
-            plan.rk4_step_mhd(u, b, 2)
+            call = lambda: plan.rk4_step_mhd(u, b, 2)
         elif kind == "adjoint":
             work = torch.empty(plan.adjoint_work_bytes(2), dtype=torch.uint8, device=cuda)
-            plan.adjoint_window(u, 2, b, work)
+            call = lambda: plan.adjoint_window(u, 2, b, work)
         else:
-            plan.rk4_step(u, 2)
+            call = lambda: plan.rk4_step(u, 2)
+        call()
         plan.status()
         got.append((u.cpu().numpy(), b.cpu().numpy()))
+        pitch = (N[2] // 3 + 1 + 15) // 16 * 16
+        tiles = (3 if kind == "conservative" else 6) * N[0] * pitch // 16
+        assert (tiles in captured(plan, call)[0]) == (prec == "f32" and N[2] >= 128 and not tuning)
     tol = 16 * math.log2(np.prod(N)) * EPS[prec]
     for x, y in zip(*got):
         assert rel(x, y) < tol

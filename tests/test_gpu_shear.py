@@ -18,6 +18,7 @@ pytestmark = pytest.mark.gpu
 
 EPS = {"f32": 2.0 ** -23, "f64": 2.0 ** -52}
 STEPS, NU = 2, 0.01
+LONG = 800
 
 
 def flow(basis, N, axis, rng):
@@ -50,11 +51,11 @@ def flow(basis, N, axis, rng):
     return A
 
 
-def decay(basis, N, kf, dt):
+def decay(basis, N, kf, time):
     ks = [np.arange(N[ax]) if basis[ax] == "S" else np.fft.fftfreq(N[ax], 1 / N[ax]) for ax in range(3)]
     ks[2] = np.arange(N[2] // 2 + 1)
     K = np.meshgrid(*[k * f for k, f in zip(ks, kf)], indexing="ij")
-    return np.exp(-NU * dt * STEPS * sum(k ** 2 for k in K))
+    return np.exp(-NU * time * sum(k ** 2 for k in K))
 
 
 CASES = [("FFF", kind, axis, N) for kind in ("fluid", "scalar", "mhd") for axis in range(3)
@@ -87,6 +88,34 @@ def test_parallel_flows_only_decay(cuda, basis, kind, axis, N, prec):
         assert noise == 0
     else:
         assert noise < 4 * EPS[prec] * math.log2(np.prod(N)) * STEPS * dt * kmax * 20 * np.linalg.norm(start)
-    want = start * decay(basis, N, kf, dt)
+    want = start * decay(basis, N, kf, STEPS * dt)
     err = np.linalg.norm(u[axis].cpu().numpy() - want) / np.linalg.norm(want)
     assert err < 2 * STEPS * EPS[prec]
+
+
+@pytest.mark.parametrize("basis,kind,N", [("FFF", k, N) for k in ("fluid", "scalar", "mhd")
+                                          for N in ((32, 16, 32), (128, 16, 16), (256, 16, 16), (512, 16, 16))]
+                         + [("SFF", "rbc", (32, 16, 16)), ("SSF", "fluid", (32, 16, 16)), ("SSF", "rbc", (96, 48, 16))])
+def test_integrating_factors_have_no_bias(cuda, basis, kind, N):
+    """A flow along z in FP32 over LONG steps: every step is one rounding of u0 exp(-nu K^2 dt), so the
+    state stays within a rounding of the same product rounded in numpy.  A factor rounded to FP32
+    leaves it by 1e-5."""
+    import torch
+    import tarang_b200 as tb
+    kf = {"FFF": (1.0,) * 3, "SFF": (math.pi, 2 * math.pi, 2 * math.pi), "SSF": (math.pi,) * 3}[basis]
+    K2max = sum((f * n / (1 if b == "S" else 2)) ** 2 for f, n, b in zip(kf, N, basis))
+    dt = 1.0 / (LONG * NU * K2max)  # the smallest scales lose a factor e
+    plan = tb.Plan(N, basis=basis, precision="f32", kfactor=kf, dealias="reference", nu=NU, kappa=NU, dt=dt, Ra=1e4, Pr=1.0)
+    u, other = plan.field(3), plan.field(3 if kind == "mhd" else 1)
+    u[2] = torch.from_numpy(flow(basis, N, 2, np.random.default_rng(2))).to(plan.torch_dtype())
+    u[2, 0, 0, 0] = 0
+    want = u[2].cpu().numpy()
+    for _ in range(LONG):
+        want = (want.astype(np.complex128) * decay(basis, N, kf, dt)).astype(np.complex64)
+    if kind == "fluid":
+        plan.rk4_step(u, LONG)
+    else:
+        {"scalar": plan.rk4_step_scalar, "rbc": plan.rk4_step_rbc, "mhd": plan.rk4_step_mhd}[kind](u, other, LONG)
+    plan.status()
+    err = np.linalg.norm(u[2].cpu().numpy() - want) / np.linalg.norm(want)
+    assert err < 2.0 ** -24
