@@ -102,7 +102,13 @@ typedef struct ts_plan ts_plan;
 void ts_config_default(ts_config* cfg);
 
 /* Replaces the FFF_PENCIL / SFF_PENCIL constructor + fftk.Init
- * (FFF_pencil.cc:31-135, SFF_pencil.cc:38-): allocates twiddles and workspace. */
+ * (FFF_pencil.cc:31-135, SFF_pencil.cc:38-): allocates twiddles and workspace.
+ * Workspace in components of elems_per_comp: FFF 12, SFF 17, SSF 12, SSS 18, more on the
+ * first call of a step that needs it (scalar and SSF convection 17, SSS convection 20,
+ * MHD 21, adjoint and flux 15).  FP32 FFF plans with two-thirds dealiasing and 128, 256 or
+ * 512 points along z take 1 to 1.5 components more (MHD 3.5), unless that workspace is more
+ * than a quarter of what the device has free: then, or when the allocation fails, their
+ * steps run in place, some 5 % slower. */
 int ts_plan_create(const ts_config* cfg, ts_plan** plan);
 int ts_plan_destroy(ts_plan* plan);
 /* Stream for every later call (cudaStream_t; NULL = legacy default stream). */

@@ -4,7 +4,7 @@
 // (basis/FFF/pencil/FFF_pencil.cc:31-277) and the static work arrays of
 // Time_advance_incompress::RK4 (RK.cc:95-96: Vcopy, tot_Vrhs).  The caller's
 // u_hat is the state (the reference's U.cvf); the plan owns the stage field,
-// the RK accumulator, six product / transform work fields and twiddle tables.
+// the RK accumulator, the product / transform work fields and twiddle tables.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <string.h>
@@ -310,7 +310,9 @@ static int compact_pitch(const ts_plan* p, const Geo& g, int form) {
 
 // Work fields for nprod components in place, or for nin compact inverse-transformed fields
 // followed by nout products where a step of product form `form` takes that layout.  The second,
-// larger size is a wish: without the memory for it the step runs in place.
+// larger size (up to 39 % more) is a wish: where it is more than a quarter of what the device has
+// free, or cannot be had, the step runs in place, so that programs that fill the device keep the
+// memory they had.
 static int alloc_work(ts_plan* p, int nprod, int form, int nin, int nout) {
   Geo g = p->g;
   for (int c = 0; c < TUNE_NCLASS; ++c) g.tv[c] = g.tb[c] = 0;
@@ -324,7 +326,12 @@ static int alloc_work(ts_plan* p, int nprod, int form, int nin, int nout) {
   p->P_elems = 0;
   const long long most = std::max(want, p->P_asked);
   long long got = most;
-  if (cudaMalloc(&p->P, most * p->cb) != cudaSuccess) {
+  size_t free_bytes = 0, total = 0;
+  if (most > base) {
+    CK(cudaMemGetInfo(&free_bytes, &total));
+    if ((size_t)most * p->cb > free_bytes / 4) got = base;
+  }
+  if (cudaMalloc(&p->P, got * p->cb) != cudaSuccess) {
     cudaGetLastError();
     got = base;
     CK(cudaMalloc(&p->P, base * p->cb));
@@ -1078,7 +1085,7 @@ static Geo y_as_x(const Geo& g) {
 // SSF fluid step (sin/cos along x and y; sincostr_switch "SCF"), conservative form,
 // unforced: RK4(U,P,F) (RK.cc:91-170) with standalone transforms; with a temperature
 // T the Boussinesq step RK4(U,T,P,F) (RK_SF.cc:97-221, PRLARGE / ULARGE buoyancy).
-// With nf = 3 (fluid) or 4 (U, T) fields and np = 6 or 9 products, P holds [0, np):
+// With nf = 3 (fluid) or 4 (U, T) fields and np = 5 or 8 products, P holds [0, np):
 // the nf spectra after the x and y inverses, which the fused z pass turns into the
 // np product spectra in place.
 // ---------------------------------------------------------------------------
@@ -1090,8 +1097,8 @@ static int ssf_step_supported(ts_plan* p, bool rbc) {
                        : "the SSF / SSS step is the conservative, unforced fluid step";
     return TS_ERR_UNSUPPORTED;
   }
-  const int nf = rbc ? 4 : 3, np = rbc ? 9 : 6;
-  return ensure_work(p, nf, np);
+  // work fields: eight or five products (with nine the flux needs no others)
+  return ensure_work(p, rbc ? 4 : 3, rbc ? 9 : 6);
 }
 
 // the RBC epilogue's arguments (U, T in place; stage fields U then T in Ucur, tot)

@@ -7,6 +7,7 @@ The steps are compared with the FP64 oracle from states with energy in every mod
 lost or wrongly dealiased row shows.  The time step is such that a step moves the state by at
 most CHANGE = 5 %: its error is the rounding of the stored state (half an ulp in FP32, where one
 fma chain ends it; three roundings in FP64) plus CHANGE times that of the transforms (step_tol)."""
+import gc
 import math
 
 import numpy as np
@@ -254,6 +255,36 @@ def test_compact_inverse_lines_match_in_place(cuda, N, kind, prec):
     tol = 16 * math.log2(np.prod(N)) * EPS[prec]
     for x, y in zip(*got):
         assert rel(x, y) < tol
+
+
+@pytest.mark.parametrize("kind,spare", [("fluid", 140 << 20), ("mhd", 200 << 20)])
+def test_compact_lines_leave_a_full_device_its_memory(cuda, kind, spare):
+    """With little memory free a plan keeps the work fields of the in-place step and takes that step;
+    results as with the compact lines."""
+    import torch
+    import tarang_b200 as tb
+    N = (128, 64, 128)  # 4.3 MB a component
+    V, dt = lively(R.Grid(N), 0), small_dt(N)
+    got, took = [], []
+    for full in (False, True):
+        gc.collect()
+        torch.cuda.empty_cache()
+        hog = torch.empty(max(0, torch.cuda.mem_get_info()[0] - spare) if full else 0, dtype=torch.uint8, device=cuda)
+        before = torch.cuda.mem_get_info()[0]
+        u = torch.from_numpy(V).to(torch.complex64).to(cuda)
+        b = u.flip(0).contiguous()
+        plan = tb.Plan(N, precision="f32", nlin_form="conservative", dealias="two_thirds", nu=0.01, kappa=0.02, dt=dt)
+        call = (lambda: plan.rk4_step_mhd(u, b, 1)) if kind == "mhd" else (lambda: plan.rk4_step(u, 1))
+        call()
+        plan.status()
+        got.append((u.cpu().numpy(), b.cpu().numpy()))
+        took.append(before - torch.cuda.mem_get_info()[0])
+        tiles = (6 if kind == "mhd" else 3) * N[0] * 48 // 16
+        assert (tiles in captured(plan, call)[0]) == (not full)
+        del hog, plan, call, u, b
+    assert took[1] < took[0]
+    for x, y in zip(*got):
+        assert rel(x, y) < 16 * math.log2(np.prod(N)) * EPS["f32"]
 
 
 @pytest.mark.parametrize("prec,tol", [("f64", 1e-12), ("f32", 2e-6)])
