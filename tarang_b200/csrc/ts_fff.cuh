@@ -690,13 +690,12 @@ template <int FORM> __host__ __device__ constexpr int zreg_threads() { return 64
 // from global memory (a line spread over several warps; the second read of the
 // line hits L1), then the length-M inverse FFT (forward radix schedule) leaves
 // the packed real line in registers
-// Register layout of a line: with a first radix equal to E (powers of two), slot
+// Register layout of a line: with a first radix equal to E (powers of two, and 12), slot
 // s of lane t holds row t + s*TPL on input (forward schedule) and on output
 // (reversed schedule), and the pair terms X[M-k] sit in the partner lane of the
-// same warp (TPL <= 32): warp shuffles.  Otherwise (a line over two warps, or a
-// radix-3 schedule whose rows follow load_row / final_row) the inverse reads the
-// pair terms from global memory (L1 hits) and the forward swaps them through the
-// line's exchange buffer.
+// same warp (TPL <= 32): warp shuffles.  Otherwise (a line over two warps) the inverse
+// reads the pair terms from global memory (L1 hits) and the forward swaps them through
+// the line's exchange buffer.
 template <int M, int E, int TPL> __host__ __device__ constexpr bool zreg_shfl() {
   return radix_at(M, E, 0) == E && TPL <= 32;
 }
@@ -783,7 +782,7 @@ __device__ __forceinline__ void zreg_forward_store(C<T> (&p)[E], C<T>* Xo, bool 
 }
 
 // blocks per SM the register z kernel is compiled for: 6 (170 registers), 3 for
-// the 12-element radix-3 lines (which would spill at 170), 4 for 512-point lines
+// the 12-element lines with a factor 3 (which would spill at 170), 4 for 512-point lines
 // (two warps per line, the pair terms through the exchange line; spilled at 170)
 // (8 for the 4-element variant)
 // (4 for the MHD and flux-giver forms, which hold six lines while they make eight or nine products)
@@ -792,7 +791,7 @@ template <int NZ, int EZ = 0, int FORM = 0> __host__ __device__ constexpr int zr
 }
 
 // EZ = 0: 8 elements per thread, 12 for a line length with a factor 3 (radices
-// 4, 2|4, 3); EZ = 4: 4 elements per thread (twice the lanes per line).
+// 12, 2|4); EZ = 4: 4 elements per thread (twice the lanes per line).
 // BATCH: a line over two warps also issues every component's loads before the first
 // transform (one load latency per line instead of one per component)
 template <typename T, int NZ, int FORM, int EZ = 0, bool BATCH = false>
@@ -865,6 +864,9 @@ __global__ void __launch_bounds__(zreg_threads<FORM>(), zreg_min_blocks<NZ, EZ, 
 // needs warp barriers only, and the mirrored rows N - k come from the partner lane by
 // shuffles (SH); otherwise they are read again (L1) and, on the way out, taken from the
 // exchange line.
+// Rounding: both lines carry that of the stronger one (a line of zeros beside another comes out
+// as noise of eps times it, and equal lines differ by eps, the modes ky = Ny / 2).  In the norm
+// over a field that is the rounding of single lines: the y and x passes mix its lines anyway.
 // ---------------------------------------------------------------------------
 template <typename T, int NZ, int E> __host__ __device__ constexpr bool zpair_shfl() {
   return radix_at(NZ, E, 0) == E && NZ / E <= 32 && E >= 2;
@@ -1818,11 +1820,11 @@ __global__ void __launch_bounds__(z_nout(FORM) * CW * (L / E), 1)
 }
 
 // ---------------------------------------------------------------------------
-// Elementwise spectral epilogue, used where the fused x kernel's column tiles
-// would have rows narrower than 64 bytes (FP32 and FP64 at Nx >= 512): the NF
-// product fields have already been forward-transformed along x in place
-// (k_strided_fft); one thread per spectral element, every array access
-// coalesced.  Same arithmetic as k_fwd_x's epilogue (spec_epilogue).
+// Elementwise spectral epilogue of the split form: a step's wherever the pipelined kernel
+// has no tile (fwd_x_impl), every mode's where the fused kernel's column tiles would have
+// rows narrower than 64 bytes (Nx >= 512).  The NF product fields have already been
+// forward-transformed along x in place (k_strided_ld); one thread per spectral element, every
+// array access coalesced.  Same arithmetic as k_fwd_x's epilogue (spec_epilogue).
 // ---------------------------------------------------------------------------
 template <typename T, int FORM, int MODE>
 __global__ void __launch_bounds__(256) k_spec_epi(const C<T>* P, Geo g, StageArgs a) {

@@ -125,10 +125,10 @@ inline unsigned grid1d(long long n, int threads) {
 
 }  // namespace
 
-// strided passes at L = 1024 in FP32: 16 elements per thread and 8-column tiles
-// (64-byte rows) with the exchange in the consumed staging tile; on B200 this
-// moved the x pass from 1.2 to 2.35 TB/s and the y pass from 2.0 to 2.9 TB/s
-// against 4-column tiles
+// persistent strided kernel (the candidates of the y passes; ld_tile is the rule): elements per
+// thread, tile columns, staging tiles.  At L = 1024 in FP32 16 elements per thread and 8-column
+// tiles (64-byte rows) with the exchange in the consumed staging tile: 2.9 TB/s in the y pass
+// against 2.0 with 4-column tiles
 constexpr bool wide1024(int L) { return std::is_same<T, float>::value && L == 1024; }
 constexpr int str_e(int L) { return wide1024(L) ? 16 : e_mixed(L, e_reg(L)); }
 constexpr int str_cw(int L) { return wide1024(L) ? 8 : cw_for(L, str_e(L)); }
@@ -191,11 +191,13 @@ constexpr LdTile ix_tile(int L) {
 }
 
 // ---------------------------------------------------------------------------
-// Launch-tuning candidates.  Candidate 0 of every pass class is the fixed rule;
-// the others change the radix schedule (elements per thread E: the Stockham
-// passes use radix min(E, remaining)), the column-tile width CW or the number of
-// staging tiles NT.  A candidate that does not fit (threads per block, shared
-// memory) or repeats an earlier one is invalid and launches as the rule.
+// Launch-tuning candidates.  Candidate 0 of every pass class is the rule; the others are the
+// kernels that were the rules before the direct-load, line-pair and pipelined ones, and their
+// variants: elements per thread E (the Stockham passes use radix min(E, remaining)), column-tile
+// width CW, number of staging tiles NT.  On B200 they are slower than the rules at the sizes
+// beside the tile tables (13-60 %); their numbers stay valid for stored tunings.  One that does not fit
+// (threads per block, shared memory) or repeats another of the candidates' tables is refused
+// (str_cand, ix_cand and sx_cand 0 are the tiles that the tables start from, not the rule's).
 // ---------------------------------------------------------------------------
 constexpr int NCAND = TUNE_NCAND;
 struct Tile { int E, CW, NT; };
@@ -257,7 +259,8 @@ constexpr bool ix_valid(int L, int v) {
 // (12 with a factor 3), 2 = the slot kernel with 4 (power-of-two lines), 3 = the
 // FP32 register kernel with 4 elements per thread (lines of up to 256 points),
 // 4 = on 1024-point lines in FP32, the register kernel that loads each component just
-// before its transform (the rule there issues every load up front)
+// before its transform (the rule there issues every load up front).  Candidate 1 exists where the
+// slot kernel was not itself candidate 0 when the numbers were given
 template <int NZ, int FORM> constexpr bool z_rule_slots() {
   constexpr int M = NZ / 2;
   return !(std::is_same<T, float>::value && M <= 512) &&
@@ -268,7 +271,12 @@ template <int NZ, int FORM> constexpr bool z_rule_slots() {
 struct ZTile { int E, NTHR, MINB, NB; };
 constexpr ZTile zp_tile(int NZ, int form) {
   const bool f32 = std::is_same<T, float>::value;
-  // FP64 with six inputs at 128 points: 4 elements per thread (187 us against 195; 8 spill)
+  // FP64 lines: measured as whole steps only, against the shared-memory slot kernel that was the
+  // rule before (64x64x512 rotational 1291 -> 712 us, 64x64x1024 2422 -> 1505, MHD 64x64x512 2507 ->
+  // 1292, 256^3 17900 -> 9150, SFF 96^3 Boussinesq 1229 -> 627, SSS 64x64x1024 4450 -> 2449); from 256
+  // points, at 48 and 96, and in forms 2, 5 and 6 they spill 0.1-1 KB a thread.  The rotational
+  // form at 128 points takes 4 elements per thread: 47.5 us against 48.5 with 8, which spill; at 256
+  // points it is the other way round (109.9 against 94.2)
   const int E = NZ % 3 == 0 ? 12 : (!f32 && form == 1 && NZ == 128 ? 4 : 8);
   const int tpl = NZ / E, thr = tpl > 64 ? tpl : 64;
   // the three products of the rotational form together: twiddles and barriers shared (138 -> 134 us)
@@ -317,7 +325,8 @@ constexpr PipeTile pipe_tile(int L, int form) {
 constexpr bool fx_rule_split(int L) { return L <= 64 || std::is_same<T, float>::value || L > 128; }
 
 // forward x candidates (MODE_STEP): 1 = the split form (strided x FFT, then the
-// elementwise epilogue) where the rule is the fused TMA kernel; 2 = the fused
+// elementwise epilogue) where the fused TMA kernel's tiles fit (the rule's own form where
+// neither the pipelined nor the fused kernel is the rule, see fwd_x_impl); 2 = the fused
 // kernel with half-width column tiles (32-byte rows in FP32; where the rule
 // splits, the fused kernel at the rule's tile width); 3 = the fused kernel with
 // 8 elements per thread (half the threads)
@@ -329,9 +338,9 @@ constexpr bool fx_valid(int L, int v) {
 }
 
 
-// SFF x candidates. Inverse: 1 = 4 elements per thread (power-of-two lengths),
-// 2 = half-width column tiles. Forward: 1 = the other split choice (fused
-// epilogue from 64 points on, split below), 2 = half-width column tiles.
+// SFF x candidates (k_sff_inv_x, k_sff_fwd_x; the rule is k_sc_x). Inverse: 1 = 4 elements per
+// thread (power-of-two lengths), 2 = half-width column tiles. Forward: 1 = fused epilogue from 64
+// points on, split below, 2 = half-width column tiles (split from 64 points on, fused below).
 constexpr int sx_e(int N, int dir) { return e_mixed(N, dir > 0 ? 8 : (std::is_same<T, float>::value ? 8 : 4)); }
 constexpr Tile sx_cand(int N, int dir, int v) {
   return v == 0 ? Tile{sx_e(N, dir), cw_for(N, sx_e(N, dir)), 1}
@@ -623,7 +632,7 @@ template <> cudaError_t Launch<T>::z_fused(const Geo& g, int form, void* P, cons
   return err;
 }
 
-// SSS z pass (forms 0, 2, 6): line pairs, tiles as the Fourier z pass
+// SSS z pass (forms 7, 2, 6): line pairs, tiles as the Fourier z pass
 template <int NZ, int FORM>
 static cudaError_t sss_z_pairs(const Geo& g, void* P, const void* tw, const void* tq, int zin, int zout,
                                cudaStream_t st) {

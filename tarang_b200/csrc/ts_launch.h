@@ -1,5 +1,5 @@
-// Host-side launchers of the templated kernels, instantiated per precision in
-// ts_kern_f32.cu / ts_kern_f64.cu (compiled in parallel).
+// Host-side launchers of the templated kernels, instantiated per group and precision in the
+// ts_kern_<part>_<precision>.cu files (compiled in parallel).
 #pragma once
 #include <cuda_runtime.h>
 #include "ts_fff.cuh"
@@ -19,7 +19,7 @@ inline unsigned shell_blocks(const Geo& g, unsigned cap) {
 
 template <typename T> struct Launch {
   // strided-axis FFT on nf fields in place: axis 0 = x (L = Nx), 1 = y (L = Ny);
-  // dir -1 forward, +1 inverse; outputs scaled by `scale`
+  // dir -1 forward, +1 inverse
   // per > 0: the nf fields are nf / per members of per fields each, members mstride complex apart
   // inner_eff > 0: transform only the first inner_eff columns (y axis: kz < inner_eff);
   // zero_hi: rows with 3|k| > L are zero and not read (two-thirds dealiased input)
@@ -27,16 +27,14 @@ template <typename T> struct Launch {
   static cudaError_t strided(const Geo& g, int axis, int dir, void* data, int nf, const void* tw, cudaStream_t st,
                              int per = 0, long long mstride = 0, int inner_eff = 0, int zero_hi = 0,
                              void* dst = nullptr, double scl = 1.0);
-  // form 0 conservative (3 fields out), 1 rotational (6), 3 adjoint of the rotational form (9: also
-  // lsc c^-1 P lam from the cotangent lam)
+  // form 0 conservative (3 fields out), 1 rotational (6), 4 the adjoint's cotangent (lsc c^-1 P lam
+  // into fields 6-8), 5 the giver of the per-sphere energy flux (u inside |K| <= rad into fields 3-5)
   // forms 0, 1, 5: W has lines of g.Hp and components of g.Sp elements
   // kept != 0 (forms 0, 1 with two-thirds dealiasing): write only the columns with 3|ky| <= Ny, 3 kz <= Nz
-  // form 4: the adjoint's cotangent fields 6-8; form 5: the giver, u inside |K| <= rad, into
-  // fields 3-5 for the per-sphere energy flux
   static cudaError_t inv_x(const Geo& g, int form, const void* U, void* W, const void* tw, const void* lam,
                            double lsc, cudaStream_t st, int kept = 0, double rad = 0.0);
-  // form 0 conservative, 1 rotational, 2 Boussinesq (u, T), 3 adjoint of the rotational form,
-  // 5 MHD (Elsasser products), 6 flux giver (u_i g_j)
+  // form 0 conservative (whole tensor), 7 conservative step, 1 rotational, 2 Boussinesq or scalar
+  // (u, T), 3 adjoint of the rotational form, 5 MHD, 6 flux giver (u_i g_j)
   // nmem members, member fields msP complex apart
   // zkeep >= 0: input rows kz > zkeep are zero and not read
   // q (form 6): u is read there (three components) instead of from P
@@ -45,17 +43,17 @@ template <typename T> struct Launch {
                              int nmem = 1, long long msP = 0, int zkeep = -1, const void* q = nullptr,
                              const void* x = nullptr);
   static cudaError_t z_single(const Geo& g, int dir, const void* in, void* out, int ncomp, const void* tw, cudaStream_t st);
-  // SSS: the fused z pass on real coefficients (form 0 / 2 products; zin / zout sine masks)
+  // SSS: the fused z pass on real coefficients (products of form 7, 2 or 6; zin / zout sine masks)
   static cudaError_t sss_z_fused(const Geo& g, int form, void* P, const void* tw, const void* tq, int zin, int zout,
                                  cudaStream_t st);
   // line pitch of the inverse-transformed fields for a right-hand side of product form `form`
   // (g.Hz: the fields' own, and the products go in place)
   static int inverse_pitch(const Geo& g, int form);
   // a.U0 / a.Ud / a.tot must be 16-byte aligned (TMA)
-  // form 0 / 1 / 3 as inv_x; mode MODE_STEP, MODE_FLUX, MODE_NLIN (forms 0, 1) or MODE_ADJ (form 3)
+  // product form as z_fused: MODE_STEP with 1 or 7, MODE_FLUX and MODE_NLIN with 0 or 1, MODE_ADJ with 3
   static cudaError_t fwd_x(const Geo& g, int form, int mode, const void* P, const StageArgs& a, const void* tw,
                            cudaStream_t st);
-  // SFF x passes (sin/cos along x): inverse of u1,u2,u3,T into P[0..3]; forward of the nine
+  // SFF x passes (sin/cos along x): inverse of u1,u2,u3,T into P[0..3]; forward of the eight
   // Boussinesq products + force, projection and the IF-RK4 stage update
   // nmem members: member strides (complex elements) of U, Tf, W; SffArgs carries its own
   static cudaError_t sff_inv_x(const Geo& g, const void* U, const void* Tf, void* W, const void* tq, cudaStream_t st,
@@ -70,7 +68,7 @@ template <typename T> struct Launch {
                            int deal = 0);
   static cudaError_t sc_x(const Geo& g, int dir, const ScArgs& a, const void* tq, cudaStream_t st, int nf,
                           int nmem = 1);
-  // FFF passive scalar: elementwise epilogue of the nine x-transformed products in P
+  // FFF passive scalar: elementwise epilogue of the eight x-transformed products in P
   static cudaError_t scalar_epi(const Geo& g, const void* P, const SffArgs& a, cudaStream_t st);
   // SSS z sin/cos helpers on nlines lines of N reals (padded to N + 2)
   static cudaError_t sss_zperm_fwd(const void* u, void* v, long long nlines, int N, int sine, cudaStream_t st);
@@ -82,12 +80,12 @@ template <typename T> struct Launch {
   // SSS fluid step: dealiased copy of real coefficients, and the epilogue
   static cudaError_t sss_dealias_copy(const Geo& g, const void* A, void* B, int ncomp, cudaStream_t st);
   static cudaError_t sss_epi(const Geo& g, const void* P, const StageArgs& a, cudaStream_t st);
-  // SSF fluid step: elementwise epilogue of the six forward-transformed products in P
+  // SSF fluid step: elementwise epilogue of the five forward-transformed products in P
   static cudaError_t ssf_epi(const Geo& g, const void* P, const StageArgs& a, cudaStream_t st);
-  // SSF / SSS Boussinesq step: epilogues of the nine forward-transformed products in P
+  // SSF / SSS Boussinesq step: epilogues of the eight forward-transformed products in P
   static cudaError_t ssf_rbc_epi(const Geo& g, const void* P, const SffArgs& a, cudaStream_t st);
   static cudaError_t sss_rbc_epi(const Geo& g, const void* P, const SffArgs& a, cudaStream_t st);
-  // FFF MHD: elementwise epilogue of the nine x-transformed Elsasser products in P
+  // FFF MHD: elementwise epilogue of the eight x-transformed products of form 5 in P
   static cudaError_t mhd_epi(const Geo& g, const void* P, const SffArgs& a, cudaStream_t st);
   static cudaError_t reality(const Geo& g, void* A, int ncomp, cudaStream_t st);
   static cudaError_t rbc_slave(const Geo& g, void* U, void* Tf, int slave, double vs, cudaStream_t st);

@@ -225,9 +225,6 @@ __global__ void k_energy(const C<T>* __restrict__ A, const C<T>* __restrict__ B,
   if (threadIdx.x == 0) out[1 + blockIdx.x] = s;  // partial sums, added in a fixed order by k_sum_partials
 }
 
-// out[0] = sum of the n partial sums out[1..n], in an order that does not depend
-// on scheduling (one block), so energies and the normalised initial condition are
-// reproducible bit for bit
 // res[r] = the sum of the n partials at out + r * pitch + 1 (block r; the order of k_sum_partials)
 static __global__ void k_sum_partials_many(const double* out, long long pitch, int n, double* res) {
   const double* o = out + blockIdx.x * pitch;
@@ -236,6 +233,9 @@ static __global__ void k_sum_partials_many(const double* out, long long pitch, i
   s = block_sum(s);
   if (threadIdx.x == 0) res[blockIdx.x] = s;
 }
+// out[0] = sum of the n partial sums out[1..n], in an order that does not depend
+// on scheduling (one block), so energies and the normalised initial condition are
+// reproducible bit for bit
 static __global__ void k_sum_partials(double* out, int n) {
   double s = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += out[1 + i];
