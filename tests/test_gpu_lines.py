@@ -280,8 +280,10 @@ def test_compact_lines_leave_a_full_device_its_memory(cuda, kind, spare):
         got.append((u.cpu().numpy(), b.cpu().numpy()))
         took.append(before - torch.cuda.mem_get_info()[0])
         tiles = (6 if kind == "mhd" else 3) * N[0] * 48 // 16
-        assert (tiles in captured(plan, call)[0]) == (not full)
+        compact = tiles in captured(plan, call)[0]
         del hog, plan, call, u, b
+        torch.cuda.empty_cache()  # the library allocates beside torch's cache
+        assert compact == (not full)
     assert took[1] < took[0]
     for x, y in zip(*got):
         assert rel(x, y) < 16 * math.log2(np.prod(N)) * EPS["f32"]
