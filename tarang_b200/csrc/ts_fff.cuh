@@ -548,8 +548,8 @@ template <int M> __host__ __device__ constexpr int zslot() { return M + M / 16 +
 //         divergence of S and B.nlin that of A (compute_nlin_VF_MHD.cc:40-95, MHD.cc:75-84,150-161).
 //         Every product is rounded by itself (mul_rn), so that the products of an aligned state,
 //         u = b or u = -b, cancel exactly, as Zp_i Zm_j does: with an fma its rounding is left.
-//         256^3 FP32 step 4350 us with fma, 4388 so; on Zp and Zm held in the registers of u and b 4392
-//         (FP64 9150, 9160 and 9330)
+//         256^3 FP32 step 4350 us with fma and so (FP64 9150 and 9285); on Zp and Zm held in the
+//         registers of u and b 4392 (9330)
 // FORM 6 (flux giver):    in u1..3, g1..3   -> u_i g_j (f = 3 i + j), for the giver nonlinear
 //                         term N_i = sum_j D_j F[u_j g_i] (compute_nlin_ET_VF.cc:71-87)
 __host__ __device__ constexpr int z_nin(int form) {
@@ -569,6 +569,11 @@ template <typename V> __device__ __forceinline__ V prod_pk(V a, V b) { return mk
 template <typename V> __device__ __forceinline__ V diff_pk(V a, V c, V b, V d) {
   return mk<V>(a.x * c.x - b.x * d.x, a.y * c.y - b.y * d.y);
 }
+// a copy that the compiler takes for another value: what is computed from it is computed again
+// instead of being kept in registers over the transform of the product before (256^3 FP32 MHD step
+// 4410 us with u1u1 kept, which spills 172 bytes a thread, 4348 so)
+__device__ __forceinline__ float2 again(float2 a) { asm("" : "+f"(a.x), "+f"(a.y)); return a; }
+__device__ __forceinline__ double2 again(double2 a) { asm("" : "+d"(a.x), "+d"(a.y)); return a; }
 // product f of a form from its inputs at a point (f known at compile time; not FORM 3)
 template <int FORM, typename V> __device__ __forceinline__ V z_product(int f, const V* in) {
   if constexpr (FORM == 1) {
@@ -579,11 +584,17 @@ template <int FORM, typename V> __device__ __forceinline__ V z_product(int f, co
     return prod_pk(in[f / 3], in[3 + f % 3]);
   } else if constexpr (FORM == 5) {
     auto dif = [&](int a, int c, int b, int d) { return sub(mul_rn(in[a], in[c]), mul_rn(in[b], in[d])); };
-    if (f < 2) return sub(dif(f + 1, f + 1, f + 4, f + 4), dif(0, 0, 3, 3));
+    if (f < 2) {
+      const V a = f == 0 ? in[0] : again(in[0]), b = f == 0 ? in[3] : again(in[3]);
+      return sub(dif(f + 1, f + 1, f + 4, f + 4), sub(mul_rn(a, a), mul_rn(b, b)));
+    }
     const int i = (f - 2) % 3, j = (i + 1) % 3;
     return f < 5 ? dif(i, j, 3 + i, 3 + j) : dif(3 + i, j, i, 3 + j);
   } else {
-    if (f < 2) return diff_pk(in[f + 1], in[f + 1], in[0], in[0]);
+    if (f < 2) {
+      const V a = f == 0 ? in[0] : again(in[0]);
+      return diff_pk(in[f + 1], in[f + 1], a, a);
+    }
     return f < 5 ? prod_pk(in[f - 2], in[(f - 1) % 3]) : prod_pk(in[f - 5], in[3]);
   }
 }
