@@ -308,6 +308,30 @@ static int compact_pitch(const ts_plan* p, const Geo& g, int form) {
   return h != g.Hz ? h : 0;
 }
 
+// *buf of `had` complex elements becomes one of n, contents lost; without the memory for it the plan
+// keeps a buffer of the old size, so that the calls that ran before still do
+static int regrow(ts_plan* p, void** buf, long long n, long long had) {
+  CK(cudaFree(*buf));
+  *buf = nullptr;
+  if (cudaMalloc(buf, n * p->cb) == cudaSuccess) return TS_OK;
+  cudaGetLastError();  // not for a later launch to report
+  *buf = nullptr;
+  if (had && cudaMalloc(buf, had * p->cb) != cudaSuccess) {
+    cudaGetLastError();
+    *buf = nullptr;
+  }
+  g_last_error = "no device memory for " + std::to_string(n * p->cb) + " bytes of work fields";
+  return TS_ERR_NOMEM;
+}
+
+// a work field that regrow could not give back at its old size either (another program took the
+// memory in between): the call is refused, and a call that grows the field tries again
+static int has_work(const ts_plan* p) {
+  if (p->P && p->Ucur && p->tot) return TS_OK;
+  g_last_error = "the plan's work fields were lost to a failed allocation";
+  return TS_ERR_NOMEM;
+}
+
 // Work fields for nprod components in place, or for nin compact inverse-transformed fields
 // followed by nout products where a step of product form `form` takes that layout.  The second,
 // larger size (up to 39 % more) is a wish: where it is more than a quarter of what the device has
@@ -320,21 +344,17 @@ static int alloc_work(ts_plan* p, int nprod, int form, int nin, int nout) {
   const long long want = std::max(base, h ? nin * (long long)g.Nx * g.Ny * h + nout * g.S : 0);
   if (want <= p->P_asked && p->nP >= nprod) return TS_OK;
   CK(cudaStreamSynchronize(p->st));
-  CK(cudaFree(p->P));
-  p->P = nullptr;
-  p->nP = 0;
-  p->P_elems = 0;
-  const long long most = std::max(want, p->P_asked);
+  const long long most = std::max(want, p->P_asked), had = p->P_elems;
   long long got = most;
   size_t free_bytes = 0, total = 0;
-  if (most > base) {
-    CK(cudaMemGetInfo(&free_bytes, &total));
-    if ((size_t)most * p->cb > free_bytes / 4) got = base;
-  }
-  if (cudaMalloc(&p->P, got * p->cb) != cudaSuccess) {
-    cudaGetLastError();
+  if (most > base &&
+      (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || (size_t)most * p->cb > (free_bytes + had * p->cb) / 4))
     got = base;
-    CK(cudaMalloc(&p->P, base * p->cb));
+  int rc = regrow(p, &p->P, got, had);
+  if (rc != TS_OK && got > base) rc = regrow(p, &p->P, got = base, had);
+  if (rc != TS_OK) {
+    if (!p->P) p->nP = 0, p->P_elems = 0;
+    return rc;
   }
   p->P_asked = most;
   p->P_elems = got;
@@ -990,12 +1010,13 @@ static int step_scalar_fff(ts_plan* p, void* U0, void* T0) {
 static int ensure_work(ts_plan* p, int nstage, int nprod, int form, int nin, int nout) {
   if (p->nS < nstage) {
     CK(cudaStreamSynchronize(p->st));
-    CK(cudaFree(p->Ucur));
-    CK(cudaFree(p->tot));
-    p->Ucur = p->tot = nullptr;
-    p->nS = 0;
-    CK(cudaMalloc(&p->Ucur, nstage * p->g.S * p->cb));
-    CK(cudaMalloc(&p->tot, nstage * p->g.S * p->cb));
+    const long long n = nstage * p->g.S, had = p->nS * p->g.S;
+    int rc = regrow(p, &p->Ucur, n, had);
+    if (rc == TS_OK && (rc = regrow(p, &p->tot, n, had)) != TS_OK) regrow(p, &p->Ucur, had, 0);
+    if (rc != TS_OK) {
+      if (!p->Ucur || !p->tot) p->nS = 0;
+      return rc;
+    }
     p->nS = nstage;
   }
   CKS(alloc_work(p, std::max(p->nP, nprod), form, nin, nout));
@@ -1291,6 +1312,7 @@ int ts_rk4_step(ts_plan* p, void* u_hat, int nsteps) {
     CKS(ssf_step_supported(p, false));
     // the health word of earlier calls (copied back without a sync)
     if (*p->err_h) return health_status(p);
+    CKS(has_work(p));
     int rc = with_device(p, &p->stage_u, u_hat, 3 * p->g.S * p->cb, true, [&](void* U) -> int {
       for (int s = 0; s < nsteps; ++s) CKS(sss ? step_sss(p, U) : step_ssf(p, U));
       return (int)TS_OK;
@@ -1302,6 +1324,7 @@ int ts_rk4_step(ts_plan* p, void* u_hat, int nsteps) {
   // a bounded device wait that gave up in an earlier call (read without a sync)
   // the health word of earlier calls (copied back without a sync)
   if (*p->err_h) return health_status(p);
+  CKS(has_work(p));
   int rc = with_device(p, &p->stage_u, u_hat, 3 * p->g.S * p->cb, true, [&](void* U) -> int {
     for (int s = 0; s < nsteps; ++s) CKS(step_fff(p, U));
     return (int)TS_OK;
@@ -1322,6 +1345,7 @@ int ts_rk4_step_keep(ts_plan* p, const void* u_hat, void* u_next, void* stages) 
   }
   // the health word of earlier calls (copied back without a sync)
   if (*p->err_h) return health_status(p);
+  CKS(has_work(p));
   CKS(step_fff(p, const_cast<void*>(u_hat), u_next, stages));
   CK(cudaMemcpyAsync(p->err_h, p->err_d, sizeof(int), cudaMemcpyDeviceToHost, p->st));
   return TS_OK;
@@ -1336,6 +1360,7 @@ int ts_adjoint_step(ts_plan* p, const void* u_hat, const void* stages, void* lam
   }
   // the health word of earlier calls (copied back without a sync)
   if (*p->err_h) return health_status(p);
+  CKS(has_work(p));
   CKS(adjoint_step_fff(p, u_hat, stages, lam_hat));
   CK(cudaMemcpyAsync(p->err_h, p->err_d, sizeof(int), cudaMemcpyDeviceToHost, p->st));
   return TS_OK;
@@ -1363,6 +1388,7 @@ int ts_adjoint_window(ts_plan* p, const void* u_start, int nsteps, void* lam_hat
   }
   // the health word of earlier calls (copied back without a sync)
   if (*p->err_h) return health_status(p);
+  CKS(has_work(p));
   // work slot n = [U_n (3 components), U1, U2, U3 of step n (9)]; U_0 is u_start itself
   const size_t cs = 3 * (size_t)p->g.S * p->cb, slot = 4 * cs;
   char* w = (char*)work;
@@ -1387,6 +1413,7 @@ int ts_rk4_step_rbc(ts_plan* p, void* u_hat, void* T_hat, int nsteps) {
     CKS(ssf_step_supported(p, true));
     // the health word of earlier calls (copied back without a sync)
     if (*p->err_h) return health_status(p);
+    CKS(has_work(p));
     const size_t bu = 3 * p->g.S * p->cb, bt = p->g.S * p->cb;
     int rc = with_device(p, &p->stage_u, u_hat, bu, true, [&](void* U) -> int {
       return with_device(p, &p->stage_t, T_hat, bt, true, [&](void* T) -> int {
@@ -1400,6 +1427,7 @@ int ts_rk4_step_rbc(ts_plan* p, void* u_hat, void* T_hat, int nsteps) {
   if (p->cfg.basis != TS_BASIS_SFF) return TS_ERR_UNSUPPORTED;
   // the health word of earlier calls (copied back without a sync)
   if (*p->err_h) return health_status(p);
+  CKS(has_work(p));
   const size_t bu = 3 * p->g.S * p->cb, bt = p->g.S * p->cb;
   int rc = with_device(p, &p->stage_u, u_hat, bu, true, [&](void* U) -> int {
     return with_device(p, &p->stage_t, T_hat, bt, true, [&](void* T) -> int {
@@ -1416,6 +1444,7 @@ int ts_rk4_step_scalar(ts_plan* p, void* u_hat, void* T_hat, int nsteps) {
   CKS(scalar_supported(p));
   // the health word of earlier calls (copied back without a sync)
   if (*p->err_h) return health_status(p);
+  CKS(has_work(p));
   const size_t bu = 3 * p->g.S * p->cb, bt = p->g.S * p->cb;
   int rc = with_device(p, &p->stage_u, u_hat, bu, true, [&](void* U) -> int {
     return with_device(p, &p->stage_t, T_hat, bt, true, [&](void* T) -> int {
@@ -1432,6 +1461,7 @@ int ts_rk4_step_mhd(ts_plan* p, void* u_hat, void* b_hat, int nsteps) {
   CKS(mhd_supported(p));
   // the health word of earlier calls (copied back without a sync)
   if (*p->err_h) return health_status(p);
+  CKS(has_work(p));
   const size_t bu = 3 * p->g.S * p->cb;
   int rc = with_device(p, &p->stage_u, u_hat, bu, true, [&](void* U) -> int {
     return with_device(p, &p->stage_b, b_hat, bu, true, [&](void* B) -> int {
@@ -1461,6 +1491,7 @@ int ts_nlin(ts_plan* p, void* u_hat, void* nlin_hat) {
   if (p && (p->cfg.basis == TS_BASIS_SSF || p->cfg.basis == TS_BASIS_SSS)) return ssf_transforms_only();
   if (!p || !u_hat || !nlin_hat) return TS_ERR_ARG;
   if (p->cfg.basis != TS_BASIS_FFF) return TS_ERR_UNSUPPORTED;
+  CKS(has_work(p));
   const size_t bytes = 3 * p->g.S * p->cb;
   return with_device(p, &p->stage_u, u_hat, bytes, true, [&](void* U) -> int {
     // the reference dealiases U in place before the transforms (compute_nlin.cc:61-62)
@@ -1657,6 +1688,7 @@ int ts_flux(ts_plan* p, const void* u_hat, const double* radii, int n_radii, dou
     g_last_error = "ts_flux: at most " + std::to_string(FLUX_MAX_BINS - 1) + " radii";
     return TS_ERR_ARG;
   }
+  CKS(has_work(p));
   // the reference's default radii need not ascend on small grids
   // (Global_process_advanced_vars.cc:133-154); the one-pass form bins ascending radii
   bool ascending = true;
@@ -1840,6 +1872,7 @@ int ts_fft_forward(ts_plan* p, const char* parity, const void* real_in, void* sp
     return TS_ERR_ARG;
   }
   if (!is_device_ptr(real_in) || !is_device_ptr(spec_out)) return TS_ERR_ARG;
+  CKS(has_work(p));
   const Geo& g = p->g;
   if (zp) {
     // SSS: sin/cos / (2 Nz) along z on the real lines, then y and x on the coefficient
@@ -1883,6 +1916,7 @@ int ts_fft_inverse(ts_plan* p, const char* parity, const void* spec_in, void* re
     return TS_ERR_ARG;
   }
   if (!is_device_ptr(spec_in) || !is_device_ptr(real_out)) return TS_ERR_ARG;
+  CKS(has_work(p));
   const Geo& g = p->g;
   // the reference copies the input to X_transform first (FFF_pencil_tr.cc:59); here the x
   // pass reads the input and writes the work fields.  It reads whole complex values: an input
@@ -2498,6 +2532,7 @@ int ts_plan_set_tuning(ts_plan* p, const ts_tuning* t) {
 int ts_plan_autotune(ts_plan* p, int reps, char* report, size_t report_len) {
   if (p && (p->cfg.basis == TS_BASIS_SSF || p->cfg.basis == TS_BASIS_SSS)) return ssf_transforms_only();
   if (!p || reps < 1) return TS_ERR_ARG;
+  CKS(has_work(p));
   const bool sff = p->cfg.basis == TS_BASIS_SFF;
   const size_t bu = 3 * (size_t)p->g.S * p->cb, bt = (size_t)p->g.S * p->cb;
   void *U = nullptr, *T = nullptr;

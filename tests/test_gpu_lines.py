@@ -289,6 +289,40 @@ def test_compact_lines_leave_a_full_device_its_memory(cuda, kind, spare):
         assert rel(x, y) < 16 * math.log2(np.prod(N)) * EPS["f32"]
 
 
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_a_step_that_finds_no_memory_leaves_the_plan_usable(cuda, prec):
+    """MHD needs larger stage, accumulator and work fields than the plan has; on a full device it
+    says so, and the plan's fluid step, transform and flux run as before."""
+    import torch
+    import tarang_b200 as tb
+    N = (64, 64, 64)
+    V, dt = lively(R.Grid(N), 0), small_dt(N)
+    plan = tb.Plan(N, precision=prec, dealias="two_thirds", nu=0.01, kappa=0.02, dt=dt)
+    u = torch.from_numpy(V).to(plan.torch_dtype()).to(cuda)
+    w = u.clone()
+    plan.rk4_step(w, 1)
+    want, flux = w.clone(), plan.flux(u, [2.0, 5.0])
+    x, b = u.clone(), u.clone()
+    gc.collect()
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (4 << 20), dtype=torch.uint8, device=cuda)
+    try:
+        for _ in range(2):
+            with pytest.raises(tb.TsError) as e:
+                plan.rk4_step_mhd(x, b, 1)
+            assert e.value.status == 6  # TS_ERR_NOMEM
+        w.copy_(u)
+        plan.rk4_step(w, 1)
+        plan.status()
+        assert torch.equal(w, want)
+        assert np.array_equal(plan.flux(u, [2.0, 5.0]), flux)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    plan.rk4_step_mhd(x, b, 1)
+    plan.status()
+
+
 @pytest.mark.parametrize("prec,tol", [("f64", 1e-12), ("f32", 2e-6)])
 @pytest.mark.parametrize("N", [(16, 16, 16), (1024, 16, 16), (512, 16, 32), (64, 32, 16), (256, 16, 16), (128, 16, 64)])
 def test_flux_at_line_edges(cuda, N, prec, tol):
