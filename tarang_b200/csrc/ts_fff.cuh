@@ -370,7 +370,8 @@ __global__ void __launch_bounds__(CW * (L / E), MINB)
 // ---------------------------------------------------------------------------
 // inverse x pass of the adjoint's cotangent: W_6..8 = IFFT_x(lsc c^-1 P Lam), the
 // Leray-projected cotangent divided by the C2R weight c (2 on the planes 0 < kz < Nz/2, else
-// 1).  The three components of a column stay in registers from the projection to their transforms, one after the other through one exchange tile.
+// 1).  The three components of a column stay in registers from the projection to their
+// transforms, one after the other through one exchange tile.
 // ---------------------------------------------------------------------------
 template <typename T, int L, int E, int CW, int MINB>
 __global__ void __launch_bounds__(CW * (L / E), MINB)
